@@ -313,9 +313,12 @@ __global__ void __launch_bounds__(128) k_adj_p2m(int64_t nl, const double *__res
 // ---- A6: Hessian-vector P2P over the near lists (symmetric at leaf level):
 //   g_x,i += sum_k J(x_k - x_i) (m_i lam_k - m_k lam_i),  J(d) = I/r^3 - 3 d d^T / r^5
 //   g_m,i -= sum_k lam_k . (x_k - x_i) / r^3           (r^2 = |d|^2 + eps^2, k != i)
-// Work items as in the forward P2P: one warp per (target leaf, <= 32 source leaves),
-// partial sums per item, summed in item order afterwards.
-__global__ void __launch_bounds__(128) k_adj_p2p_items(int64_t n_items, const int32_t *__restrict__ item_leaf,
+// Work items as in the forward P2P: one warp (FP64: one block) per (target leaf, <= 32
+// source leaves), partial sums per item, summed in item order afterwards.  FP64-pipe bound like the
+// forward P2P: r^-3 and 3 r^-5 come from the integer pipes (gx_r3_3r5), 18 FP64
+// instructions are left of 31, and leaves of at most 16 bodies give each half-warp every
+// other source.
+__global__ void __launch_bounds__(128) k_adj_p2p_items(const int32_t *__restrict__ item_leaf,
                                                        const int64_t *__restrict__ item_qb,
                                                        const int32_t *__restrict__ item_nq, const double *__restrict__ x,
                                                        const double *__restrict__ y, const double *__restrict__ m,
@@ -323,53 +326,72 @@ __global__ void __launch_bounds__(128) k_adj_p2p_items(int64_t n_items, const in
                                                        const int32_t *__restrict__ bs, const int32_t *__restrict__ be,
                                                        const int32_t *__restrict__ src_idx, double eps2, int tchunks,
                                                        double4 *__restrict__ part) {
-    __shared__ double4 sb[4][32];
-    __shared__ double sm_[4][32];
-    int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (it >= n_items) return;
-    int32_t leaf = item_leaf[it];
-    int64_t qb = item_qb[it];
-    int nq = item_nq[it];
-    int32_t t0 = bs[leaf], t1 = be[leaf];
-    int sl = lane < nq ? src_idx[qb + lane] : -1;
-    int sbeg = sl >= 0 ? bs[sl] : 0, send = sl >= 0 ? be[sl] : 0;
+    __shared__ P2PRows rows;
+    __shared__ double4 sb[128];
+    __shared__ double smass[128];
+    __shared__ int32_t sj[128];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t it = blockIdx.x;
+    const int32_t leaf = item_leaf[it];
+    const int nq = item_nq[it];
+    const int32_t t0 = bs[leaf], t1 = be[leaf];
+    p2p_rows_load(rows, nq, src_idx + item_qb[it], nullptr, bs, be);
+    __syncthreads();
+    const bool halves = t1 - t0 <= 16;
+    const int step = halves ? 2 : 1, sub = halves ? lane >> 4 : 0, tl = halves ? lane & 15 : lane;
+    const int nchunks = nq * tchunks;
     for (int tc = 0; tc < tchunks; tc++) {
-        int32_t i = t0 + tc * 32 + lane;
-        bool valid = i < t1;
-        double xi = valid ? x[i] : 0.0, yi = valid ? y[i] : 0.0, mi = valid ? m[i] : 0.0;
-        double lxi = valid ? lx[i] : 0.0, lyi = valid ? ly[i] : 0.0;
+        const int32_t i = t0 + tc * 32 + tl;
+        const bool valid = i < t1;
+        const double xi = valid ? x[i] : 0.0, yi = valid ? y[i] : 0.0, mi = valid ? m[i] : 0.0;
+        const double lxi = valid ? lx[i] : 0.0, lyi = valid ? ly[i] : 0.0;
         double gxa = 0.0, gya = 0.0, gma = 0.0;
         if (t0 + tc * 32 < t1) {
-            for (int k = 0; k < nq; k++) {
-                int s0 = __shfl_sync(0xffffffffu, sbeg, k), s1 = __shfl_sync(0xffffffffu, send, k);
-                for (int sc = s0; sc < s1; sc += 32) {
-                    int j = sc + lane;
-                    __syncwarp();
-                    if (j < s1) {
-                        sb[w][lane] = make_double4(x[j], y[j], lx[j], ly[j]);
-                        sm_[w][lane] = m[j];
-                    }
-                    __syncwarp();
-                    int ns = min(32, s1 - sc);
-                    for (int kk = 0; kk < ns; kk++) {
-                        if (sc + kk == i) continue;
-                        double4 bj = sb[w][kk];
-                        double mj = sm_[w][kk];
-                        double dx = bj.x - xi, dy = bj.y - yi;
-                        double r2 = dx * dx + dy * dy + eps2;
-                        double ir = rsqrt(r2);
-                        double ir3 = ir * ir * ir, ir5 = ir3 * ir * ir;
-                        double wx = mi * bj.z - mj * lxi, wy = mi * bj.w - mj * lyi;
-                        double dw = dx * wx + dy * wy;
-                        gxa += ir3 * wx - 3.0 * ir5 * dx * dw;
-                        gya += ir3 * wy - 3.0 * ir5 * dy * dw;
-                        gma -= (bj.z * dx + bj.w * dy) * ir3;
-                    }
+            for (int base = 0; base < nchunks; base += 4) {
+                int32_t j;
+                int ns;
+                const int slot = p2p_run_slot(rows, nq, tchunks, base, j, ns);
+                __syncthreads();  // the last run has been read
+                if (slot >= 0) {
+                    sb[slot] = make_double4(x[j], y[j], lx[j], ly[j]);
+                    smass[slot] = m[j];
+                    sj[slot] = j;
+                }
+                __syncthreads();
+                const int q1 = (w + 1) * ns / 4;
+                for (int q = w * ns / 4 + sub; q < q1; q += step) {
+                    if (sj[q] == i) continue;
+                    const double4 bj = sb[q];
+                    const double mj = smass[q];
+                    const double dx = bj.x - xi, dy = bj.y - yi;
+                    double ir3, ir5x3;
+                    gx_r3_3r5(fma(dx, dx, fma(dy, dy, eps2)), ir3, ir5x3);
+                    const double wx = mi * bj.z - mj * lxi, wy = mi * bj.w - mj * lyi;
+                    const double dw = ir5x3 * (dx * wx + dy * wy);
+                    gxa = fma(ir3, wx, fma(-dw, dx, gxa));
+                    gya = fma(ir3, wy, fma(-dw, dy, gya));
+                    gma = fma(-ir3, bj.z * dx + bj.w * dy, gma);
                 }
             }
         }
-        part[(it * tchunks + tc) * 32 + lane] = make_double4(gxa, gya, gma, 0.0);
+        if (halves) {
+            const double ox = __shfl_xor_sync(0xffffffffu, gxa, 16), oy = __shfl_xor_sync(0xffffffffu, gya, 16),
+                         om = __shfl_xor_sync(0xffffffffu, gma, 16);
+            gxa = sub ? ox + gxa : gxa + ox;
+            gya = sub ? oy + gya : gya + oy;
+            gma = sub ? om + gma : gma + om;
+        }
+        __syncthreads();  // sb becomes the four warps' sums
+        sb[threadIdx.x] = make_double4(gxa, gya, gma, 0.0);
+        __syncthreads();
+        if (w == 0) {
+            double4 s = sb[lane], u = sb[64 + lane];
+            vadd(s, sb[32 + lane]);
+            vadd(u, sb[96 + lane]);
+            vadd(s, u);
+            part[(it * tchunks + tc) * 32 + lane] = s;
+        }
+        __syncthreads();
     }
 }
 
@@ -703,10 +725,10 @@ int run_force_vjp(gx_ctx *ctx, const double *X, const double *Y, const void *lf_
                                                             dptr<int32_t>(ctx->near_idx), (float)eps2, tchunks,
                                                             dptr<float4>(ctx->part));
         else
-            k_adj_p2p_items<<<gi, 128, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
-                                                          dptr<int32_t>(I.nq), X, Y, Mb, lx, ly, bs, be,
-                                                          dptr<int32_t>(ctx->near_idx), eps2, tchunks,
-                                                          dptr<double4>(ctx->part));
+            k_adj_p2p_items<<<(unsigned)I.n, 128, 0, ctx->stream2>>>(dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
+                                                                     dptr<int32_t>(I.nq), X, Y, Mb, lx, ly, bs, be,
+                                                                     dptr<int32_t>(ctx->near_idx), eps2, tchunks,
+                                                                     dptr<double4>(ctx->part));
         if (I.n > GX_FOLD_MIN) {
             const unsigned gf = (unsigned)(((I.n + GX_FOLD - 1) / GX_FOLD * 32 + 127) / 128);
             if (F32)

@@ -19,6 +19,7 @@
 // factor is applied once per target after the sum over its sources.
 #pragma once
 #include "gx_internal.cuh"
+#include "gx_mass_r3.cuh"
 
 namespace {
 
@@ -811,87 +812,141 @@ __device__ __forceinline__ void l2p_eval(const T *__restrict__ Ll, T du, T dv, T
 // kernel evaluates L2P and adds the partials of each leaf in item order, so the
 // result does not depend on scheduling.
 
-// FP64 partials: sum_j m_j (x_j - x_i) / (r^2+eps^2)^(3/2)
-__global__ void __launch_bounds__(128) k_p2p64_items(int64_t n_items, const int32_t *__restrict__ item_leaf,
+// The source side of an FP64 work item, shared by a block of four warps: the item's rows
+// (source leaves, in chunks of 32 bodies) are taken four at a time, a warp loading each, and
+// their kept bodies are packed into one run of shared memory that the four warps then
+// divide.  An item is then four warps of work however few rows it has, which is what a
+// small problem needs (an FP64 instruction holds its scheduler for 64 clocks, so one warp on
+// 32 rows took 540 us at N = 1000), and no extra partials are written for it.
+struct P2PRows {
+    int32_t beg[32], end[32];
+    uint32_t skip[32];  // bodies of the row left out (the body-level P2L)
+};
+
+__device__ __forceinline__ void p2p_rows_load(P2PRows &r, int nq, const int32_t *__restrict__ src,
+                                              const uint32_t *__restrict__ mask, const int32_t *__restrict__ bs,
+                                              const int32_t *__restrict__ be) {
+    if ((int)threadIdx.x < nq) {
+        const int32_t sl = src[threadIdx.x];
+        r.beg[threadIdx.x] = bs[sl];
+        r.end[threadIdx.x] = be[sl];
+        r.skip[threadIdx.x] = mask ? mask[threadIdx.x] : 0u;
+    }
+}
+
+// chunk c of the rows (row c / chunks, its bodies from (c % chunks) 32 on): first body and
+// the bits of the bodies kept; empty past the last chunk
+__device__ __forceinline__ uint32_t p2p_chunk(const P2PRows &r, int nq, int chunks, int c, int32_t &j0) {
+    const int row = chunks == 1 ? c : c / chunks;
+    j0 = 0;
+    if (row >= nq) return 0u;
+    j0 = r.beg[row] + (c - row * chunks) * 32;
+    const int nb = r.end[row] - j0;
+    return nb <= 0 ? 0u : ((nb >= 32 ? 0xffffffffu : (1u << nb) - 1u) & ~r.skip[row]);
+}
+
+// This lane's place in the run of the four chunks base .. base + 3 (its warp's chunk is
+// base + w), -1 if its body is not kept; j its body, total the run's length
+__device__ __forceinline__ int p2p_run_slot(const P2PRows &r, int nq, int chunks, int base, int32_t &j, int &total) {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int before = 0;
+    int32_t j0 = 0;
+    uint32_t mine = 0;
+    total = 0;
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+        int32_t jv;
+        const uint32_t k = p2p_chunk(r, nq, chunks, base + v, jv);
+        if (v == w) {
+            before = total;
+            mine = k;
+            j0 = jv;
+        }
+        total += __popc(k);
+    }
+    j = j0 + lane;
+    return ((mine >> lane) & 1u) ? before + __popc(mine & ((1u << lane) - 1u)) : -1;
+}
+
+// FP64 partials: sum_j m_j (x_j - x_i) / (r^2+eps^2)^(3/2), a block per item.  Bound by the
+// FP64 pipe (two lanes a clock and SM), so m r^-3 comes from the integer pipes (gx_mass_r3)
+// and an interaction keeps six FP64 instructions of 18.  A leaf of at most 16 bodies leaves
+// half the lanes without a target, and the pipe's cost is per warp: there each half-warp
+// takes every other source.  Halves and warps are added in a fixed order.
+__global__ void __launch_bounds__(128) k_p2p64_items(const int32_t *__restrict__ item_leaf,
                                                      const int64_t *__restrict__ item_qb, const int32_t *__restrict__ item_nq,
                                                      const double *__restrict__ x, const double *__restrict__ y,
                                                      const double *__restrict__ m, const int32_t *__restrict__ bs,
                                                      const int32_t *__restrict__ be, const int32_t *__restrict__ src_idx,
                                                      const uint32_t *__restrict__ p2p_mask, double eps2, int tchunks,
                                                      double2 *__restrict__ part) {
-    __shared__ double3 sb[4][32];
-    int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (it >= n_items) return;
-    int32_t leaf = item_leaf[it];
-    int64_t qb = item_qb[it];
-    int nq = item_nq[it];
+    __shared__ P2PRows rows;
+    __shared__ double2 spos[128];
+    __shared__ GxMass sgm[128];
+    __shared__ double smass[128];
+    __shared__ int32_t sj[128];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t it = blockIdx.x;
+    const int nq = item_nq[it];
     if (nq < 0) return;  // an M2P item of the near-list split (k_m2p)
-    int32_t t0 = bs[leaf], t1 = be[leaf];
-    int sl = lane < nq ? src_idx[qb + lane] : -1;
-    int sbeg = sl >= 0 ? bs[sl] : 0, send = sl >= 0 ? be[sl] : 0;
-    // the body-level P2L (p2p_mask != null): a row's masked bodies are skipped here
-    const uint32_t skip = (p2p_mask && sl >= 0) ? p2p_mask[qb + lane] : 0u;
-    auto fetch = [&](int k, int sc) -> double3 {
-        int s0 = __shfl_sync(0xffffffffu, sbeg, k) + sc, s1 = __shfl_sync(0xffffffffu, send, k);
-        int j = s0 + lane;
-        return (j < s1) ? make_double3(x[j], y[j], m[j]) : make_double3(0.0, 0.0, 0.0);
-    };
+    const int32_t leaf = item_leaf[it];
+    const int64_t qb = item_qb[it];
+    const int32_t t0 = bs[leaf], t1 = be[leaf];
+    p2p_rows_load(rows, nq, src_idx + qb, p2p_mask ? p2p_mask + qb : nullptr, bs, be);
+    __syncthreads();
+    const bool halves = t1 - t0 <= 16;
+    const int step = halves ? 2 : 1, sub = halves ? lane >> 4 : 0, tl = halves ? lane & 15 : lane;
+    const int nchunks = nq * tchunks;  // a source leaf has at most as many chunks as the largest target
     for (int tc = 0; tc < tchunks; tc++) {
-        int32_t i = t0 + tc * 32 + lane;
-        bool valid = i < t1;
-        double xi = valid ? x[i] : 0.0, yi = valid ? y[i] : 0.0;
+        const int32_t i = t0 + tc * 32 + tl;
+        const bool valid = i < t1;
+        const double xi = valid ? x[i] : 0.0, yi = valid ? y[i] : 0.0;
         double accx = 0.0, accy = 0.0;
         if (t0 + tc * 32 < t1) {
-            double3 cur = fetch(0, 0);
-            for (int k = 0; k < nq; k++) {
-                int s0 = __shfl_sync(0xffffffffu, sbeg, k), s1 = __shfl_sync(0xffffffffu, send, k);
-                int srcl = __shfl_sync(0xffffffffu, sl, k);
-                const uint32_t sk = __shfl_sync(0xffffffffu, skip, k);
-                for (int sc = 0; sc < s1 - s0; sc += 32) {
-                    double3 nxt;
-                    if (sc + 32 < s1 - s0) nxt = fetch(k, sc + 32);
-                    else nxt = (k + 1 < nq) ? fetch(k + 1, 0) : make_double3(0.0, 0.0, 0.0);
-                    __syncwarp();
-                    sb[w][lane] = cur;
-                    __syncwarp();
-                    int ns = min(32, s1 - s0 - sc);
-                    if (srcl == leaf) {
-                        for (int kk = 0; kk < ns; kk++) {
-                            double3 bb = sb[w][kk];
-                            double dx = bb.x - xi, dy = bb.y - yi;
-                            double ir = rsqrt(dx * dx + dy * dy + eps2);
-                            double f = bb.z * (ir * ir * ir);
-                            if (s0 + sc + kk == i) f = 0.0;
-                            accx += f * dx;
-                            accy += f * dy;
-                        }
-                    } else if (sk) {
-                        for (int kk = 0; kk < ns; kk++) {
-                            if ((sk >> kk) & 1u) continue;  // leaves of at most 32 bodies: sc = 0
-                            double3 bb = sb[w][kk];
-                            double dx = bb.x - xi, dy = bb.y - yi;
-                            double ir = rsqrt(dx * dx + dy * dy + eps2);
-                            double f = bb.z * (ir * ir * ir);
-                            accx += f * dx;
-                            accy += f * dy;
-                        }
-                    } else {
-#pragma unroll 4
-                        for (int kk = 0; kk < ns; kk++) {
-                            double3 bb = sb[w][kk];
-                            double dx = bb.x - xi, dy = bb.y - yi;
-                            double ir = rsqrt(dx * dx + dy * dy + eps2);
-                            double f = bb.z * (ir * ir * ir);
-                            accx += f * dx;
-                            accy += f * dy;
-                        }
-                    }
-                    cur = nxt;
+            int32_t j;
+            int total;
+            int slot = p2p_run_slot(rows, nq, tchunks, 0, j, total);
+            double3 b = slot >= 0 ? make_double3(x[j], y[j], m[j]) : make_double3(0.0, 0.0, 0.0);
+            for (int base = 0; base < nchunks; base += 4) {
+                __syncthreads();  // the last run has been read
+                if (slot >= 0) {
+                    spos[slot] = make_double2(b.x, b.y);
+                    sgm[slot] = gx_mass_split(b.z);
+                    smass[slot] = b.z;
+                    sj[slot] = j;
+                }
+                const int ns = total;
+                __syncthreads();
+                if (base + 4 < nchunks) {  // the next run's loads are in flight while this one is computed
+                    slot = p2p_run_slot(rows, nq, tchunks, base + 4, j, total);
+                    if (slot >= 0) b = make_double3(x[j], y[j], m[j]);
+                }
+                const int q1 = (w + 1) * ns / 4;
+#pragma unroll 2
+                for (int q = w * ns / 4; q < q1; q += step) {
+                    const int kk = min(q + sub, q1 - 1);
+                    const double2 p = spos[kk];
+                    const double dx = p.x - xi, dy = p.y - yi;
+                    const double f = (q + sub < q1 && sj[kk] != i)
+                                         ? gx_mass_r3(fma(dx, dx, fma(dy, dy, eps2)), sgm[kk], smass[kk])
+                                         : 0.0;
+                    accx = fma(f, dx, accx);
+                    accy = fma(f, dy, accy);
                 }
             }
         }
-        part[(it * tchunks + tc) * 32 + lane] = make_double2(accx, accy);
+        if (halves) {
+            const double ox = __shfl_xor_sync(0xffffffffu, accx, 16), oy = __shfl_xor_sync(0xffffffffu, accy, 16);
+            accx = sub ? ox + accx : accx + ox;
+            accy = sub ? oy + accy : accy + oy;
+        }
+        __syncthreads();  // spos becomes the four warps' sums
+        spos[threadIdx.x] = make_double2(accx, accy);
+        __syncthreads();
+        if (w == 0) {
+            const double2 a = spos[lane], b = spos[32 + lane], c = spos[64 + lane], d = spos[96 + lane];
+            part[(it * tchunks + tc) * 32 + lane] = make_double2((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y));
+        }
     }
 }
 
@@ -2379,9 +2434,9 @@ int run_forces(gx_ctx *ctx, bool timed) {
                                                             dptr<int32_t>(I.nq), pos, comx, comy, bs, be, src_idx,
                                                             (float)eps2, tchunks, dptr<float2>(ctx->part));
             else
-                k_p2p64_items<<<gi, 128, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
-                                                            dptr<int32_t>(I.nq), X, Y, Mb, bs, be, src_idx, p2p_mask, eps2,
-                                                            tchunks, dptr<double2>(ctx->part));
+                k_p2p64_items<<<(unsigned)I.n, 128, 0, ctx->stream2>>>(dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
+                                                                       dptr<int32_t>(I.nq), X, Y, Mb, bs, be, src_idx,
+                                                                       p2p_mask, eps2, tchunks, dptr<double2>(ctx->part));
             ctx->launches++;
         }
         if (timed) GX_CUDA(ctx, cudaEventRecord(ctx->ev[15], ctx->stream2));  // the P2P kernel alone

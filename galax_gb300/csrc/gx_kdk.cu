@@ -5,9 +5,12 @@
 //  * diagnostics (galax-core/src/lib.rs:1638-1683): KE, FMM PE, momentum, Lz as
 //    deterministic two-stage block reductions (fixed grid, fixed tree order);
 //  * validate_fmm's exact sum (lib.rs:1537-1553) for sampled targets.
+#include <cooperative_groups.h>
+
 #include <mutex>
 
 #include "gx_internal.cuh"
+#include "gx_mass_r3.cuh"
 
 namespace {
 
@@ -79,28 +82,62 @@ __global__ void k_diag_final(const double *part, int nb, double *out) {
     }
 }
 
-// one block per sampled target
-__global__ void k_n2_sampled(int64_t n, const double *x, const double *y, const double *m, double eps2,
-                             const int64_t *idx, double *ax, double *ay) {
+// One cluster of blocks per sampled target, the bodies dealt out over its threads; the
+// blocks' sums are added in rank order through distributed shared memory, so the result
+// does not depend on scheduling and no scratch is needed.  Bound by the FP64 pipe: m r^-3
+// comes from the integer pipes (gx_mass_r3), which leaves six FP64 instructions a pair.
+__global__ void __launch_bounds__(RED_THREADS) k_n2_sampled(int64_t n, const double *__restrict__ x,
+                                                            const double *__restrict__ y,
+                                                            const double *__restrict__ m, double eps2,
+                                                            const int64_t *__restrict__ idx, double *ax, double *ay) {
+    namespace cg = cooperative_groups;
     __shared__ double sh[RED_THREADS / 32];
-    int64_t i = idx[blockIdx.x];
-    double xi = x[i], yi = y[i];
+    __shared__ double2 tot;
+    cg::cluster_group cl = cg::this_cluster();
+    const unsigned nb = cl.num_blocks(), rank = cl.block_rank();
+    const int64_t s = blockIdx.x / nb, i = idx[s];
+    const double xi = x[i], yi = y[i];
     double fx = 0.0, fy = 0.0;
-    for (int64_t j = threadIdx.x; j < n; j += blockDim.x) {
-        if (j == i) continue;
-        double dx = x[j] - xi, dy = y[j] - yi;
-        double r2 = dx * dx + dy * dy + eps2;
-        double ir = 1.0 / sqrt(r2);
-        double f = m[j] * (ir * (ir * ir));
-        fx += f * dx;
-        fy += f * dy;
+#pragma unroll 2
+    for (int64_t j = (int64_t)rank * blockDim.x + threadIdx.x; j < n; j += (int64_t)nb * blockDim.x) {
+        const double mj = m[j], dx = x[j] - xi, dy = y[j] - yi;
+        const double f = j == i ? 0.0 : gx_mass_r3(fma(dx, dx, fma(dy, dy, eps2)), gx_mass_split(mj), mj);
+        fx = fma(f, dx, fx);
+        fy = fma(f, dy, fy);
     }
-    double tx = block_sum(fx, sh);
-    double ty = block_sum(fy, sh);
-    if (threadIdx.x == 0) {
-        ax[blockIdx.x] = tx;
-        ay[blockIdx.x] = ty;
+    const double tx = block_sum(fx, sh);
+    const double ty = block_sum(fy, sh);
+    if (threadIdx.x == 0) tot = make_double2(tx, ty);
+    cl.sync();
+    if (rank == 0 && threadIdx.x == 0) {
+        double sx = 0.0, sy = 0.0;
+        for (unsigned b = 0; b < nb; b++) {
+            const double2 v = *cl.map_shared_rank(&tot, b);
+            sx += v.x;
+            sy += v.y;
+        }
+        ax[s] = sx;
+        ay[s] = sy;
     }
+    cl.sync();  // the other blocks' sums stay in place until rank 0 has read them
+}
+
+// Blocks of a cluster: enough to fill the GPU (eight blocks an SM) when the samples alone do not.
+cudaError_t launch_n2(int64_t n, const double *x, const double *y, const double *m, double eps2, const int64_t *idx,
+                      int64_t n_idx, double *ax, double *ay, int sms, cudaStream_t st) {
+    unsigned c = 1;
+    while (c < 8 && n_idx * c < (int64_t)sms * 8 && (int64_t)c * RED_THREADS < n) c *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)n_idx * c);
+    cfg.blockDim = dim3(RED_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = c;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_n2_sampled, n, x, y, m, eps2, idx, ax, ay);
 }
 
 }  // namespace
@@ -168,9 +205,8 @@ int gx_n2_device(gx_ctx *ctx, const int64_t *idx, int64_t n_idx, double *ax, dou
     for (int64_t k = 0; k < n_idx; k++)
         if (idx[k] < 0 || idx[k] >= ctx->n_bodies) return gx_fail(ctx, GX_ERR_INVALID_ARG, "n2: index out of range");
     GX_CUDA(ctx, cudaMemcpyAsync(didx, idx, sizeof(int64_t) * n_idx, cudaMemcpyHostToDevice, ctx->stream));
-    k_n2_sampled<<<(unsigned)n_idx, RED_THREADS, 0, ctx->stream>>>(ctx->n_bodies, dptr<double>(ctx->x),
-                                                                   dptr<double>(ctx->y), dptr<double>(ctx->m),
-                                                                   ctx->eps * ctx->eps, didx, dax, day);
+    GX_CUDA(ctx, launch_n2(ctx->n_bodies, dptr<double>(ctx->x), dptr<double>(ctx->y), dptr<double>(ctx->m),
+                           ctx->eps * ctx->eps, didx, n_idx, dax, day, ctx->sm_count, ctx->stream));
     ctx->launches++;
     GX_CUDA(ctx, cudaGetLastError());
     GX_CUDA(ctx, cudaMemcpyAsync(ax, dax, sizeof(double) * n_idx, cudaMemcpyDeviceToHost, ctx->stream));
@@ -237,8 +273,12 @@ extern "C" int gx_n2_sampled_static(const double *x, const double *y, const doub
         cudaGetLastError();
         return GX_ERR_CUDA;
     }
-    k_n2_sampled<<<(unsigned)n_idx, RED_THREADS, 0, st>>>(n, x, y, m, eps * eps, didx, dax, day);
-    if (cudaGetLastError() != cudaSuccess) return GX_ERR_CUDA;
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        launch_n2(n, x, y, m, eps * eps, didx, n_idx, dax, day, sms, st) != cudaSuccess) {
+        cudaGetLastError();
+        return GX_ERR_CUDA;
+    }
     if (cudaMemcpyAsync(ax, dax, sizeof(double) * n_idx, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaMemcpyAsync(ay, day, sizeof(double) * n_idx, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess) {

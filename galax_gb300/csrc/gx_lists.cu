@@ -1575,7 +1575,23 @@ int gx_plan_near_split(gx_ctx *ctx) {
 }
 
 namespace {
-constexpr int P2P_K = 32;  // source leaves per P2P work item
+constexpr int P2P_K = 32;  // most source leaves per P2P (or M2P) work item
+
+// Source leaves per P2P item: a small problem's lists are cut finer, down to one leaf an
+// item, until there are enough items for the GPU to balance: 8 an SM for the reference's
+// lists (FP64; at N = 1000 their 306 near pairs were 32 items), 2 an SM for the
+// opening-angle lists, whose mixed form gains less from it than its final sum pays for the
+// extra partials (N = 10,000, 14,561 near pairs, 8 an SM: P2P 28 -> 20 us beside the far
+// field, sum 8 -> 10 us after it).
+static int p2p_item_leaves(const gx_ctx *ctx, int64_t near_pairs, bool accurate) {
+    const int64_t want = (int64_t)ctx->sm_count * (accurate ? 2 : 8);
+    int k = P2P_K;
+    while (k > 1 && near_pairs / k < want) k /= 2;
+    return k;
+}
+// Source leaves per M2P item: not below eight (k_m2p_x2 sets up its moments a lane per
+// source and its half-warps take every other one).
+static int m2p_item_leaves(int p2p_leaves) { return p2p_leaves < 8 ? 8 : p2p_leaves; }
 
 // ancestor table: anc[level * nl + leaf] = the leaf's ancestor at that level
 __global__ void k_ancestors(int64_t nl, int n_levels, const int32_t *parent, int32_t *anc) {
@@ -1600,25 +1616,25 @@ __global__ void k_comhl(int64_t nn, const double *comx, const double *comy, floa
 // per leaf: number of items; start/count from either list layout.  With the near-list
 // split (split != null) the leaf's P2P items are followed by its M2P items, whose
 // source count is stored negated; split[2a] is the leaf's M2P count.
-__global__ void k_items_count(int64_t nl, const int64_t *start, const int32_t *cnt, const int32_t *split,
+__global__ void k_items_count(int64_t nl, int K, int KM, const int64_t *start, const int32_t *cnt, const int32_t *split,
                               int64_t *nitems) {
     int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (a > nl) return;
     if (a == nl) { nitems[a] = 0; return; }
     int64_t c = cnt ? cnt[a] : start[a + 1] - start[a];
     int64_t cm = split ? split[2 * a] : 0;
-    nitems[a] = (c + P2P_K - 1) / P2P_K + (cm + P2P_K - 1) / P2P_K;
+    nitems[a] = (c + K - 1) / K + (cm + KM - 1) / KM;
 }
 
 // per leaf: number of M2P items (the compact list the M2P kernel runs over)
-__global__ void k_m2p_items_count(int64_t nl, const int32_t *split, int64_t *n) {
+__global__ void k_m2p_items_count(int64_t nl, int KM, const int32_t *split, int64_t *n) {
     int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (a > nl) return;
-    n[a] = a == nl ? 0 : (split[2 * a] + P2P_K - 1) / P2P_K;
+    n[a] = a == nl ? 0 : (split[2 * a] + KM - 1) / KM;
 }
 
 // one warp per leaf, lanes over its items: the widest halo leaves have ~1000 items
-__global__ void k_items_fill(int64_t nl, const int64_t *start, const int32_t *cnt, const int32_t *split,
+__global__ void k_items_fill(int64_t nl, int K, int KM, const int64_t *start, const int32_t *cnt, const int32_t *split,
                              const int64_t *off, int32_t *leaf, int64_t *qb, int32_t *nq, const int64_t *m2p_off,
                              int32_t *m2p_list) {
     const int64_t a = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1626,18 +1642,18 @@ __global__ void k_items_fill(int64_t nl, const int64_t *start, const int32_t *cn
     if (a >= nl) return;
     const int64_t s0 = start[a];
     const int64_t c = cnt ? cnt[a] : start[a + 1] - start[a];
-    const int64_t it0 = off[a], np = (c + P2P_K - 1) / P2P_K;
+    const int64_t it0 = off[a], np = (c + K - 1) / K;
     for (int64_t k = lane; k < np; k += 32) {
         leaf[it0 + k] = (int32_t)a;
-        qb[it0 + k] = s0 + k * P2P_K;
-        nq[it0 + k] = (int32_t)min((int64_t)P2P_K, c - k * P2P_K);
+        qb[it0 + k] = s0 + k * K;
+        nq[it0 + k] = (int32_t)min((int64_t)K, c - k * K);
     }
-    const int64_t cm = split ? split[2 * a] : 0, nm = (cm + P2P_K - 1) / P2P_K;
+    const int64_t cm = split ? split[2 * a] : 0, nm = (cm + KM - 1) / KM;
     for (int64_t k = lane; k < nm; k += 32) {
         const int64_t it = it0 + np + k;
         leaf[it] = (int32_t)a;
-        qb[it] = s0 + c + k * P2P_K;
-        nq[it] = -(int32_t)min((int64_t)P2P_K, cm - k * P2P_K);
+        qb[it] = s0 + c + k * KM;
+        nq[it] = -(int32_t)min((int64_t)KM, cm - k * KM);
         m2p_list[m2p_off[a] + k] = (int32_t)it;
     }
 }
@@ -1855,10 +1871,12 @@ int gx_plan_items(gx_ctx *ctx, bool accurate) {
     const bool body = split && nl > 0 && gx_body_split_on(ctx);  // body-level P2L units after the leaf-level ones
     if (accurate) ctx->plan_body_split = false;  // the masks follow these items (gx_plan_body_masks)
     const int32_t *scnt = split ? dptr<int32_t>(ctx->split_cnt) : nullptr;
+    const int K = p2p_item_leaves(ctx, accurate ? ctx->n_near_pairs : ctx->n_p2p_pairs, accurate);
+    const int KM = m2p_item_leaves(K);
     GX_TRY(gx_ensure(ctx, I.off, sizeof(int64_t) * (size_t)(nl + 1)));
     GX_TRY(gx_ensure(ctx, ctx->scratch_c, sizeof(int64_t) * (size_t)(nl + 1)));
     int64_t *nit = dptr<int64_t>(ctx->scratch_c);
-    k_items_count<<<gx_blocks(nl + 1, 256), 256, 0, ctx->stream>>>(nl, start, cnt, scnt, nit);
+    k_items_count<<<gx_blocks(nl + 1, 256), 256, 0, ctx->stream>>>(nl, K, KM, start, cnt, scnt, nit);
     GX_TRY(gx_exclusive_scan_i64(ctx, nit, dptr<int64_t>(I.off), nl + 1));
     int64_t tot[5] = {0, 0, 0, 0, 0};
     unsigned long long stot[4] = {0, 0, 0, 0};
@@ -1867,7 +1885,7 @@ int gx_plan_items(gx_ctx *ctx, bool accurate) {
         GX_TRY(gx_ensure(ctx, ctx->m2p_off, sizeof(int64_t) * (size_t)(nl + 1)));
         GX_TRY(gx_ensure(ctx, ctx->scratch_e, sizeof(int64_t) * (size_t)(nl + 1)));  // free after the plan
         int64_t *nm = dptr<int64_t>(ctx->scratch_e);
-        k_m2p_items_count<<<gx_blocks(nl + 1, 256), 256, 0, ctx->stream>>>(nl, scnt, nm);
+        k_m2p_items_count<<<gx_blocks(nl + 1, 256), 256, 0, ctx->stream>>>(nl, KM, scnt, nm);
         GX_TRY(gx_exclusive_scan_i64(ctx, nm, dptr<int64_t>(ctx->m2p_off), nl + 1));
         GX_CUDA(ctx, cudaMemcpyAsync(&tot[3], dptr<int64_t>(ctx->m2p_off) + nl, sizeof(int64_t),
                                      cudaMemcpyDeviceToHost, ctx->stream));
@@ -1913,7 +1931,7 @@ int gx_plan_items(gx_ctx *ctx, bool accurate) {
     GX_TRY(gx_ensure(ctx, I.nq, sizeof(int32_t) * (size_t)(tot[0] + 1)));
     if (split) GX_TRY(gx_ensure(ctx, ctx->m2p_list, sizeof(int32_t) * (size_t)(tot[3] + 1)));
     k_items_fill<<<gx_blocks(nl * 32, 256), 256, 0, ctx->stream>>>(
-        nl, start, cnt, scnt, dptr<int64_t>(I.off), dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb), dptr<int32_t>(I.nq),
+        nl, K, KM, start, cnt, scnt, dptr<int64_t>(I.off), dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb), dptr<int32_t>(I.nq),
         split ? dptr<int64_t>(ctx->m2p_off) : nullptr, split ? dptr<int32_t>(ctx->m2p_list) : nullptr);
     ctx->launches += 2;
     I.n = tot[0];
