@@ -95,51 +95,10 @@ __global__ void __launch_bounds__(128) k_adj_l2p(int64_t nl, const double *__res
     }
 }
 
-// ---- A2: L2L^T, one level of the upward pass: dL[P][U] = sum_c sum_{T<=U} dL[c][T] C(U,T) e^(U-T),
-// e = com_c - com_P.  The leaves' rows are already in place; internal rows are written here.
-template <int P, class T>
-__global__ void __launch_bounds__(128) k_adj_l2l_up(int64_t s, int64_t e, const int4 *__restrict__ child,
-                                                    const double *__restrict__ comx, const double *__restrict__ comy,
-                                                    T *__restrict__ dL) {
-    constexpr int NC = nc2(P);
-    constexpr int NS = row_stride<T>(NC);
-    const int PP = gx_rt_order(P);
-    const int NCr = (PP + 1) * (PP + 2) / 2;
-    int64_t node = s + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (node >= e) return;
-    int4 c4 = child[node];
-    int cc[4] = {c4.x, c4.y, c4.z, c4.w};
-    T out[NC];
-#pragma unroll
-    for (int k = 0; k < NCr; k++) out[k] = T(0);
-    for (int q = 0; q < 4; q++) {
-        int c = cc[q];
-        if (c < 0) continue;
-        T ex = (T)(comx[c] - comx[node]), ey = (T)(comy[c] - comy[node]);
-        T px[P + 1], py[P + 1];
-        px[0] = T(1);
-        py[0] = T(1);
-#pragma unroll
-        for (int k = 1; k <= PP; k++) {
-            px[k] = px[k - 1] * ex;
-            py[k] = py[k - 1] * ey;
-        }
-        T dc[NC];
-        load_row<NC>(dL + (int64_t)c * NS, dc);
-#pragma unroll
-        for (int ui = 0; ui <= PP; ui++)
-#pragma unroll
-            for (int uj = 0; uj <= PP - ui; uj++)
-#pragma unroll
-                for (int ti = 0; ti <= ui; ti++)
-#pragma unroll
-                    for (int tj = 0; tj <= uj; tj++)
-                        out[gx_mi(ui, uj)] += dc[gx_mi(ti, tj)] * (tab_binom<T>(ui, ti) * tab_binom<T>(uj, tj)) *
-                                              px[ui - ti] * py[uj - tj];
-    }
-#pragma unroll
-    for (int k = 0; k < NCr; k++) dL[node * NS + k] = out[k];
-}
+// ---- A2: L2L^T, an upward pass: dL[P][U] = sum_c sum_{T<=U} dL[c][T] C(U,T) e^(U-T),
+// e = com_c - com_P (run_up with ADJ; the leaves' rows are already in place).  As in M2M the
+// chain levels are one shift from the leaves to the top one: those below it have no far
+// lists, so A3 never reads their rows.
 
 // ---- A3: M2L^T as a gather over far(s) (far lists are symmetric):
 //   dM[s][S] = -(-1)^|S| sum_{t in far(s)} sum_T A(com_t - com_s)[S+T] dL[t][T] / T!
@@ -686,7 +645,6 @@ int run_force_vjp(gx_ctx *ctx, const double *X, const double *Y, const void *lf_
     const double *Mb = dptr<double>(ctx->m);
     const double *comx = dptr<double>(ctx->comx), *comy = dptr<double>(ctx->comy);
     const int32_t *bs = dptr<int32_t>(ctx->bs), *be = dptr<int32_t>(ctx->be);
-    const int4 *child = dptr<int4>(ctx->child);
     const double eps2 = ctx->eps * ctx->eps;
     const unsigned gw = (unsigned)((nl * 32 + 127) / 128);
     const T *Lf = reinterpret_cast<const T *>(lf_rows);
@@ -740,11 +698,9 @@ int run_force_vjp(gx_ctx *ctx, const double *X, const double *Y, const void *lf_
         }
     }
     GX_CUDA(ctx, cudaEventRecord(ctx->ev_join, ctx->stream2));
-    // A2: L2L^T upward, level by level (leaves are level 0)
-    for (int lv = 1; lv < ctx->n_levels; lv++) {
-        int64_t s = ctx->level_start[lv], e = ctx->level_start[lv + 1];
-        k_adj_l2l_up<P, T><<<gx_blocks(e - s, 128), 128, 0, st>>>(s, e, child, comx, comy, dL);
-    }
+    // A2: L2L^T
+    const int lc = ctx->chain_levels >= 2 ? ctx->chain_levels : 0;
+    GX_TRY((run_up<P, T, true>(ctx, lc, lc, dL, nullptr)));
     // A3: M2L^T
     const gx_ctx::M2LUnits &U = ctx->m2l_units;
     if (U.n > 0) {
@@ -770,7 +726,7 @@ int run_force_vjp(gx_ctx *ctx, const double *X, const double *Y, const void *lf_
     else
         k_adj_p2p_reduce<double4, double><<<gw, 128, 0, st>>>(nl, bs, be, dptr<int64_t>(I.off), tchunks,
                                                               dptr<double4>(ctx->part), gx, gy, gm);
-    ctx->launches += 6 + (ctx->n_levels - 1) + (I.n > GX_FOLD_MIN ? 1 : 0);
+    ctx->launches += 6 + (I.n > GX_FOLD_MIN ? 1 : 0);
     GX_CUDA(ctx, cudaGetLastError());
     return GX_OK;
 }

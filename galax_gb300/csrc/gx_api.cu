@@ -80,6 +80,7 @@ void gx_tree_plan_swap(gx_ctx *ctx, gx_tree_plan &t) {
     std::swap(ctx->m2l_units.n, t.units_n);
     std::swap(ctx->n_levels, t.n_levels);
     std::swap(ctx->chain_levels, t.chain_levels);
+    std::swap(ctx->unary_levels, t.unary_levels);
     std::swap(ctx->have_tree, t.have_tree);
     std::swap(ctx->aux_valid, t.aux_valid);
     std::swap(ctx->plan_acc_valid, t.plan_acc_valid);
@@ -264,6 +265,16 @@ __global__ void k_gather_i32(int64_t n, const uint32_t *perm, const int32_t *in,
 }
 }  // namespace
 
+// The levels of a device-built tree that are single-child chains over the leaves: a level
+// with as many nodes as there are leaves grouped nothing, and Tree::build numbers it in the
+// order of the level below.
+static int count_unary_levels(const gx_ctx *ctx) {
+    const std::vector<int64_t> &s = ctx->level_start;
+    int l = 0;
+    while (l + 1 < ctx->n_levels && s[l + 2] - s[l + 1] == s[1] - s[0]) l++;
+    return l;
+}
+
 // Device Tree::build over the resident bodies with the last build's parameters.
 int gx_rebuild_internal(gx_ctx *ctx) {
     if (ctx->build_n_max <= 0) return gx_fail(ctx, GX_ERR_STATE, "no tree parameters: build a tree first");
@@ -288,6 +299,7 @@ int gx_rebuild_internal(gx_ctx *ctx) {
     if (ctx->cfg.max_nodes && (uint64_t)ctx->n_nodes > ctx->cfg.max_nodes)
         return gx_fail(ctx, GX_ERR_CAP_EXCEEDED, "tree node count exceeds max_nodes");
     ctx->max_leaf = std::min<int64_t>(ctx->build_n_max, n);
+    ctx->unary_levels = count_unary_levels(ctx);
     ctx->have_tree = true;
     GX_CUDA(ctx, cudaGetLastError());
     return GX_OK;
@@ -379,6 +391,7 @@ int gx_build_tree(gx_ctx *ctx, int64_t n, double *x, double *y, double *vx, doub
     // the reference's V/U lists are built when first needed (REF mode, gx_export_lists)
     ctx->ref_lists_valid = false;
     ctx->max_leaf = std::min<int64_t>(n_max, n);
+    ctx->unary_levels = count_unary_levels(ctx);
     // Tree::build permutes the caller's arrays (lib.rs:204); so do we.
     if (!(flags & GX_BUILD_BALANCED)) GX_TRY(gx_download_bodies(ctx, x, y, vx, vy, m, ax, ay));
     GX_TRY(gx_ids_reset(ctx));  // the caller's arrays are now in tree order
@@ -456,6 +469,14 @@ int gx_upload_tree(gx_ctx *ctx, int64_t n_nodes, int64_t n_bodies, const double 
     ctx->n_bodies = n_bodies;
     ctx->max_leaf = 0;
     for (int64_t i = 0; i < nl; i++) ctx->max_leaf = std::max(ctx->max_leaf, body_end[i] - body_start[i]);
+    ctx->unary_levels = 0;
+    for (int l = 1; l < ctx->n_levels; l++) {  // single-child levels, checked node by node
+        bool chain = ls[l + 1] - ls[l] == nl;
+        for (int64_t i = ls[l]; chain && i < ls[l + 1]; i++)
+            chain = child[4 * i] == i - nl && child[4 * i + 1] < 0 && child[4 * i + 2] < 0 && child[4 * i + 3] < 0;
+        if (!chain) break;
+        ctx->unary_levels = l;
+    }
     ctx->ref_lists_valid = true;  // the caller's lists
     ctx->have_tree = true;
     return GX_OK;

@@ -6,7 +6,7 @@
 // so a warp reading one node's row reads one contiguous segment.
 //
 //   P2M   (lib.rs:848-887)   warp per leaf, lane per body, warp-shuffle reduction
-//   M2M   (lib.rs:890-938)   warp per parent, lane per output coefficient, per level
+//   M2M   (lib.rs:890-938)   four lanes per parent, one child each; small levels in one launch
 //   M2L   (lib.rs:1199-1259) warp per target node, lane per list entry, warp reduction
 //   L2L   (lib.rs:1262-1302) REF: node-id-ascending order means every leaf receives
 //                            its own M2L local plus one shift of its parent's M2L local;
@@ -18,6 +18,8 @@
 // reference's plan (lib.rs:1160-1196) is L[T] = (1/T!) sum_S M'[S] G[S+T]; the 1/T!
 // factor is applied once per target after the sum over its sources.
 #pragma once
+#include <cooperative_groups.h>
+
 #include "gx_internal.cuh"
 #include "gx_mass_r3.cuh"
 
@@ -274,95 +276,230 @@ __global__ void __launch_bounds__(128) k_p2m(int64_t nl, const double *__restric
     }
 }
 
-// ---------------------------------------------------------------- M2M
-// One thread per parent: M_P[I,J] = sum_children sum_{i<=I, j<=J} M_c[i,j] dx^(I-i) dy^(J-j) / ((I-i)!(J-j)!)
-template <int P, class T>
-__global__ void __launch_bounds__(128) k_m2m(int64_t s, int64_t e, const int4 *__restrict__ child,
-                                             const double *__restrict__ comx, const double *__restrict__ comy,
-                                             T *__restrict__ M) {
-    constexpr int NC = nc2(P);
+// ---------------------------------------------------------------- M2M (and L2L^T)
+// One upward shift, rows of a child moved to its parent's centre:
+//   M_P[I,J] += sum_{i<=I, j<=J} M_c[i,j] dx^(I-i)/(I-i)! dy^(J-j)/(J-j)!
+// done in place one axis at a time (descending, so the lower terms are still the old ones):
+// 20 + 20 multiply-adds at p = 4 against 70 products of three for the two axes together.
+// The transpose of L2L is the same shift on rows scaled by 1/(i! j!) before and i! j! after
+// (ADJ).
+template <int P, class T, bool ADJ>
+__device__ __forceinline__ void shift_up(T dx, T dy, T *c) {
+    const int PP = gx_rt_order(P);
+    if constexpr (ADJ) {
+#pragma unroll
+        for (int i = 0; i <= PP; i++)
+#pragma unroll
+            for (int j = 0; j <= PP - i; j++)
+                if (i > 1 || j > 1) c[gx_mi(i, j)] *= tab_ifp<T>(i, j);
+    }
+    T pw[P + 1];
+    pw[0] = T(1);
+#pragma unroll
+    for (int k = 1; k <= PP; k++) pw[k] = pw[k - 1] * (dy * tab_inv<T>(k));
+#pragma unroll
+    for (int i = 0; i <= PP; i++)
+#pragma unroll
+        for (int J = PP - i; J >= 1; J--)
+#pragma unroll
+            for (int j = 0; j < J; j++) c[gx_mi(i, J)] += c[gx_mi(i, j)] * pw[J - j];
+#pragma unroll
+    for (int k = 1; k <= PP; k++) pw[k] = pw[k - 1] * (dx * tab_inv<T>(k));
+#pragma unroll
+    for (int J = 0; J <= PP; J++)
+#pragma unroll
+        for (int I = PP - J; I >= 1; I--)
+#pragma unroll
+            for (int i = 0; i < I; i++) c[gx_mi(I, J)] += c[gx_mi(i, J)] * pw[I - i];
+    if constexpr (ADJ) {
+#pragma unroll
+        for (int i = 0; i <= PP; i++)
+#pragma unroll
+            for (int j = 0; j <= PP - i; j++)
+                if (i > 1 || j > 1) c[gx_mi(i, j)] *= tab_ff<T>(i, j);
+    }
+}
+
+// One parent by four lanes, one child each: the four shifted rows are summed by a
+// reduce-scatter (three additions per group of four coefficients instead of eight), lane q
+// ending with coefficients q, q + 4, ...  All 32 lanes of the warp call it; node < 0 stores
+// nothing.  Returns whether a stored value was not finite.
+template <int P, class T, bool ADJ>
+__device__ __forceinline__ bool up_node(int64_t node, const int4 *__restrict__ child,
+                                        const double *__restrict__ comx, const double *__restrict__ comy, T *M) {
+    constexpr int NC = nc2(P), NC4 = (NC + 3) / 4 * 4;
     constexpr int NS = row_stride<T>(NC);
     const int PP = gx_rt_order(P);
     const int NCr = (PP + 1) * (PP + 2) / 2;
-    int64_t node = s + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (node >= e) return;
-    int4 c4 = child[node];
-    int cc[4] = {c4.x, c4.y, c4.z, c4.w};
-    double pcx = comx[node], pcy = comy[node];
-    T out[NC];
+    const unsigned full = 0xffffffffu;
+    const int q = threadIdx.x & 3;
+    T c[NC4];
 #pragma unroll
-    for (int k = 0; k < NCr; k++) out[k] = T(0);
-    for (int q = 0; q < 4; q++) {
-        int c = cc[q];
-        if (c < 0) continue;
-        T dx = (T)(comx[c] - pcx), dy = (T)(comy[c] - pcy);
-        T px[P + 1], py[P + 1];
-        px[0] = T(1);
-        py[0] = T(1);
+    for (int k = 0; k < NC4; k++) c[k] = T(0);
+    if (node >= 0) {
+        const int ch = reinterpret_cast<const int *>(child + node)[q];
+        if (ch >= 0) {
 #pragma unroll
-        for (int k = 1; k <= PP; k++) {
-            px[k] = px[k - 1] * dx * tab_inv<T>(k);  // dx^k / k!
-            py[k] = py[k - 1] * dy * tab_inv<T>(k);
+            for (int k = 0; k < NCr; k++) c[k] = M[(int64_t)ch * NS + k];
+            shift_up<P, T, ADJ>((T)(comx[ch] - comx[node]), (T)(comy[ch] - comy[node]), c);
         }
-        T mc[NC];
-        load_row<NC>(M + (int64_t)c * NS, mc);
-#pragma unroll
-        for (int oi = 0; oi <= PP; oi++)
-#pragma unroll
-            for (int oj = 0; oj <= PP - oi; oj++)
-#pragma unroll
-                for (int i = 0; i <= oi; i++)
-#pragma unroll
-                    for (int j = 0; j <= oj; j++) out[gx_mi(oi, oj)] += mc[gx_mi(i, j)] * px[oi - i] * py[oj - j];
     }
+    bool bad = false;
 #pragma unroll
-    for (int k = 0; k < NCr; k++) M[node * NS + k] = out[k];
+    for (int g = 0; g < (NCr + 3) / 4; g++) {
+        const bool hi = q & 2, od = q & 1;
+        T k0 = hi ? c[4 * g + 2] : c[4 * g], k1 = hi ? c[4 * g + 3] : c[4 * g + 1];
+        k0 += __shfl_xor_sync(full, hi ? c[4 * g] : c[4 * g + 2], 2);
+        k1 += __shfl_xor_sync(full, hi ? c[4 * g + 1] : c[4 * g + 3], 2);
+        const T v = (od ? k1 : k0) + __shfl_xor_sync(full, od ? k0 : k1, 1);
+        if (node >= 0 && 4 * g + q < NCr) {
+            M[node * NS + 4 * g + q] = v;
+            bad |= !isfinite(v);
+        }
+    }
+    return bad;
 }
 
-// Levels 1 .. L of single-child chains over the leaves (Morton rounds that grouped
-// nothing): the level-L ancestor of leaf x is node x + L nl and holds the same bodies,
-// so its moments are the leaf's shifted once to its COM (translations compose exactly);
-// the chain nodes in between have no far interactions in the ACCURATE lists and their
-// moments are never read.
-template <int P, class T>
-__global__ void __launch_bounds__(128) k_m2m_chain(int64_t nl, int64_t up, const double *__restrict__ comx,
-                                                   const double *__restrict__ comy, T *__restrict__ M) {
+// A level of more nodes than the cluster kernel below takes: four lanes a parent.  bad: set
+// where a stored moment is not finite (null for the adjoint).
+template <int P, class T, bool ADJ>
+__global__ void __launch_bounds__(128) k_up_level(int64_t s, int64_t e, const int4 *__restrict__ child,
+                                                  const double *__restrict__ comx, const double *__restrict__ comy,
+                                                  T *M, unsigned *bad) {
+    const int64_t node = s + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 2);
+    if (up_node<P, T, ADJ>(node < e ? node : -1, child, comx, comy, M) && bad) atomicOr(bad, 1u);
+}
+
+// Levels l0 .. l1 of single-child chains over the leaves (Morton rounds that grouped
+// nothing): node x + l nl holds the bodies of leaf x, so its row is the leaf's shifted once
+// (translations compose exactly).  ACCURATE takes the top level only (the chain nodes below
+// it have no far lists and are never read), the reference's lists need them all.
+template <int P, class T, bool ADJ>
+__device__ __forceinline__ bool chain_node(int64_t x, int64_t node, const double *__restrict__ comx,
+                                           const double *__restrict__ comy, T *M) {
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<T>(NC);
     const int PP = gx_rt_order(P);
     const int NCr = (PP + 1) * (PP + 2) / 2;
-    int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nl) return;
-    const int64_t node = c + up;
-    T dx = (T)(comx[c] - comx[node]), dy = (T)(comy[c] - comy[node]);
-    T px[P + 1], py[P + 1];
-    px[0] = T(1);
-    py[0] = T(1);
+    T c[NC];
+    bool bad = false;
 #pragma unroll
-    for (int k = 1; k <= PP; k++) {
-        px[k] = px[k - 1] * dx * tab_inv<T>(k);
-        py[k] = py[k - 1] * dy * tab_inv<T>(k);
+    for (int k = 0; k < NCr; k++) c[k] = M[x * NS + k];
+    shift_up<P, T, ADJ>((T)(comx[x] - comx[node]), (T)(comy[x] - comy[node]), c);
+#pragma unroll
+    for (int k = 0; k < NCr; k++) {
+        M[node * NS + k] = c[k];
+        bad |= !isfinite(c[k]);
     }
-    T mc[NC], out[NC];
-    load_row<NC>(M + c * NS, mc);
-#pragma unroll
-    for (int k = 0; k < NCr; k++) out[k] = T(0);
-#pragma unroll
-    for (int oi = 0; oi <= PP; oi++)
-#pragma unroll
-        for (int oj = 0; oj <= PP - oi; oj++)
-#pragma unroll
-            for (int i = 0; i <= oi; i++)
-#pragma unroll
-                for (int j = 0; j <= oj; j++) out[gx_mi(oi, oj)] += mc[gx_mi(i, j)] * px[oi - i] * py[oj - j];
-#pragma unroll
-    for (int k = 0; k < NCr; k++) M[node * NS + k] = out[k];
+    return bad;
+}
+template <int P, class T, bool ADJ>
+__global__ void __launch_bounds__(128) k_up_chain(int64_t nl, int l0, int l1, const double *__restrict__ comx,
+                                                  const double *__restrict__ comy, T *M, unsigned *bad) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nl * (l1 - l0 + 1)) return;
+    const int64_t x = t % nl;
+    if (chain_node<P, T, ADJ>(x, x + (l0 + t / nl) * nl, comx, comy, M) && bad) atomicOr(bad, 1u);
 }
 
-template <class T>
-__global__ void k_scrub(int64_t n, T *v) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && !isfinite(v[i])) v[i] = T(0);
+// The small levels, bottom-up in one launch: a cluster of UP_BLOCKS blocks does a level's
+// nodes at once and meets at a cluster barrier before the next (a launch a level, a thread a
+// parent, took 8 us each in FP64 and 2 us in FP32, most of the evaluation of a small
+// problem: M2M 169 -> 25 us at N = 1000 FP64, 241 -> 39 us at 10,000, 48 -> 23 us mixed;
+// 178 -> 129 us mixed at 1M, beside P2P).  A cluster and not
+// one block, for its FP64 pipes.  With chain levels l0 .. l1 > 0 it does those first.  At
+// the end, if a level of this or an earlier launch stored a moment that is not finite, it
+// zeroes all such moments (they spread upward before that) and clears the mark.
+constexpr int UP_BLOCKS = 8, UP_THREADS = 256;
+constexpr int UP_NODES = UP_BLOCKS * UP_THREADS / 4;  // a level done in one pass
+constexpr int UP_MAX_LEVELS = 60;
+struct UpLevels {
+    int n;
+    int32_t start[UP_MAX_LEVELS + 1];  // level k: nodes start[k] .. start[k + 1]
+};
+template <int P, class T, bool ADJ>
+__global__ void __launch_bounds__(UP_THREADS) k_up_small(UpLevels lv, int64_t nl, int l0, int l1,
+                                                         const int4 *__restrict__ child,
+                                                         const double *__restrict__ comx,
+                                                         const double *__restrict__ comy, T *M, int64_t n_rows,
+                                                         unsigned *bad) {
+    constexpr int NS = row_stride<T>(nc2(P));
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const int tid = cl.block_rank() * UP_THREADS + threadIdx.x;
+    constexpr int stride = UP_BLOCKS * UP_THREADS;
+    bool b = false;
+    if (l0 > 0) {
+        const int64_t n = nl * (l1 - l0 + 1);
+        for (int64_t t = tid; t < n; t += stride) b |= chain_node<P, T, ADJ>(t % nl, t % nl + (l0 + t / nl) * nl, comx, comy, M);
+        cl.sync();
+    }
+    for (int k = 0; k < lv.n; k++) {
+        const int64_t e = lv.start[k + 1];
+        for (int64_t s = lv.start[k]; s < e; s += UP_NODES) {
+            const int64_t node = s + (tid >> 2);
+            b |= up_node<P, T, ADJ>(node < e ? node : -1, child, comx, comy, M);
+        }
+        cl.sync();
+    }
+    if (!bad) return;
+    if (b) atomicOr(bad, 1u);
+    cl.sync();
+    const bool any = *reinterpret_cast<volatile unsigned *>(bad) != 0;
+    if (any)
+        for (int64_t i = tid; i < n_rows * NS; i += stride)
+            if (!isfinite(M[i])) M[i] = T(0);
+    cl.sync();
+    if (any && tid == 0) *bad = 0;
+}
+
+// The whole upward pass over the rows of the leaves: the chain levels l0 .. l1 (0: none)
+// straight from the leaves, the levels above them one by one down to UP_NODES nodes, the
+// rest in k_up_small.  bad: the mark of moments to be zeroed (null: none are).
+template <int P, class T, bool ADJ>
+int run_up(gx_ctx *ctx, int l0, int l1, T *M, unsigned *bad) {
+    const int64_t nl = ctx->n_leaves;
+    const double *comx = dptr<double>(ctx->comx), *comy = dptr<double>(ctx->comy);
+    const int4 *child = dptr<int4>(ctx->child);
+    cudaStream_t st = ctx->stream;
+    if (ctx->n_levels <= 1) return GX_OK;
+    const int64_t chains = l0 > 0 ? nl * (l1 - l0 + 1) : 0;
+    int lv = l1 + 1;
+    auto size = [&](int l) { return ctx->level_start[l + 1] - ctx->level_start[l]; };
+    // the chain levels in a launch of their own where they are many, or a large level follows
+    const bool apart = chains > 2 * UP_BLOCKS * UP_THREADS || (chains > 0 && lv < ctx->n_levels && size(lv) > UP_NODES);
+    if (apart) {
+        k_up_chain<P, T, ADJ><<<gx_blocks(chains, 128), 128, 0, st>>>(nl, l0, l1, comx, comy, M, bad);
+        ctx->launches++;
+    }
+    for (; lv < ctx->n_levels && size(lv) > UP_NODES; lv++) {
+        k_up_level<P, T, ADJ><<<gx_blocks(size(lv) * 4, 128), 128, 0, st>>>(
+            ctx->level_start[lv], ctx->level_start[lv + 1], child, comx, comy, M, bad);
+        ctx->launches++;
+    }
+    bool chain_here = chains > 0 && !apart;
+    do {  // once, or more often for a tree of very many levels
+        UpLevels L;
+        L.n = 0;
+        for (; lv < ctx->n_levels && L.n < UP_MAX_LEVELS; lv++) {
+            L.start[L.n++] = (int32_t)ctx->level_start[lv];
+            L.start[L.n] = (int32_t)ctx->level_start[lv + 1];
+        }
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(UP_BLOCKS);
+        cfg.blockDim = dim3(UP_THREADS);
+        cfg.stream = st;
+        cudaLaunchAttribute at = {};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = UP_BLOCKS;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        GX_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_up_small<P, T, ADJ>, L, nl, chain_here ? l0 : 0, chain_here ? l1 : 0,
+                                        child, comx, comy, M, ctx->n_nodes, lv < ctx->n_levels ? nullptr : bad));
+        ctx->launches++;
+        chain_here = false;
+    } while (lv < ctx->n_levels);
+    return GX_OK;
 }
 
 // ---------------------------------------------------------------- M2L
@@ -2373,7 +2510,6 @@ int run_forces(gx_ctx *ctx, bool timed) {
     const double *X = dptr<double>(ctx->x), *Y = dptr<double>(ctx->y), *Mb = dptr<double>(ctx->m);
     const double *comx = dptr<double>(ctx->comx), *comy = dptr<double>(ctx->comy);
     const int32_t *bs = dptr<int32_t>(ctx->bs), *be = dptr<int32_t>(ctx->be), *parent = dptr<int32_t>(ctx->parent);
-    const int4 *child = dptr<int4>(ctx->child);
     const unsigned gw = (unsigned)((nl * 32 + 127) / 128);  // warp per leaf
     const double eps2 = ctx->eps * ctx->eps;
     const gx_ctx::Items &I = mode == GX_MODE_ACCURATE ? ctx->items_acc : ctx->items_ref;
@@ -2481,24 +2617,10 @@ int run_forces(gx_ctx *ctx, bool timed) {
         // the near field starts beside the far-field chain; for a measurement of the
         // near field alone (gx_bench_forces) it starts after the chain
         if (!ctx->near_after_far) GX_TRY(near_field());
-        // M2M, bottom-up by level; in ACCURATE mode the single-child chain levels over the
-        // leaves are one direct shift (their nodes have no far lists)
-        int lv_m2m = 1;
-        if (mode == GX_MODE_ACCURATE && ctx->chain_levels >= 2) {
-            const int64_t up = ctx->level_start[ctx->chain_levels];
-            k_m2m_chain<P, T><<<gx_blocks(nl, 128), 128, 0, st>>>(nl, up, comx, comy, M);
-            ctx->launches++;
-            lv_m2m = ctx->chain_levels + 1;
-        }
-        for (int lv = lv_m2m; lv < ctx->n_levels; lv++) {
-            int64_t s = ctx->level_start[lv], e = ctx->level_start[lv + 1];
-            k_m2m<P, T><<<gx_blocks(e - s, 128), 128, 0, st>>>(s, e, child, comx, comy, M);
-            ctx->launches++;
-        }
-        if (ctx->n_levels > 1) {
-            k_scrub<T><<<gx_blocks(NS * nn, 256), 256, 0, st>>>(NS * nn, M);
-            ctx->launches++;
-        }
+        // M2M: in ACCURATE mode the chain levels are one direct shift to the top one
+        const int lc = mode == GX_MODE_ACCURATE ? (ctx->chain_levels >= 2 ? ctx->chain_levels : 0) : ctx->unary_levels;
+        GX_TRY((run_up<P, T, false>(ctx, mode == GX_MODE_ACCURATE ? lc : (lc > 0 ? 1 : 0), lc, M,
+                                    dptr<unsigned>(ctx->status) + 1)));
         tm.mark();  // 3
         // M2L
         const unsigned gn = (unsigned)((nn * 32 + 127) / 128);

@@ -34,7 +34,7 @@ struct gx_tree_plan {
     int64_t n_nodes = 0, n_leaves = 0, max_leaf = 0, n_far_pairs = 0, n_near_pairs = 0, n_p2p_inter = 0;
     int64_t items_n = 0, units_n = 0;
     int32_t n_levels = 0;
-    int chain_levels = 0;
+    int chain_levels = 0, unary_levels = 0;
     bool have_tree = false, aux_valid = false, plan_acc_valid = false, plan_ref_valid = false,
          ref_lists_valid = false, items_valid = false;
     int plan_p = -1;
@@ -183,6 +183,9 @@ struct gx_ctx {
     // (level l holds node x + l nl above leaf x); with chain_levels >= 2 the plan and M2M
     // skip levels 1 .. chain_levels - 1 (no far lists there), else 0
     int chain_levels = 0;
+    // levels 1 .. unary_levels are single-child chains over the leaves, node x + l nl above
+    // leaf x in level l (by the level sizes of a device build; checked for an uploaded tree)
+    int unary_levels = 0;
     bool near_after_far = false;  // measurement only: the near field after the far-field chain
     // gx_compute_forces into page-locked host arrays: their device addresses, written by
     // the final sum of the evaluation being enqueued (null otherwise)
