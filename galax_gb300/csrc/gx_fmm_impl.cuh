@@ -630,7 +630,69 @@ __device__ __forceinline__ void m2l_fused(T dx, T dy, T eps2, const T *in, T *ou
     }
 }
 
-// REF mode: derivative sets from the first-inserter table (FP64).
+// v != 0 on the integer pipe: a comparison of FP64 values holds the FP64 pipe as long as the
+// multiply-add behind it (2.0 against 1.1 ms for the kernel below at N = 200k), and nvcc
+// turns the plain integer test of the bits back into one.
+__device__ __forceinline__ bool nonzero_bits(double v) {
+    uint32_t nz;
+    asm("{\n.reg .b32 l, h;\nmov.b64 {l, h}, %1;\nshl.b32 h, h, 1;\nor.b32 %0, l, h;\n}" : "=r"(nz) : "d"(v));
+    return nz != 0;
+}
+
+// REF mode: derivative sets from the first-inserter table (FP64).  A warp per node, a lane
+// per output coefficient, as many sources side by side as fit (two at p = 4): a list of 23
+// sources, the mean at N = 200k, takes 12 x 15 multiply-adds a lane instead of a round of
+// 225 with a quarter of the lanes idle and a warp sum of each of the 15 coefficients, and a
+// derivative set is read as 15 neighbouring values instead of 32 sets at once.
+template <int P>
+__global__ void __launch_bounds__(128) k_m2l_ref_rows(int64_t nn, const uint32_t *__restrict__ vdata,
+                                                      const uint8_t *__restrict__ vlen,
+                                                      const int64_t *__restrict__ voff,
+                                                      const int32_t *__restrict__ did, const double *__restrict__ G,
+                                                      const double *__restrict__ M, double *__restrict__ L) {
+    constexpr int NC = nc2(P);
+    constexpr int NS = row_stride<double>(NC);
+    constexpr int S = 2 * P + 1;
+    constexpr int SIDE = 32 / NC;
+    static_assert(SIDE >= 1 && GX_LIST_CAP <= 64, "a lane per coefficient, two list entries per lane");
+    const unsigned full = 0xffffffffu;
+    const int64_t node = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (node >= nn) return;
+    const int len = vlen[node];
+    const int64_t v0 = node * GX_LIST_CAP, d0 = voff[node];
+    const int srcA = lane < len ? (int)vdata[v0 + lane] : 0, srcB = lane + 32 < len ? (int)vdata[v0 + 32 + lane] : 0;
+    const int didA = lane < len ? did[d0 + lane] : 0, didB = lane + 32 < len ? did[d0 + 32 + lane] : 0;
+    const int slot = lane / NC, k = lane - slot * NC;
+    int n = 0;  // coefficient k = gx_mi(oi, oj) with oi + oj = n
+    while ((n + 1) * (n + 2) / 2 <= k) n++;
+    const int oj = k - n * (n + 1) / 2, oi = n - oj;
+    const double *g0 = G + gx_kdi(oi, oj, P);
+    double acc = 0.0;
+    for (int s0 = 0; s0 < len; s0 += SIDE) {
+        const int s = s0 + slot;
+        const int sa = __shfl_sync(full, srcA, s & 31), sb = __shfl_sync(full, srcB, s & 31);
+        const int da = __shfl_sync(full, didA, s & 31), db = __shfl_sync(full, didB, s & 31);
+        if (slot >= SIDE || s >= len) continue;
+        const double *g = g0 + (int64_t)(s < 32 ? da : db) * (S * S);
+        double ms[NC];
+        load_row<NC>(M + (int64_t)(s < 32 ? sa : sb) * NS, ms);
+#pragma unroll
+        for (int i = 0; i <= P; i++)
+#pragma unroll
+            for (int j = 0; j <= P - i; j++) {
+                const double mv = ms[gx_mi(i, j)];
+                if (nonzero_bits(mv))  // lib.rs:1252: zero source terms are skipped
+                    acc = fma(((i + j) & 1) ? -mv : mv, __ldg(g + gx_kdi(i, j, P)), acc);
+            }
+    }
+    double v = acc;
+#pragma unroll
+    for (int q = 1; q < SIDE; q++) v += __shfl_sync(full, acc, (lane + q * NC) & 31);
+    if (lane < NC) L[node * NS + lane] = v * tab_ifp<double>(oi, oj);
+}
+
+// The same with a lane per source, for the orders whose coefficients do not fit a warp.
 template <int P>
 __global__ void __launch_bounds__(128) k_m2l_ref(int64_t nn, const uint32_t *__restrict__ vdata,
                                                  const uint8_t *__restrict__ vlen, const int64_t *__restrict__ voff,
@@ -2625,10 +2687,14 @@ int run_forces(gx_ctx *ctx, bool timed) {
         // M2L
         const unsigned gn = (unsigned)((nn * 32 + 127) / 128);
         if (mode == GX_MODE_REF && !mixed) {
-            k_m2l_ref<P><<<gn, 128, 0, st>>>(nn, dptr<uint32_t>(ctx->vdata), dptr<uint8_t>(ctx->vlen),
-                                             dptr<int64_t>(ctx->ref_voff), dptr<int32_t>(ctx->ref_did),
-                                             dptr<double>(ctx->ref_G), reinterpret_cast<const double *>(M),
-                                             reinterpret_cast<double *>(L));
+            const auto launch = [&](auto kernel) {
+                kernel<<<gn, 128, 0, st>>>(nn, dptr<uint32_t>(ctx->vdata), dptr<uint8_t>(ctx->vlen),
+                                           dptr<int64_t>(ctx->ref_voff), dptr<int32_t>(ctx->ref_did),
+                                           dptr<double>(ctx->ref_G), reinterpret_cast<const double *>(M),
+                                           reinterpret_cast<double *>(L));
+            };
+            if constexpr (NC <= 32) launch(k_m2l_ref_rows<P>);
+            else launch(k_m2l_ref<P>);
         } else if (mode == GX_MODE_ACCURATE) {
             // nodes without far sources keep whatever L holds: has_far = 0 keeps L2L from reading it
             const gx_ctx::M2LUnits &U = ctx->m2l_units;
