@@ -190,33 +190,45 @@ constexpr int RS_WARP_ITEMS = 32 * RS_ROUNDS;          // 256
 constexpr int RS_TILE = RS_WARPS * RS_WARP_ITEMS;      // 2048
 constexpr int RS_BINS = 256;
 
-__global__ void k_rs_hist(const uint64_t *keys, int64_t n, int shift, unsigned mask, unsigned *hist, int64_t nb) {
+// digit counts of a tile, digit-major: hist[d * nb + tile]
+__global__ void k_rs_hist(const uint64_t *__restrict__ keys, int64_t n, int shift, int bins, unsigned *hist,
+                          int64_t nb) {
     __shared__ unsigned h[RS_BINS];
-    for (int i = threadIdx.x; i < RS_BINS; i += blockDim.x) h[i] = 0;
+    for (int i = threadIdx.x; i < bins; i += blockDim.x) h[i] = 0;
     __syncthreads();
-    int64_t base = (int64_t)blockIdx.x * RS_TILE;
-    for (int k = threadIdx.x; k < RS_TILE; k += blockDim.x) {
-        int64_t i = base + k;
-        if (i < n) atomicAdd(&h[(unsigned)(keys[i] >> shift) & mask], 1u);
+    const int64_t base = (int64_t)blockIdx.x * RS_TILE;
+    uint64_t k[RS_TILE / 256];
+#pragma unroll
+    for (int r = 0; r < RS_TILE / 256; r++) {
+        const int64_t i = base + r * 256 + threadIdx.x;
+        k[r] = i < n ? keys[i] : 0;
     }
+#pragma unroll
+    for (int r = 0; r < RS_TILE / 256; r++)
+        if (base + r * 256 + threadIdx.x < n) atomicAdd(&h[(unsigned)(k[r] >> shift) & (unsigned)(bins - 1)], 1u);
     __syncthreads();
-    for (int d = threadIdx.x; d < RS_BINS; d += blockDim.x) hist[(int64_t)d * nb + blockIdx.x] = h[d];
+    for (int d = threadIdx.x; d < bins; d += blockDim.x) hist[(int64_t)d * nb + blockIdx.x] = h[d];
 }
 
-// flag = 1 if every key has the same digit (the pass copies instead of scattering)
-__global__ void k_rs_uniform(const unsigned *offs, int64_t nb, int64_t n, unsigned *flag) {
-    int d = threadIdx.x;
-    if (d >= RS_BINS) return;
-    int64_t lo = offs[(int64_t)d * nb];
-    int64_t hi = (d + 1 < RS_BINS) ? (int64_t)offs[(int64_t)(d + 1) * nb] : n;
-    if (hi - lo == n) *flag = 1u;
+// One block per digit: its tiles' counts become their exclusive scan, tot[d] the digit's
+// count.  The scan over the digits themselves (256 values) is left to the scatter's blocks,
+// so a pass is three launches and no scan of the whole count matrix.
+__global__ void __launch_bounds__(SCAN_THREADS) k_rs_rows(unsigned *hist, int64_t nb, unsigned *tot) {
+    scan_single_block<unsigned>(hist + blockIdx.x * nb, nb, tot + blockIdx.x);
 }
 
-__global__ void __launch_bounds__(RS_WARPS * 32) k_rs_scatter(const uint64_t *kin, const uint32_t *vin,
-                                                             uint64_t *kout, uint32_t *vout, int64_t n,
-                                                             int shift, unsigned mask, const unsigned *offs,
-                                                             int64_t nb, const unsigned *uniform) {
-    if (*uniform) {  // every key has the same digit: the stable order is the present one
+__global__ void __launch_bounds__(RS_WARPS * 32) k_rs_scatter(const uint64_t *__restrict__ kin,
+                                                             const uint32_t *__restrict__ vin, uint64_t *kout,
+                                                             uint32_t *vout, int64_t n, int shift, int bins,
+                                                             const unsigned *__restrict__ offs, int64_t nb,
+                                                             const unsigned *__restrict__ tot) {
+    static_assert(RS_WARPS * 32 == RS_BINS && RS_BINS == SCAN_THREADS, "a thread per digit");
+    const unsigned mask = (unsigned)(bins - 1);
+    __shared__ unsigned first[RS_BINS], sum;  // where this tile's items of a digit begin
+    const unsigned mine = (int)threadIdx.x < bins ? tot[threadIdx.x] : 0u;
+    const unsigned before = block_exclusive_scan<unsigned>(mine, &sum);
+    if ((int)threadIdx.x < bins) first[threadIdx.x] = before + offs[(int64_t)threadIdx.x * nb + blockIdx.x];
+    if (__syncthreads_or(mine == (unsigned)n)) {  // every key has the same digit: the stable order is the present one
         for (int64_t i = (int64_t)blockIdx.x * RS_TILE + threadIdx.x; i < n && i < (int64_t)(blockIdx.x + 1) * RS_TILE;
              i += blockDim.x) {
             kout[i] = kin[i];
@@ -225,7 +237,7 @@ __global__ void __launch_bounds__(RS_WARPS * 32) k_rs_scatter(const uint64_t *ki
         return;
     }
     __shared__ unsigned cnt[RS_WARPS][RS_BINS];
-    for (int i = threadIdx.x; i < RS_WARPS * RS_BINS; i += blockDim.x) (&cnt[0][0])[i] = 0;
+    for (int i = threadIdx.x; i < RS_WARPS * RS_BINS; i += blockDim.x) (&cnt[0][0])[i] = 0u;
     __syncthreads();
     int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     unsigned lt = (1u << lane) - 1u;
@@ -249,8 +261,8 @@ __global__ void __launch_bounds__(RS_WARPS * 32) k_rs_scatter(const uint64_t *ki
         rk[r] = c + __popc(peers & lt);
     }
     __syncthreads();
-    for (int dd = threadIdx.x; dd < RS_BINS; dd += blockDim.x) {
-        unsigned run = 0;
+    for (int dd = threadIdx.x; dd < bins; dd += blockDim.x) {
+        unsigned run = first[dd];
         for (int ww = 0; ww < RS_WARPS; ww++) {
             unsigned t = cnt[ww][dd];
             cnt[ww][dd] = run;
@@ -261,7 +273,7 @@ __global__ void __launch_bounds__(RS_WARPS * 32) k_rs_scatter(const uint64_t *ki
 #pragma unroll
     for (int r = 0; r < RS_ROUNDS; r++) {
         if (d[r] == 0xFFFFFFFFu) continue;
-        int64_t pos = (int64_t)offs[(int64_t)d[r] * nb + blockIdx.x] + cnt[w][d[r]] + rk[r];
+        const unsigned pos = cnt[w][d[r]] + rk[r];
         kout[pos] = k[r];
         vout[pos] = v[r];
     }
@@ -306,28 +318,22 @@ int gx_radix_sort_u64(gx_ctx *ctx, uint64_t *keys, uint32_t *vals, int64_t n, in
     int64_t nb = (n + RS_TILE - 1) / RS_TILE;
     if (nb * RS_BINS > 0x7fffffffLL) return gx_fail(ctx, GX_ERR_CAP_EXCEEDED, "radix sort: too many items");
     GX_TRY(gx_ensure(ctx, ctx->scratch_e, sizeof(unsigned) * (size_t)(nb * RS_BINS + 1)));
-    GX_TRY(gx_ensure(ctx, ctx->scratch_f, sizeof(unsigned) * 4));
+    GX_TRY(gx_ensure(ctx, ctx->scratch_f, sizeof(unsigned) * RS_BINS));
     unsigned *hist = dptr<unsigned>(ctx->scratch_e);
-    unsigned *flag = dptr<unsigned>(ctx->scratch_f);
+    unsigned *tot = dptr<unsigned>(ctx->scratch_f);
     uint64_t *ki = keys, *ko = keys_alt;
     uint32_t *vi = vals, *vo = vals_alt;
-    for (int shift = begin_bit; shift < end_bit; shift += 8) {
-        int bits = end_bit - shift < 8 ? end_bit - shift : 8;
-        unsigned mask = (1u << bits) - 1u;
-        k_rs_hist<<<(unsigned)nb, 256, 0, ctx->stream>>>(ki, n, shift, mask, hist, nb);
-        ctx->launches++;
-        int32_t total = 0;
-        GX_TRY(scan_impl<int32_t>(ctx, reinterpret_cast<int32_t *>(hist), reinterpret_cast<int32_t *>(hist),
-                                  nb * RS_BINS, nullptr));
-        GX_CUDA(ctx, cudaMemsetAsync(flag, 0, sizeof(unsigned), ctx->stream));
-        k_rs_uniform<<<1, RS_BINS, 0, ctx->stream>>>(hist, nb, n, flag);
-        ctx->launches++;
-        (void)total;
-        // the uniform-digit case is decided on the device (a copy instead of the scatter),
-        // so the passes run without a host round trip
-        k_rs_scatter<<<(unsigned)nb, RS_WARPS * 32, 0, ctx->stream>>>(ki, vi, ko, vo, n, shift, mask, hist, nb, flag);
-        ctx->launches++;
+    // passes of at most 8 bits, as even as the key allows (42 bits: six of 7, whose runs in
+    // the scatter are twice as long as those of 8)
+    const int passes = (end_bit - begin_bit + 7) / 8;
+    for (int q = 0, shift = begin_bit; q < passes; q++) {
+        const int bits = (end_bit - shift + passes - q - 1) / (passes - q), bins = 1 << bits;
+        k_rs_hist<<<(unsigned)nb, 256, 0, ctx->stream>>>(ki, n, shift, bins, hist, nb);
+        k_rs_rows<<<(unsigned)bins, SCAN_THREADS, 0, ctx->stream>>>(hist, nb, tot);
+        k_rs_scatter<<<(unsigned)nb, RS_WARPS * 32, 0, ctx->stream>>>(ki, vi, ko, vo, n, shift, bins, hist, nb, tot);
+        ctx->launches += 3;
         GX_CUDA(ctx, cudaGetLastError());
+        shift += bits;
         uint64_t *tk = ki; ki = ko; ko = tk;
         uint32_t *tv = vi; vi = vo; vo = tv;
     }

@@ -6,6 +6,8 @@
 // __dsub_rn, which the compiler never contracts into FMA), in the reference's
 // order: Morton normalisation, leaf mass and COM sums (body order), parent sums
 // (child slot order), box centres and half-widths.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "gx_internal.cuh"
@@ -181,9 +183,10 @@ enum {
 enum { TS_DONE = 1, TS_OVERFLOW = 2, TS_STUCK = 4 };
 constexpr int TS_MAX_ROUNDS = 400;  // level starts kept: TS_MAX_ROUNDS + 2
 
-constexpr int TS_SMALL = 2048;  // levels of at most this many nodes: k_rounds_small
+constexpr int TS_SMALL = 512;     // levels of at most this many nodes: k_rounds_small
+constexpr int TS_CLUSTER = 65536;  // larger ones, up to this many nodes: k_rounds_cluster
 // the multi-block round kernels do nothing once the build is over or the level is small
-__device__ __forceinline__ bool round_off(const int64_t *st) { return st[TS_FLAGS] != 0 || st[TS_C] <= TS_SMALL; }
+__device__ __forceinline__ bool round_off(const int64_t *st) { return st[TS_FLAGS] != 0 || st[TS_C] <= TS_CLUSTER; }
 
 __global__ void k_round_heads(const int64_t *st, const uint64_t *__restrict__ keys, const int32_t *__restrict__ bs,
                               int64_t *head) {
@@ -335,7 +338,7 @@ __global__ void k_chain_depth(int64_t nl, const uint64_t *__restrict__ keys, con
 __global__ void k_chain_rounds(int64_t *st, int64_t *level_start, int64_t nl, int64_t cap_nodes, double *cx,
                                double *cy, double *hw, double *mass, double *comx, double *comy, int32_t *bs,
                                int32_t *be, int4 *child, int32_t *parent, uint8_t *is_leaf) {
-    if (st[TS_FLAGS] != 0 || nl <= TS_SMALL) return;
+    if (st[TS_FLAGS] != 0) return;
     int64_t L = st[TS_CHAIN_M] >= 2 ? st[TS_CHAIN_M] / 2 : 0;
     L = min(L, cap_nodes / nl - 1);
     L = min(L, (int64_t)TS_MAX_ROUNDS - 2);
@@ -396,7 +399,7 @@ __global__ void __launch_bounds__(RS_SMALL_THREADS) k_rounds_small(int64_t *st, 
                                                                   double *cy, double *hw, double *mass, double *comx,
                                                                   double *comy, int32_t *bs, int32_t *be, int32_t *child,
                                                                   int32_t *parent, uint8_t *is_leaf) {
-    constexpr int PER = TS_SMALL / RS_SMALL_THREADS;  // items per thread
+    constexpr int PER = (TS_SMALL + RS_SMALL_THREADS - 1) / RS_SMALL_THREADS;  // items per thread
     __shared__ int head[TS_SMALL], segex[TS_SMALL], segstart[TS_SMALL], goff[TS_SMALL];
     __shared__ int warp_tot[32], tot;
     __shared__ int64_t sh_s, sh_e, sh_c, sh_flags, sh_rounds;
@@ -490,6 +493,167 @@ __global__ void __launch_bounds__(RS_SMALL_THREADS) k_rounds_small(int64_t *st, 
     }
 }
 
+// The rounds of levels of more than TS_SMALL and at most TS_CLUSTER nodes, all in one
+// cluster of blocks that meets at cluster barriers: a round was 13 launches of 4 us each
+// (with the sort's passes of three launches instead of seven, upload, build and read-back at
+// N = 200k, n_max = 16 take 0.80 ms, 1.13 before).
+// Every thread owns a run of consecutive nodes of the level; two scans over the cluster
+// (block scans, the blocks' results exchanged through distributed shared memory) give each
+// node the head of its segment and its group, the same groups in the same order as the
+// multi-block rounds: a segment's nodes by fours.  One cluster has the FP64 pipes of as many
+// SMs as it has blocks, and parent_fields_one is FP64: above TS_CLUSTER nodes a round over
+// the whole GPU is as fast.
+constexpr int RC_THREADS = 1024;
+constexpr int RC_MAX_BLOCKS = 16;
+
+__device__ __forceinline__ int warp_max_scan(int v) {
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, v, o);
+        if ((int)(threadIdx.x & 31) >= o) v = max(v, t);
+    }
+    return v;
+}
+
+__global__ void __launch_bounds__(RC_THREADS) k_rounds_cluster(int64_t *st, int64_t *level_start, int64_t cap_nodes,
+                                                               const uint64_t *__restrict__ keys, double *cx,
+                                                               double *cy, double *hw, double *mass, double *comx,
+                                                               double *comy, int32_t *bs, int32_t *be, int32_t *child,
+                                                               int32_t *parent, uint8_t *is_leaf) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const int nb = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int gt = rank * RC_THREADS + t, stride = nb * RC_THREADS;
+    __shared__ int wt[32], blast, bcnt, prev_last, prev_cnt, all_cnt;
+    // the round state, kept by every thread alike and written back at the end
+    int64_t s = st[TS_S], e = st[TS_E], flags = st[TS_FLAGS], rounds = st[TS_ROUNDS], shift = st[TS_SHIFT];
+    int c = (int)st[TS_C];
+    cl.sync();  // all blocks have read the state before one writes it
+    if (flags != 0 || c > TS_CLUSTER || c <= TS_SMALL) return;
+    while (flags == 0 && c > TS_SMALL) {
+        const unsigned sh = (unsigned)shift & 63u;
+        const int per = (c + stride - 1) / stride;  // at most 8 (TS_CLUSTER nodes on 8 blocks)
+        const int i0 = min(c, gt * per), i1 = min(c, i0 + per);
+        // heads of segments (nodes whose key prefix differs from the one before)
+        unsigned heads = 0;
+        int last = -1;
+        bool next_head = true;  // the node after this run begins a segment (or there is none)
+        if (i0 < i1) {
+            uint64_t p = i0 > 0 ? keys[bs[s + i0 - 1]] >> sh : 0;
+            for (int i = i0; i < i1; i++) {
+                const uint64_t g = keys[bs[s + i]] >> sh;
+                if (i == 0 || g != p) {
+                    heads |= 1u << (i - i0);
+                    last = i;
+                }
+                p = g;
+            }
+            next_head = i1 >= c || (keys[bs[s + i1]] >> sh) != p;
+        }
+        // the last head before this run: max scan over the cluster
+        int m = warp_max_scan(last);
+        if (lane == 31) wt[w] = m;
+        __syncthreads();
+        if (w == 0) {
+            const int v = warp_max_scan(wt[lane]);
+            wt[lane] = v;
+            if (lane == 31) blast = v;
+        }
+        __syncthreads();
+        int head = __shfl_up_sync(0xffffffffu, m, 1);
+        if (lane == 0) head = -1;
+        if (w > 0) head = max(head, wt[w - 1]);
+        cl.sync();
+        if (t == 0) {
+            int v = -1;
+            for (int r = 0; r < rank; r++) v = max(v, *cl.map_shared_rank(&blast, r));
+            prev_last = v;
+        }
+        __syncthreads();
+        head = max(head, prev_last);
+        // groups of four within each segment: count those that begin in this run
+        int h = head, cnt = 0;
+        for (int i = i0; i < i1; i++) {
+            if ((heads >> (i - i0)) & 1u) h = i;
+            cnt += ((i - h) & 3) == 0;
+        }
+        int inc = cnt;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += v;
+        }
+        __syncthreads();  // wt has been read
+        if (lane == 31) wt[w] = inc;
+        __syncthreads();
+        if (w == 0) {
+            int v = wt[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane >= o) v += u;
+            }
+            if (lane == 31) bcnt = v;
+            wt[lane] = v;
+        }
+        __syncthreads();
+        int g = inc - cnt + (w > 0 ? wt[w - 1] : 0);
+        cl.sync();
+        if (t == 0) {
+            int before = 0, total = 0;
+            for (int r = 0; r < nb; r++) {
+                const int v = *cl.map_shared_rank(&bcnt, r);
+                if (r < rank) before += v;
+                total += v;
+            }
+            prev_cnt = before;
+            all_cnt = total;
+        }
+        __syncthreads();
+        g += prev_cnt - 1;
+        const int ng = all_cnt;
+        if (e + ng > cap_nodes) {
+            flags |= TS_OVERFLOW;
+            break;
+        }
+        if (rounds >= TS_MAX_ROUNDS) {
+            flags |= TS_STUCK;
+            break;
+        }
+        h = head;
+        for (int i = i0; i < i1; i++) {
+            if ((heads >> (i - i0)) & 1u) h = i;
+            const int pos = (i - h) & 3;
+            g += pos == 0;
+            const int64_t q = e + g;
+            parent[s + i] = (int32_t)q;
+            child[q * 4 + pos] = (int32_t)(s + i);
+            const bool end = i + 1 < i1 ? (heads >> (i + 1 - i0)) & 1u : next_head;
+            if (end)
+                for (int k = pos + 1; k < 4; k++) child[q * 4 + k] = -1;
+        }
+        cl.sync();
+        for (int k = gt; k < ng; k += stride)
+            parent_fields_one(e + k, cx, cy, hw, mass, comx, comy, bs, be, reinterpret_cast<const int4 *>(child),
+                              parent, is_leaf);
+        s = e;
+        e += ng;
+        c = ng;
+        shift += 2;
+        rounds++;
+        if (gt == 0) level_start[rounds + 1] = e;
+        if (ng <= 1) flags |= TS_DONE;
+        cl.sync();
+    }
+    cl.sync();  // no block leaves while another may read its shared memory
+    if (gt == 0) {
+        st[TS_S] = s;
+        st[TS_E] = e;
+        st[TS_C] = c;
+        st[TS_SHIFT] = shift;
+        st[TS_FLAGS] = flags;
+        st[TS_ROUNDS] = rounds;
+    }
+}
+
 // ---- build_constrained helpers (lib.rs:541-694) ----
 // leaf ranges bounded by n_max and by the sorted split points (lib.rs:603-613):
 // computed on the host from the split list, which is small.
@@ -518,13 +682,45 @@ static int ensure_nodes(gx_ctx *ctx, int64_t need) {
     return GX_OK;
 }
 
+// The cluster of k_rounds_cluster: 16 blocks where the device takes them, else the portable 8.
+static int launch_rounds_cluster(gx_ctx *ctx, int64_t *st, int64_t *lstart, int64_t cap) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.blockDim = dim3(RC_THREADS);
+    cfg.stream = ctx->stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (ctx->rounds_blocks == 0) {
+        ctx->rounds_blocks = 8;
+        at.val.clusterDim.x = RC_MAX_BLOCKS;
+        cfg.gridDim = dim3(RC_MAX_BLOCKS);
+        int fit = 0;
+        if (cudaFuncSetAttribute(k_rounds_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&fit, k_rounds_cluster, &cfg) == cudaSuccess && fit > 0)
+            ctx->rounds_blocks = RC_MAX_BLOCKS;
+        cudaGetLastError();  // a device without the larger cluster is no error
+    }
+    at.val.clusterDim.x = (unsigned)ctx->rounds_blocks;
+    cfg.gridDim = dim3((unsigned)ctx->rounds_blocks);
+    GX_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_rounds_cluster, st, lstart, cap, (const uint64_t *)dptr<uint64_t>(ctx->keys),
+                                    dptr<double>(ctx->cx), dptr<double>(ctx->cy), dptr<double>(ctx->hw),
+                                    dptr<double>(ctx->mass), dptr<double>(ctx->comx), dptr<double>(ctx->comy),
+                                    dptr<int32_t>(ctx->bs), dptr<int32_t>(ctx->be), dptr<int32_t>(ctx->child),
+                                    dptr<int32_t>(ctx->parent), dptr<uint8_t>(ctx->is_leaf)));
+    ctx->launches++;
+    return GX_OK;
+}
+
 // Builds nodes from leaf ranges already in scratch (rs, re as int32), using ctx->keys
 // (Morton keys of the tree-ordered bodies).
 static int build_from_ranges(gx_ctx *ctx, const int32_t *rs, const int32_t *re, int64_t nl) {
     if (nl <= 0) return gx_fail(ctx, GX_ERR_STATE, "tree build: no leaves");
     // node storage: the last build's node count (a rebuild every step keeps it), else a
-    // guess; a round that overflows it makes the build start again with more
-    int64_t cap = std::max<int64_t>(nl * 4 + 64, ctx->hint_nodes + ctx->hint_nodes / 8 + 64);
+    // guess (10 to 20 nodes a leaf: the single-child levels); a round that overflows it makes
+    // the build start again with more
+    int64_t cap = std::max<int64_t>(nl * 12 + 512, ctx->hint_nodes + ctx->hint_nodes / 8 + 64);
     // per-round scratch: head, segex, segstart, gcnt, goff (int64, <= nl each)
     GX_TRY(gx_ensure(ctx, ctx->scratch_a, sizeof(int64_t) * (size_t)(nl + 1) * 5));
     GX_TRY(gx_ensure(ctx, ctx->tree_state, sizeof(int64_t) * (TS_N + TS_MAX_ROUNDS + 2)));
@@ -534,7 +730,7 @@ static int build_from_ranges(gx_ctx *ctx, const int32_t *rs, const int32_t *re, 
     int64_t *segex = head + (nl + 1), *segstart = segex + (nl + 1), *gcnt = segstart + (nl + 1),
             *goff = gcnt + (nl + 1);
     const unsigned gb = gx_blocks(nl, 256);
-    int64_t hs[TS_N];
+    int64_t hs[TS_N + TS_MAX_ROUNDS + 2];  // the state and, behind it, the level starts
     for (int attempt = 0;; attempt++) {
         if (attempt == 8) return gx_fail(ctx, GX_ERR_ALLOC, "tree build: node storage keeps overflowing");
         GX_TRY(ensure_nodes(ctx, cap));
@@ -548,7 +744,7 @@ static int build_from_ranges(gx_ctx *ctx, const int32_t *rs, const int32_t *re, 
         const int64_t ls01[2] = {0, nl};
         GX_CUDA(ctx, cudaMemcpyAsync(st, init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream));
         GX_CUDA(ctx, cudaMemcpyAsync(lstart, ls01, sizeof(ls01), cudaMemcpyHostToDevice, ctx->stream));
-        if (nl > TS_SMALL) {
+        if (nl > 1) {
             k_chain_depth<<<gx_blocks(nl, 256), 256, 0, ctx->stream>>>(nl, dptr<uint64_t>(ctx->keys),
                                                                       dptr<int32_t>(ctx->bs), st);
             k_chain_rounds<<<gx_blocks(nl, 128), 128, 0, ctx->stream>>>(
@@ -558,10 +754,9 @@ static int build_from_ranges(gx_ctx *ctx, const int32_t *rs, const int32_t *re, 
                 dptr<uint8_t>(ctx->is_leaf));
             ctx->launches += 2;
         }
-        // rounds in batches: the last build's round count first, then 8 at a time
-        // multi-block rounds in batches (the last build's count first), each batch followed
-        // by the single-block kernel for the small levels
-        int batch = std::max(4, ctx->hint_big_rounds + 1);
+        // multi-block rounds, if any level may need them, in batches (the last build's count
+        // first), each batch followed by the cluster's and the single block's rounds
+        int batch = nl > TS_CLUSTER ? std::max(4, ctx->hint_big_rounds + 1) : 0;
         int issued = 0;
         for (;;) {
             for (int r = 0; r < batch; r++) {
@@ -580,6 +775,7 @@ static int build_from_ranges(gx_ctx *ctx, const int32_t *rs, const int32_t *re, 
                 k_round_close<<<1, 1, 0, ctx->stream>>>(st, lstart);
                 ctx->launches += 7;
             }
+            if (nl > TS_SMALL) GX_TRY(launch_rounds_cluster(ctx, st, lstart, cap));
             k_rounds_small<<<1, RS_SMALL_THREADS, 0, ctx->stream>>>(
                 st, lstart, cap, dptr<uint64_t>(ctx->keys), dptr<double>(ctx->cx), dptr<double>(ctx->cy),
                 dptr<double>(ctx->hw), dptr<double>(ctx->mass), dptr<double>(ctx->comx), dptr<double>(ctx->comy),
@@ -598,13 +794,11 @@ static int build_from_ranges(gx_ctx *ctx, const int32_t *rs, const int32_t *re, 
         cap *= 2;
     }
     const int64_t rounds = hs[TS_ROUNDS];
-    std::vector<int64_t> ls((size_t)rounds + 2);
-    GX_CUDA(ctx, cudaMemcpyAsync(ls.data(), lstart, sizeof(int64_t) * ls.size(), cudaMemcpyDeviceToHost, ctx->stream));
-    GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    std::vector<int64_t> ls(hs + TS_N, hs + TS_N + rounds + 2);
     ctx->level_start.assign(ls.begin(), ls.end());
     ctx->hint_big_rounds = 0;  // multi-block rounds after the single-child ones
     for (size_t l = 0; l + 2 < ls.size(); l++)
-        if (ls[l + 1] - ls[l] > TS_SMALL) ctx->hint_big_rounds++;
+        if (ls[l + 1] - ls[l] > TS_CLUSTER) ctx->hint_big_rounds++;
     ctx->hint_big_rounds = std::max<int64_t>(0, ctx->hint_big_rounds - hs[TS_CHAIN_L]);
     const int64_t nn = ls.back();
     ctx->n_nodes = nn;
