@@ -179,6 +179,7 @@ struct gx_ctx {
     // (their arrays may be fresh ones swapped in from a gx_tree_plan)
     int64_t hint_nodes = 0, hint_far = 0, hint_near = 0;
     int hint_big_rounds = 0;  // tree build: rounds of the last build run by the multi-block kernels
+    int hint_field_levels = 0;  // tree build: levels of the last build whose fields took a launch each
     int rounds_blocks = 0;    // tree build: blocks of the rounds' cluster (0: not yet asked for)
     // ACCURATE plan: levels 1 .. chain_levels are single-child chains over the leaves
     // (level l holds node x + l nl above leaf x); with chain_levels >= 2 the plan and M2M

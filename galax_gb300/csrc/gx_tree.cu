@@ -178,13 +178,13 @@ enum {
     TS_S = 0, TS_E = 1, TS_C = 2, TS_SHIFT = 3, TS_NSEG = 4, TS_NG = 5, TS_FLAGS = 6, TS_ROUNDS = 7,
     TS_CHAIN_M = 8,  // min over adjacent leaves of the highest bit in which their first keys differ
     TS_CHAIN_L = 9,  // single-child rounds built by k_chain_rounds
-    TS_N = 10
+    TS_BEFORE = 10,  // rounds built before k_rounds_cluster
+    TS_N = 11
 };
 enum { TS_DONE = 1, TS_OVERFLOW = 2, TS_STUCK = 4 };
 constexpr int TS_MAX_ROUNDS = 400;  // level starts kept: TS_MAX_ROUNDS + 2
 
-constexpr int TS_SMALL = 512;     // levels of at most this many nodes: k_rounds_small
-constexpr int TS_CLUSTER = 65536;  // larger ones, up to this many nodes: k_rounds_cluster
+constexpr int TS_CLUSTER = 65536;  // levels of at most this many nodes: k_rounds_cluster
 // the multi-block round kernels do nothing once the build is over or the level is small
 __device__ __forceinline__ bool round_off(const int64_t *st) { return st[TS_FLAGS] != 0 || st[TS_C] <= TS_CLUSTER; }
 
@@ -291,7 +291,7 @@ __device__ __forceinline__ void parent_fields_one(int64_t q, double *cx, double 
     comy[q] = ms > 0.0 ? __ddiv_rn(sy, ms) : c_y;
     bs[q] = bs[first];
     be[q] = be[last];
-    parent[q] = -1;
+    if (parent) parent[q] = -1;  // null: the topology is already there
     is_leaf[q] = 0;
 }
 
@@ -363,253 +363,118 @@ __global__ void k_chain_rounds(int64_t *st, int64_t *level_start, int64_t nl, in
     }
 }
 
-// The rounds of levels of at most TS_SMALL nodes, all in one block: each phase of a
-// round is a loop over the level with a block barrier after it, so the tail of the
-// tree (a dozen rounds at 1M) costs one launch instead of a dozen per round.
-constexpr int RS_SMALL_THREADS = 1024;
-
-__device__ int64_t block_excl_scan_small(int v, int *warp_tot, int *total) {
-    // exclusive scan of one int per thread over RS_SMALL_THREADS threads
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int inc = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        int t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
-    }
-    if (lane == 31) warp_tot[w] = inc;
-    __syncthreads();
-    if (w == 0) {
-        int s = warp_tot[lane];
-        int si = s;
-        for (int o = 1; o < 32; o <<= 1) {
-            int t = __shfl_up_sync(0xffffffffu, si, o);
-            if (lane >= o) si += t;
-        }
-        warp_tot[lane] = si - s;
-        if (lane == 31) *total = si;
-    }
-    __syncthreads();
-    int r = warp_tot[w] + inc - v;
-    __syncthreads();
-    return r;
-}
-
-__global__ void __launch_bounds__(RS_SMALL_THREADS) k_rounds_small(int64_t *st, int64_t *level_start, int64_t cap_nodes,
-                                                                  const uint64_t *__restrict__ keys, double *cx,
-                                                                  double *cy, double *hw, double *mass, double *comx,
-                                                                  double *comy, int32_t *bs, int32_t *be, int32_t *child,
-                                                                  int32_t *parent, uint8_t *is_leaf) {
-    constexpr int PER = (TS_SMALL + RS_SMALL_THREADS - 1) / RS_SMALL_THREADS;  // items per thread
-    __shared__ int head[TS_SMALL], segex[TS_SMALL], segstart[TS_SMALL], goff[TS_SMALL];
-    __shared__ int warp_tot[32], tot;
-    __shared__ int64_t sh_s, sh_e, sh_c, sh_flags, sh_rounds;
-    __shared__ unsigned sh_shift;
-    const int t = threadIdx.x;
-    for (;;) {
-        if (t == 0) {
-            sh_s = st[TS_S];
-            sh_e = st[TS_E];
-            sh_c = st[TS_C];
-            sh_flags = st[TS_FLAGS];
-            sh_rounds = st[TS_ROUNDS];
-            sh_shift = (unsigned)st[TS_SHIFT] & 63u;
-        }
-        __syncthreads();
-        const int64_t s = sh_s, e = sh_e, c = sh_c;
-        if (sh_flags != 0 || c > TS_SMALL) return;
-        // heads and their exclusive scan (segment of each node)
-        int loc[PER], lsum = 0;
-        for (int k = 0; k < PER; k++) {
-            const int i = t * PER + k;
-            int h = 0;
-            if (i < c) {
-                const uint64_t g = keys[bs[s + i]] >> sh_shift;
-                h = (i == 0) ? 1 : (g != (keys[bs[s + i - 1]] >> sh_shift));
-                head[i] = h;
-            }
-            loc[k] = h;
-            lsum += h;
-        }
-        int run = (int)block_excl_scan_small(lsum, warp_tot, &tot);
-        const int nseg = tot;
-        for (int k = 0; k < PER; k++) {
-            const int i = t * PER + k;
-            if (i < c) segex[i] = run;
-            run += loc[k];
-        }
-        __syncthreads();
-        for (int k = 0; k < PER; k++) {
-            const int i = t * PER + k;
-            if (i < c && head[i]) segstart[segex[i]] = i;
-        }
-        __syncthreads();
-        // groups of at most 4 per segment and their exclusive scan
-        lsum = 0;
-        for (int k = 0; k < PER; k++) {
-            const int j = t * PER + k;
-            int g = 0;
-            if (j < nseg) g = (int)((((j + 1 < nseg) ? segstart[j + 1] : (int)c) - segstart[j] + 3) / 4);
-            loc[k] = g;
-            lsum += g;
-        }
-        run = (int)block_excl_scan_small(lsum, warp_tot, &tot);
-        const int ng = tot;
-        for (int k = 0; k < PER; k++) {
-            const int j = t * PER + k;
-            if (j < nseg) goff[j] = run;
-            run += loc[k];
-        }
-        if (e + ng > cap_nodes || sh_rounds >= TS_MAX_ROUNDS) {
-            if (t == 0) st[TS_FLAGS] |= (e + ng > cap_nodes) ? TS_OVERFLOW : TS_STUCK;
-            return;  // uniform: every thread saw the same counts
-        }
-        for (int g = t; g < ng; g += RS_SMALL_THREADS)
-            reinterpret_cast<int4 *>(child)[e + g] = make_int4(-1, -1, -1, -1);
-        __syncthreads();
-        for (int k = 0; k < PER; k++) {
-            const int i = t * PER + k;
-            if (i >= c) continue;
-            const int seg = segex[i] + head[i] - 1;
-            const int pos = i - segstart[seg];
-            const int64_t g = goff[seg] + pos / 4;
-            parent[s + i] = (int32_t)(e + g);
-            child[(e + g) * 4 + (pos & 3)] = (int32_t)(s + i);
-        }
-        __syncthreads();
-        for (int g = t; g < ng; g += RS_SMALL_THREADS)
-            parent_fields_one(e + g, cx, cy, hw, mass, comx, comy, bs, be, reinterpret_cast<const int4 *>(child),
-                              parent, is_leaf);
-        __syncthreads();
-        if (t == 0) {
-            const int64_t r = ++st[TS_ROUNDS];
-            level_start[r + 1] = e + ng;
-            st[TS_S] = e;
-            st[TS_E] = e + ng;
-            st[TS_C] = ng;
-            st[TS_SHIFT] += 2;
-            if (ng <= 1) st[TS_FLAGS] |= TS_DONE;
-        }
-        __syncthreads();
-    }
-}
-
-// The rounds of levels of more than TS_SMALL and at most TS_CLUSTER nodes, all in one
-// cluster of blocks that meets at cluster barriers: a round was 13 launches of 4 us each
-// (with the sort's passes of three launches instead of seven, upload, build and read-back at
-// N = 200k, n_max = 16 take 0.80 ms, 1.13 before).
-// Every thread owns a run of consecutive nodes of the level; two scans over the cluster
-// (block scans, the blocks' results exchanged through distributed shared memory) give each
-// node the head of its segment and its group, the same groups in the same order as the
-// multi-block rounds: a segment's nodes by fours.  One cluster has the FP64 pipes of as many
-// SMs as it has blocks, and parent_fields_one is FP64: above TS_CLUSTER nodes a round over
-// the whole GPU is as fast.
+// The rounds of levels of at most TS_CLUSTER nodes: their topology in one launch
+// (k_rounds_cluster), then the nodes' fields level by level.
+//
+// Which nodes a round groups depends on the leaves alone.  Let d be the highest bit in which
+// a node's first key differs from the first key of the node before it; the node begins a
+// segment of the round with shift sh exactly when d >= sh.  A parent inherits the d of its
+// first child: if that child began a segment, the children before it have smaller d, so its
+// d is the parents' too, and if not, d < sh and neither it nor its parent begins a segment
+// again.  So a thread loads the d of a run of consecutive nodes once (a byte each, in one
+// register pair), and every round is two scans over the cluster, of the last segment head
+// and of the groups begun, with nothing read from global memory; the thread that holds a
+// group's first node keeps the parent.  The groups and their order are those of the
+// multi-block rounds: a segment's nodes by fours.
 constexpr int RC_THREADS = 1024;
 constexpr int RC_MAX_BLOCKS = 16;
+constexpr int RC_RUN = 8;  // nodes a thread holds at most: TS_CLUSTER nodes on 8 blocks
+static_assert(TS_CLUSTER <= 8 * RC_THREADS * RC_RUN, "a level fits the smaller cluster");
 
-__device__ __forceinline__ int warp_max_scan(int v) {
+// Inclusive scan over the block (op: max or sum) of one int a thread; wt: 33 ints, the last
+// one the block's result.
+template <class Op>
+__device__ __forceinline__ int rc_block_scan(int v, int *wt, Op op, int zero) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, v, o);
-        if ((int)(threadIdx.x & 31) >= o) v = max(v, t);
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v = op(v, u);
     }
-    return v;
+    if (lane == 31) wt[w] = v;
+    __syncthreads();
+    if (w == 0) {
+        int x = wt[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x = op(x, u);
+        }
+        wt[lane] = x;
+        if (lane == 31) wt[32] = x;
+    }
+    __syncthreads();
+    return w > 0 ? op(v, wt[w - 1]) : op(v, zero);
 }
 
 __global__ void __launch_bounds__(RC_THREADS) k_rounds_cluster(int64_t *st, int64_t *level_start, int64_t cap_nodes,
-                                                               const uint64_t *__restrict__ keys, double *cx,
-                                                               double *cy, double *hw, double *mass, double *comx,
-                                                               double *comy, int32_t *bs, int32_t *be, int32_t *child,
-                                                               int32_t *parent, uint8_t *is_leaf) {
+                                                               const uint64_t *__restrict__ keys,
+                                                               const int32_t *__restrict__ bs, int32_t *child,
+                                                               int32_t *parent) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     const int nb = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const int gt = rank * RC_THREADS + t, stride = nb * RC_THREADS;
-    __shared__ int wt[32], blast, bcnt, prev_last, prev_cnt, all_cnt;
+    const int t = threadIdx.x, lane = t & 31;
+    __shared__ int wmax[2][33], wsum[2][33];  // by the round's parity: a block reads the others' after one barrier
+    __shared__ int prev_last, prev_cnt, all_cnt;
     // the round state, kept by every thread alike and written back at the end
     int64_t s = st[TS_S], e = st[TS_E], flags = st[TS_FLAGS], rounds = st[TS_ROUNDS], shift = st[TS_SHIFT];
-    int c = (int)st[TS_C];
+    int64_t c = st[TS_C];
     cl.sync();  // all blocks have read the state before one writes it
-    if (flags != 0 || c > TS_CLUSTER || c <= TS_SMALL) return;
-    while (flags == 0 && c > TS_SMALL) {
-        const unsigned sh = (unsigned)shift & 63u;
-        const int per = (c + stride - 1) / stride;  // at most 8 (TS_CLUSTER nodes on 8 blocks)
-        const int i0 = min(c, gt * per), i1 = min(c, i0 + per);
-        // heads of segments (nodes whose key prefix differs from the one before)
-        unsigned heads = 0;
+    if (flags != 0 || c > TS_CLUSTER) return;
+    // this thread's nodes i0 .. i0 + n - 1 and their d + 1 (0: equal keys; 255: the first node)
+    const int per = (int)((c + nb * RC_THREADS - 1) / (nb * RC_THREADS));
+    int i0 = (int)min(c, (int64_t)(rank * RC_THREADS + t) * per), n = (int)min(c, (int64_t)i0 + per) - i0;
+    uint64_t dv = 0;
+    if (n > 0) {
+        uint64_t p = i0 > 0 ? keys[bs[s + i0 - 1]] : 0;
+        for (int k = 0; k < n; k++) {
+            const uint64_t g = keys[bs[s + i0 + k]], x = g ^ p;
+            const int d1 = i0 + k == 0 ? 255 : (x ? 64 - __clzll((long long)x) : 0);
+            dv |= (uint64_t)d1 << (8 * k);
+            p = g;
+        }
+    }
+    const auto mx = [](int a, int b) { return max(a, b); };
+    const auto sm = [](int a, int b) { return a + b; };
+    for (int par = 0; flags == 0; par ^= 1) {
+        const int sh = (int)min(shift, (int64_t)63);
+        // the last segment head before this thread's run
         int last = -1;
-        bool next_head = true;  // the node after this run begins a segment (or there is none)
-        if (i0 < i1) {
-            uint64_t p = i0 > 0 ? keys[bs[s + i0 - 1]] >> sh : 0;
-            for (int i = i0; i < i1; i++) {
-                const uint64_t g = keys[bs[s + i]] >> sh;
-                if (i == 0 || g != p) {
-                    heads |= 1u << (i - i0);
-                    last = i;
-                }
-                p = g;
-            }
-            next_head = i1 >= c || (keys[bs[s + i1]] >> sh) != p;
-        }
-        // the last head before this run: max scan over the cluster
-        int m = warp_max_scan(last);
-        if (lane == 31) wt[w] = m;
-        __syncthreads();
-        if (w == 0) {
-            const int v = warp_max_scan(wt[lane]);
-            wt[lane] = v;
-            if (lane == 31) blast = v;
-        }
-        __syncthreads();
+        for (int k = 0; k < n; k++)
+            if ((int)((dv >> (8 * k)) & 255u) > sh) last = i0 + k;
+        const int m = rc_block_scan(last, wmax[par], mx, -1);
         int head = __shfl_up_sync(0xffffffffu, m, 1);
-        if (lane == 0) head = -1;
-        if (w > 0) head = max(head, wt[w - 1]);
+        if (lane == 0) head = t > 0 ? wmax[par][(t >> 5) - 1] : -1;
         cl.sync();
-        if (t == 0) {
-            int v = -1;
-            for (int r = 0; r < rank; r++) v = max(v, *cl.map_shared_rank(&blast, r));
-            prev_last = v;
+        if (t < 32) {
+            int v = t < rank ? *cl.map_shared_rank(&wmax[par][32], t) : -1;
+            for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+            if (t == 0) prev_last = v;
         }
         __syncthreads();
         head = max(head, prev_last);
-        // groups of four within each segment: count those that begin in this run
-        int h = head, cnt = 0;
-        for (int i = i0; i < i1; i++) {
-            if ((heads >> (i - i0)) & 1u) h = i;
-            cnt += ((i - h) & 3) == 0;
+        // groups of four within each segment: those that begin in this run
+        int cnt = 0, h = head;
+        for (int k = 0; k < n; k++) {
+            if ((int)((dv >> (8 * k)) & 255u) > sh) h = i0 + k;
+            cnt += ((i0 + k - h) & 3) == 0;
         }
-        int inc = cnt;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += v;
-        }
-        __syncthreads();  // wt has been read
-        if (lane == 31) wt[w] = inc;
-        __syncthreads();
-        if (w == 0) {
-            int v = wt[lane];
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, v, o);
-                if (lane >= o) v += u;
-            }
-            if (lane == 31) bcnt = v;
-            wt[lane] = v;
-        }
-        __syncthreads();
-        int g = inc - cnt + (w > 0 ? wt[w - 1] : 0);
+        int g = rc_block_scan(cnt, wsum[par], sm, 0) - cnt;
         cl.sync();
-        if (t == 0) {
-            int before = 0, total = 0;
-            for (int r = 0; r < nb; r++) {
-                const int v = *cl.map_shared_rank(&bcnt, r);
-                if (r < rank) before += v;
-                total += v;
+        if (t < 32) {
+            const int v = t < nb ? *cl.map_shared_rank(&wsum[par][32], t) : 0;
+            int before = t < rank ? v : 0, total = v;
+            for (int o = 16; o > 0; o >>= 1) {
+                before += __shfl_xor_sync(0xffffffffu, before, o);
+                total += __shfl_xor_sync(0xffffffffu, total, o);
             }
-            prev_cnt = before;
-            all_cnt = total;
+            if (t == 0) {
+                prev_cnt = before;
+                all_cnt = total;
+            }
         }
         __syncthreads();
-        g += prev_cnt - 1;
-        const int ng = all_cnt;
+        g += prev_cnt;
+        const int64_t ng = all_cnt;
         if (e + ng > cap_nodes) {
             flags |= TS_OVERFLOW;
             break;
@@ -618,33 +483,36 @@ __global__ void __launch_bounds__(RC_THREADS) k_rounds_cluster(int64_t *st, int6
             flags |= TS_STUCK;
             break;
         }
+        // parents and child slots; the parents of the groups begun here are this thread's next run
+        int q = g - 1, kept = 0;
+        uint64_t nd = 0;
         h = head;
-        for (int i = i0; i < i1; i++) {
-            if ((heads >> (i - i0)) & 1u) h = i;
+        for (int k = 0; k < n; k++) {
+            const int i = i0 + k;
+            const uint64_t d = (dv >> (8 * k)) & 255u;
+            if ((int)d > sh) h = i;
             const int pos = (i - h) & 3;
-            g += pos == 0;
-            const int64_t q = e + g;
-            parent[s + i] = (int32_t)q;
-            child[q * 4 + pos] = (int32_t)(s + i);
-            const bool end = i + 1 < i1 ? (heads >> (i + 1 - i0)) & 1u : next_head;
-            if (end)
-                for (int k = pos + 1; k < 4; k++) child[q * 4 + k] = -1;
+            if (pos == 0) {
+                q++;
+                nd |= d << (8 * kept++);
+            }
+            parent[s + i] = (int32_t)(e + q);
+            child[(e + q) * 4 + pos] = (int32_t)(s + i);
         }
-        cl.sync();
-        for (int k = gt; k < ng; k += stride)
-            parent_fields_one(e + k, cx, cy, hw, mass, comx, comy, bs, be, reinterpret_cast<const int4 *>(child),
-                              parent, is_leaf);
+        dv = nd;
+        n = kept;
+        i0 = g;
         s = e;
         e += ng;
         c = ng;
         shift += 2;
         rounds++;
-        if (gt == 0) level_start[rounds + 1] = e;
+        if (rank == 0 && t == 0) level_start[rounds + 1] = e;
         if (ng <= 1) flags |= TS_DONE;
-        cl.sync();
     }
+    if ((flags & TS_DONE) && rank == 0 && t == 0) parent[s] = -1;  // the root
     cl.sync();  // no block leaves while another may read its shared memory
-    if (gt == 0) {
+    if (rank == 0 && t == 0) {
         st[TS_S] = s;
         st[TS_E] = e;
         st[TS_C] = c;
@@ -653,6 +521,47 @@ __global__ void __launch_bounds__(RC_THREADS) k_rounds_cluster(int64_t *st, int6
         st[TS_ROUNDS] = rounds;
     }
 }
+
+// every child slot of the new levels starts empty
+__global__ void k_slots_clear(const int64_t *st, int64_t cap_nodes, int4 *child) {
+    if (st[TS_FLAGS] != 0) return;
+    const int64_t q = st[TS_E] + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < cap_nodes) child[q] = make_int4(-1, -1, -1, -1);
+}
+
+// The fields of the nodes built by k_rounds_cluster: the levels after the first `from`
+// (built before it), the k-th of them by launch k of k_fields_level over the whole GPU
+// while it has more than FIELDS_SMALL nodes, the rest in one cluster (k_fields_small).
+constexpr int FIELDS_SMALL = 2048;
+constexpr int FIELDS_BLOCKS = 8, FIELDS_THREADS = 256;
+__global__ void k_fields_level(const int64_t *st, const int64_t *level_start, int64_t lv, double *cx, double *cy,
+                               double *hw, double *mass, double *comx, double *comy, int32_t *bs, int32_t *be,
+                               const int4 *child, uint8_t *is_leaf) {
+    lv += st[TS_BEFORE];
+    if (!(st[TS_FLAGS] & TS_DONE) || lv > st[TS_ROUNDS]) return;
+    const int64_t s = level_start[lv], c = level_start[lv + 1] - s;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c <= FIELDS_SMALL || i >= c) return;
+    parent_fields_one(s + i, cx, cy, hw, mass, comx, comy, bs, be, child, nullptr, is_leaf);
+}
+__global__ void __launch_bounds__(FIELDS_THREADS) k_fields_small(const int64_t *st, const int64_t *level_start,
+                                                                int64_t launched, double *cx, double *cy, double *hw,
+                                                                double *mass, double *comx, double *comy, int32_t *bs,
+                                                                int32_t *be, const int4 *child, uint8_t *is_leaf) {
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    if (!(st[TS_FLAGS] & TS_DONE)) return;
+    const int64_t n = st[TS_ROUNDS], from = st[TS_BEFORE] + 1;
+    for (int64_t lv = from; lv <= n; lv++) {
+        const int64_t s = level_start[lv], c = level_start[lv + 1] - s;
+        if (c > FIELDS_SMALL && lv < from + launched) continue;
+        for (int64_t i = cl.block_rank() * FIELDS_THREADS + threadIdx.x; i < c; i += FIELDS_BLOCKS * FIELDS_THREADS)
+            parent_fields_one(s + i, cx, cy, hw, mass, comx, comy, bs, be, child, nullptr, is_leaf);
+        cl.sync();
+    }
+}
+
+// the rounds built so far: the cluster's levels come after them
+__global__ void k_mark_before(int64_t *st) { st[TS_BEFORE] = st[TS_ROUNDS]; }
 
 // ---- build_constrained helpers (lib.rs:541-694) ----
 // leaf ranges bounded by n_max and by the sorted split points (lib.rs:603-613):
@@ -682,8 +591,9 @@ static int ensure_nodes(gx_ctx *ctx, int64_t need) {
     return GX_OK;
 }
 
-// The cluster of k_rounds_cluster: 16 blocks where the device takes them, else the portable 8.
-static int launch_rounds_cluster(gx_ctx *ctx, int64_t *st, int64_t *lstart, int64_t cap) {
+// k_rounds_cluster: one block while its threads hold the level, else 16 where the device
+// takes them, else the portable 8.
+static int launch_rounds_cluster(gx_ctx *ctx, int64_t *st, int64_t *lstart, int64_t cap, int64_t nl) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at = {};
     at.id = cudaLaunchAttributeClusterDimension;
@@ -702,13 +612,12 @@ static int launch_rounds_cluster(gx_ctx *ctx, int64_t *st, int64_t *lstart, int6
             ctx->rounds_blocks = RC_MAX_BLOCKS;
         cudaGetLastError();  // a device without the larger cluster is no error
     }
-    at.val.clusterDim.x = (unsigned)ctx->rounds_blocks;
-    cfg.gridDim = dim3((unsigned)ctx->rounds_blocks);
+    const unsigned blocks = nl <= 2 * RC_THREADS ? 1 : (unsigned)ctx->rounds_blocks;
+    at.val.clusterDim.x = blocks;
+    cfg.gridDim = dim3(blocks);
     GX_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_rounds_cluster, st, lstart, cap, (const uint64_t *)dptr<uint64_t>(ctx->keys),
-                                    dptr<double>(ctx->cx), dptr<double>(ctx->cy), dptr<double>(ctx->hw),
-                                    dptr<double>(ctx->mass), dptr<double>(ctx->comx), dptr<double>(ctx->comy),
-                                    dptr<int32_t>(ctx->bs), dptr<int32_t>(ctx->be), dptr<int32_t>(ctx->child),
-                                    dptr<int32_t>(ctx->parent), dptr<uint8_t>(ctx->is_leaf)));
+                                    (const int32_t *)dptr<int32_t>(ctx->bs), dptr<int32_t>(ctx->child),
+                                    dptr<int32_t>(ctx->parent)));
     ctx->launches++;
     return GX_OK;
 }
@@ -740,7 +649,7 @@ static int build_from_ranges(gx_ctx *ctx, const int32_t *rs, const int32_t *re, 
             dptr<double>(ctx->comy), dptr<int32_t>(ctx->bs), dptr<int32_t>(ctx->be), dptr<int4>(ctx->child),
             dptr<int32_t>(ctx->parent), dptr<uint8_t>(ctx->is_leaf));
         ctx->launches++;
-        const int64_t init[TS_N] = {0, nl, nl, 2, 0, 0, nl > 1 ? 0 : TS_DONE, 0, 64, 0};
+        const int64_t init[TS_N] = {0, nl, nl, 2, 0, 0, nl > 1 ? 0 : TS_DONE, 0, 64, 0, 0};
         const int64_t ls01[2] = {0, nl};
         GX_CUDA(ctx, cudaMemcpyAsync(st, init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream));
         GX_CUDA(ctx, cudaMemcpyAsync(lstart, ls01, sizeof(ls01), cudaMemcpyHostToDevice, ctx->stream));
@@ -755,7 +664,7 @@ static int build_from_ranges(gx_ctx *ctx, const int32_t *rs, const int32_t *re, 
             ctx->launches += 2;
         }
         // multi-block rounds, if any level may need them, in batches (the last build's count
-        // first), each batch followed by the cluster's and the single block's rounds
+        // first), each batch followed by the cluster's rounds
         int batch = nl > TS_CLUSTER ? std::max(4, ctx->hint_big_rounds + 1) : 0;
         int issued = 0;
         for (;;) {
@@ -775,13 +684,34 @@ static int build_from_ranges(gx_ctx *ctx, const int32_t *rs, const int32_t *re, 
                 k_round_close<<<1, 1, 0, ctx->stream>>>(st, lstart);
                 ctx->launches += 7;
             }
-            if (nl > TS_SMALL) GX_TRY(launch_rounds_cluster(ctx, st, lstart, cap));
-            k_rounds_small<<<1, RS_SMALL_THREADS, 0, ctx->stream>>>(
-                st, lstart, cap, dptr<uint64_t>(ctx->keys), dptr<double>(ctx->cx), dptr<double>(ctx->cy),
-                dptr<double>(ctx->hw), dptr<double>(ctx->mass), dptr<double>(ctx->comx), dptr<double>(ctx->comy),
-                dptr<int32_t>(ctx->bs), dptr<int32_t>(ctx->be), dptr<int32_t>(ctx->child), dptr<int32_t>(ctx->parent),
-                dptr<uint8_t>(ctx->is_leaf));
-            ctx->launches++;
+            // the rest of the topology, then the fields of its levels (the last build's number
+            // of large ones, four on a first build)
+            k_mark_before<<<1, 1, 0, ctx->stream>>>(st);
+            k_slots_clear<<<gx_blocks(cap - nl, 256), 256, 0, ctx->stream>>>(st, cap, dptr<int4>(ctx->child));
+            GX_TRY(launch_rounds_cluster(ctx, st, lstart, cap, nl));
+            const int large = nl > FIELDS_SMALL ? (ctx->hint_field_levels > 0 ? ctx->hint_field_levels : 4) : 0;
+            const unsigned gf = gx_blocks(std::min<int64_t>(nl, TS_CLUSTER), 128);
+            for (int k = 1; k <= large; k++)
+                k_fields_level<<<gf, 128, 0, ctx->stream>>>(
+                    st, lstart, k, dptr<double>(ctx->cx), dptr<double>(ctx->cy), dptr<double>(ctx->hw),
+                    dptr<double>(ctx->mass), dptr<double>(ctx->comx), dptr<double>(ctx->comy), dptr<int32_t>(ctx->bs),
+                    dptr<int32_t>(ctx->be), dptr<int4>(ctx->child), dptr<uint8_t>(ctx->is_leaf));
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute at = {};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = FIELDS_BLOCKS;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.gridDim = dim3(FIELDS_BLOCKS);
+            cfg.blockDim = dim3(FIELDS_THREADS);
+            cfg.stream = ctx->stream;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            GX_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_fields_small, (const int64_t *)st, (const int64_t *)lstart,
+                                            (int64_t)large, dptr<double>(ctx->cx), dptr<double>(ctx->cy),
+                                            dptr<double>(ctx->hw), dptr<double>(ctx->mass), dptr<double>(ctx->comx),
+                                            dptr<double>(ctx->comy), dptr<int32_t>(ctx->bs), dptr<int32_t>(ctx->be),
+                                            (const int4 *)dptr<int4>(ctx->child), dptr<uint8_t>(ctx->is_leaf)));
+            ctx->launches += 3 + large;
             GX_CUDA(ctx, cudaGetLastError());
             issued += batch;
             GX_CUDA(ctx, cudaMemcpyAsync(hs, st, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream));
@@ -800,6 +730,9 @@ static int build_from_ranges(gx_ctx *ctx, const int32_t *rs, const int32_t *re, 
     for (size_t l = 0; l + 2 < ls.size(); l++)
         if (ls[l + 1] - ls[l] > TS_CLUSTER) ctx->hint_big_rounds++;
     ctx->hint_big_rounds = std::max<int64_t>(0, ctx->hint_big_rounds - hs[TS_CHAIN_L]);
+    ctx->hint_field_levels = 0;  // levels of k_fields_level
+    for (int64_t l = hs[TS_BEFORE] + 1; l <= rounds; l++)
+        if (ls[l + 1] - ls[l] > FIELDS_SMALL) ctx->hint_field_levels++;
     const int64_t nn = ls.back();
     ctx->n_nodes = nn;
     ctx->hint_nodes = nn;
