@@ -88,11 +88,7 @@ __global__ void __launch_bounds__(128) k_adj_l2p(int64_t nl, const double *__res
         gx[i] = -(double)(hxx * lam_x + hxy * lam_y);
         gy[i] = -(double)(hxy * lam_x + hyy * lam_y);
     }
-#pragma unroll
-    for (int k = 0; k < NCr; k++) {
-        T s = warp_sum_t<T>(acc[k]);
-        if (lane == (k & 31)) dL[leaf * NS + k] = s;
-    }
+    warp_coeffs<NC>(acc, [&](int k, T s) { dL[leaf * NS + k] = s; });
 }
 
 // ---- A2: L2L^T, an upward pass: dL[P][U] = sum_c sum_{T<=U} dL[c][T] C(U,T) e^(U-T),
@@ -105,15 +101,15 @@ __global__ void __launch_bounds__(128) k_adj_l2p(int64_t nl, const double *__res
 // The FP32 form forms com_t - com_s from the FP32 (hi, lo) COMs exactly as the
 // forward M2L forms it for the pair (t, s).  Work units as in the forward M2L (far
 // lists cut into pieces of at most GX_M2L_UNIT entries, one warp each); a node with
-// one unit writes dM directly, otherwise k_adj_m2l_combine sums the units' partials
-// in unit order.  Nodes without far entries are not written: has_far = 0 keeps A4
+// one unit writes dM directly, otherwise the unit that finishes last sums the units'
+// partials in unit order.  Nodes without far entries are not written: has_far = 0 keeps A4
 // from reading them.
 template <int P, class T>
 __global__ void __launch_bounds__(128, (sizeof(T) == 4 && P <= 4) ? 8 : 1)
     k_adj_m2l(int64_t n_units, const int32_t *__restrict__ unode, const int64_t *__restrict__ ustart,
               const int32_t *__restrict__ ulen, const int64_t *__restrict__ node_u, const int32_t *__restrict__ idx,
               const double *__restrict__ comx, const double *__restrict__ comy, const float4 *__restrict__ comhl,
-              double eps2d, const T *__restrict__ dL, T *__restrict__ dM, T *__restrict__ part) {
+              double eps2d, const T *__restrict__ dL, T *__restrict__ dM, T *part, unsigned *count) {
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<T>(NC);
     const int PP = gx_rt_order(P);
@@ -122,7 +118,6 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && P <= 4) ? 8 : 1)
     int lane = threadIdx.x & 31;
     if (u >= n_units) return;
     const int64_t node = unode[u];
-    const bool single = node_u[node + 1] - node_u[node] == 1;
     const int64_t st = ustart[u];
     const int len = ulen[u];
     double scx = comx[node], scy = comy[node];
@@ -153,37 +148,18 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && P <= 4) ? 8 : 1)
         m2l_fused<P, T>(dx, dy, eps2, lt, acc);
         t = nt;
     }
-#pragma unroll
-    for (int si = 0; si <= PP; si++)
-#pragma unroll
-        for (int sj = 0; sj <= PP - si; sj++) {
-            int k = gx_mi(si, sj);
-            T v = warp_sum_t<T>(acc[k]);
-            if (lane == (k & 31)) {
-                if (single) dM[node * NS + k] = ((si + sj) & 1) ? v : -v;
-                else part[u * NS + k] = v;
-            }
-        }
-}
-
-template <int P, class T>
-__global__ void k_adj_m2l_combine(int64_t nn, const int64_t *__restrict__ node_u, const T *__restrict__ part,
-                                  T *__restrict__ dM) {
-    constexpr int NC = nc2(P);
-    constexpr int NS = row_stride<T>(NC);
-    const int PP = gx_rt_order(P);
-    const int NCr = (PP + 1) * (PP + 2) / 2;
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int64_t node = t / NC;
-    int k = (int)(t - node * NC);
-    if (node >= nn || k >= NCr) return;
-    int64_t u0 = node_u[node], u1 = node_u[node + 1];
-    if (u1 - u0 < 2) return;
-    T s = T(0);
-    for (int64_t u = u0; u < u1; u++) s += part[u * NS + k];
-    int n = 0;  // coefficient k = gx_mi(si, sj) with si + sj = n
-    while ((n + 1) * (n + 2) / 2 <= k) n++;
-    dM[node * NS + k] = (n & 1) ? s : -s;
+    const int64_t u0 = node_u[node], u1 = node_u[node + 1];
+    const auto store = [&](int k, T v) {
+        int i, j;
+        mi_split(k, i, j);
+        dM[node * NS + k] = ((i + j) & 1) ? v : -v;
+    };
+    if (u1 - u0 == 1) {
+        warp_coeffs<NC>(acc, store);
+    } else {
+        warp_coeffs<NC>(acc, [&](int k, T v) { part[u * NS + k] = v; });
+        last_unit_sums<NC, NS>(node, u0, u1, part, count, store);
+    }
 }
 
 // ---- A4: M2M^T straight to the leaves: the moments of an ancestor a are the leaf's
@@ -210,24 +186,11 @@ __global__ void __launch_bounds__(128) k_adj_m2m_direct(int64_t nl, int n_levels
         if (a < 0 || !has_far[a]) continue;
         T da[NC];
         load_row<NC>(dM + (int64_t)a * NS, da);
-        T px[P + 1], py[P + 1];
-        pow_fact<P, T>((T)(comx[leaf] - comx[a]), px);
-        pow_fact<P, T>((T)(comy[leaf] - comy[a]), py);
+        shift_down<P, T>((T)(comx[leaf] - comx[a]), (T)(comy[leaf] - comy[a]), da);
 #pragma unroll
-        for (int si = 0; si <= PP; si++)
-#pragma unroll
-            for (int sj = 0; sj <= PP - si; sj++)
-#pragma unroll
-                for (int ti = si; ti <= PP; ti++)
-#pragma unroll
-                    for (int tj = sj; tj <= PP - ti; tj++)
-                        out[gx_mi(si, sj)] += da[gx_mi(ti, tj)] * px[ti - si] * py[tj - sj];
+        for (int k = 0; k < NCr; k++) out[k] += da[k];
     }
-#pragma unroll
-    for (int k = 0; k < NCr; k++) {
-        T v = warp_sum_t<T>(out[k]);
-        if (lane == (k & 31)) dMleaf[leaf * NS + k] = v;
-    }
+    warp_coeffs<NC>(out, [&](int k, T v) { dMleaf[leaf * NS + k] = v; });
 }
 
 // ---- A5: P2M^T: g_m,j += sum_S dM[S] u^S/S!,  g_x,j += m_j sum_S dM[S] grad(u^S/S!).
@@ -709,8 +672,7 @@ int run_force_vjp(gx_ctx *ctx, const double *X, const double *Y, const void *lf_
         k_adj_m2l<P, T><<<(unsigned)((U.n * 32 + 127) / 128), 128, 0, st>>>(
             U.n, dptr<int32_t>(U.node), dptr<int64_t>(U.start), dptr<int32_t>(U.len), node_u,
             dptr<int32_t>(ctx->far_idx), comx, comy, F32 ? dptr<float4>(ctx->comhl) : nullptr, eps2, dL, dM,
-            dptr<T>(ctx->m2l_part));
-        k_adj_m2l_combine<P, T><<<gx_blocks(nn * NC, 256), 256, 0, st>>>(nn, node_u, dptr<T>(ctx->m2l_part), dM);
+            dptr<T>(ctx->m2l_part), dptr<unsigned>(ctx->m2l_count));
     }
     // A4: M2M^T to the leaves
     k_adj_m2m_direct<P, T><<<gw, 128, 0, st>>>(nl, ctx->n_levels, dptr<int32_t>(ctx->anc),

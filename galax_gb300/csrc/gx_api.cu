@@ -158,6 +158,8 @@ int gx_create(const gx_config *cfg, gx_ctx **out) {
     }
     for (auto &e : ctx->ev) cudaEventCreate(&e);
     if (cudaStreamCreateWithPriority(&ctx->stream2, cudaStreamNonBlocking, prio_lo) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&ctx->stream3, cudaStreamNonBlocking, prio_lo) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_join3, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess) {
         gx_destroy(ctx);
@@ -190,7 +192,7 @@ int gx_destroy(gx_ctx *ctx) {
                       &ctx->Lff32, &ctx->pos32, &ctx->fl32, &ctx->part, &ctx->items_ref.leaf, &ctx->items_ref.qb, &ctx->items_ref.nq, &ctx->items_ref.off, &ctx->items_acc.leaf, &ctx->items_acc.qb, &ctx->items_acc.nq, &ctx->items_acc.off, &ctx->scratch_a, &ctx->scratch_b, &ctx->scratch_c, &ctx->scratch_d,
                       &ctx->scratch_e, &ctx->scratch_f, &ctx->scratch_g, &ctx->status, &ctx->red, &ctx->flush, &ctx->adj_lx, &ctx->adj_ly, &ctx->adj_lvx, &ctx->adj_lvy, &ctx->adj_lm, &ctx->adj_gx, &ctx->adj_gy, &ctx->adj_gm, &ctx->adj_lax, &ctx->adj_lay, &ctx->adj_lf, &ctx->adj_dL, &ctx->adj_dM, &ctx->adj_dMleaf, &ctx->adj_lam32, &ctx->ckpt, &ctx->seg, &ctx->ids, &ctx->perm, &ctx->roll_perms, &ctx->radius32,
                       &ctx->m2l_units.node, &ctx->m2l_units.start, &ctx->m2l_units.len, &ctx->m2l_units.node_u,
-                      &ctx->m2l_part, &ctx->plan_ctr, &ctx->tree_state, &ctx->m2l_cnt, &ctx->split_cnt,
+                      &ctx->m2l_part, &ctx->m2l_count, &ctx->plan_ctr, &ctx->tree_state, &ctx->m2l_cnt, &ctx->split_cnt,
                       &ctx->split_tot, &ctx->p2l_units.leaf, &ctx->p2l_units.start, &ctx->p2l_units.len,
                       &ctx->p2l_units.leaf_u, &ctx->p2l_units.body_u, &ctx->p2l_part, &ctx->m2p_list,
                       &ctx->m2p_off, &ctx->p2p_mask, &ctx->body_off32};
@@ -203,6 +205,11 @@ int gx_destroy(gx_ctx *ctx) {
         cudaStreamSynchronize(ctx->stream2);
         cudaStreamDestroy(ctx->stream2);
     }
+    if (ctx->stream3) {
+        cudaStreamSynchronize(ctx->stream3);
+        cudaStreamDestroy(ctx->stream3);
+    }
+    if (ctx->ev_join3) cudaEventDestroy(ctx->ev_join3);
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -300,6 +307,7 @@ int gx_rebuild_internal(gx_ctx *ctx) {
         return gx_fail(ctx, GX_ERR_CAP_EXCEEDED, "tree node count exceeds max_nodes");
     ctx->max_leaf = std::min<int64_t>(ctx->build_n_max, n);
     ctx->unary_levels = count_unary_levels(ctx);
+    ctx->leaves_cover = true;
     ctx->have_tree = true;
     GX_CUDA(ctx, cudaGetLastError());
     return GX_OK;
@@ -392,6 +400,7 @@ int gx_build_tree(gx_ctx *ctx, int64_t n, double *x, double *y, double *vx, doub
     ctx->ref_lists_valid = false;
     ctx->max_leaf = std::min<int64_t>(n_max, n);
     ctx->unary_levels = count_unary_levels(ctx);
+    ctx->leaves_cover = true;
     // Tree::build permutes the caller's arrays (lib.rs:204); so do we.
     if (!(flags & GX_BUILD_BALANCED)) GX_TRY(gx_download_bodies(ctx, x, y, vx, vy, m, ax, ay));
     GX_TRY(gx_ids_reset(ctx));  // the caller's arrays are now in tree order
@@ -477,6 +486,13 @@ int gx_upload_tree(gx_ctx *ctx, int64_t n_nodes, int64_t n_bodies, const double 
         if (!chain) break;
         ctx->unary_levels = l;
     }
+    std::vector<std::pair<int64_t, int64_t>> lr;  // the leaves' ranges, in body order
+    for (int64_t i = 0; i < nl; i++) lr.emplace_back(body_start[i], body_end[i]);
+    std::sort(lr.begin(), lr.end());
+    int64_t reach = 0;
+    for (const auto &r : lr)
+        if (r.first <= reach) reach = std::max(reach, r.second);
+    ctx->leaves_cover = reach == n_bodies;
     ctx->ref_lists_valid = true;  // the caller's lists
     ctx->have_tree = true;
     return GX_OK;

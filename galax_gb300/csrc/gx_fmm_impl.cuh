@@ -105,6 +105,45 @@ __device__ __forceinline__ T warp_sum_t(T v) {
     return v;
 }
 
+// Sums over the warp of N = 16 or 32 values a lane, as a reduce-scatter: each exchange
+// halves what a lane still carries, 16 or 31 additions instead of five a value.  Lane l ends
+// with the sum of value l (N = 16: value l & 15, in both half-warps).
+template <int N, class T>
+__device__ __forceinline__ T warp_scatter_sum(T *v) {
+    static_assert(N == 16 || N == 32, "");
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = N / 2; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int k = 0; k < o; k++) {
+            const T keep = up ? v[k + o] : v[k], send = up ? v[k] : v[k + o];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    if (N == 16) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
+    return v[0];
+}
+// f(k, sum of a[k] over the warp) for k < NC, called by one lane for each k
+template <int NC, int BASE = 0, class T, class F>
+__device__ __forceinline__ void warp_coeffs(const T *a, const F &f) {
+    constexpr int N = NC - BASE > 16 ? 32 : 16;
+    const int lane = threadIdx.x & 31;
+    T v[N];
+#pragma unroll
+    for (int k = 0; k < N; k++) v[k] = BASE + k < NC ? a[BASE + k] : T(0);
+    const T s = warp_scatter_sum<N>(v);
+    if (lane < N && BASE + lane < NC) f(BASE + lane, s);
+    if constexpr (BASE + N < NC) warp_coeffs<NC, BASE + N>(a, f);
+}
+// coefficient k = gx_mi(i, j)
+__device__ __forceinline__ void mi_split(int k, int &i, int &j) {
+    int n = 0;
+    while ((n + 1) * (n + 2) / 2 <= k) n++;
+    j = k - n * (n + 1) / 2;
+    i = n - j;
+}
+
 // FP32 reciprocal square root as the single PTX instruction rsqrt.approx.ftz.f32:
 // the arguments here are r^2 + eps^2 > 0, far from the denormal range, so the
 // denormal handling the library function adds around it is dead weight.
@@ -233,12 +272,16 @@ __global__ void k_prepare_from(int64_t n, const double *__restrict__ hx, const d
 }
 
 // ---------------------------------------------------------------- P2M
+// The evaluation's first kernel when the leaves hold every body: it also sanitises the
+// inputs (lib.rs:1474-1482, as k_prepare), reading them from the caller's page-locked arrays
+// (hx, hy, hm, then stored) where there are some; the final sum writes every a, so none is
+// zeroed.  A warp per leaf, a lane per body; the moments are summed by reduce-scatter.
 template <int P, class T>
-__global__ void __launch_bounds__(128) k_p2m(int64_t nl, const double *__restrict__ x, const double *__restrict__ y,
-                                             const double *__restrict__ m, const double *__restrict__ comx,
-                                             const double *__restrict__ comy, const int32_t *__restrict__ bs,
-                                             const int32_t *__restrict__ be, T *__restrict__ M,
-                                             float4 *__restrict__ pos) {
+__global__ void __launch_bounds__(128) k_p2m(int64_t nl, const double *__restrict__ hx, const double *__restrict__ hy,
+                                             const double *__restrict__ hm, double *x, double *y, double *m,
+                                             const double *__restrict__ comx, const double *__restrict__ comy,
+                                             const int32_t *__restrict__ bs, const int32_t *__restrict__ be,
+                                             T *__restrict__ M, float4 *__restrict__ pos, unsigned *status) {
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<T>(NC);
     const int PP = gx_rt_order(P);
@@ -253,27 +296,39 @@ __global__ void __launch_bounds__(128) k_p2m(int64_t nl, const double *__restric
 #pragma unroll
     for (int k = 0; k < NCr; k++) acc[k] = T(0);
     for (int32_t b = b0 + lane; b < b1; b += 32) {
-        T dx = (T)(x[b] - cxl), dy = (T)(y[b] - cyl), mm = (T)m[b];
-        if (pos) pos[b] = make_float4((float)dx, (float)dy, (float)m[b], 0.f);
-        T px[P + 1], py[P + 1];
-        px[0] = T(1);
+        double xb = hx ? hx[b] : x[b], yb = hx ? hy[b] : y[b], mb = hx ? hm[b] : m[b];
+        bool bad = false;
+        if (fabs(xb) > 1e100 || fabs(yb) > 1e100 || !isfinite(xb) || !isfinite(yb)) {
+            xb = 0.0;
+            yb = 0.0;
+            bad = true;
+        }
+        if (!isfinite(mb) || mb <= 0.0) {
+            mb = 1.0;
+            bad = true;
+        }
+        if (hx || bad) {
+            x[b] = xb;
+            y[b] = yb;
+            m[b] = mb;
+        }
+        if (bad) atomicOr(status, GX_DEV_NONFINITE_INPUT);
+        T dx = (T)(xb - cxl), dy = (T)(yb - cyl), mm = (T)mb;
+        if (pos) pos[b] = make_float4((float)dx, (float)dy, (float)mb, 0.f);
+        T px[P + 1], py[P + 1];  // m dx^k / k!, dy^k / k!
+        px[0] = mm;
         py[0] = T(1);
 #pragma unroll
         for (int k = 1; k <= PP; k++) {
-            px[k] = px[k - 1] * dx;
-            py[k] = py[k - 1] * dy;
+            px[k] = px[k - 1] * (dx * tab_inv<T>(k));
+            py[k] = py[k - 1] * (dy * tab_inv<T>(k));
         }
 #pragma unroll
         for (int i = 0; i <= PP; i++)
 #pragma unroll
-            for (int j = 0; j <= PP - i; j++)
-                acc[gx_mi(i, j)] += mm * px[i] * py[j] * tab_ifp<T>(i, j);
+            for (int j = 0; j <= PP - i; j++) acc[gx_mi(i, j)] += px[i] * py[j];
     }
-#pragma unroll
-    for (int k = 0; k < NCr; k++) {
-        T v = warp_sum_t<T>(acc[k]);
-        if (lane == (k & 31)) M[leaf * NS + k] = isfinite(v) ? v : T(0);
-    }
+    warp_coeffs<NC>(acc, [&](int k, T v) { M[leaf * NS + k] = isfinite(v) ? v : T(0); });
 }
 
 // ---------------------------------------------------------------- M2M (and L2L^T)
@@ -805,27 +860,47 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && P <= 4) ? 8 : 1) k_m2l
     for (int k = 0; k < NCr; k++) acc[k] = T(0);
     m2l_sources<P, T, IDX>(idx, st, len, lane, comx[node], comy[node], thl, comx, comy, comhl, (T)eps2d, M, acc);
     // G = -A: L[T] = -(1/T!) sum_S M'[S] A[S+T]
-#pragma unroll
-    for (int oi = 0; oi <= PP; oi++)
-#pragma unroll
-        for (int oj = 0; oj <= PP - oi; oj++) {
-            int k = gx_mi(oi, oj);
-            T v = warp_sum_t<T>(acc[k]);
-            if (lane == (k & 31)) L[node * NS + k] = v * -tab_ifp<T>(oi, oj);
-        }
+    warp_coeffs<NC>(acc, [&](int k, T v) {
+        int i, j;
+        mi_split(k, i, j);
+        L[node * NS + k] = v * -tab_ifp<T>(i, j);
+    });
+}
+
+// A node cut into several units: each warp leaves its unit's sums in part and counts itself
+// off; the one that comes last (no warp waits for another) has all of them and adds them in
+// unit order, so the result does not depend on which one that is.  count is zero before and
+// after.  Calls store(k, sum) for the node's coefficients.
+template <int NC, int NS, class T, class F>
+__device__ __forceinline__ void last_unit_sums(int64_t node, int64_t u0, int64_t u1, const T *part, unsigned *count,
+                                               const F &store) {
+    const int lane = threadIdx.x & 31;
+    __threadfence();
+    __syncwarp();
+    unsigned before = 0;
+    if (lane == 0) before = atomicAdd(&count[node], 1u);
+    before = __shfl_sync(0xffffffffu, before, 0);
+    if (before + 1 != (unsigned)(u1 - u0)) return;
+    __threadfence();
+    for (int k = lane; k < NC; k += 32) {
+        T s = T(0);
+#pragma unroll 4
+        for (int64_t u = u0; u < u1; u++) s += __ldcg(part + u * NS + k);
+        store(k, s);
+    }
+    if (lane == 0) count[node] = 0;
 }
 
 // ACCURATE M2L over work units: every far list is cut into units of at most
 // GX_M2L_UNIT sources (one warp each), so a node near the centre of a wide halo, with
 // tens of thousands of far sources, is spread over many warps instead of running as
-// one straggler.  A node with one unit writes its local directly; otherwise each unit
-// writes its warp-reduced partial and k_m2l_combine sums them in unit order.
+// one straggler.  A node with one unit writes its local directly, the others as above.
 template <int P, class T>
 __global__ void __launch_bounds__(128, (sizeof(T) == 4 && P <= 4) ? 8 : 1) k_m2l_units(
     int64_t n_units, const int32_t *__restrict__ unode, const int64_t *__restrict__ ustart,
     const int32_t *__restrict__ ulen, const int64_t *__restrict__ node_u, const int32_t *__restrict__ idx,
     const double *__restrict__ comx, const double *__restrict__ comy, const float4 *__restrict__ comhl, double eps2d,
-    const T *__restrict__ M, T *__restrict__ L, T *__restrict__ part) {
+    const T *__restrict__ M, T *__restrict__ L, T *part, unsigned *count) {
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<T>(NC);
     const int PP = gx_rt_order(P);
@@ -835,7 +910,6 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && P <= 4) ? 8 : 1) k_m2l
     int lane = threadIdx.x & 31;
     if (u >= n_units) return;
     const int64_t node = unode[u];
-    const bool single = node_u[node + 1] - node_u[node] == 1;
     float4 thl = make_float4(0.f, 0.f, 0.f, 0.f);
     if constexpr (sizeof(T) == 4) thl = comhl[node];
     T acc[NC];
@@ -843,108 +917,141 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && P <= 4) ? 8 : 1) k_m2l
     for (int k = 0; k < NCr; k++) acc[k] = T(0);
     m2l_sources<P, T, int32_t>(idx, ustart[u], ulen[u], lane, comx[node], comy[node], thl, comx, comy, comhl,
                                (T)eps2d, M, acc);
-#pragma unroll
-    for (int oi = 0; oi <= PP; oi++)
-#pragma unroll
-        for (int oj = 0; oj <= PP - oi; oj++) {
-            int k = gx_mi(oi, oj);
-            T v = warp_sum_t<T>(acc[k]);
-            if (lane == (k & 31)) {
-                if (single) L[node * NS + k] = v * -tab_ifp<T>(oi, oj);
-                else part[u * NS + k] = v;
-            }
-        }
-}
-
-// Nodes cut into several M2L units: the local is the sum of the units' partials in
-// unit order.  One thread per (node, coefficient).
-template <int P, class T>
-__global__ void k_m2l_combine(int64_t nn, const int64_t *__restrict__ node_u, const T *__restrict__ part,
-                              T *__restrict__ L) {
-    constexpr int NC = nc2(P);
-    constexpr int NS = row_stride<T>(NC);
-    const int PP = gx_rt_order(P);
-    const int NCr = (PP + 1) * (PP + 2) / 2;
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int64_t node = t / NC;
-    int k = (int)(t - node * NC);
-    if (node >= nn || k >= NCr) return;
-    int64_t u0 = node_u[node], u1 = node_u[node + 1];
-    if (u1 - u0 < 2) return;
-    T s = T(0);
-    for (int64_t u = u0; u < u1; u++) s += part[u * NS + k];
-    int n = 0;  // coefficient k = gx_mi(oi, oj): n(n+1)/2 + oj with n = oi + oj
-    while ((n + 1) * (n + 2) / 2 <= k) n++;
-    const int oj = k - n * (n + 1) / 2, oi = n - oj;
-    L[node * NS + k] = s * -tab_ifp<T>(oi, oj);
+    const int64_t u0 = node_u[node], u1 = node_u[node + 1];
+    const auto store = [&](int k, T v) {
+        int i, j;
+        mi_split(k, i, j);
+        L[node * NS + k] = v * -tab_ifp<T>(i, j);
+    };
+    if (u1 - u0 == 1) {
+        warp_coeffs<NC>(acc, store);
+    } else {
+        warp_coeffs<NC>(acc, [&](int k, T v) { part[u * NS + k] = v; });
+        last_unit_sums<NC, NS>(node, u0, u1, part, count, store);
+    }
 }
 
 // ---------------------------------------------------------------- L2L
-// L_c[I,J] += sum_{i>=I, j>=J} L_P[i,j] C(i,I) C(j,J) dx^(i-I) dy^(j-J), one thread per child.
+// c[I,J] = sum_{i>=I, j>=J} c[i,j] dx^(i-I)/(i-I)! dy^(j-J)/(j-J)! in place, one axis at a
+// time (ascending: the higher terms are still the old ones).
 template <int P, class T>
-__device__ __forceinline__ void l2l_shift(const T *__restrict__ LP, T dx, T dy, T *out) {
+__device__ __forceinline__ void shift_down(T dx, T dy, T *c) {
     const int PP = gx_rt_order(P);
-    T px[P + 1], py[P + 1];
-    px[0] = T(1);
-    py[0] = T(1);
+    T pw[P + 1];
+    pw[0] = T(1);
 #pragma unroll
-    for (int q = 1; q <= PP; q++) {
-        px[q] = px[q - 1] * dx;
-        py[q] = py[q - 1] * dy;
-    }
-    T lp[nc2(P)];
-    load_row<nc2(P)>(LP, lp);
+    for (int k = 1; k <= PP; k++) pw[k] = pw[k - 1] * (dy * tab_inv<T>(k));
 #pragma unroll
-    for (int oi = 0; oi <= PP; oi++)
+    for (int i = 0; i <= PP; i++)
 #pragma unroll
-        for (int oj = 0; oj <= PP - oi; oj++) {
-            T sum = T(0);
+        for (int J = 0; J < PP - i; J++)
 #pragma unroll
-            for (int i = oi; i <= PP; i++)
+            for (int j = J + 1; j <= PP - i; j++) c[gx_mi(i, J)] += c[gx_mi(i, j)] * pw[j - J];
 #pragma unroll
-                for (int j = oj; j <= PP - i; j++)
-                    sum += lp[gx_mi(i, j)] * (tab_binom<T>(i, oi) * tab_binom<T>(j, oj)) * px[i - oi] * py[j - oj];
-            out[gx_mi(oi, oj)] += sum;
-        }
+    for (int k = 1; k <= PP; k++) pw[k] = pw[k - 1] * (dx * tab_inv<T>(k));
+#pragma unroll
+    for (int J = 0; J <= PP; J++)
+#pragma unroll
+        for (int I = 0; I < PP - J; I++)
+#pragma unroll
+            for (int i = I + 1; i <= PP - J; i++) c[gx_mi(I, J)] += c[gx_mi(i, J)] * pw[i - I];
+}
+// A local's row with its coefficients times i! j!: there L2L,
+//   L_c[I,J] = sum_{i>=I, j>=J} L_P[i,j] C(i,I) C(j,J) dx^(i-I) dy^(j-J),
+// is shift_down.
+template <int P, class T>
+__device__ __forceinline__ void load_local(const T *__restrict__ row, T *c) {
+    const int PP = gx_rt_order(P);
+    load_row<nc2(P)>(row, c);
+#pragma unroll
+    for (int i = 0; i <= PP; i++)
+#pragma unroll
+        for (int j = 0; j <= PP - i; j++)
+            if (i > 1 || j > 1) c[gx_mi(i, j)] *= tab_ff<T>(i, j);
 }
 
-// Top-down modes: only the leaves' locals are consumed (by L2P), and translating a
-// local expansion is exact for polynomials, so shifting every ancestor's M2L local
-// straight to the leaf equals the level-by-level L2L chain.  One warp per leaf, one
-// lane per ancestor (from the ancestor table anc[level * nl + leaf]), then a warp
-// reduction: a single launch instead of one per level.  Ancestors without far
-// interactions (has_far = 0) hold a zero local and are skipped.
+// L2P (lib.rs:1321-1345) for one body at (du, dv) from the leaf COM: the gradient of the
+// local polynomial, by Horner in u for every power of v and in v over those.
 template <int P, class T>
-__global__ void __launch_bounds__(128) k_l2l_direct(int64_t nl, int n_levels, const int32_t *__restrict__ anc,
+__device__ __forceinline__ void l2p_eval(const T *__restrict__ Ll, T du, T dv, T &fx, T &fy) {
+    const int PP = gx_rt_order(P);
+    T q = T(0), qy = T(0), qx = T(0);
+#pragma unroll
+    for (int b = PP; b >= 0; b--) {
+        T s = Ll[gx_mi(PP - b, b)], d = T(0);
+#pragma unroll
+        for (int a = PP - b - 1; a >= 0; a--) {
+            d = d * du + s;
+            s = s * du + Ll[gx_mi(a, b)];
+        }
+        qy = qy * dv + q;
+        q = q * dv + s;
+        qx = qx * dv + d;
+    }
+    fx = qx;
+    fy = qy;
+}
+
+// The leaves' locals, top-down modes: only they are consumed (by L2P), and translating a
+// local expansion is exact for polynomials, so every ancestor's M2L local is shifted straight
+// to the leaf, which equals the level-by-level chain.  One warp per leaf, a lane per ancestor
+// (the table anc[level * nl + leaf]; ancestors without far interactions, has_far = 0, hold no
+// local), summed by reduce-scatter; the P2L units of the leaf (u0 .. u1, then the body-level
+// ones) are subtracted in unit order; and in the mixed form L2P of the leaf's bodies follows
+// from the local still in shared memory (fl: their (fx, fy)).  One launch and one pass over
+// the locals for what were three kernels.  With P2L off the main stream, the inputs sanitised
+// by P2M and the unit sums of M2L in its own kernel, ten leapfrog steps at N = 10,000 went from 1.24
+// to 0.87 ms and the evaluation at 1M (host arrays in and out) from 2.52 to 2.40 ms.
+template <int P, class T>
+__global__ void __launch_bounds__(128) k_leaf_local(int64_t nl, int n_levels, const int32_t *__restrict__ anc,
                                                     const uint8_t *__restrict__ has_far, const double *__restrict__ comx,
                                                     const double *__restrict__ comy, const T *__restrict__ L,
-                                                    T *__restrict__ Lout) {
+                                                    const int64_t *__restrict__ leaf_u,
+                                                    const int64_t *__restrict__ body_u, int64_t n_leafu,
+                                                    const T *__restrict__ ppart, T *__restrict__ Lout,
+                                                    const float4 *__restrict__ pos, const int32_t *__restrict__ bs,
+                                                    const int32_t *__restrict__ be, float2 *__restrict__ fl) {
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<T>(NC);
     const int PP = gx_rt_order(P);
     const int NCr = (PP + 1) * (PP + 2) / 2;
-    int lane = threadIdx.x & 31;
-    int64_t leaf = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    __shared__ T sl[4][NC];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t leaf = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (leaf >= nl) return;
     T out[NC];
 #pragma unroll
     for (int k = 0; k < NCr; k++) out[k] = T(0);
     for (int j = lane; j < n_levels; j += 32) {
-        int32_t a = anc[(int64_t)j * nl + leaf];
+        const int32_t a = anc[(int64_t)j * nl + leaf];
         if (a < 0 || !has_far[a]) continue;
-        if (a == (int32_t)leaf) {
-            T own[NC];
-            load_row<NC>(L + leaf * NS, own);
+        T c[NC];
+        load_local<P, T>(L + (int64_t)a * NS, c);
+        if (a != (int32_t)leaf) shift_down<P, T>((T)(comx[leaf] - comx[a]), (T)(comy[leaf] - comy[a]), c);
 #pragma unroll
-            for (int k = 0; k < NCr; k++) out[k] += own[k];
-        } else {
-            l2l_shift<P, T>(L + (int64_t)a * NS, (T)(comx[leaf] - comx[a]), (T)(comy[leaf] - comy[a]), out);
-        }
+        for (int k = 0; k < NCr; k++) out[k] += c[k];
     }
-#pragma unroll
-    for (int k = 0; k < NCr; k++) {
-        T v = warp_sum_t<T>(out[k]);
-        if (lane == (k & 31)) Lout[leaf * NS + k] = v;
+    const int64_t u0 = leaf_u ? leaf_u[leaf] : 0, u1 = leaf_u ? leaf_u[leaf + 1] : 0;
+    const int64_t b0 = body_u ? n_leafu + body_u[leaf] : 0, b1 = body_u ? n_leafu + body_u[leaf + 1] : 0;
+    warp_coeffs<NC>(out, [&](int k, T v) {
+        int i, j;
+        mi_split(k, i, j);
+        v *= tab_ifp<T>(i, j);
+        T s = T(0);
+        for (int64_t q = u0; q < u1; q++) s += ppart[q * NS + k];
+        for (int64_t q = b0; q < b1; q++) s += ppart[q * NS + k];
+        v -= s;
+        Lout[leaf * NS + k] = v;
+        sl[w][k] = v;
+    });
+    if (!fl) return;
+    __syncwarp();
+    const int32_t t1 = be[leaf];
+    for (int32_t i = bs[leaf] + lane; i < t1; i += 32) {
+        const float4 me = pos[i];
+        T fx, fy;
+        l2p_eval<P, T>(sl[w], (T)me.x, (T)me.y, fx, fy);
+        fl[i] = make_float2((float)fx, (float)fy);
     }
 }
 
@@ -956,17 +1063,24 @@ __global__ void __launch_bounds__(128) k_l2l_ref_leaves(int64_t nl, const int32_
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<T>(NC);
     const int PP = gx_rt_order(P);
-    const int NCr = (PP + 1) * (PP + 2) / 2;
     int64_t leaf = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (leaf >= nl) return;
-    int32_t par = parent[leaf];
-    T out[NC];
+    const int32_t par = parent[leaf];
+    T c[NC];
 #pragma unroll
-    for (int k = 0; k < NCr; k++) out[k] = L[leaf * NS + k];
-    if (par >= 0)
-        l2l_shift<P, T>(L + (int64_t)par * NS, (T)(comx[leaf] - comx[par]), (T)(comy[leaf] - comy[par]), out);
+    for (int k = 0; k < NC; k++) c[k] = T(0);
+    if (par >= 0) {
+        load_local<P, T>(L + (int64_t)par * NS, c);
+        shift_down<P, T>((T)(comx[leaf] - comx[par]), (T)(comy[leaf] - comy[par]), c);
+    }
 #pragma unroll
-    for (int k = 0; k < NCr; k++) Lout[leaf * NS + k] = out[k];
+    for (int i = 0; i <= PP; i++)
+#pragma unroll
+        for (int j = 0; j <= PP - i; j++) {
+            const int k = gx_mi(i, j);
+            const T own = L[leaf * NS + k];
+            Lout[leaf * NS + k] = par >= 0 ? own + c[k] * tab_ifp<T>(i, j) : own;
+        }
 }
 
 // ---------------------------------------------------------------- L2P + P2P
@@ -977,32 +1091,6 @@ __global__ void __launch_bounds__(128) k_l2l_ref_leaves(int64_t nl, const int32_
 // load is issued before the current leaf is computed, so its latency is hidden.
 // The target leaf itself is handled in a separate branch (i == j is skipped there),
 // keeping the common loop free of the self test.
-
-// L2P (lib.rs:1321-1345) for one body at (du, dv) from the leaf COM
-template <int P, class T>
-__device__ __forceinline__ void l2p_eval(const T *__restrict__ Ll, T du, T dv, T &fx, T &fy) {
-    const int PP = gx_rt_order(P);
-    const int NCr = (PP + 1) * (PP + 2) / 2;
-    (void)NCr;
-    T px[P + 1], py[P + 1];
-    px[0] = T(1);
-    py[0] = T(1);
-#pragma unroll
-    for (int q = 1; q <= PP; q++) {
-        px[q] = px[q - 1] * du;
-        py[q] = py[q - 1] * dv;
-    }
-    fx = T(0);
-    fy = T(0);
-#pragma unroll
-    for (int a = 0; a <= PP; a++)
-#pragma unroll
-        for (int b = 0; b <= PP - a; b++) {
-            T c = Ll[gx_mi(a, b)];
-            if (a >= 1) fx += c * (T)a * px[a - 1] * py[b];
-            if (b >= 1) fy += c * (T)b * px[a] * py[b - 1];
-        }
-}
 
 // Work items: the source list of every target leaf is cut into items of at most
 // P2P_K source leaves; one warp per item writes per-body partial accelerations to
@@ -1960,11 +2048,10 @@ constexpr int P2L_RING = 4;  // rounds of P2L source bodies in flight per warp (
 template <int P>
 __global__ void __launch_bounds__(128, 6) k_p2l_x2(int64_t n_units, const int32_t *__restrict__ uleaf,
                                                 const int64_t *__restrict__ ustart, const int32_t *__restrict__ ulen,
-                                                const int64_t *__restrict__ leaf_u, const int64_t *__restrict__ body_u,
                                                 const int32_t *__restrict__ src_idx, const float4 *__restrict__ pos,
                                                 const double *__restrict__ comx, const double *__restrict__ comy,
                                                 const int32_t *__restrict__ bs, const int32_t *__restrict__ be,
-                                                float eps2, float *__restrict__ Lf, float *__restrict__ ppart) {
+                                                float eps2, float *__restrict__ ppart) {
     static_assert(P <= 5, "paired accumulators are sized for p <= 5");
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<float>(NC);
@@ -2045,17 +2132,14 @@ __global__ void __launch_bounds__(128, 6) k_p2l_x2(int64_t n_units, const int32_
         }
     }
     cp_async_wait<0>();
-    const bool single = (leaf_u[a + 1] - leaf_u[a]) + (body_u ? body_u[a + 1] - body_u[a] : 0) == 1;
+    float sum[NC];
 #pragma unroll
     for (int q = 0; q < NC; q++) {
         float lo, hi;
         upk2(acc[q].v, lo, hi);
-        const float v = warp_sum_t<float>(lo + hi);
-        if (lane == (q & 31)) {
-            if (single) Lf[(int64_t)a * NS + q] -= v;
-            else ppart[u * NS + q] = v;
-        }
+        sum[q] = lo + hi;
     }
+    warp_coeffs<NC>(sum, [&](int q, float v) { ppart[u * NS + q] = v; });
 }
 
 // Body-level P2L units, mixed form, p <= 5: a unit is up to GX_BODY_UNIT consecutive
@@ -2064,20 +2148,17 @@ __global__ void __launch_bounds__(128, 6) k_p2l_x2(int64_t n_units, const int32_
 // its masked bodies to the unit's stream in shared memory (entry (row << 5) | body, row
 // and body order).  The stream is taken two bodies per lane, 64 at a time (positions
 // c + lane and c + 32 + lane), each with its row's com_a - com_s; a padding slot has zero
-// mass at a unit offset.  Writes like k_p2l_x2 (the leaf's units are summed in unit
-// order, or a leaf with one unit subtracts its sum from its local directly).
+// mass at a unit offset.  Writes the unit's partial like k_p2l_x2.
 template <int P>
 __global__ void __launch_bounds__(128, 6) k_p2l_body_x2(int64_t u_base, int64_t n_units,
                                                      const int32_t *__restrict__ uleaf,
                                                      const int64_t *__restrict__ ustart,
                                                      const int32_t *__restrict__ ulen,
-                                                     const int64_t *__restrict__ leaf_u,
-                                                     const int64_t *__restrict__ body_u,
                                                      const int32_t *__restrict__ src_idx,
                                                      const uint32_t *__restrict__ p2p_mask,
                                                      const float4 *__restrict__ pos, const double *__restrict__ comx,
                                                      const double *__restrict__ comy, const int32_t *__restrict__ bs,
-                                                     float eps2, float *__restrict__ Lf, float *__restrict__ ppart) {
+                                                     float eps2, float *__restrict__ ppart) {
     static_assert(P <= 5, "paired accumulators are sized for p <= 5");
     static_assert(GX_BODY_UNIT % 32 == 0 && GX_BODY_UNIT * 32 <= 65536, "whole rows per lane, 16-bit entries");
     constexpr int RPL = GX_BODY_UNIT / 32;  // rows per lane
@@ -2178,24 +2259,21 @@ __global__ void __launch_bounds__(128, 6) k_p2l_body_x2(int64_t u_base, int64_t 
         oA = pA;
         oB = pB;
     }
-    const bool single = (leaf_u[a + 1] - leaf_u[a]) + (body_u ? body_u[a + 1] - body_u[a] : 0) == 1;
+    float sum[NC];
 #pragma unroll
     for (int q = 0; q < NC; q++) {
         float lo, hi;
         upk2(acc[q].v, lo, hi);
-        const float v = warp_sum_t<float>(lo + hi);
-        if (lane == (q & 31)) {
-            if (single) Lf[(int64_t)a * NS + q] -= v;
-            else ppart[u * NS + q] = v;
-        }
+        sum[q] = lo + hi;
     }
+    warp_coeffs<NC>(sum, [&](int q, float v) { ppart[u * NS + q] = v; });
 }
 
 // P2L units: one warp per unit (a target leaf and at most GX_P2L_UNIT of its P2L source
 // leaves), lane per source body.  L_a[T] += m_j G^(T)(com_a - x_j) / T! = -m_j a_T(com_a - x_j),
-// summed per lane in body order, then over the warp; a leaf with one unit subtracts the
-// sum from its local directly, otherwise the unit writes a partial and k_p2l_combine
-// adds the partials in unit order.  Runs after L2L (the leaf locals exist) and before L2P.
+// summed per lane in body order, then over the warp, into the unit's partial; k_leaf_local
+// subtracts a leaf's partials in unit order.  Needs nothing but the bodies, so the units run
+// on a stream of their own beside M2M and M2L.
 // Lane q holds source q's body range and COM offset (one load round for the unit); the
 // bodies of the next source are requested before the current ones are used.
 template <int P, class T>
@@ -2222,14 +2300,13 @@ __device__ __forceinline__ void p2l_body(T dx, T dy, T mj, T eps2, T *acc) {
 template <int P, class T>
 __global__ void __launch_bounds__(128) k_p2l(int64_t n_units, const int32_t *__restrict__ uleaf,
                                              const int64_t *__restrict__ ustart, const int32_t *__restrict__ ulen,
-                                             const int64_t *__restrict__ leaf_u, const int64_t *__restrict__ body_u,
                                              const int32_t *__restrict__ src_idx,
                                              const float4 *__restrict__ pos, const double *__restrict__ X,
                                              const double *__restrict__ Y, const double *__restrict__ Mb,
                                              const double *__restrict__ comx, const double *__restrict__ comy,
                                              const int32_t *__restrict__ bs, const int32_t *__restrict__ be, T eps2,
                                              const uint32_t *__restrict__ p2p_mask, int body_units,
-                                             T *__restrict__ Lf, T *__restrict__ ppart) {
+                                             T *__restrict__ ppart) {
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<T>(NC);
     const int PP = gx_rt_order(P);
@@ -2316,36 +2393,7 @@ __global__ void __launch_bounds__(128) k_p2l(int64_t n_units, const int32_t *__r
             cm = nm;
         }
     }
-    const bool single = (leaf_u[a + 1] - leaf_u[a]) + (body_u ? body_u[a + 1] - body_u[a] : 0) == 1;
-#pragma unroll
-    for (int k = 0; k < NCr; k++) {
-        const T v = warp_sum_t<T>(acc[k]);
-        if (lane == (k & 31)) {
-            if (single) Lf[(int64_t)a * NS + k] -= v;
-            else ppart[u * NS + k] = v;
-        }
-    }
-}
-
-// Leaves with several P2L units: the partials in unit order, subtracted from the local.
-template <int P, class T>
-__global__ void k_p2l_combine(int64_t nl, const int64_t *__restrict__ leaf_u, const int64_t *__restrict__ body_u,
-                              int64_t n_leafu, const T *__restrict__ ppart, T *__restrict__ Lf) {
-    constexpr int NC = nc2(P);
-    constexpr int NS = row_stride<T>(NC);
-    const int PP = gx_rt_order(P);
-    const int NCr = (PP + 1) * (PP + 2) / 2;
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t a = t / NC;
-    const int k = (int)(t - a * NC);
-    if (a >= nl || k >= NCr) return;
-    const int64_t u0 = leaf_u[a], u1 = leaf_u[a + 1];
-    const int64_t b0 = body_u ? n_leafu + body_u[a] : 0, b1 = body_u ? n_leafu + body_u[a + 1] : 0;
-    if ((u1 - u0) + (b1 - b0) < 2) return;
-    T s = T(0);
-    for (int64_t q = u0; q < u1; q++) s += ppart[q * NS + k];  // leaf-level units, then body-level ones
-    for (int64_t q = b0; q < b1; q++) s += ppart[q * NS + k];
-    Lf[a * NS + k] -= s;
+    warp_coeffs<NC>(acc, [&](int k, T v) { ppart[u * NS + k] = v; });
 }
 
 // Folding of long item ranges.  A wide halo leaf can have ~1000 P2P items (977 at 1M
@@ -2485,29 +2533,10 @@ __global__ void __launch_bounds__(128) k_l2p_reduce64(int64_t nl, const double *
     }
 }
 
-// Mixed form, in two kernels: the L2P of every body on the main stream while the near
-// field still runs (fl = the local expansion's (fx, fy) in FP32), and after the join the
-// ordered sum of the P2P partials, a = sum - f in FP64.  The sum kernel has nothing but
-// its loads to wait for, so more of its warps are resident and its loads (the leaf's
-// item range, then the partials and fl together) are two dependent rounds.
-template <int P>
-__global__ void __launch_bounds__(128) k_l2p32(int64_t nl, const float4 *__restrict__ pos,
-                                               const int32_t *__restrict__ bs, const int32_t *__restrict__ be,
-                                               const float *__restrict__ Lf, float2 *__restrict__ fl) {
-    constexpr int NC = nc2(P);
-    constexpr int NS = row_stride<float>(NC);
-    int lane = threadIdx.x & 31;
-    int64_t leaf = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (leaf >= nl) return;
-    int32_t t0 = bs[leaf], t1 = be[leaf];
-    for (int32_t i = t0 + lane; i < t1; i += 32) {
-        float4 me = pos[i];
-        float fx, fy;
-        l2p_eval<P, float>(Lf + leaf * NS, me.x, me.y, fx, fy);
-        fl[i] = make_float2(fx, fy);
-    }
-}
-
+// Mixed form: L2P has run with the leaves' locals (k_leaf_local) beside the near field; after
+// the join only the ordered sum of the P2P partials is left, a = sum - f in FP64.  The kernel
+// has nothing but its loads to wait for, so more of its warps are resident and its loads (the
+// leaf's item range, then the partials and fl together) are two dependent rounds.
 __global__ void __launch_bounds__(128) k_reduce32(int64_t nl, const int32_t *__restrict__ bs,
                                                   const int32_t *__restrict__ be, const int64_t *__restrict__ item_off,
                                                   int tchunks, const float2 *__restrict__ part,
@@ -2555,14 +2584,20 @@ int run_forces(gx_ctx *ctx, bool timed) {
     Timer tm{ctx, timed};
     int64_t launches0 = ctx->launches;
     tm.mark();  // 0
-    if (ctx->in_x)
-        k_prepare_from<<<gx_blocks(n, 256), 256, 0, st>>>(n, ctx->in_x, ctx->in_y, ctx->in_m, dptr<double>(ctx->x),
-                                                          dptr<double>(ctx->y), dptr<double>(ctx->m), dptr<double>(ctx->ax),
-                                                          dptr<double>(ctx->ay), dptr<unsigned>(ctx->status));
-    else
-        k_prepare<<<gx_blocks(n, 256), 256, 0, st>>>(n, dptr<double>(ctx->x), dptr<double>(ctx->y), dptr<double>(ctx->m),
-                                                     dptr<double>(ctx->ax), dptr<double>(ctx->ay), dptr<unsigned>(ctx->status));
-    ctx->launches++;
+    // where the leaves do not hold every body (an uploaded tree may leave some out), a kernel
+    // of its own sanitises them all and zeroes their a; else P2M does the first on its way
+    const bool apart = nn == 0 || !ctx->leaves_cover;
+    if (apart) {
+        if (ctx->in_x)
+            k_prepare_from<<<gx_blocks(n, 256), 256, 0, st>>>(
+                n, ctx->in_x, ctx->in_y, ctx->in_m, dptr<double>(ctx->x), dptr<double>(ctx->y), dptr<double>(ctx->m),
+                dptr<double>(ctx->ax), dptr<double>(ctx->ay), dptr<unsigned>(ctx->status));
+        else
+            k_prepare<<<gx_blocks(n, 256), 256, 0, st>>>(n, dptr<double>(ctx->x), dptr<double>(ctx->y),
+                                                         dptr<double>(ctx->m), dptr<double>(ctx->ax),
+                                                         dptr<double>(ctx->ay), dptr<unsigned>(ctx->status));
+        ctx->launches++;
+    }
     tm.mark();  // 1
     if (nn == 0) {
         GX_CUDA(ctx, cudaGetLastError());
@@ -2599,13 +2634,16 @@ int run_forces(gx_ctx *ctx, bool timed) {
             pos = dptr<float4>(ctx->pos32);
         }
         // P2M (+ FP32 body packing in the mixed form)
-        k_p2m<P, T><<<gw, 128, 0, st>>>(nl, X, Y, Mb, comx, comy, bs, be, M, pos);
+        k_p2m<P, T><<<gw, 128, 0, st>>>(nl, apart ? nullptr : ctx->in_x, ctx->in_y, ctx->in_m, dptr<double>(ctx->x),
+                                        dptr<double>(ctx->y), dptr<double>(ctx->m), comx, comy, bs, be, M, pos,
+                                        dptr<unsigned>(ctx->status));
         ctx->launches++;
         tm.mark();  // 2
-        // near field on the second stream, beside M2M -> M2L -> L2L on this one: both
-        // are FP32-pipe bound but neither fills it alone (latency, occupancy), and
+        // near field on the second stream and P2L on a third, beside M2M -> M2L -> L2L on
+        // this one: all are FP32-pipe bound but none fills it alone (latency, occupancy), and
         // their blocks share the SMs.  Deterministic: P2P writes per-item partials
-        // that L2P sums in order after the join.
+        // that the final sum adds in order after the join, P2L per-unit ones for the leaves'
+        // locals.
         const size_t pbytes = (mixed ? sizeof(float2) : sizeof(double2)) * 32 * (size_t)tchunks * (size_t)(I.n + 1);
         GX_TRY(gx_ensure(ctx, ctx->part, pbytes));
         auto near_field = [&]() -> int {
@@ -2676,9 +2714,46 @@ int run_forces(gx_ctx *ctx, bool timed) {
         GX_CUDA(ctx, cudaEventRecord(ctx->ev_join, ctx->stream2));
         return GX_OK;
         };
+        // P2L of the near-list split (leaf-level units, then the body-level ones)
+        const gx_ctx::P2LUnits &PU = ctx->p2l_units;
+        const bool p2l = split && PU.n > 0;
+        if (p2l) GX_TRY(gx_ensure(ctx, ctx->p2l_part, sizeof(T) * NS * (size_t)(PU.n + 1)));
+        auto p2l_field = [&](cudaStream_t sp) -> int {
+            bool packed = false;
+            if constexpr (P <= 5 && sizeof(T) == 4) {
+                if (PU.n_leafu > 0) {
+                    k_p2l_x2<P><<<gx_blocks(PU.n_leafu * 32, 128), 128, 0, sp>>>(
+                        PU.n_leafu, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start), dptr<int32_t>(PU.len), src_idx,
+                        pos, comx, comy, bs, be, (float)eps2, dptr<float>(ctx->p2l_part));
+                    ctx->launches++;
+                }
+                if (body && PU.n_body > 0) {
+                    k_p2l_body_x2<P><<<gx_blocks(PU.n_body * 32, 128), 128, 0, sp>>>(
+                        PU.n_leafu, PU.n_body, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start),
+                        dptr<int32_t>(PU.len), src_idx, p2p_mask, pos, comx, comy, bs, (float)eps2,
+                        dptr<float>(ctx->p2l_part));
+                    ctx->launches++;
+                }
+                packed = true;
+            }
+            if (!packed) {
+                k_p2l<P, T><<<gx_blocks(PU.n * 32, 128), 128, 0, sp>>>(
+                    PU.n, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start), dptr<int32_t>(PU.len), src_idx, pos, X, Y,
+                    Mb, comx, comy, bs, be, (T)eps2, p2p_mask, body ? 1 : 0, dptr<T>(ctx->p2l_part));
+                ctx->launches++;
+            }
+            return GX_OK;
+        };
         // the near field starts beside the far-field chain; for a measurement of the
         // near field alone (gx_bench_forces) it starts after the chain
-        if (!ctx->near_after_far) GX_TRY(near_field());
+        if (!ctx->near_after_far) {
+            GX_TRY(near_field());
+            if (p2l) {
+                GX_CUDA(ctx, cudaStreamWaitEvent(ctx->stream3, ctx->ev_fork, 0));
+                GX_TRY(p2l_field(ctx->stream3));
+                GX_CUDA(ctx, cudaEventRecord(ctx->ev_join3, ctx->stream3));
+            }
+        }
         // M2M: in ACCURATE mode the chain levels are one direct shift to the top one
         const int lc = mode == GX_MODE_ACCURATE ? (ctx->chain_levels >= 2 ? ctx->chain_levels : 0) : ctx->unary_levels;
         GX_TRY((run_up<P, T, false>(ctx, mode == GX_MODE_ACCURATE ? lc : (lc > 0 ? 1 : 0), lc, M,
@@ -2704,9 +2779,7 @@ int run_forces(gx_ctx *ctx, bool timed) {
                 k_m2l_units<P, T><<<(unsigned)((U.n * 32 + 127) / 128), 128, 0, st>>>(
                     U.n, dptr<int32_t>(U.node), dptr<int64_t>(U.start), dptr<int32_t>(U.len), node_u,
                     dptr<int32_t>(ctx->far_idx), comx, comy, mixed ? dptr<float4>(ctx->comhl) : nullptr, eps2, M, L,
-                    dptr<T>(ctx->m2l_part));
-                k_m2l_combine<P, T><<<gx_blocks(nn * NC, 256), 256, 0, st>>>(nn, node_u, dptr<T>(ctx->m2l_part), L);
-                ctx->launches++;
+                    dptr<T>(ctx->m2l_part), dptr<unsigned>(ctx->m2l_count));
             }
         } else {
             k_m2l_exact<P, T, uint32_t><<<gn, 128, 0, st>>>(nn, dptr<uint32_t>(ctx->vdata), nullptr, nullptr,
@@ -2715,61 +2788,23 @@ int run_forces(gx_ctx *ctx, bool timed) {
         }
         ctx->launches++;
         tm.mark();  // 4
-        // L2L
-        const T *Lleaf = L;
-        if (mode == GX_MODE_REF) {
-            k_l2l_ref_leaves<P, T><<<gx_blocks(nl, 128), 128, 0, st>>>(nl, parent, comx, comy, L, Lf);
-            ctx->launches++;
-            Lleaf = Lf;
-        } else {
-            k_l2l_direct<P, T><<<gw, 128, 0, st>>>(nl, ctx->n_levels, dptr<int32_t>(ctx->anc),
-                                                   dptr<uint8_t>(mode == GX_MODE_ACCURATE ? ctx->has_far_acc
-                                                                                          : ctx->has_far_ref),
-                                                   comx, comy, L, Lf);
-            ctx->launches++;
-            Lleaf = Lf;
-        }
-        if (split && ctx->p2l_units.n > 0) {
-            // P2L of the near-list split into the leaf locals, before L2P reads them
-            const gx_ctx::P2LUnits &PU = ctx->p2l_units;
-            GX_TRY(gx_ensure(ctx, ctx->p2l_part, sizeof(T) * NS * (size_t)(PU.n + 1)));
-            const int64_t *leaf_u = dptr<int64_t>(PU.leaf_u);
-            const int64_t *body_u = body ? dptr<int64_t>(PU.body_u) : nullptr;
-            const unsigned gu = (unsigned)((PU.n * 32 + 127) / 128);
-            const unsigned gl = (unsigned)((PU.n_leafu * 32 + 127) / 128);
-            const unsigned gb = (unsigned)((PU.n_body * 32 + 127) / 128);
-            bool packed = false;
-            if constexpr (P <= 5 && sizeof(T) == 4) {
-                // leaf-level units, then (body-level P2L) the body-level ones
-                if (PU.n_leafu > 0)
-                    k_p2l_x2<P><<<gl, 128, 0, st>>>(PU.n_leafu, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start),
-                                                    dptr<int32_t>(PU.len), leaf_u, body_u, src_idx, pos, comx, comy,
-                                                    bs, be, (float)eps2, Lf, dptr<float>(ctx->p2l_part));
-                if (body && PU.n_body > 0) {
-                    k_p2l_body_x2<P><<<gb, 128, 0, st>>>(PU.n_leafu, PU.n_body, dptr<int32_t>(PU.leaf),
-                                                         dptr<int64_t>(PU.start), dptr<int32_t>(PU.len), leaf_u,
-                                                         body_u, src_idx, p2p_mask, pos, comx, comy, bs, (float)eps2,
-                                                         Lf, dptr<float>(ctx->p2l_part));
-                    ctx->launches++;
-                }
-                packed = true;
-            }
-            if (!packed)
-                k_p2l<P, T><<<gu, 128, 0, st>>>(PU.n, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start),
-                                                dptr<int32_t>(PU.len), leaf_u, body_u, src_idx, pos, X, Y, Mb, comx,
-                                                comy, bs, be, (T)eps2, p2p_mask, body ? 1 : 0, Lf,
-                                                dptr<T>(ctx->p2l_part));
-            k_p2l_combine<P, T><<<gx_blocks(nl * NC, 256), 256, 0, st>>>(nl, leaf_u, body_u, PU.n_leafu,
-                                                                         dptr<T>(ctx->p2l_part), Lf);
-            ctx->launches += 2;
-        }
+        // L2L and the P2L partials into the leaves' locals (+ L2P in the mixed form)
         float2 *fl = nullptr;
-        if (mixed) {  // L2P beside the near field
+        if (mixed) {
             GX_TRY(gx_ensure(ctx, ctx->fl32, sizeof(float2) * (size_t)n));
             fl = dptr<float2>(ctx->fl32);
-            k_l2p32<P><<<gw, 128, 0, st>>>(nl, pos, bs, be, reinterpret_cast<const float *>(Lleaf), fl);
-            ctx->launches++;
         }
+        if (p2l && ctx->near_after_far) GX_TRY(p2l_field(st));
+        if (p2l && !ctx->near_after_far) GX_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_join3, 0));
+        if (mode == GX_MODE_REF && !mixed)
+            k_l2l_ref_leaves<P, T><<<gx_blocks(nl, 128), 128, 0, st>>>(nl, parent, comx, comy, L, Lf);
+        else  // REF lists: the leaf's own local and its parent's
+            k_leaf_local<P, T><<<gw, 128, 0, st>>>(
+                nl, mode == GX_MODE_REF ? std::min(2, (int)ctx->n_levels) : (int)ctx->n_levels, dptr<int32_t>(ctx->anc),
+                dptr<uint8_t>(mode == GX_MODE_ACCURATE ? ctx->has_far_acc : ctx->has_far_ref), comx, comy, L,
+                p2l ? dptr<int64_t>(PU.leaf_u) : nullptr, p2l && body ? dptr<int64_t>(PU.body_u) : nullptr, PU.n_leafu,
+                dptr<T>(ctx->p2l_part), Lf, pos, bs, be, fl);
+        ctx->launches++;
         tm.mark();  // 5
         if (ctx->near_after_far) GX_TRY(near_field());
         // join the near field, then the ordered sum of the P2P partials (+ L2P in FP64)
@@ -2778,7 +2813,7 @@ int run_forces(gx_ctx *ctx, bool timed) {
             k_reduce32<<<gw, 128, 0, st>>>(nl, bs, be, dptr<int64_t>(I.off), tchunks, dptr<float2>(ctx->part), fl,
                                            dptr<double>(ctx->ax), dptr<double>(ctx->ay), ctx->out_ax, ctx->out_ay);
         } else {
-            k_l2p_reduce64<P><<<gw, 128, 0, st>>>(nl, X, Y, comx, comy, bs, be, reinterpret_cast<const double *>(Lleaf),
+            k_l2p_reduce64<P><<<gw, 128, 0, st>>>(nl, X, Y, comx, comy, bs, be, reinterpret_cast<const double *>(Lf),
                                                   dptr<int64_t>(I.off), tchunks, dptr<double2>(ctx->part),
                                                   dptr<double>(ctx->ax), dptr<double>(ctx->ay), ctx->out_ax,
                                                   ctx->out_ay);

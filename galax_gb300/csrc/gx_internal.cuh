@@ -84,7 +84,9 @@ struct gx_ctx {
     // second stream: the near field (P2P) runs beside the far-field chain
     // (M2M, M2L, L2L) of the same evaluation; forked after P2M, joined before L2P
     cudaStream_t stream2 = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    // third stream: P2L, beside both; joined before the leaves' locals
+    cudaStream_t stream3 = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr;
     std::string err;
     int sm_count = 0;
 
@@ -144,7 +146,8 @@ struct gx_ctx {
         DevBuf node, start, len, node_u;  // int32, int64, int32, int64[n_nodes+1]
         int64_t n = 0;
     } m2l_units;
-    DevBuf m2l_part;  // per-unit partial locals of nodes cut into several units
+    DevBuf m2l_part;   // per-unit partial locals of nodes cut into several units
+    DevBuf m2l_count;  // uint32 per node: its units that have finished (zero between evaluations)
     // ACCURATE near-list split (theta_w > 0): every leaf's near list is partitioned in
     // place into [P2P | M2P | P2L] sources; the leaf's near count becomes its P2P count
     // and split_cnt holds (M2P count, P2L count) per leaf.  M2P sources become extra work
@@ -188,6 +191,7 @@ struct gx_ctx {
     // levels 1 .. unary_levels are single-child chains over the leaves, node x + l nl above
     // leaf x in level l (by the level sizes of a device build; checked for an uploaded tree)
     int unary_levels = 0;
+    bool leaves_cover = false;  // every body is in a leaf (an uploaded tree may leave some out)
     bool near_after_far = false;  // measurement only: the near field after the far-field chain
     // gx_compute_forces into page-locked host arrays: their device addresses, written by
     // the final sum of the evaluation being enqueued (null otherwise)

@@ -1963,6 +1963,9 @@ int gx_plan_items(gx_ctx *ctx, bool accurate) {
         GX_TRY(gx_ensure(ctx, U.node, sizeof(int32_t) * (size_t)(nun + 1)));
         GX_TRY(gx_ensure(ctx, U.start, sizeof(int64_t) * (size_t)(nun + 1)));
         GX_TRY(gx_ensure(ctx, U.len, sizeof(int32_t) * (size_t)(nun + 1)));
+        // the units' count-off starts at zero and every evaluation leaves it there
+        GX_TRY(gx_ensure(ctx, ctx->m2l_count, sizeof(unsigned) * (size_t)(nn + 1)));
+        GX_CUDA(ctx, cudaMemsetAsync(ctx->m2l_count.p, 0, sizeof(unsigned) * (size_t)(nn + 1), ctx->stream));
         k_m2l_units_fill<<<gx_blocks(nn, 256), 256, 0, ctx->stream>>>(nn, fstart, fcnt, dptr<int64_t>(U.node_u),
                                                                       dptr<int32_t>(U.node), dptr<int64_t>(U.start),
                                                                       dptr<int32_t>(U.len));

@@ -49,3 +49,23 @@ def test_non_finite_moments_are_zeroed_once(G, oracle):
             ctx.compute_forces(b.x, b.y, np.ascontiguousarray(ref.mass), ax, ay)
             if scale == 1.0:
                 assert (rel_vec_err(ax, ay, ref.ax, ref.ay) <= 1e-10).all()
+
+
+def test_uploaded_tree_that_leaves_a_body_out(G, oracle):
+    """A body in no leaf keeps a = 0 and is still sanitised; the others are those of the tree."""
+    n, n_max, p = 400, 16, 4
+    b = presets.uniform(n, seed=12)
+    ob, t, v, u, eps = oracle_case(oracle, b, n_max, presets.BOUNDS["uniform"], p)
+    t.body_start[t.body_start == 0] = 1
+    ob.mass[0] = -1.0
+    ctx = G.GpuContext(G.GpuConfig(max_n=n, max_nodes=0, p=p))
+    ctx.set_params(p, eps)
+    ctx.upload_tree_data(t, v, u)
+    ax, ay = np.full(n, 7.0), np.full(n, 7.0)
+    for _ in range(2):
+        ctx.compute_forces(ob.x, ob.y, ob.mass, ax, ay)
+        assert ax[0] == 0.0 and ay[0] == 0.0 and np.isfinite(ax).all() and np.abs(ax[1:]).min() > 0.0
+        assert ctx.last_status() == G.STATUS_SANITIZED
+    out = G.Bodies.new(n)
+    ctx.download_bodies(out)
+    assert out.mass[0] == 1.0
