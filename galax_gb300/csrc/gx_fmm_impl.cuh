@@ -188,7 +188,7 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 template <class T>
 __device__ __forceinline__ T rsqrt_t(T v);
 template <>
-__device__ __forceinline__ double rsqrt_t<double>(double v) { return rsqrt(v); }
+__device__ __forceinline__ double rsqrt_t<double>(double v) { return gx_rsqrt(v); }  // six FP64 instructions fewer
 template <>
 __device__ __forceinline__ float rsqrt_t<float>(float v) { return rsqrt_fast(v); }
 
@@ -581,13 +581,12 @@ __host__ __device__ constexpr double ff_const(int k, int l) {
 }
 
 template <int P, int N, class T>
-__device__ __forceinline__ void m2l_order(T dx, T dy, T ir2, T *a, const T *in, T *out) {
+__device__ __forceinline__ void m2l_order(T X, T Y, T ir2, T *a, const T *in, T *out) {
     if constexpr (N <= 2 * P) {
-        const T in_ = tab_inv<T>(N) * ir2;
-        // c1 (dx a_{k-1,l} + dy a_{k,l-1}) + c2 (a_{k-2,l} + a_{k,l-2}) with c1 dx, c1 dy
-        // formed once per order: one multiply fewer per term
-        const T c1 = -(T)(2 * N - 1) * in_, c2 = -(T)(N - 1) * in_;
-        const T c1x = c1 * dx, c1y = c1 * dy;
+        // c1x a_{k-1,l} + c1y a_{k,l-1} + c2 (a_{k-2,l} + a_{k,l-2}); with X = dx / R^2 and
+        // Y = dy / R^2 formed once, three multiplies an order (none at order 1)
+        constexpr double q1 = -(double)(2 * N - 1) / N, q2 = -(double)(N - 1) / N;
+        const T c1x = (T)q1 * X, c1y = (T)q1 * Y, c2 = (T)q2 * ir2;
 #pragma unroll
         for (int k = 0; k <= N; k++) {
             const int l = N - k;
@@ -609,7 +608,7 @@ __device__ __forceinline__ void m2l_order(T dx, T dy, T ir2, T *a, const T *in, 
                     if (yi + yj <= P && xi + xj <= P) out[gx_mi(xi, xj)] += in[gx_mi(yi, yj)] * Av;
                 }
         }
-        m2l_order<P, N + 1, T>(dx, dy, ir2, a, in, out);
+        m2l_order<P, N + 1, T>(X, Y, ir2, a, in, out);
     }
 }
 
@@ -622,7 +621,7 @@ __device__ __forceinline__ void m2l_fused_core(T dx, T dy, T eps2, const T *in, 
     if constexpr (P <= 8) {
         T a[nc2(2 * P)];
         a[0] = ir;
-        m2l_order<P, 1, T>(dx, dy, ir2, a, in, out);
+        m2l_order<P, 1, T>(dx * ir2, dy * ir2, ir2, a, in, out);
     } else {
         // high orders: run-time loop bounds keep the code size bounded
         const int PP = gx_rt_order(P);
@@ -807,11 +806,11 @@ __device__ __forceinline__ void m2l_sources(const IDX *__restrict__ idx, int64_t
     const int PP = gx_rt_order(P);
     // the next source index is fetched one iteration ahead, and the source row is
     // requested before the derivatives are formed, so both latencies overlap compute
-    int64_t src = lane < len ? (int64_t)idx[st + lane] : 0;
+    int32_t src = lane < len ? (int32_t)idx[st + lane] : 0;
     for (int s = lane; s < len; s += 32) {
-        int64_t nsrc = s + 32 < len ? (int64_t)idx[st + s + 32] : 0;
+        const int32_t nsrc = s + 32 < len ? (int32_t)idx[st + s + 32] : 0;
         T ms[NC];
-        load_row<NC>(M + src * NS, ms);
+        load_row<NC>(M + (int64_t)src * NS, ms);
         T dx, dy;
         if constexpr (sizeof(T) == 4) {
             // COMs as FP32 (hi, lo) pairs: the offset is exact to FP32 rounding without
@@ -1773,17 +1772,19 @@ __global__ void __launch_bounds__(128, 8) k_p2p32_stream(
 // coefficients a_k of 1/R, R^2 = dx^2 + dy^2 + eps^2, from the three-term recurrence of
 // the fused M2L; a derivative of 1/R is k! a_k and the reference's G is its negative.
 
-// a_k for |k| <= N at (dx, dy): a[gx_mi(k, l)]; NR = N or, above the unrolled orders, a
-// run-time copy of it
-template <int N, class T>
-__device__ __forceinline__ void taylor_1r(T dx, T dy, T ir, T ir2, int NR, T *a) {
-    a[0] = ir;
+// f(n, k, l, a_kl) for |k| + |l| = n = 1 .. N at (dx, dy), a_00 = a0; NR = N or, above the
+// unrolled orders, a run-time copy of it.  With X = dx / R^2 and Y = dy / R^2 an order costs
+// three multiplies besides its terms.
+template <int N, class T, class F>
+__device__ __forceinline__ void taylor_each(T dx, T dy, T a0, T ir2, int NR, const F &f) {
+    T a[nc2(N)];
+    a[0] = a0;
+    const T X = dx * ir2, Y = dy * ir2;
 #pragma unroll
     for (int n = 1; n <= N; n++) {
         if (n > NR) break;
-        const T in_ = tab_inv<T>(n) * ir2;
-        const T c1 = -(T)(2 * n - 1) * in_, c2 = -(T)(n - 1) * in_;
-        const T c1x = c1 * dx, c1y = c1 * dy;
+        const T q1 = -(T)(2 * n - 1) * tab_inv<T>(n), q2 = -(T)(n - 1) * tab_inv<T>(n);
+        const T c1x = q1 * X, c1y = q1 * Y, c2 = q2 * ir2;
 #pragma unroll
         for (int k = 0; k <= n; k++) {
             const int l = n - k;
@@ -1794,58 +1795,60 @@ __device__ __forceinline__ void taylor_1r(T dx, T dy, T ir, T ir2, int NR, T *a)
             if (k >= 2) v += c2 * a[gx_mi(k - 2, l)];
             if (l >= 2) v += c2 * a[gx_mi(k, l - 2)];
             a[gx_mi(k, l)] = v;
+            f(n, k, l, v);
         }
     }
 }
 
-// M2P of one source multipole M (about com_s, raw coefficients) at offset
-// d = x - com_s:  a(x) = sum_S (-1)^|S| M[S] (S+e)! a_{S+e}(d), e = e_x, e_y.  FP32 at
-// p >= 6 forms the coefficients at unit distance (the 1/R kernel is homogeneous of
-// degree -1 in (d, eps)) and moves the powers of 1/R onto the moments, as the M2L does.
-template <int P, class T>
-__device__ __forceinline__ void m2p_eval(T dx, T dy, T eps2, const T *ms, T &fx, T &fy) {
-    constexpr int N = P + 1;
+template <class T> struct pair_t;
+template <> struct pair_t<float> { using type = float2; };
+template <> struct pair_t<double> { using type = double2; };
+
+// M2P of one source multipole about com_s at offset d = x - com_s:
+//   a(x) = sum_S (-1)^|S| M[S] (S+e)! a_{S+e}(d), e = e_x, e_y,
+// from w[S] = (-1)^|S| M[S] times ((S+e_x)!, (S+e_y)!), the same for every body.  FP32 at
+// p >= 6 forms the coefficients at unit distance (the 1/R kernel is homogeneous of degree -1
+// in (d, eps): a'_0 = 1 and 1/R'^2 = 1 there, eps enters through R only, and a_k(d) =
+// a'_k(d / R) R^-(|k|+1)), so the orders' sums are joined by Horner in 1/R.
+template <int P, class T, class V>
+__device__ __forceinline__ void m2p_eval(T dx, T dy, T eps2, const V *w, T &fx, T &fy) {
+    constexpr bool unit = sizeof(T) == 4 && P >= 6;
     const int PP = gx_rt_order(P);
-    const T ir = rsqrt_t<T>(dx * dx + dy * dy + eps2);
-    T a[nc2(N)];
-    T scale = T(1);
-    T mw[nc2(P)];
-    if constexpr (sizeof(T) == 4 && P >= 6) {
-        T pw = T(1);
-        for (int q = 0; q <= PP; q++) {
-            for (int j = 0; j <= q; j++) mw[gx_mi(q - j, j)] = ms[gx_mi(q - j, j)] * pw;
-            pw *= ir;
+    const T ir = rsqrt_t<T>(dx * dx + (dy * dy + eps2));
+    T sx = T(0), sy = T(0), ox[P + 1], oy[P + 1];
+    if constexpr (unit) {
+#pragma unroll
+        for (int q = 0; q <= PP; q++) ox[q] = oy[q] = T(0);
+    }
+    const auto term = [&](int n, int k, int l, T v) {
+        T &ax = unit ? ox[n - 1] : sx, &ay = unit ? oy[n - 1] : sy;
+        if (k >= 1) ax += w[gx_mi(k - 1, l)].x * v;
+        if (l >= 1) ay += w[gx_mi(k, l - 1)].y * v;
+    };
+    if constexpr (unit) {
+        taylor_each<P + 1, T>(dx * ir, dy * ir, T(1), T(1), PP + 1, term);
+#pragma unroll
+        for (int q = PP; q >= 0; q--) {
+            sx = sx * ir + ox[q];
+            sy = sy * ir + oy[q];
         }
-        // at unit distance R' = 1: a'_0 = 1 and 1/R'^2 = 1 (eps enters through R only);
-        // a_k(d) = a'_k(d / R) R^-(|k|+1)
-        taylor_1r<N, T>(dx * ir, dy * ir, T(1), T(1), PP + 1, a);
-        scale = ir * ir;
+        fx += sx * (ir * ir);
+        fy += sy * (ir * ir);
     } else {
-#pragma unroll
-        for (int k = 0; k < nc2(P); k++) mw[k] = ms[k];
-        taylor_1r<N, T>(dx, dy, ir, ir * ir, PP + 1, a);
+        taylor_each<P + 1, T>(dx, dy, ir, ir * ir, PP + 1, term);
+        fx += sx;
+        fy += sy;
     }
-    T sx = T(0), sy = T(0);
-#pragma unroll
-    for (int si = 0; si <= P; si++) {
-        if (si > PP) break;
-#pragma unroll
-        for (int sj = 0; sj <= P - si; sj++) {
-            if (si + sj > PP) break;
-            const T mv = ((si + sj) & 1) ? -mw[gx_mi(si, sj)] : mw[gx_mi(si, sj)];
-            sx += mv * (a[gx_mi(si + 1, sj)] * tab_ff<T>(si + 1, sj));
-            sy += mv * (a[gx_mi(si, sj + 1)] * tab_ff<T>(si, sj + 1));
-        }
-    }
-    fx += sx * scale;
-    fy += sy * scale;
 }
 
 // M2P items: one warp per item with item_nq < 0 (grid-stride; P2P items are skipped),
-// lane per target body (chunks of 32 above 32 bodies).  Per source leaf its lane forms
-// the offset com_a - com_s in FP64 once (rounded to T), shared through shared memory;
-// the source's moment row is a broadcast load.  Writes the item's partial slot like a
-// P2P item, so the ordered sum of the leaf's items includes it.
+// lane per target body (chunks of 32 above 32 bodies).  A source's moments are signed and
+// scaled once for the warp (a lane per coefficient, the next source's in flight meanwhile)
+// and read back from shared memory; its lane forms the offset com_a - com_s in FP64 once.
+// FP64 at 1M (1.97M leaf pairs): 15.5 -> 12.4 ms with the moments no longer scaled per body
+// and 1/R from the integer pipes; the FP64 pipe alone would take 10 ms.
+// Writes the item's partial slot like a P2P item, so the ordered sum of the leaf's items
+// includes it.
 template <int P, class T, class V>
 __global__ void __launch_bounds__(128) k_m2p(int64_t n_list, const int32_t *__restrict__ list,
                                              const int32_t *__restrict__ item_leaf,
@@ -1857,10 +1860,20 @@ __global__ void __launch_bounds__(128) k_m2p(int64_t n_list, const int32_t *__re
                                              T eps2, const T *__restrict__ M, int tchunks, V *__restrict__ part) {
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<T>(NC);
-    __shared__ T shx[4][32], shy[4][32];
-    __shared__ int32_t shs[4][32];
+    constexpr int CPL = (NC + 31) / 32;  // coefficients a lane prepares
+    __shared__ V sw[4][NC];
+    const unsigned full = 0xffffffffu;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    T scx[CPL], scy[CPL];
+#pragma unroll
+    for (int c = 0; c < CPL; c++) {
+        int si, sj;
+        mi_split(min(lane + 32 * c, NC - 1), si, sj);
+        const T sign = ((si + sj) & 1) ? T(-1) : T(1);
+        scx[c] = sign * tab_ff<T>(si + 1, sj);
+        scy[c] = sign * tab_ff<T>(si, sj + 1);
+    }
     for (int64_t li = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; li < n_list; li += nwarps) {
         const int64_t it = list[li];
         const int nq0 = item_nq[it];
@@ -1868,14 +1881,13 @@ __global__ void __launch_bounds__(128) k_m2p(int64_t n_list, const int32_t *__re
         const int nq = -nq0;
         const int32_t leaf = item_leaf[it];
         const double tcx = comx[leaf], tcy = comy[leaf];
-        __syncwarp();  // the previous item's reads of the shared arrays are done
+        int32_t sl = 0;
+        T shx = T(0), shy = T(0);
         if (lane < nq) {
-            const int32_t sl = src_idx[item_qb[it] + lane];
-            shs[w][lane] = sl;
-            shx[w][lane] = (T)(tcx - comx[sl]);
-            shy[w][lane] = (T)(tcy - comy[sl]);
+            sl = src_idx[item_qb[it] + lane];
+            shx = (T)(tcx - comx[sl]);
+            shy = (T)(tcy - comy[sl]);
         }
-        __syncwarp();
         const int32_t t0 = bs[leaf], t1 = be[leaf];
         for (int tc = 0; tc < tchunks; tc++) {
             const int32_t i = t0 + tc * 32 + lane;
@@ -1892,10 +1904,27 @@ __global__ void __launch_bounds__(128) k_m2p(int64_t n_list, const int32_t *__re
             }
             T fx = T(0), fy = T(0);
             if (t0 + tc * 32 < t1) {
+                T m[CPL];
+                const auto fetch = [&](int k) {
+                    const T *row = M + (int64_t)__shfl_sync(full, sl, k) * NS;
+#pragma unroll
+                    for (int c = 0; c < CPL; c++) m[c] = lane + 32 * c < NC ? row[lane + 32 * c] : T(0);
+                };
+                fetch(0);
                 for (int k = 0; k < nq; k++) {
-                    T ms[NC];
-                    load_row<NC>(M + (int64_t)shs[w][k] * NS, ms);
-                    m2p_eval<P, T>(px + shx[w][k], py + shy[w][k], eps2, ms, fx, fy);
+                    __syncwarp();  // the last source's moments have been read
+#pragma unroll
+                    for (int c = 0; c < CPL; c++)
+                        if (lane + 32 * c < NC) {
+                            V v;
+                            v.x = m[c] * scx[c];
+                            v.y = m[c] * scy[c];
+                            sw[w][lane + 32 * c] = v;
+                        }
+                    __syncwarp();
+                    if (k + 1 < nq) fetch(k + 1);
+                    m2p_eval<P, T, V>(px + __shfl_sync(full, shx, k), py + __shfl_sync(full, shy, k), eps2, sw[w], fx,
+                                      fy);
                 }
             }
             V r;
@@ -1917,16 +1946,16 @@ __device__ __forceinline__ f2v f2add(f2v a, f2v b) { return {add2(a.v, b.v)}; }
 __device__ __forceinline__ f2v f2sub(f2v a, f2v b) { return {sub2(a.v, b.v)}; }
 __device__ __forceinline__ f2v f2fma(f2v a, f2v b, f2v c) { return {fma2(a.v, b.v, c.v)}; }
 
-// taylor_1r on pairs: a_k for |k| <= N at two offsets at once
+// the recurrence of taylor_each on pairs: a_k for |k| <= N at two offsets at once
 template <int N>
 __device__ __forceinline__ void taylor_1r_x2(f2v dx, f2v dy, f2v ir, f2v ir2, f2v *a) {
     a[0] = ir;
+    const f2v X = f2mul(dx, ir2), Y = f2mul(dy, ir2);
 #pragma unroll
     for (int n = 1; n <= N; n++) {
-        const f2v in_ = f2mul(f2splat((float)(1.0 / n)), ir2);
-        const f2v c1 = f2mul(f2splat(-(float)(2 * n - 1)), in_);
-        const f2v c2 = f2mul(f2splat(-(float)(n - 1)), in_);
-        const f2v c1x = f2mul(c1, dx), c1y = f2mul(c1, dy);
+        const f2v c1x = f2mul(f2splat(-(float)((2.0 * n - 1.0) / n)), X);
+        const f2v c1y = f2mul(f2splat(-(float)((2.0 * n - 1.0) / n)), Y);
+        const f2v c2 = f2mul(f2splat(-(float)((n - 1.0) / n)), ir2);
 #pragma unroll
         for (int k = 0; k <= n; k++) {
             const int l = n - k;
@@ -1969,15 +1998,14 @@ __global__ void __launch_bounds__(128, 8) k_m2p_x2(int64_t n_list, const int32_t
     __shared__ __align__(8) float2 shf[4][32];        // com_a - com_s
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int half = lane >> 4, tl = lane & 15;
-    const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
     const f2v E2 = f2splat(eps2);
-    for (int64_t li = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; li < n_list; li += nwarps) {
-        const int64_t it = list[li];
+    const int64_t li = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // one item a warp
+    if (li < n_list) {
+        const int32_t it = list[li];
         const int nq0 = item_nq[it];
-        if (nq0 >= 0) continue;
+        if (nq0 >= 0) return;
         const int nq = -nq0;
         const int32_t leaf = item_leaf[it];
-        __syncwarp();  // the previous item's reads of the shared arrays are done
         if (lane < nq) {
             const int32_t sl = src_idx[item_qb[it] + lane];
             shf[w][lane] = make_float2((float)(comx[leaf] - comx[sl]), (float)(comy[leaf] - comy[sl]));
@@ -2023,7 +2051,7 @@ __global__ void __launch_bounds__(128, 8) k_m2p_x2(int64_t n_list, const int32_t
         float2 res;
         if (half == 0) res = make_float2(xA + oxA, yA + oyA);  // body tl
         else res = make_float2(oxB + xB, oyB + yB);             // body tl + 16 (half 0's part first)
-        part[it * 32 + lane] = res;
+        part[(int64_t)it * 32 + lane] = res;
     }
 }
 
@@ -2279,24 +2307,117 @@ __global__ void __launch_bounds__(128, 6) k_p2l_body_x2(int64_t u_base, int64_t 
 template <int P, class T>
 __device__ __forceinline__ void p2l_body(T dx, T dy, T mj, T eps2, T *acc) {
     const int PP = gx_rt_order(P);
-    const int NCr = (PP + 1) * (PP + 2) / 2;
-    (void)NCr;
-    const T ir = rsqrt_t<T>(dx * dx + dy * dy + eps2);
-    T c[nc2(P)];
-    if constexpr (sizeof(T) == 4 && P >= 6) {
-        taylor_1r<P, T>(dx * ir, dy * ir, T(1), T(1), PP, c);
-        T w = mj * ir;
-        for (int q = 0; q <= PP; q++) {
-            for (int i = 0; i <= q; i++) acc[gx_mi(q - i, i)] += w * c[gx_mi(q - i, i)];
-            w *= ir;
-        }
-    } else {
-        taylor_1r<P, T>(dx, dy, ir, ir * ir, PP, c);
+    const T ir = rsqrt_t<T>(dx * dx + (dy * dy + eps2));
+    if constexpr (sizeof(T) == 4 && P >= 6) {  // at unit distance, as in m2p_eval
+        T w[P + 1];  // m R^-(n+1)
+        w[0] = mj * ir;
 #pragma unroll
-        for (int k = 0; k < NCr; k++) acc[k] += mj * c[k];
+        for (int n = 1; n <= PP; n++) w[n] = w[n - 1] * ir;
+        acc[0] += w[0];
+        taylor_each<P, T>(dx * ir, dy * ir, T(1), T(1), PP, [&](int n, int k, int l, T v) { acc[gx_mi(k, l)] += w[n] * v; });
+    } else {
+        acc[0] += mj * ir;
+        taylor_each<P, T>(dx, dy, ir, ir * ir, PP, [&](int, int k, int l, T v) { acc[gx_mi(k, l)] += mj * v; });
     }
 }
 
+// P2L units over leaves of at most 32 bodies, where the packed kernels above do not apply
+// (FP64, and FP32 at p >= 6): the unit's bodies (a leaf-level unit's all, a body-level one's
+// masked) are laid out as one stream in shared memory, entry (row << 5) | body, and taken a
+// body per lane, so no lane idles on a masked or missing body.  (A row at a time, FP64 paid
+// the whole warp's evaluation for the third of a row that the masks keep: 14.0 -> 10.8 ms at
+// 1M, 8.7 ms of it the FP64 pipe's.)
+template <int P, class T>
+__global__ void __launch_bounds__(128) k_p2l_stream(int64_t n_units, const int32_t *__restrict__ uleaf,
+                                                    const int64_t *__restrict__ ustart, const int32_t *__restrict__ ulen,
+                                                    const int32_t *__restrict__ src_idx,
+                                                    const float4 *__restrict__ pos, const double *__restrict__ X,
+                                                    const double *__restrict__ Y, const double *__restrict__ Mb,
+                                                    const double *__restrict__ comx, const double *__restrict__ comy,
+                                                    const int32_t *__restrict__ bs, const int32_t *__restrict__ be, T eps2,
+                                                    const uint32_t *__restrict__ p2p_mask, T *__restrict__ ppart) {
+    constexpr int NC = nc2(P);
+    constexpr int NS = row_stride<T>(NC);
+    constexpr int ROWS = GX_BODY_UNIT > GX_P2L_UNIT ? GX_BODY_UNIT : GX_P2L_UNIT;
+    constexpr int RPL = ROWS / 32;
+    static_assert(ROWS % 32 == 0 && ROWS * 32 <= 65536, "whole rows per lane, 16-bit entries");
+    const int PP = gx_rt_order(P);
+    const int NCr = (PP + 1) * (PP + 2) / 2;
+    __shared__ int32_t rb0[4][ROWS];       // per row: the source leaf's first body
+    __shared__ float2 rsh[4][ROWS];        // FP32: com_a - com_s
+    __shared__ uint16_t strm[4][ROWS * 32];
+    const unsigned full = 0xffffffffu;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (u >= n_units) return;
+    const int32_t a = uleaf[u];
+    const int raw = ulen[u], nq = raw < 0 ? -raw : raw;  // a body-level unit's length is stored negated
+    const double tcx = comx[a], tcy = comy[a];
+    int total = 0;
+#pragma unroll
+    for (int h = 0; h < RPL; h++) {
+        uint32_t take = 0u;
+        const int r = 32 * h + lane;
+        if (r < nq) {
+            const int64_t q = ustart[u] + r;
+            const int32_t sl = src_idx[q];
+            const int nb = be[sl] - bs[sl];
+            take = raw < 0 ? p2p_mask[q] : (nb >= 32 ? full : (1u << nb) - 1u);
+            rb0[w][r] = bs[sl];
+            if constexpr (sizeof(T) == 4)
+                rsh[w][r] = make_float2((float)(tcx - comx[sl]), (float)(tcy - comy[sl]));
+        }
+        const int c = __popc(take);
+        int incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(full, incl, o);
+            if (lane >= o) incl += v;
+        }
+        int at = total + incl - c;
+        total += __shfl_sync(full, incl, 31);
+        while (take) {
+            const int j = __ffs(take) - 1;
+            take &= take - 1u;
+            strm[w][at++] = (uint16_t)((r << 5) | j);
+        }
+    }
+    __syncwarp();
+    T acc[NC];
+#pragma unroll
+    for (int k = 0; k < NCr; k++) acc[k] = T(0);
+    // com_a - x_j and m_j of stream entry p (past the end: a unit offset and no mass)
+    const auto get = [&](int p, T &dx, T &dy, T &m) {
+        dx = dy = T(1);
+        m = T(0);
+        if (p >= total) return;
+        const int e = strm[w][p], j = rb0[w][e >> 5] + (e & 31);
+        if constexpr (sizeof(T) == 4) {
+            const float4 v = pos[j];
+            const float2 o = rsh[w][e >> 5];
+            dx = o.x - v.x;
+            dy = o.y - v.y;
+            m = v.z;
+        } else {
+            dx = tcx - X[j];
+            dy = tcy - Y[j];
+            m = Mb[j];
+        }
+    };
+    T dx, dy, m;
+    get(lane, dx, dy, m);
+    for (int p = 0; p < total; p += 32) {
+        T nx, ny, nm;
+        get(p + 32 + lane, nx, ny, nm);
+        p2l_body<P, T>(dx, dy, m, eps2, acc);
+        dx = nx;
+        dy = ny;
+        m = nm;
+    }
+    warp_coeffs<NC>(acc, [&](int k, T v) { ppart[u * NS + k] = v; });
+}
+
+// P2L units over larger leaves (no body-level units there): a row at a time.
 template <int P, class T>
 __global__ void __launch_bounds__(128) k_p2l(int64_t n_units, const int32_t *__restrict__ uleaf,
                                              const int64_t *__restrict__ ustart, const int32_t *__restrict__ ulen,
@@ -2305,7 +2426,6 @@ __global__ void __launch_bounds__(128) k_p2l(int64_t n_units, const int32_t *__r
                                              const double *__restrict__ Y, const double *__restrict__ Mb,
                                              const double *__restrict__ comx, const double *__restrict__ comy,
                                              const int32_t *__restrict__ bs, const int32_t *__restrict__ be, T eps2,
-                                             const uint32_t *__restrict__ p2p_mask, int body_units,
                                              T *__restrict__ ppart) {
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<T>(NC);
@@ -2316,27 +2436,19 @@ __global__ void __launch_bounds__(128) k_p2l(int64_t n_units, const int32_t *__r
     const int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (u >= n_units) return;
     const int32_t a = uleaf[u];
-    // a body-level unit (length stored negated): up to GX_BODY_UNIT P2P rows of the leaf,
-    // their masked bodies only (source leaves of at most 32 bodies); body_units = 0 leaves
-    // them to k_p2l_body_x2
-    const int raw = ulen[u];
-    if (raw < 0 && !body_units) return;
-    const bool body = raw < 0;
-    const int nq = body ? -raw : raw;
+    const int nq = ulen[u];
     const double tcx = comx[a], tcy = comy[a];
     T acc[NC];
 #pragma unroll
     for (int k = 0; k < NCr; k++) acc[k] = T(0);
-    // the unit's rows 32 at a time (a body-level unit has up to GX_BODY_UNIT)
+    // the unit's rows 32 at a time
     for (int g0 = 0; g0 < nq; g0 += 32) {
         const int ng = min(32, nq - g0);
         int32_t sb = 0, se = 0;
-        uint32_t take = 0xffffffffu;
         T shx = T(0), shy = T(0);
         double scx = 0.0, scy = 0.0;
         if (lane < ng) {
             const int64_t q = ustart[u] + g0 + lane;
-            if (body) take = p2p_mask[q];
             const int32_t sl = src_idx[q];
             sb = bs[sl];
             se = be[sl];
@@ -2370,10 +2482,9 @@ __global__ void __launch_bounds__(128) k_p2l(int64_t n_units, const int32_t *__r
             const double ckx = __shfl_sync(0xffffffffu, scx, k), cky = __shfl_sync(0xffffffffu, scy, k);
             (void)ckx;
             (void)cky;
-            const uint32_t tk = __shfl_sync(0xffffffffu, take, k);
             // com_a - x_j = (com_a - com_s) - (x_j - com_s)
-            if (j0 + lane < j1 && ((tk >> lane) & 1u)) p2l_body<P, T>(ox - cx_, oy - cy_, cm, eps2, acc);
-            // leaves above 32 bodies (n_max > 32, never a body-level unit): the rest of the source's bodies
+            if (j0 + lane < j1) p2l_body<P, T>(ox - cx_, oy - cy_, cm, eps2, acc);
+            // the rest of the source's bodies
             for (int32_t j = j0 + 32 + lane; j < j1; j += 32) {
                 T px, py, pm;
                 if constexpr (sizeof(T) == 4) {
@@ -2719,7 +2830,6 @@ int run_forces(gx_ctx *ctx, bool timed) {
         const bool p2l = split && PU.n > 0;
         if (p2l) GX_TRY(gx_ensure(ctx, ctx->p2l_part, sizeof(T) * NS * (size_t)(PU.n + 1)));
         auto p2l_field = [&](cudaStream_t sp) -> int {
-            bool packed = false;
             if constexpr (P <= 5 && sizeof(T) == 4) {
                 if (PU.n_leafu > 0) {
                     k_p2l_x2<P><<<gx_blocks(PU.n_leafu * 32, 128), 128, 0, sp>>>(
@@ -2734,12 +2844,15 @@ int run_forces(gx_ctx *ctx, bool timed) {
                         dptr<float>(ctx->p2l_part));
                     ctx->launches++;
                 }
-                packed = true;
-            }
-            if (!packed) {
+            } else if (ctx->max_leaf <= 32) {
+                k_p2l_stream<P, T><<<gx_blocks(PU.n * 32, 128), 128, 0, sp>>>(
+                    PU.n, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start), dptr<int32_t>(PU.len), src_idx, pos, X, Y,
+                    Mb, comx, comy, bs, be, (T)eps2, p2p_mask, dptr<T>(ctx->p2l_part));
+                ctx->launches++;
+            } else {
                 k_p2l<P, T><<<gx_blocks(PU.n * 32, 128), 128, 0, sp>>>(
                     PU.n, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start), dptr<int32_t>(PU.len), src_idx, pos, X, Y,
-                    Mb, comx, comy, bs, be, (T)eps2, p2p_mask, body ? 1 : 0, dptr<T>(ctx->p2l_part));
+                    Mb, comx, comy, bs, be, (T)eps2, dptr<T>(ctx->p2l_part));
                 ctx->launches++;
             }
             return GX_OK;

@@ -50,6 +50,7 @@ __device__ __forceinline__ GxMass gx_mass_split(double m) {
 
 // z = r^2 2^(-2k) in [1, 4) with y = rsqrt(z) to 24 bits and e = 1 - z y^2
 struct GxRoot {
+    uint32_t yi;      // y 2^32
     uint64_t y2, y3;  // y^2 2^64 (exact), y^3 2^63
     int64_t e;        // e 2^63
     int k;
@@ -69,6 +70,7 @@ __device__ __forceinline__ GxRoot gx_root(uint32_t hi, uint32_t lo) {
         : "f"(__uint_as_float(((zh >> 8) & 0x7fffffu) | ((uint32_t)(127 + odd) << 23))));
     y = fminf(fmaxf(y, 0.5f), 0x1.fffffep-1f);  // [1/2, 1): one exponent, so the bits are the fraction
     const uint32_t yi = 0x80000000u | (__float_as_uint(y) << 8);  // y 2^32
+    r.yi = yi;
     r.y2 = (uint64_t)yi * yi;
     // e 2^63 = 2^63 - z y^2 2^63 (modulo 2^64: the difference fits in 44 bits)
     r.e = (int64_t)(0x8000000000000000ull - (__umul64hi(z63, r.y2) << odd));
@@ -76,7 +78,7 @@ __device__ __forceinline__ GxRoot gx_root(uint32_t hi, uint32_t lo) {
     return r;
 }
 
-// mant 2^(ex - 63) r^-N from y^N 2^63 (N = 3 or 5)
+// mant 2^(ex - 63) r^-N from y^N 2^63 (N = 1, 3 or 5)
 template <int N>
 __device__ __forceinline__ double gx_root_pow(const GxRoot &r, uint64_t yn, uint64_t mant, int ex) {
     const float ef = (float)(int32_t)(r.e >> 20);  // e 2^43
@@ -114,4 +116,12 @@ __device__ __forceinline__ void gx_r3_3r5(double r2, double &ir3, double &ir5x3)
     const GxRoot r = gx_root(hi, lo);
     ir3 = gx_root_pow<3>(r, r.y3, 0x8000000000000000ull, 0);
     ir5x3 = gx_root_pow<5>(r, __umul64hi(r.y3, r.y2), 0xc000000000000000ull, 1);
+}
+
+// r2^(-1/2)
+__device__ __forceinline__ double gx_rsqrt(double r2) {
+    const uint32_t hi = (uint32_t)__double2hiint(r2), lo = (uint32_t)__double2loint(r2);
+    if ((hi >> 20) - (uint32_t)GX_R3_EXP_LO >= GX_R3_EXP_SPAN) return rsqrt(r2);
+    const GxRoot r = gx_root(hi, lo);
+    return gx_root_pow<1>(r, (uint64_t)r.yi << 31, 0x8000000000000000ull, 0);
 }
