@@ -183,7 +183,7 @@ struct gx_ctx {
     int64_t hint_nodes = 0, hint_far = 0, hint_near = 0;
     int hint_big_rounds = 0;  // tree build: rounds of the last build run by the multi-block kernels
     int hint_field_levels = 0;  // tree build: levels of the last build whose fields took a launch each
-    int rounds_blocks = 0;    // tree build: blocks of the rounds' cluster (0: not yet asked for)
+    int cluster16 = 0;        // clusters of 16 blocks: 1 the device takes them, -1 not, 0 not yet asked
     // ACCURATE plan: levels 1 .. chain_levels are single-child chains over the leaves
     // (level l holds node x + l nl above leaf x); with chain_levels >= 2 the plan and M2M
     // skip levels 1 .. chain_levels - 1 (no far lists there), else 0
@@ -265,10 +265,6 @@ int gx_exclusive_scan_i32(gx_ctx *ctx, const int32_t *in, int32_t *out, int64_t 
 // the grand total goes to *total_dev when given
 int gx_exclusive_scan_i64_devn(gx_ctx *ctx, const int64_t *in, int64_t *out, const int64_t *n_dev, int64_t n_add,
                                int64_t n_cap, int64_t *total_dev = nullptr);
-// m arrays at a common stride (in + k * stride -> out + k * stride), one set of launches;
-// total_dev (if given) receives m totals
-int gx_exclusive_scan_i64_devn_multi(gx_ctx *ctx, const int64_t *in, int64_t *out, int m, int64_t stride,
-                                     const int64_t *n_dev, int64_t n_add, int64_t n_cap, int64_t *total_dev = nullptr);
 int gx_radix_sort_u64(gx_ctx *ctx, uint64_t *keys, uint32_t *vals, int64_t n, int begin_bit, int end_bit,
                       uint64_t *keys_alt, uint32_t *vals_alt, bool *result_in_alt);
 // gx_kdk.cu

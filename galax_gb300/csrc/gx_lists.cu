@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <set>
 
+#include "gx_cluster_scan.cuh"
 #include "gx_internal.cuh"
 
 int gx_tree_rebuild_with_splits(gx_ctx *ctx, int64_t n_max, const double bounds[4], const std::vector<int64_t> &splits);
@@ -454,19 +455,23 @@ __global__ void k_radius_chain(int64_t nl, int L, const double *comx, const doub
     }
 }
 
-// the top levels (at most RADIUS_TOP nodes each) in one block, a barrier between levels
-constexpr int RADIUS_TOP = 256;  // one SM's FP64 pipe: only the small levels
-constexpr int RADIUS_TOP_THREADS = 256;
+// the top levels (at most RADIUS_TOP nodes each) in one cluster, a barrier between levels; a
+// cluster and not a block for its FP64 pipes
+constexpr int RADIUS_TOP = 1024;
+constexpr int RADIUS_TOP_THREADS = 256, RADIUS_TOP_BLOCKS = 8;
 struct RadiusLevels {
     int64_t start[66];  // level_start of levels lo .. hi + 1
     int lo, hi;
 };
-__global__ void __launch_bounds__(RADIUS_TOP_THREADS) k_radius_top(RadiusLevels RL, const int4 *child,
-                                                                   const double *comx, const double *comy, double *R) {
+__global__ void __cluster_dims__(RADIUS_TOP_BLOCKS, 1, 1) __launch_bounds__(RADIUS_TOP_THREADS)
+    k_radius_top(RadiusLevels RL, const int4 *child, const double *comx, const double *comy, double *R) {
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     for (int lv = RL.lo; lv <= RL.hi; lv++) {
         const int64_t s = RL.start[lv - RL.lo], e = RL.start[lv - RL.lo + 1];
-        for (int64_t q = s + threadIdx.x; q < e; q += RADIUS_TOP_THREADS) R[q] = radius_node(q, child, comx, comy, R);
-        __syncthreads();
+        for (int64_t q = s + blockIdx.x * RADIUS_TOP_THREADS + threadIdx.x; q < e;
+             q += RADIUS_TOP_BLOCKS * RADIUS_TOP_THREADS)
+            R[q] = radius_node(q, child, comx, comy, R);
+        cl.sync();
     }
 }
 
@@ -503,41 +508,68 @@ constexpr int MAC_CHUNK = 128;
 // Capacities are fixed for one attempt; a level that would exceed one sets its flag,
 // every later kernel of the attempt returns at once, and the host grows the arrays
 // and plans again.
-enum { PC_FAR = 0, PC_NEAR = 1, PC_NEAR_LAST = 2, PC_OVF = 3, PC_N = 4 };
+enum {
+    PC_FAR = 0, PC_NEAR = 1, PC_NEAR_LAST = 2, PC_OVF = 3,
+    PC_FAR0 = 4, PC_NEAR0 = 5,  // the totals before the level in work
+    PC_N = 6
+};
 enum { OVF_UNITS = 1, OVF_FAR = 2, OVF_NEAR = 4, OVF_CHAIN = 8 };
 
-__global__ void k_mac_nchunks(int64_t s, int64_t e, const int32_t *parent, const int32_t *near_cnt, int64_t *nch,
-                              const int64_t *ctr) {
-    if (ctr[PC_OVF]) return;
-    int64_t x = s + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (x > e) return;
-    if (x == e) { nch[e - s] = 0; return; }
-    int32_t P = parent[x];
-    int64_t cand = P >= 0 ? near_cnt[P] : 0;
-    nch[x - s] = (cand + MAC_CHUNK - 1) / MAC_CHUNK;
+// The level's units, chunks of the nodes' candidate lists (their parents' near lists), counted
+// and scanned by one cluster: uoff[x - s] the first unit of node x, uoff[e - s] their number.
+__device__ __forceinline__ int64_t mac_chunks(int32_t P, const int32_t *near_cnt) {
+    return P >= 0 ? ((int64_t)near_cnt[P] + MAC_CHUNK - 1) / MAC_CHUNK : 0;
 }
-
-// unit -> (node, chunk) for the level's U = uoff[e - s] units; zero count slots at U
-// so the count scans below end on the level totals
-__global__ void k_mac_units(int64_t s, int64_t e, const int64_t *uoff, int64_t ucap, int32_t *unode, int32_t *uchunk,
-                            int64_t *ufar, int64_t *unear, int64_t *ctr) {
+__global__ void __launch_bounds__(CS_THREADS) k_mac_units(int64_t s, int64_t e, const int32_t *parent,
+                                                          const int32_t *near_cnt, int64_t *uoff, int64_t ucap,
+                                                          int64_t *ctr) {
     if (ctr[PC_OVF]) return;
-    int64_t x = s + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const CsVec<1> all = cluster_scan<1>(
+        e - s, [&](int64_t i) { return CsVec<1>{{mac_chunks(parent[s + i], near_cnt)}}; },
+        [&](int64_t i, const CsVec<1> &p, const CsVec<1> &) { uoff[i] = p.v[0]; });
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        uoff[e - s] = all.v[0];
+        if (all.v[0] > ucap)
+            atomicOr(reinterpret_cast<unsigned long long *>(ctr + PC_OVF), (unsigned long long)OVF_UNITS);
+    }
+}
+// unit -> (node, chunk): over the whole GPU, as a wide halo node has dozens
+__global__ void k_mac_unit_nodes(int64_t s, int64_t e, const int64_t *uoff, int32_t *unode, int32_t *uchunk,
+                                 const int64_t *ctr) {
+    if (ctr[PC_OVF]) return;
+    const int64_t x = s + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= e) return;
-    const int64_t U = uoff[e - s];
-    if (U > ucap) {
-        if (x == s) atomicOr(reinterpret_cast<unsigned long long *>(ctr + PC_OVF), (unsigned long long)OVF_UNITS);
-        return;
-    }
-    if (x == s) {
-        ufar[U] = 0;
-        unear[U] = 0;
-    }
-    int64_t a = uoff[x - s], b = uoff[x - s + 1];
+    const int64_t a = uoff[x - s], b = uoff[x - s + 1];
     for (int64_t u = a; u < b; u++) {
         unode[u] = (int32_t)x;
         uchunk[u] = (int32_t)(u - a);
     }
+}
+
+// After the counting pass, by one cluster: the units' offsets within the level (ufo, uno; one
+// more entry, the totals) and the running totals moved past the level.
+__global__ void __launch_bounds__(CS_THREADS) k_mac_offsets(const int64_t *Uptr, const int64_t *ufar,
+                                                            const int64_t *unear, int64_t *ufo, int64_t *uno,
+                                                            int64_t far_cap, int64_t near_cap, int64_t *ctr) {
+    if (ctr[PC_OVF]) return;
+    const int64_t U = *Uptr, far0 = ctr[PC_FAR], near0 = ctr[PC_NEAR];
+    const CsVec<2> all = cluster_scan<2>(
+        U, [&](int64_t u) { return CsVec<2>{{ufar[u], unear[u]}}; },
+        [&](int64_t u, const CsVec<2> &p, const CsVec<2> &) {
+            ufo[u] = p.v[0];
+            uno[u] = p.v[1];
+        });
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;  // all threads have read the totals before the scan's barriers
+    ufo[U] = all.v[0];
+    uno[U] = all.v[1];
+    ctr[PC_FAR0] = far0;
+    ctr[PC_NEAR0] = near0;
+    ctr[PC_FAR] = far0 + all.v[0];
+    ctr[PC_NEAR] = near0 + all.v[1];
+    ctr[PC_NEAR_LAST] = all.v[1];
+    const unsigned long long bad =
+        (far0 + all.v[0] > far_cap ? OVF_FAR : 0) | (near0 + all.v[1] > near_cap ? OVF_NEAR : 0);
+    if (bad) atomicOr(reinterpret_cast<unsigned long long *>(ctr + PC_OVF), bad);
 }
 
 __device__ __forceinline__ bool mac_far_v(const float4 A, float Ra, const float4 B, float Rb, float theta2) {
@@ -551,16 +583,16 @@ __device__ __forceinline__ bool mac_far_v(const float4 A, float Ra, const float4
 // pass 0: per-unit counts (ufar, unear), and each candidate's decisions in dec (one word
 // per lane and unit: byte k holds candidate k * 32 + lane's far mask in the low nibble and
 // its near mask in the high one, one bit per child slot); pass 1: the children written at
-// the running totals plus the per-unit offsets, from dec without testing again.  A
-// grid-stride loop over the level's units, one warp per unit; each lane loads its
+// the running totals plus the per-unit offsets, from dec without testing again, and every
+// node's list starts and counts.  A grid-stride loop over the level's units, one warp per unit; each lane loads its
 // MAC_ROUNDS candidates, then their children, then tests them, so that the gathers of a
 // unit are in flight together.
 constexpr int MAC_ROUNDS = MAC_CHUNK / 32;
 __global__ void __launch_bounds__(128) k_mac(const int64_t *Uptr, int pass, const int32_t *unode,
                                              const int32_t *uchunk, const int32_t *parent, const int4 *child,
                                              const float4 *hl, const float *R32, float theta2,
-                                             const int64_t *near_start, const int32_t *near_cnt,
-                                             const int32_t *near_idx_in, int64_t *ufar, int64_t *unear,
+                                             int64_t *near_start, int32_t *near_cnt, int64_t *far_start,
+                                             int32_t *far_cnt, const int32_t *near_idx_in, int64_t *ufar, int64_t *unear,
                                              int32_t *far_idx, int32_t *near_idx, int64_t far_cap, int64_t near_cap,
                                              uint32_t *dec, int64_t *ctr) {
     const unsigned full = 0xffffffffu;
@@ -568,7 +600,7 @@ __global__ void __launch_bounds__(128) k_mac(const int64_t *Uptr, int pass, cons
     const int64_t n_units = *Uptr;
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    const int64_t far0 = pass ? ctr[PC_FAR] : 0, near0 = pass ? ctr[PC_NEAR] : 0;
+    const int64_t far0 = pass ? ctr[PC_FAR0] : 0, near0 = pass ? ctr[PC_NEAR0] : 0;
     for (int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n_units; u += nwarps) {
         const int32_t x = unode[u];
         const int32_t P = parent[x];
@@ -587,6 +619,13 @@ __global__ void __launch_bounds__(128) k_mac(const int64_t *Uptr, int pass, cons
             if (bad) {
                 if (lane == 0) atomicOr(reinterpret_cast<unsigned long long *>(ctr + PC_OVF), bad);
                 continue;
+            }
+            if (uchunk[u] == 0 && lane == 0) {  // the node's first unit (every node has one: it is near itself)
+                const int64_t last = u + mac_chunks(P, near_cnt);
+                far_start[x] = fb;
+                near_start[x] = nb;
+                far_cnt[x] = (int32_t)(ufar[last] - ufar[u]);
+                near_cnt[x] = (int32_t)(unear[last] - unear[u]);
             }
         }
         int32_t cand[MAC_ROUNDS];
@@ -859,28 +898,6 @@ __global__ void __launch_bounds__(PLAN_SMALL_THREADS) k_mac_small_levels(
         }
         __syncthreads();
     }
-}
-
-// per node of the level: start (running total + first unit's offset) and count
-__global__ void k_mac_node_lists(int64_t s, int64_t e, const int64_t *uoff, const int64_t *ufo, const int64_t *uno,
-                                 const int64_t *ctr, int64_t *fstart, int32_t *fcnt, int64_t *nstart, int32_t *ncnt) {
-    if (ctr[PC_OVF]) return;
-    int64_t x = s + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= e) return;
-    int64_t a = uoff[x - s], b = uoff[x - s + 1];
-    fstart[x] = ctr[PC_FAR] + ufo[a];
-    nstart[x] = ctr[PC_NEAR] + uno[a];
-    fcnt[x] = (int32_t)(ufo[b] - ufo[a]);
-    ncnt[x] = (int32_t)(uno[b] - uno[a]);
-}
-
-// after a level: advance the running totals by the level's far / near counts
-__global__ void k_mac_advance(const int64_t *Uptr, const int64_t *ufo, const int64_t *uno, int64_t *ctr) {
-    if (ctr[PC_OVF]) return;
-    const int64_t U = *Uptr;
-    ctr[PC_FAR] += ufo[U];
-    ctr[PC_NEAR] += uno[U];
-    ctr[PC_NEAR_LAST] = uno[U];
 }
 
 // ---------------------------------------------------------------- balanced build
@@ -1239,7 +1256,7 @@ int gx_plan_accurate(gx_ctx *ctx) {
             ctx->launches++;
             lv = chain + 1;
         }
-        int top = ctx->n_levels;  // levels top .. n_levels - 1 go to one block
+        int top = ctx->n_levels;  // levels top .. n_levels - 1 go to one cluster
         while (top - 1 >= lv && ctx->level_start[top] - ctx->level_start[top - 1] <= RADIUS_TOP && top - 1 > ctx->n_levels - 65)
             top--;
         for (; lv < top; lv++) {
@@ -1254,7 +1271,7 @@ int gx_plan_accurate(gx_ctx *ctx) {
             RL.lo = top;
             RL.hi = ctx->n_levels - 1;
             for (int l = RL.lo; l <= RL.hi + 1; l++) RL.start[l - RL.lo] = ctx->level_start[l];
-            k_radius_top<<<1, RADIUS_TOP_THREADS, 0, ctx->stream>>>(RL, dptr<int4>(ctx->child),
+            k_radius_top<<<RADIUS_TOP_BLOCKS, RADIUS_TOP_THREADS, 0, ctx->stream>>>(RL, dptr<int4>(ctx->child),
                                                                    dptr<double>(ctx->comx), dptr<double>(ctx->comy), R);
             ctx->launches++;
         }
@@ -1272,19 +1289,19 @@ int gx_plan_accurate(gx_ctx *ctx) {
                                           ctx->hint_near + ctx->hint_near / 8});
     GX_TRY(gx_ensure(ctx, ctx->plan_ctr, sizeof(int64_t) * PC_N));
     int64_t *ctr = dptr<int64_t>(ctx->plan_ctr);
-    int64_t hc[PC_N] = {0, 0, 0, 0};
+    int64_t hc[PC_N] = {};
     const unsigned gmac = (unsigned)(ctx->sm_count > 0 ? ctx->sm_count * 16 : 2432);  // grid-stride k_mac
     for (int attempt = 0;; attempt++) {
         if (attempt == 8) return gx_fail(ctx, GX_ERR_CAP_EXCEEDED, "accurate plan: list storage keeps overflowing");
         const int64_t ucap = ctx->mac_ucap;
         GX_TRY(gx_ensure(ctx, ctx->far_idx, sizeof(int32_t) * (size_t)far_cap));
         GX_TRY(gx_ensure(ctx, ctx->near_idx, sizeof(int32_t) * (size_t)near_cap));
-        GX_TRY(gx_ensure(ctx, ctx->scratch_a, sizeof(int64_t) * (size_t)(cmax + 1) * 2));
+        GX_TRY(gx_ensure(ctx, ctx->scratch_a, sizeof(int64_t) * (size_t)(cmax + 1)));
         GX_TRY(gx_ensure(ctx, ctx->scratch_b, sizeof(int32_t) * (size_t)(ucap + 1) * 2));
         GX_TRY(gx_ensure(ctx, ctx->scratch_e, sizeof(int64_t) * (size_t)(ucap + 1) * 4));
         GX_TRY(gx_ensure(ctx, ctx->scratch_d, sizeof(uint32_t) * 32 * (size_t)(ucap + 1)));
         uint32_t *dec = dptr<uint32_t>(ctx->scratch_d);
-        int64_t *nch = dptr<int64_t>(ctx->scratch_a), *uoff = nch + (cmax + 1);
+        int64_t *uoff = dptr<int64_t>(ctx->scratch_a);
         int32_t *unode = dptr<int32_t>(ctx->scratch_b), *uchunk = unode + (ucap + 1);
         int64_t *ufar = dptr<int64_t>(ctx->scratch_e), *unear = ufar + (ucap + 1), *ufo = unear + (ucap + 1),
                 *uno = ufo + (ucap + 1);
@@ -1324,26 +1341,19 @@ int gx_plan_accurate(gx_ctx *ctx) {
         for (int lv = lv_big; lv >= lv_low; lv--) {
             const int64_t s = ctx->level_start[lv], e = ctx->level_start[lv + 1], c = e - s;
             // units: chunks of each node's candidate list
-            k_mac_nchunks<<<gx_blocks(c + 1, 256), 256, 0, ctx->stream>>>(s, e, dptr<int32_t>(ctx->parent), ncnt, nch,
-                                                                         ctr);
-            GX_TRY(gx_exclusive_scan_i64(ctx, nch, uoff, c + 1));
+            GX_TRY(cs_launch(ctx, c, k_mac_units, s, e, dptr<int32_t>(ctx->parent), ncnt, uoff, ucap, ctr));
+            k_mac_unit_nodes<<<gx_blocks(c, 256), 256, 0, ctx->stream>>>(s, e, uoff, unode, uchunk, ctr);
             const int64_t *Ud = uoff + c;  // the level's unit count, on the device
-            k_mac_units<<<gx_blocks(c, 256), 256, 0, ctx->stream>>>(s, e, uoff, ucap, unode, uchunk, ufar, unear,
-                                                                   ctr);
             k_mac<<<gmac, 128, 0, ctx->stream>>>(Ud, 0, unode, uchunk, dptr<int32_t>(ctx->parent),
-                                                 dptr<int4>(ctx->child), hl, R32, theta2, nstart, ncnt,
+                                                 dptr<int4>(ctx->child), hl, R32, theta2, nstart, ncnt, fstart, fcnt,
                                                  dptr<int32_t>(ctx->near_idx), ufar, unear, nullptr, nullptr, far_cap,
                                                  near_cap, dec, ctr);
-            // ufar, unear -> ufo, uno (arrays ucap + 1 apart) in one scan
-            GX_TRY(gx_exclusive_scan_i64_devn_multi(ctx, ufar, ufo, 2, ucap + 1, Ud, 1, ucap + 1));
+            GX_TRY(cs_launch(ctx, CS_MAX_N, k_mac_offsets, Ud, ufar, unear, ufo, uno, far_cap, near_cap, ctr));
             k_mac<<<gmac, 128, 0, ctx->stream>>>(Ud, 1, unode, uchunk, dptr<int32_t>(ctx->parent),
-                                                 dptr<int4>(ctx->child), hl, R32, theta2, nstart, ncnt,
+                                                 dptr<int4>(ctx->child), hl, R32, theta2, nstart, ncnt, fstart, fcnt,
                                                  dptr<int32_t>(ctx->near_idx), ufo, uno, dptr<int32_t>(ctx->far_idx),
                                                  dptr<int32_t>(ctx->near_idx), far_cap, near_cap, dec, ctr);
-            k_mac_node_lists<<<gx_blocks(c, 256), 256, 0, ctx->stream>>>(s, e, uoff, ufo, uno, ctr, fstart, fcnt,
-                                                                        nstart, ncnt);
-            k_mac_advance<<<1, 1, 0, ctx->stream>>>(Ud, ufo, uno, ctr);
-            ctx->launches += 6;
+            ctx->launches += 3;
             GX_CUDA(ctx, cudaGetLastError());
         }
         if (lv_low >= 2) {
@@ -1408,19 +1418,20 @@ __device__ __forceinline__ int near_kind(const float4 A, float Ra, const float4 
 constexpr int NS_CHUNK = 256;
 constexpr int NS_ROUNDS = NS_CHUNK / 32;
 
-__global__ void k_ns_nchunks(int64_t nl, const int32_t *ncnt, int64_t *nch) {
-    const int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (a > nl) return;
-    nch[a] = a == nl ? 0 : (ncnt[a] + NS_CHUNK - 1) / NS_CHUNK;
-}
-
-__global__ void k_ns_units(int64_t nl, const int32_t *ncnt, const int64_t *uoff, int4 *unit, int32_t *split_cnt) {
-    const int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= nl) return;
-    const int32_t c = ncnt[a];
-    const int64_t u0 = uoff[a];
-    for (int32_t j = 0; j * NS_CHUNK < c; j++) unit[u0 + j] = make_int4((int32_t)a, j, min(NS_CHUNK, c - j * NS_CHUNK), 0);
-    if (c == 0) split_cnt[2 * a] = split_cnt[2 * a + 1] = 0;  // no unit writes them
+// unit -> (leaf, chunk, entries), by one cluster; uoff[nl]: their number
+__global__ void __launch_bounds__(CS_THREADS) k_ns_units(int64_t nl, const int32_t *ncnt, int64_t *uoff, int4 *unit,
+                                                         int32_t *split_cnt) {
+    const CsVec<1> all = cluster_scan<1>(
+        nl, [&](int64_t a) { return CsVec<1>{{(ncnt[a] + NS_CHUNK - 1) / NS_CHUNK}}; },
+        [&](int64_t a, const CsVec<1> &p, const CsVec<1> &) {
+            const int32_t c = ncnt[a];
+            const int64_t u0 = p.v[0];
+            uoff[a] = u0;
+            for (int32_t j = 0; j * NS_CHUNK < c; j++)
+                unit[u0 + j] = make_int4((int32_t)a, j, min(NS_CHUNK, c - j * NS_CHUNK), 0);
+            if (c == 0) split_cnt[2 * a] = split_cnt[2 * a + 1] = 0;  // no unit writes them
+        });
+    if (blockIdx.x == 0 && threadIdx.x == 0) uoff[nl] = all.v[0];
 }
 
 __global__ void __launch_bounds__(128) k_ns_kinds(const int64_t *__restrict__ Ud, const int4 *__restrict__ unit,
@@ -1553,14 +1564,12 @@ int gx_plan_near_split(gx_ctx *ctx) {
         const int64_t ncap = (int64_t)(ctx->near_idx.bytes / sizeof(int32_t));
         const int64_t ucap = nl + ncap / NS_CHUNK + 1;
         GX_TRY(gx_ensure(ctx, ctx->scratch_f, sizeof(int32_t) * (size_t)(ncap + 1)));
-        GX_TRY(gx_ensure(ctx, ctx->scratch_a, sizeof(int64_t) * 2 * (size_t)(nl + 1)));
+        GX_TRY(gx_ensure(ctx, ctx->scratch_a, sizeof(int64_t) * (size_t)(nl + 1)));
         GX_TRY(gx_ensure(ctx, ctx->scratch_b, sizeof(int4) * (size_t)ucap));
         GX_TRY(gx_ensure(ctx, ctx->scratch_d, sizeof(int4) * (size_t)ucap));
-        int64_t *nch = dptr<int64_t>(ctx->scratch_a), *uoff = nch + (nl + 1);
+        int64_t *uoff = dptr<int64_t>(ctx->scratch_a);
         int4 *unit = dptr<int4>(ctx->scratch_b), *ucnt = dptr<int4>(ctx->scratch_d);
-        k_ns_nchunks<<<gx_blocks(nl + 1, 256), 256, 0, ctx->stream>>>(nl, ncnt, nch);
-        GX_TRY(gx_exclusive_scan_i64(ctx, nch, uoff, nl + 1));
-        k_ns_units<<<gx_blocks(nl, 256), 256, 0, ctx->stream>>>(nl, ncnt, uoff, unit, dptr<int32_t>(ctx->split_cnt));
+        GX_TRY(cs_launch(ctx, nl, k_ns_units, nl, ncnt, uoff, unit, dptr<int32_t>(ctx->split_cnt)));
         const unsigned g = (unsigned)(ctx->sm_count > 0 ? ctx->sm_count * 16 : 2432);  // grid-stride, 4 warps a block
         k_ns_kinds<<<g, 128, 0, ctx->stream>>>(uoff + nl, unit, nstart, dptr<int32_t>(ctx->near_idx),
                                                dptr<int32_t>(ctx->scratch_f), dptr<float4>(ctx->comhl),
@@ -1568,7 +1577,7 @@ int gx_plan_near_split(gx_ctx *ctx) {
         k_ns_write<<<g, 128, 0, ctx->stream>>>(uoff + nl, unit, uoff, nstart, dptr<int32_t>(ctx->scratch_f), ucnt,
                                                dptr<int32_t>(ctx->near_idx), ncnt, dptr<int32_t>(ctx->split_cnt),
                                                dptr<unsigned long long>(ctx->split_tot));
-        ctx->launches += 4;
+        ctx->launches += 2;
     }
     GX_CUDA(ctx, cudaGetLastError());
     return GX_OK;
@@ -1616,21 +1625,38 @@ __global__ void k_comhl(int64_t nn, const double *comx, const double *comy, floa
 // per leaf: number of items; start/count from either list layout.  With the near-list
 // split (split != null) the leaf's P2P items are followed by its M2P items, whose
 // source count is stored negated; split[2a] is the leaf's M2P count.
-__global__ void k_items_count(int64_t nl, int K, int KM, const int64_t *start, const int32_t *cnt, const int32_t *split,
-                              int64_t *nitems) {
-    int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (a > nl) return;
-    if (a == nl) { nitems[a] = 0; return; }
-    int64_t c = cnt ? cnt[a] : start[a + 1] - start[a];
-    int64_t cm = split ? split[2 * a] : 0;
-    nitems[a] = (c + K - 1) / K + (cm + KM - 1) / KM;
-}
-
-// per leaf: number of M2P items (the compact list the M2P kernel runs over)
-__global__ void k_m2p_items_count(int64_t nl, int KM, const int32_t *split, int64_t *n) {
-    int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (a > nl) return;
-    n[a] = a == nl ? 0 : (split[2 * a] + KM - 1) / KM;
+// Per leaf, scanned together by one cluster: its work items (K source leaves each of its P2P
+// sources, KM of its M2P ones), its M2P items, its P2L units (of at most GX_P2L_UNIT source
+// leaves) and with the body-level P2L its units of at most GX_BODY_UNIT of its P2P rows.
+// Each array's entry nl is the total; tot receives all four.
+__global__ void __launch_bounds__(CS_THREADS) k_item_offsets(int64_t nl, int K, int KM, const int64_t *start,
+                                                             const int32_t *cnt, const int32_t *split, int body,
+                                                             int64_t *off, int64_t *m2p_off, int64_t *leaf_u,
+                                                             int64_t *body_u, int64_t *tot) {
+    const CsVec<4> all = cluster_scan<4>(
+        nl,
+        [&](int64_t a) {
+            const int64_t c = cnt ? cnt[a] : start[a + 1] - start[a];
+            const int64_t cm = split ? split[2 * a] : 0, cl = split ? split[2 * a + 1] : 0, m = (cm + KM - 1) / KM;
+            return CsVec<4>{{(c + K - 1) / K + m, m, (cl + GX_P2L_UNIT - 1) / GX_P2L_UNIT,
+                             body ? (c + GX_BODY_UNIT - 1) / GX_BODY_UNIT : 0}};
+        },
+        [&](int64_t a, const CsVec<4> &p, const CsVec<4> &) {
+            off[a] = p.v[0];
+            if (split) {
+                m2p_off[a] = p.v[1];
+                leaf_u[a] = p.v[2];
+                if (body) body_u[a] = p.v[3];
+            }
+        });
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    off[nl] = all.v[0];
+    if (split) {
+        m2p_off[nl] = all.v[1];
+        leaf_u[nl] = all.v[2];
+        if (body) body_u[nl] = all.v[3];
+    }
+    for (int k = 0; k < 4; k++) tot[k] = all.v[k];
 }
 
 // one warp per leaf, lanes over its items: the widest halo leaves have ~1000 items
@@ -1658,23 +1684,10 @@ __global__ void k_items_fill(int64_t nl, int K, int KM, const int64_t *start, co
     }
 }
 
-// P2L units: per leaf the number of units of at most GX_P2L_UNIT source leaves (its P2L
-// sources follow its P2P and M2P sources), and with the body-level P2L the number of
-// units of at most GX_BODY_UNIT of its P2P rows (the masked bodies: length stored
-// negated); then unit -> (leaf, first, length), every leaf-level unit (leaf by leaf)
-// before every body-level one, so that each kernel's grid covers its own units only
-__global__ void k_p2l_units_count(int64_t nl, const int32_t *split, int64_t *nunits) {
-    int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (a > nl) return;
-    nunits[a] = a == nl ? 0 : (split[2 * a + 1] + GX_P2L_UNIT - 1) / GX_P2L_UNIT;
-}
-
-__global__ void k_body_units_count(int64_t nl, const int32_t *cnt, int64_t *nunits) {
-    int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (a > nl) return;
-    nunits[a] = a == nl ? 0 : (cnt[a] + GX_BODY_UNIT - 1) / GX_BODY_UNIT;
-}
-
+// P2L units (a leaf's P2L sources follow its P2P and M2P sources; a body-level unit is some of
+// its P2P rows, its length stored negated): unit -> (leaf, first, length), every leaf-level
+// unit (leaf by leaf) before every body-level one, so that each kernel's grid covers its own
+// units only
 __global__ void k_p2l_units_fill(int64_t nl, const int64_t *start, const int32_t *cnt, const int32_t *split, int body,
                                  const int64_t *leaf_u, const int64_t *body_u, int32_t *uleaf, int64_t *ustart,
                                  int32_t *ulen) {
@@ -1874,42 +1887,20 @@ int gx_plan_items(gx_ctx *ctx, bool accurate) {
     const int K = p2p_item_leaves(ctx, accurate ? ctx->n_near_pairs : ctx->n_p2p_pairs, accurate);
     const int KM = m2p_item_leaves(K);
     GX_TRY(gx_ensure(ctx, I.off, sizeof(int64_t) * (size_t)(nl + 1)));
-    GX_TRY(gx_ensure(ctx, ctx->scratch_c, sizeof(int64_t) * (size_t)(nl + 1)));
-    int64_t *nit = dptr<int64_t>(ctx->scratch_c);
-    k_items_count<<<gx_blocks(nl + 1, 256), 256, 0, ctx->stream>>>(nl, K, KM, start, cnt, scnt, nit);
-    GX_TRY(gx_exclusive_scan_i64(ctx, nit, dptr<int64_t>(I.off), nl + 1));
-    int64_t tot[5] = {0, 0, 0, 0, 0};
+    GX_TRY(gx_ensure(ctx, ctx->scratch_c, sizeof(int64_t) * 4));
+    int64_t *dtot = dptr<int64_t>(ctx->scratch_c);
+    int64_t tot[5] = {0, 0, 0, 0, 0};  // items, M2P items, P2L units, body-level units, M2L units
     unsigned long long stot[4] = {0, 0, 0, 0};
     gx_ctx::P2LUnits &PU = ctx->p2l_units;
     if (split) {
         GX_TRY(gx_ensure(ctx, ctx->m2p_off, sizeof(int64_t) * (size_t)(nl + 1)));
-        GX_TRY(gx_ensure(ctx, ctx->scratch_e, sizeof(int64_t) * (size_t)(nl + 1)));  // free after the plan
-        int64_t *nm = dptr<int64_t>(ctx->scratch_e);
-        k_m2p_items_count<<<gx_blocks(nl + 1, 256), 256, 0, ctx->stream>>>(nl, KM, scnt, nm);
-        GX_TRY(gx_exclusive_scan_i64(ctx, nm, dptr<int64_t>(ctx->m2p_off), nl + 1));
-        GX_CUDA(ctx, cudaMemcpyAsync(&tot[3], dptr<int64_t>(ctx->m2p_off) + nl, sizeof(int64_t),
-                                     cudaMemcpyDeviceToHost, ctx->stream));
-        ctx->launches++;
         GX_TRY(gx_ensure(ctx, PU.leaf_u, sizeof(int64_t) * (size_t)(nl + 1)));
-        GX_TRY(gx_ensure(ctx, ctx->scratch_b, sizeof(int64_t) * (size_t)(nl + 1)));
-        int64_t *npu = dptr<int64_t>(ctx->scratch_b);
-        k_p2l_units_count<<<gx_blocks(nl + 1, 256), 256, 0, ctx->stream>>>(nl, scnt, npu);
-        GX_TRY(gx_exclusive_scan_i64(ctx, npu, dptr<int64_t>(PU.leaf_u), nl + 1));
-        GX_CUDA(ctx, cudaMemcpyAsync(&tot[2], dptr<int64_t>(PU.leaf_u) + nl, sizeof(int64_t), cudaMemcpyDeviceToHost,
-                                     ctx->stream));
         GX_TRY(gx_ensure(ctx, PU.body_u, sizeof(int64_t) * (size_t)(nl + 1)));
-        if (body) {
-            k_body_units_count<<<gx_blocks(nl + 1, 256), 256, 0, ctx->stream>>>(nl, cnt, npu);
-            GX_TRY(gx_exclusive_scan_i64(ctx, npu, dptr<int64_t>(PU.body_u), nl + 1));
-            GX_CUDA(ctx, cudaMemcpyAsync(&tot[4], dptr<int64_t>(PU.body_u) + nl, sizeof(int64_t),
-                                         cudaMemcpyDeviceToHost, ctx->stream));
-            ctx->launches++;
-        }
         GX_CUDA(ctx, cudaMemcpyAsync(stot, ctx->split_tot.p, sizeof(stot), cudaMemcpyDeviceToHost, ctx->stream));
-        ctx->launches++;
     }
-    GX_CUDA(ctx, cudaMemcpyAsync(&tot[0], dptr<int64_t>(I.off) + nl, sizeof(int64_t), cudaMemcpyDeviceToHost,
-                                 ctx->stream));
+    GX_TRY(cs_launch(ctx, nl, k_item_offsets, nl, K, KM, start, cnt, scnt, body ? 1 : 0, dptr<int64_t>(I.off),
+                     dptr<int64_t>(ctx->m2p_off), dptr<int64_t>(PU.leaf_u), dptr<int64_t>(PU.body_u), dtot));
+    GX_CUDA(ctx, cudaMemcpyAsync(tot, dtot, sizeof(int64_t) * 4, cudaMemcpyDeviceToHost, ctx->stream));
     gx_ctx::M2LUnits &U = ctx->m2l_units;
     const int64_t *fstart = accurate ? dptr<int64_t>(ctx->far_off) : nullptr;
     const int32_t *fcnt = accurate ? reinterpret_cast<const int32_t *>(fstart + nn) : nullptr;
@@ -1919,7 +1910,7 @@ int gx_plan_items(gx_ctx *ctx, bool accurate) {
         int64_t *nu = dptr<int64_t>(ctx->m2l_cnt);
         k_m2l_units_count<<<gx_blocks(nn + 1, 256), 256, 0, ctx->stream>>>(nn, fcnt, nu);
         GX_TRY(gx_exclusive_scan_i64(ctx, nu, dptr<int64_t>(U.node_u), nn + 1));
-        GX_CUDA(ctx, cudaMemcpyAsync(&tot[1], dptr<int64_t>(U.node_u) + nn, sizeof(int64_t), cudaMemcpyDeviceToHost,
+        GX_CUDA(ctx, cudaMemcpyAsync(&tot[4], dptr<int64_t>(U.node_u) + nn, sizeof(int64_t), cudaMemcpyDeviceToHost,
                                      ctx->stream));
         ctx->launches++;
     }
@@ -1929,16 +1920,16 @@ int gx_plan_items(gx_ctx *ctx, bool accurate) {
     GX_TRY(gx_ensure(ctx, I.leaf, sizeof(int32_t) * (size_t)(tot[0] + 1)));
     GX_TRY(gx_ensure(ctx, I.qb, sizeof(int64_t) * (size_t)(tot[0] + 1)));
     GX_TRY(gx_ensure(ctx, I.nq, sizeof(int32_t) * (size_t)(tot[0] + 1)));
-    if (split) GX_TRY(gx_ensure(ctx, ctx->m2p_list, sizeof(int32_t) * (size_t)(tot[3] + 1)));
+    if (split) GX_TRY(gx_ensure(ctx, ctx->m2p_list, sizeof(int32_t) * (size_t)(tot[1] + 1)));
     k_items_fill<<<gx_blocks(nl * 32, 256), 256, 0, ctx->stream>>>(
         nl, K, KM, start, cnt, scnt, dptr<int64_t>(I.off), dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb), dptr<int32_t>(I.nq),
         split ? dptr<int64_t>(ctx->m2p_off) : nullptr, split ? dptr<int32_t>(ctx->m2p_list) : nullptr);
-    ctx->launches += 2;
+    ctx->launches++;
     I.n = tot[0];
     if (accurate) {
         // the near-list split's state belongs to the ACCURATE plan: a REF plan made in
         // between (its own items) leaves it as it is
-        ctx->n_m2p_items = split ? tot[3] : 0;
+        ctx->n_m2p_items = split ? tot[1] : 0;
         PU.n = PU.n_leafu = PU.n_body = 0;
         ctx->n_m2p_pairs = ctx->n_p2l_pairs = 0;
     }
@@ -1946,7 +1937,7 @@ int gx_plan_items(gx_ctx *ctx, bool accurate) {
         ctx->n_near_pairs = (int64_t)stot[0];
         ctx->n_m2p_pairs = (int64_t)stot[1];
         ctx->n_p2l_pairs = (int64_t)stot[2];
-        const int64_t npu = tot[2] + (body ? tot[4] : 0);
+        const int64_t npu = tot[2] + (body ? tot[3] : 0);
         GX_TRY(gx_ensure(ctx, PU.leaf, sizeof(int32_t) * (size_t)(npu + 1)));
         GX_TRY(gx_ensure(ctx, PU.start, sizeof(int64_t) * (size_t)(npu + 1)));
         GX_TRY(gx_ensure(ctx, PU.len, sizeof(int32_t) * (size_t)(npu + 1)));
@@ -1956,10 +1947,10 @@ int gx_plan_items(gx_ctx *ctx, bool accurate) {
         ctx->launches++;
         PU.n = npu;
         PU.n_leafu = tot[2];
-        PU.n_body = body ? tot[4] : 0;
+        PU.n_body = body ? tot[3] : 0;
     }
     if (accurate) {
-        const int64_t nun = tot[1];
+        const int64_t nun = tot[4];
         GX_TRY(gx_ensure(ctx, U.node, sizeof(int32_t) * (size_t)(nun + 1)));
         GX_TRY(gx_ensure(ctx, U.start, sizeof(int64_t) * (size_t)(nun + 1)));
         GX_TRY(gx_ensure(ctx, U.len, sizeof(int32_t) * (size_t)(nun + 1)));

@@ -1,11 +1,13 @@
 // gx_scan.cu -- device-wide exclusive scan and a stable LSD radix sort.
 //
-// The radix sort replaces the stable `indices.sort_by_key(|&i| keys[i])` of
+// Up to 131,072 entries a scan is one launch (gx_cluster_scan.cuh), above that
+// reduce-then-scan in three.  The radix sort replaces the stable `indices.sort_by_key(|&i| keys[i])` of
 // Tree::build (galax-core/src/lib.rs:192).  It is a three-kernel
 // reduce-then-scan design: no kernel waits on another CTA, so there is no
 // inter-block spin anywhere.  Stability: within a tile each warp owns a
 // contiguous run of 256 items and ranks them in index order with
 // __match_any_sync; warps and tiles are ordered by the digit-major offset scan.
+#include "gx_cluster_scan.cuh"
 #include "gx_internal.cuh"
 
 namespace {
@@ -114,14 +116,10 @@ __device__ __forceinline__ int64_t dev_len(const int64_t *n_dev, int64_t n_add, 
     return n < n_cap ? n : n_cap;
 }
 
-// blockIdx.y selects one of gridDim.y arrays: in + y * stride, out + y * stride, and
-// the block sums of array y at sums + y * (gridDim.x + 1)
-__global__ void k_scan_sums_dn(const int64_t *in, const int64_t *n_dev, int64_t n_add, int64_t n_cap, int64_t *sums,
-                               int64_t stride) {
+__global__ void k_scan_sums_dn(const int64_t *in, const int64_t *n_dev, int64_t n_add, int64_t n_cap,
+                               int64_t *sums) {
     __shared__ int64_t tot;
     const int64_t n = dev_len(n_dev, n_add, n_cap);
-    in += blockIdx.y * stride;
-    sums += blockIdx.y * (int64_t)(gridDim.x + 1);
     int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
     int64_t s = 0;
     if (base < n)
@@ -133,20 +131,12 @@ __global__ void k_scan_sums_dn(const int64_t *in, const int64_t *n_dev, int64_t 
     if (threadIdx.x == 0) sums[blockIdx.x] = tot;
 }
 
-__global__ void k_scan_single_dn(int64_t *sums, int64_t nb, int64_t *total) {
-    const int64_t y = blockIdx.x;
-    scan_single_block<int64_t>(sums + y * (nb + 1), nb, total ? total + y : sums + y * (nb + 1) + nb);
-}
-
 __global__ void k_scan_apply_dn(const int64_t *in, int64_t *out, const int64_t *n_dev, int64_t n_add, int64_t n_cap,
-                                const int64_t *sums, int64_t stride) {
+                                const int64_t *sums) {
     __shared__ int64_t tot;
     const int64_t n = dev_len(n_dev, n_add, n_cap);
     int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
     if (base >= n) return;  // uniform per block
-    in += blockIdx.y * stride;
-    out += blockIdx.y * stride;
-    sums += blockIdx.y * (int64_t)(gridDim.x + 1);
     int64_t v[SCAN_ITEMS];
     int64_t s = 0;
     for (int k = 0; k < SCAN_ITEMS; k++) {
@@ -162,6 +152,17 @@ __global__ void k_scan_apply_dn(const int64_t *in, int64_t *out, const int64_t *
     }
 }
 
+// one array of n entries, or of min(*n_dev + n_add, n)
+template <class T>
+__global__ void __launch_bounds__(CS_THREADS) k_scan_cluster(const T *in, T *out, int64_t n, const int64_t *n_dev,
+                                                             int64_t n_add, T *total) {
+    const int64_t len = n_dev ? dev_len(n_dev, n_add, n) : n;
+    const CsVec<1> all = cluster_scan<1>(
+        len, [&](int64_t i) { return CsVec<1>{{(int64_t)in[i]}}; },
+        [&](int64_t i, const CsVec<1> &p, const CsVec<1> &) { out[i] = (T)p.v[0]; });
+    if (total && blockIdx.x == 0 && threadIdx.x == 0) *total = (T)all.v[0];
+}
+
 template <class T>
 int scan_impl(gx_ctx *ctx, const T *in, T *out, int64_t n, T *total_host) {
     if (n <= 0) {
@@ -171,6 +172,14 @@ int scan_impl(gx_ctx *ctx, const T *in, T *out, int64_t n, T *total_host) {
     int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
     GX_TRY(gx_ensure(ctx, ctx->scratch_g, sizeof(T) * (nb + 1)));
     T *sums = dptr<T>(ctx->scratch_g);
+    if (n <= CS_MAX_N) {
+        GX_TRY(cs_launch(ctx, n, k_scan_cluster<T>, in, out, n, nullptr, 0, sums + nb));
+        if (total_host) {
+            GX_CUDA(ctx, cudaMemcpyAsync(total_host, sums + nb, sizeof(T), cudaMemcpyDeviceToHost, ctx->stream));
+            GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        }
+        return GX_OK;
+    }
     k_scan_sums<T><<<(unsigned)nb, SCAN_THREADS, 0, ctx->stream>>>(in, n, sums);
     k_scan_single<T><<<1, SCAN_THREADS, 0, ctx->stream>>>(sums, nb, sums + nb);
     k_scan_apply<T><<<(unsigned)nb, SCAN_THREADS, 0, ctx->stream>>>(in, out, n, sums);
@@ -287,19 +296,14 @@ int gx_exclusive_scan_i64(gx_ctx *ctx, const int64_t *in, int64_t *out, int64_t 
 
 int gx_exclusive_scan_i64_devn(gx_ctx *ctx, const int64_t *in, int64_t *out, const int64_t *n_dev, int64_t n_add,
                                int64_t n_cap, int64_t *total_dev) {
-    return gx_exclusive_scan_i64_devn_multi(ctx, in, out, 1, 0, n_dev, n_add, n_cap, total_dev);
-}
-
-int gx_exclusive_scan_i64_devn_multi(gx_ctx *ctx, const int64_t *in, int64_t *out, int m, int64_t stride,
-                                     const int64_t *n_dev, int64_t n_add, int64_t n_cap, int64_t *total_dev) {
-    if (n_cap <= 0 || m <= 0) return GX_OK;
+    if (n_cap <= 0) return GX_OK;
+    if (n_cap <= CS_MAX_N) return cs_launch(ctx, n_cap, k_scan_cluster<int64_t>, in, out, n_cap, n_dev, n_add, total_dev);
     int64_t nb = (n_cap + SCAN_TILE - 1) / SCAN_TILE;
-    GX_TRY(gx_ensure(ctx, ctx->scratch_g, sizeof(int64_t) * (size_t)m * (nb + 1)));
+    GX_TRY(gx_ensure(ctx, ctx->scratch_g, sizeof(int64_t) * (size_t)(nb + 1)));
     int64_t *sums = dptr<int64_t>(ctx->scratch_g);
-    const dim3 grid((unsigned)nb, (unsigned)m);
-    k_scan_sums_dn<<<grid, SCAN_THREADS, 0, ctx->stream>>>(in, n_dev, n_add, n_cap, sums, stride);
-    k_scan_single_dn<<<(unsigned)m, SCAN_THREADS, 0, ctx->stream>>>(sums, nb, total_dev);
-    k_scan_apply_dn<<<grid, SCAN_THREADS, 0, ctx->stream>>>(in, out, n_dev, n_add, n_cap, sums, stride);
+    k_scan_sums_dn<<<(unsigned)nb, SCAN_THREADS, 0, ctx->stream>>>(in, n_dev, n_add, n_cap, sums);
+    k_scan_single<int64_t><<<1, SCAN_THREADS, 0, ctx->stream>>>(sums, nb, total_dev ? total_dev : sums + nb);
+    k_scan_apply_dn<<<(unsigned)nb, SCAN_THREADS, 0, ctx->stream>>>(in, out, n_dev, n_add, n_cap, sums);
     ctx->launches += 3;
     GX_CUDA(ctx, cudaGetLastError());
     return GX_OK;

@@ -10,6 +10,7 @@
 
 #include <algorithm>
 
+#include "gx_cluster_scan.cuh"
 #include "gx_internal.cuh"
 
 namespace {
@@ -376,8 +377,7 @@ __global__ void k_chain_rounds(int64_t *st, int64_t *level_start, int64_t nl, in
 // and of the groups begun, with nothing read from global memory; the thread that holds a
 // group's first node keeps the parent.  The groups and their order are those of the
 // multi-block rounds: a segment's nodes by fours.
-constexpr int RC_THREADS = 1024;
-constexpr int RC_MAX_BLOCKS = 16;
+constexpr int RC_THREADS = CS_THREADS;
 constexpr int RC_RUN = 8;  // nodes a thread holds at most: TS_CLUSTER nodes on 8 blocks
 static_assert(TS_CLUSTER <= 8 * RC_THREADS * RC_RUN, "a level fits the smaller cluster");
 
@@ -591,37 +591,6 @@ static int ensure_nodes(gx_ctx *ctx, int64_t need) {
     return GX_OK;
 }
 
-// k_rounds_cluster: one block while its threads hold the level, else 16 where the device
-// takes them, else the portable 8.
-static int launch_rounds_cluster(gx_ctx *ctx, int64_t *st, int64_t *lstart, int64_t cap, int64_t nl) {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at = {};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.blockDim = dim3(RC_THREADS);
-    cfg.stream = ctx->stream;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    if (ctx->rounds_blocks == 0) {
-        ctx->rounds_blocks = 8;
-        at.val.clusterDim.x = RC_MAX_BLOCKS;
-        cfg.gridDim = dim3(RC_MAX_BLOCKS);
-        int fit = 0;
-        if (cudaFuncSetAttribute(k_rounds_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&fit, k_rounds_cluster, &cfg) == cudaSuccess && fit > 0)
-            ctx->rounds_blocks = RC_MAX_BLOCKS;
-        cudaGetLastError();  // a device without the larger cluster is no error
-    }
-    const unsigned blocks = nl <= 2 * RC_THREADS ? 1 : (unsigned)ctx->rounds_blocks;
-    at.val.clusterDim.x = blocks;
-    cfg.gridDim = dim3(blocks);
-    GX_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_rounds_cluster, st, lstart, cap, (const uint64_t *)dptr<uint64_t>(ctx->keys),
-                                    (const int32_t *)dptr<int32_t>(ctx->bs), dptr<int32_t>(ctx->child),
-                                    dptr<int32_t>(ctx->parent)));
-    ctx->launches++;
-    return GX_OK;
-}
-
 // Builds nodes from leaf ranges already in scratch (rs, re as int32), using ctx->keys
 // (Morton keys of the tree-ordered bodies).
 static int build_from_ranges(gx_ctx *ctx, const int32_t *rs, const int32_t *re, int64_t nl) {
@@ -688,7 +657,8 @@ static int build_from_ranges(gx_ctx *ctx, const int32_t *rs, const int32_t *re, 
             // of large ones, four on a first build)
             k_mark_before<<<1, 1, 0, ctx->stream>>>(st);
             k_slots_clear<<<gx_blocks(cap - nl, 256), 256, 0, ctx->stream>>>(st, cap, dptr<int4>(ctx->child));
-            GX_TRY(launch_rounds_cluster(ctx, st, lstart, cap, nl));
+            GX_TRY(cs_launch(ctx, nl, k_rounds_cluster, st, lstart, cap, dptr<uint64_t>(ctx->keys),
+                             dptr<int32_t>(ctx->bs), dptr<int32_t>(ctx->child), dptr<int32_t>(ctx->parent)));
             const int large = nl > FIELDS_SMALL ? (ctx->hint_field_levels > 0 ? ctx->hint_field_levels : 4) : 0;
             const unsigned gf = gx_blocks(std::min<int64_t>(nl, TS_CLUSTER), 128);
             for (int k = 1; k <= large; k++)
