@@ -1,6 +1,8 @@
 // gx_api.cu -- the extern "C" boundary of libgalaxcu.so (declared in
 // include/galax_gb300.h).  Host-side orchestration only; all compute is in the
 // kernels of gx_tree.cu, gx_lists.cu, gx_fmm.cu and gx_kdk.cu.
+#include <unistd.h>
+
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -107,9 +109,52 @@ void gx_tree_plan_free(gx_tree_plan &t) {
 }
 
 static int sync_status(gx_ctx *ctx, unsigned *out) {
-    GX_CUDA(ctx, cudaMemcpyAsync(out, ctx->status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+    GX_CUDA(ctx, cudaMemcpyAsync(ctx->pin, ctx->status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
     GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    *out = *ctx->pin;
     return GX_OK;
+}
+
+// ---- host arrays read and written by kernels ----
+// On a host whose page tables the GPU shares (Grace: every host address is a device address,
+// over NVLink-C2C), a kernel reads or writes ordinary memory as it does page-locked memory.
+// For small arrays that saves the copies' calls: seven arrays of 10,000 doubles go in in 15 us
+// instead of 63 and out in 13 instead of 63; at 1,000,000 the copies run at the link's rate
+// either way.  The pages are touched by the host first (written back to, where the kernel
+// will write), so that an address that is not the caller's fails here as it would in a copy
+// and the GPU meets no page fault.
+constexpr int64_t GX_COPY_KERNEL = 262144;  // bodies moved by one kernel at most (the copy engines do more as fast)
+constexpr size_t GX_DIRECT_PAGES = 128;  // of an array; above, touching them costs what the copy does
+
+// The device address of a host array of bytes bytes, or null where it takes a copy: page-locked
+// memory (cudaHostAlloc or cudaHostRegister: its first and its last byte must resolve to the
+// same allocation, as a registered range shorter than the array would let a kernel run past
+// it), or few pages of ordinary memory on a host as above.
+static void *direct_host(const gx_ctx *ctx, const void *p, size_t bytes, bool write) {
+    if (!p || bytes == 0) return nullptr;
+    const char *first = static_cast<const char *>(p), *last = first + bytes - 1;
+    cudaPointerAttributes at{}, at_last{};
+    if (cudaPointerGetAttributes(&at, first) != cudaSuccess || cudaPointerGetAttributes(&at_last, last) != cudaSuccess) {
+        cudaGetLastError();  // pageable memory on older runtimes: not an error of the call
+        return nullptr;
+    }
+    if (at.type == cudaMemoryTypeHost) {
+        if (!at.devicePointer || at_last.type != cudaMemoryTypeHost ||
+            static_cast<const char *>(at_last.devicePointer) != static_cast<const char *>(at.devicePointer) + (bytes - 1))
+            return nullptr;
+        return at.devicePointer;
+    }
+    if (at.type != cudaMemoryTypeUnregistered || at_last.type != cudaMemoryTypeUnregistered || !ctx->host_pages)
+        return nullptr;
+    const size_t page = (size_t)ctx->host_pages;
+    if (bytes > GX_DIRECT_PAGES * page) return nullptr;
+    for (size_t k = 0;; k += page) {
+        volatile char *c = const_cast<volatile char *>(k < bytes ? first + k : last);
+        const char v = *c;
+        if (write) *c = v;
+        if (k >= bytes) break;
+    }
+    return const_cast<void *>(p);
 }
 
 extern "C" {
@@ -171,6 +216,15 @@ int gx_create(const gx_config *cfg, gx_ctx **out) {
         gx_destroy(ctx);
         return s;
     }
+    if (cudaMallocHost(&ctx->pin, 64) != cudaSuccess) {
+        cudaGetLastError();
+        gx_destroy(ctx);
+        return GX_ERR_ALLOC;
+    }
+    int pageable = 0, tables = 0;
+    cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, cfg->device);
+    cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, cfg->device);
+    if (pageable && tables) ctx->host_pages = sysconf(_SC_PAGESIZE);
     cudaMemsetAsync(ctx->status.p, 0, 64, ctx->stream);
     if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
         gx_destroy(ctx);
@@ -199,6 +253,7 @@ int gx_destroy(gx_ctx *ctx) {
     for (DevBuf *b : bufs) free_buf(*b);
     for (DevBuf &b : ctx->body_alt) free_buf(b);
     for (gx_tree_plan &t : ctx->tp_cache) gx_tree_plan_free(t);
+    if (ctx->pin) cudaFreeHost(ctx->pin);
     for (auto &e : ctx->ev)
         if (e) cudaEventDestroy(e);
     if (ctx->stream2) {
@@ -266,6 +321,25 @@ __global__ void k_iota_i32(int64_t n, int32_t *v) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) v[i] = (int32_t)i;
 }
+// out[k] = in[k], or zero where in[k] is null, for the arrays whose out[k] is not
+struct Copy7 {
+    const double *in[7];
+    double *out[7];
+};
+__global__ void k_copy7(int64_t n, Copy7 c) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double v[7];
+#pragma unroll
+    for (int k = 0; k < 7; k++) v[k] = c.in[k] ? c.in[k][i] : 0.0;
+#pragma unroll
+    for (int k = 0; k < 7; k++)
+        if (c.out[k]) c.out[k][i] = v[k];
+}
+__global__ void k_widen(int64_t n, const int32_t *in, int64_t *out) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = in[i];
+}
 __global__ void k_gather_i32(int64_t n, const uint32_t *perm, const int32_t *in, int32_t *out) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = in[perm[i]];
@@ -332,11 +406,34 @@ static int upload_bodies_impl(gx_ctx *ctx, int64_t n, const double *x, const dou
     DevBuf *dst[7] = {&ctx->x, &ctx->y, &ctx->vx, &ctx->vy, &ctx->m, &ctx->ax, &ctx->ay};
     const double *src[7] = {x, y, vx, vy, m, ax, ay};
     bool same_n = ctx->have_bodies && ctx->n_bodies == n;
+    bool keep[7];
+    const double *dsrc[7];
+    bool direct = n > 0;
     for (int k = 0; k < 7; k++) {
         void *before = dst[k]->p;
         GX_TRY(gx_ensure(ctx, *dst[k], bytes));
-        if (n == 0) continue;
-        if (!src[k] && !zero_missing && same_n && before == dst[k]->p) continue;
+        keep[k] = !src[k] && !zero_missing && same_n && before == dst[k]->p;
+    }
+    for (int k = 0; k < 7 && direct; k++) {
+        dsrc[k] = src[k] ? static_cast<const double *>(direct_host(ctx, src[k], sizeof(double) * n, false)) : nullptr;
+        direct = !src[k] || (dsrc[k] && n <= GX_COPY_KERNEL);
+    }
+    if (direct) {
+        Copy7 c;
+        int used = 0;
+        for (int k = 0; k < 7; k++) {
+            c.in[k] = dsrc[k];
+            c.out[k] = keep[k] ? nullptr : dptr<double>(*dst[k]);
+            used += !keep[k];
+        }
+        if (used) {
+            k_copy7<<<gx_blocks(n, 256), 256, 0, ctx->stream>>>(n, c);
+            GX_CUDA(ctx, cudaGetLastError());
+            ctx->launches++;
+        }
+    }
+    for (int k = 0; k < 7 && n > 0 && !direct; k++) {
+        if (keep[k]) continue;
         if (src[k]) {
             GX_CUDA(ctx, cudaMemcpyAsync(dst[k]->p, src[k], sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
         } else {
@@ -365,7 +462,19 @@ int gx_download_bodies(gx_ctx *ctx, double *x, double *y, double *vx, double *vy
     int64_t n = ctx->n_bodies;
     DevBuf *srcb[7] = {&ctx->x, &ctx->y, &ctx->vx, &ctx->vy, &ctx->m, &ctx->ax, &ctx->ay};
     double *dst[7] = {x, y, vx, vy, m, ax, ay};
-    for (int k = 0; k < 7; k++)
+    Copy7 c;
+    bool direct = n > 0 && n <= GX_COPY_KERNEL;
+    for (int k = 0; k < 7 && direct; k++) {
+        c.in[k] = dst[k] ? dptr<double>(*srcb[k]) : nullptr;
+        c.out[k] = dst[k] ? static_cast<double *>(direct_host(ctx, dst[k], sizeof(double) * n, true)) : nullptr;
+        direct = !dst[k] || c.out[k];
+    }
+    if (direct) {
+        k_copy7<<<gx_blocks(n, 256), 256, 0, ctx->stream>>>(n, c);
+        GX_CUDA(ctx, cudaGetLastError());
+        ctx->launches++;
+    }
+    for (int k = 0; k < 7 && !direct; k++)
         if (dst[k] && n > 0)
             GX_CUDA(ctx, cudaMemcpyAsync(dst[k], srcb[k]->p, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
     GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -380,6 +489,7 @@ int gx_build_tree(gx_ctx *ctx, int64_t n, double *x, double *y, double *vx, doub
     ctx->have_tree = false;
     ctx->plan_ref_valid = ctx->plan_acc_valid = ctx->aux_valid = ctx->roll_valid = false;
     GX_TRY(upload_bodies_impl(ctx, n, x, y, vx, vy, m, ax, ay));
+    GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // the caller's arrays have been read, whatever fails from here
     ctx->n_bodies = n;
     ctx->build_n_max = n_max;
     for (int k = 0; k < 4; k++) ctx->build_bounds[k] = bounds[k];
@@ -498,6 +608,22 @@ int gx_upload_tree(gx_ctx *ctx, int64_t n_nodes, int64_t n_bodies, const double 
     return GX_OK;
 }
 
+// n 32-bit indices (< 2^31) to a host array of 64-bit ones, widened on the device
+static int widen_to_host(gx_ctx *ctx, const int32_t *in, int64_t n, int64_t *out) {
+    int64_t *dev = n <= GX_COPY_KERNEL ? static_cast<int64_t *>(direct_host(ctx, out, sizeof(int64_t) * n, true)) : nullptr;
+    const bool direct = dev != nullptr;
+    if (!direct) {
+        GX_TRY(gx_ensure(ctx, ctx->scratch_a, sizeof(int64_t) * (size_t)n));
+        dev = dptr<int64_t>(ctx->scratch_a);
+    }
+    k_widen<<<gx_blocks(n, 256), 256, 0, ctx->stream>>>(n, in, dev);
+    GX_CUDA(ctx, cudaGetLastError());
+    ctx->launches++;
+    if (!direct) GX_CUDA(ctx, cudaMemcpyAsync(out, dev, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, ctx->stream));
+    GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return GX_OK;
+}
+
 int gx_rebuild_resident(gx_ctx *ctx, int64_t n_max, const double bounds[4], int flags, int64_t *perm) {
     GX_TRY(check_ctx(ctx));
     if (n_max <= 0 || !bounds) return gx_fail(ctx, GX_ERR_INVALID_ARG, "bad n_max or bounds");
@@ -512,11 +638,7 @@ int gx_rebuild_resident(gx_ctx *ctx, int64_t n_max, const double bounds[4], int 
         if (flags & GX_BUILD_BALANCED) {
             for (int64_t i = 0; i < n; i++) perm[i] = i;  // build_constrained does not reorder
         } else {
-            std::vector<uint32_t> p32((size_t)n);
-            GX_CUDA(ctx, cudaMemcpyAsync(p32.data(), ctx->perm.p, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost,
-                                         ctx->stream));
-            GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            for (int64_t i = 0; i < n; i++) perm[i] = p32[(size_t)i];
+            GX_TRY(widen_to_host(ctx, dptr<int32_t>(ctx->perm), n, perm));
         }
     }
     return GX_OK;
@@ -529,11 +651,7 @@ int gx_body_ids(gx_ctx *ctx, int64_t *ids) {
     const int64_t n = ctx->n_bodies;
     if (n == 0) return GX_OK;
     if (ctx->ids.bytes < sizeof(int32_t) * (size_t)n) GX_TRY(gx_ids_reset(ctx));
-    std::vector<int32_t> v((size_t)n);
-    GX_CUDA(ctx, cudaMemcpyAsync(v.data(), ctx->ids.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, ctx->stream));
-    GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    for (int64_t i = 0; i < n; i++) ids[i] = v[(size_t)i];
-    return GX_OK;
+    return widen_to_host(ctx, dptr<int32_t>(ctx->ids), n, ids);
 }
 
 int gx_morton_encode(gx_ctx *ctx, int64_t n, const double *x, const double *y, const double bounds[4],
@@ -730,29 +848,6 @@ int gx_plan_info(gx_ctx *ctx, int64_t *n_far_pairs, int64_t *n_near_pairs, int64
     return GX_OK;
 }
 
-// The device address of a page-locked host array of n doubles (cudaHostAlloc or
-// cudaHostRegister), or null for any other memory.
-// The array counts as mapped only when its first and its last element resolve to the
-// same page-locked allocation (a registered range shorter than the array would let a
-// kernel run past it over the host link); otherwise it takes the staged copies.
-static double *mapped_host(const double *p, int64_t n) {
-    if (!p || n <= 0) return nullptr;
-    cudaPointerAttributes at{}, at_last{};
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();  // pageable memory on older runtimes: not an error of the call
-        return nullptr;
-    }
-    if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
-    if (cudaPointerGetAttributes(&at_last, p + (n - 1)) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    if (at_last.type != cudaMemoryTypeHost ||
-        static_cast<const double *>(at_last.devicePointer) != static_cast<const double *>(at.devicePointer) + (n - 1))
-        return nullptr;
-    return static_cast<double *>(at.devicePointer);
-}
-
 // Whether ensure_plan has nothing to do (the plan of the current tree and mode exists).
 static bool plan_current(const gx_ctx *ctx) {
     if (!ctx->have_tree || !ctx->have_bodies || !ctx->aux_valid) return false;
@@ -797,13 +892,17 @@ int gx_compute_forces(gx_ctx *ctx, const double *x, const double *y, const doubl
     if (!ctx->have_tree) return gx_fail(ctx, GX_ERR_STATE, "no tree: call gx_build_tree or gx_upload_tree first");
     if (!x || !y || !m || !ax || !ay) return gx_fail(ctx, GX_ERR_INVALID_ARG, "null array");
     int64_t n = ctx->n_bodies;
-    // page-locked inputs are read by the evaluation's first kernel itself (no separate
-    // copies), page-locked outputs written by its last one, so that the transfers over
-    // the host link overlap those kernels instead of preceding or following them
-    const double *hx = mapped_host(x, n), *hy = mapped_host(y, n), *hm = mapped_host(m, n);
-    double *hax = mapped_host(ax, n), *hay = mapped_host(ay, n);
+    // inputs that kernels can read (direct_host) are read by the evaluation's first kernel
+    // itself, such outputs written by its last one, so that the transfers over the host link
+    // overlap those kernels instead of preceding or following them
+    const size_t b = sizeof(double) * (size_t)n;
+    const auto *hx = static_cast<const double *>(direct_host(ctx, x, b, false)),
+               *hy = static_cast<const double *>(direct_host(ctx, y, b, false)),
+               *hm = static_cast<const double *>(direct_host(ctx, m, b, false));
+    auto *hax = static_cast<double *>(direct_host(ctx, ax, b, true)),
+         *hay = static_cast<double *>(direct_host(ctx, ay, b, true));
     const bool direct_in = hx && hy && hm && plan_current(ctx);  // a plan built now would read the old positions
-    const bool direct = hax && hay && ctx->n_nodes > 0;
+    const bool direct = hax && hay && ctx->n_nodes > 0 && ctx->leaves_cover;  // the sum writes the leaves' bodies
     if (direct_in) {
         GX_TRY(upload_bodies_impl(ctx, n, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, false));
         ctx->in_x = hx;
@@ -821,7 +920,7 @@ int gx_compute_forces(gx_ctx *ctx, const double *x, const double *y, const doubl
     ctx->in_x = ctx->in_y = ctx->in_m = nullptr;
     // kernels enqueued before a failure may still read or write the caller's arrays:
     // let them finish before the call returns
-    if (rc != GX_OK && (direct || direct_in)) cudaStreamSynchronize(ctx->stream);
+    if (rc != GX_OK) cudaStreamSynchronize(ctx->stream);
     GX_TRY(rc);
     // otherwise the read-back is queued behind the evaluation: one wait for both
     if (n > 0 && !direct) {

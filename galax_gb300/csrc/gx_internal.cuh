@@ -89,6 +89,8 @@ struct gx_ctx {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr;
     std::string err;
     int sm_count = 0;
+    unsigned *pin = nullptr;  // 64 page-locked bytes: small results on their way to the host
+    long host_pages = 0;      // the host's page size where the GPU shares its page tables, else 0
 
     // tree (device, SoA); node ids are int32, body indices int32
     int64_t n_nodes = 0, n_bodies = 0, n_leaves = 0;
