@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(128) k_adj_l2p(int64_t nl, const double *__res
 // partials in unit order.  Nodes without far entries are not written: has_far = 0 keeps A4
 // from reading them.
 template <int P, class T>
-__global__ void __launch_bounds__(128, (sizeof(T) == 4 && P <= 4) ? 8 : 1)
+__global__ void __launch_bounds__(32 * WPB, (sizeof(T) == 4 && P <= 4) ? 32 / WPB : 1)
     k_adj_m2l(int64_t n_units, const int32_t *__restrict__ unode, const int64_t *__restrict__ ustart,
               const int32_t *__restrict__ ulen, const int64_t *__restrict__ node_u, const int32_t *__restrict__ idx,
               const double *__restrict__ comx, const double *__restrict__ comy, const float4 *__restrict__ comhl,
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(128) k_adj_p2p_items(const int32_t *__restrict
 // leaves run on packed .f32x2 arithmetic, two sources per instruction (the lo half
 // of every accumulator takes the even sources, the hi half the odd ones); the own
 // leaf and partial rows run the scalar loop, which also skips the body itself.
-__global__ void __launch_bounds__(128, 6) k_adj_p2p32_items(int64_t n_items, const int32_t *__restrict__ item_leaf,
+__global__ void __launch_bounds__(32 * WPB, 24 / WPB) k_adj_p2p32_items(int64_t n_items, const int32_t *__restrict__ item_leaf,
                                                          const int64_t *__restrict__ item_qb,
                                                          const int32_t *__restrict__ item_nq,
                                                          const float4 *__restrict__ pos, const float2 *__restrict__ lam,
@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(128, 6) k_adj_p2p32_items(int64_t n_items, con
                                                          const int32_t *__restrict__ bs, const int32_t *__restrict__ be,
                                                          const int32_t *__restrict__ src_idx, float eps2, int tchunks,
                                                          float4 *__restrict__ part) {
-    __shared__ __align__(16) float sx[4][32], sy[4][32], sm[4][32], slx[4][32], sly[4][32];
+    __shared__ __align__(16) float sx[WPB][32], sy[WPB][32], sm[WPB][32], slx[WPB][32], sly[WPB][32];
     int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (it >= n_items) return;
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(128, 6) k_adj_p2p32_items(int64_t n_items, con
 // is one row, the item's source-leaf table is written to shared memory once per item,
 // and the next row's bodies and cotangents are fetched while the current row computes.
 // Same arithmetic and accumulation order as k_adj_p2p32_items with one target chunk.
-__global__ void __launch_bounds__(128, 6) k_adj_p2p32_rows(int64_t n_items, const int32_t *__restrict__ item_leaf,
+__global__ void __launch_bounds__(32 * WPB, 24 / WPB) k_adj_p2p32_rows(int64_t n_items, const int32_t *__restrict__ item_leaf,
                                                         const int64_t *__restrict__ item_qb,
                                                         const int32_t *__restrict__ item_nq,
                                                         const float4 *__restrict__ pos, const float2 *__restrict__ lam,
@@ -444,8 +444,8 @@ __global__ void __launch_bounds__(128, 6) k_adj_p2p32_rows(int64_t n_items, cons
                                                         const int32_t *__restrict__ bs, const int32_t *__restrict__ be,
                                                         const int32_t *__restrict__ src_idx, float eps2,
                                                         float4 *__restrict__ part) {
-    __shared__ __align__(16) float sx[4][32], sy[4][32], sm[4][32], slx[4][32], sly[4][32];
-    __shared__ __align__(16) int4 meta[4][32];  // per source leaf: begin, end, shift x, shift y (FP32 bits)
+    __shared__ __align__(16) float sx[WPB][32], sy[WPB][32], sm[WPB][32], slx[WPB][32], sly[WPB][32];
+    __shared__ __align__(16) int4 meta[WPB][32];  // per source leaf: begin, end, shift x, shift y (FP32 bits)
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (it >= n_items) return;
@@ -630,18 +630,18 @@ int run_force_vjp(gx_ctx *ctx, const double *X, const double *Y, const void *lf_
     // bodies packed by A1 and writes per-item partials, summed in order after the join
     const gx_ctx::Items &I = ctx->items_acc;
     const int tchunks = (int)std::max<int64_t>(1, (ctx->max_leaf + 31) / 32);
-    const unsigned gi = (unsigned)((I.n * 32 + 127) / 128);
+    const unsigned gi = gx_blocks(I.n, WPB);
     GX_TRY(gx_ensure(ctx, ctx->part, (F32 ? sizeof(float4) : sizeof(double4)) * 32 * (size_t)tchunks * (size_t)(I.n + 1)));
     GX_CUDA(ctx, cudaEventRecord(ctx->ev_fork, st));
     GX_CUDA(ctx, cudaStreamWaitEvent(ctx->stream2, ctx->ev_fork, 0));
     if (I.n > 0) {
         if (F32 && tchunks == 1)
-            k_adj_p2p32_rows<<<gi, 128, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
+            k_adj_p2p32_rows<<<gi, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
                                                            dptr<int32_t>(I.nq), pos32, lam32, comx, comy, bs, be,
                                                            dptr<int32_t>(ctx->near_idx), (float)eps2,
                                                            dptr<float4>(ctx->part));
         else if (F32)
-            k_adj_p2p32_items<<<gi, 128, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
+            k_adj_p2p32_items<<<gi, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
                                                             dptr<int32_t>(I.nq), pos32, lam32, comx, comy, bs, be,
                                                             dptr<int32_t>(ctx->near_idx), (float)eps2, tchunks,
                                                             dptr<float4>(ctx->part));
@@ -669,7 +669,7 @@ int run_force_vjp(gx_ctx *ctx, const double *X, const double *Y, const void *lf_
     if (U.n > 0) {
         const int64_t *node_u = dptr<int64_t>(U.node_u);
         GX_TRY(gx_ensure(ctx, ctx->m2l_part, sizeof(T) * NS * (size_t)(U.n + 1)));
-        k_adj_m2l<P, T><<<(unsigned)((U.n * 32 + 127) / 128), 128, 0, st>>>(
+        k_adj_m2l<P, T><<<gx_blocks(U.n, WPB), 32 * WPB, 0, st>>>(
             U.n, dptr<int32_t>(U.node), dptr<int64_t>(U.start), dptr<int32_t>(U.len), node_u,
             dptr<int32_t>(ctx->far_idx), comx, comy, F32 ? dptr<float4>(ctx->comhl) : nullptr, eps2, dL, dM,
             dptr<T>(ctx->m2l_part), dptr<unsigned>(ctx->m2l_count));

@@ -105,6 +105,11 @@ __device__ __forceinline__ T warp_sum_t(T v) {
     return v;
 }
 
+// Warps a block of the kernels that give a warp a work item or unit: one, as a block's place
+// on an SM is free again only when its last warp is done, and items differ in length (disk 4M,
+// p = 6: 18.65 -> 17.9 ms an evaluation; Plummer 1M, whose items are mostly full, 2.40 -> 2.37).
+constexpr int WPB = 1;
+
 // Sums over the warp of N = 16 or 32 values a lane, as a reduce-scatter: each exchange
 // halves what a lane still carries, 16 or 31 additions instead of five a value.  Lane l ends
 // with the sum of value l (N = 16: value l & 15, in both half-warps).
@@ -895,7 +900,7 @@ __device__ __forceinline__ void last_unit_sums(int64_t node, int64_t u0, int64_t
 // tens of thousands of far sources, is spread over many warps instead of running as
 // one straggler.  A node with one unit writes its local directly, the others as above.
 template <int P, class T>
-__global__ void __launch_bounds__(128, (sizeof(T) == 4 && P <= 4) ? 8 : 1) k_m2l_units(
+__global__ void __launch_bounds__(32 * WPB, (sizeof(T) == 4 && P <= 4) ? 32 / WPB : 1) k_m2l_units(
     int64_t n_units, const int32_t *__restrict__ unode, const int64_t *__restrict__ ustart,
     const int32_t *__restrict__ ulen, const int64_t *__restrict__ node_u, const int32_t *__restrict__ idx,
     const double *__restrict__ comx, const double *__restrict__ comy, const float4 *__restrict__ comhl, double eps2d,
@@ -1240,7 +1245,7 @@ __global__ void __launch_bounds__(128) k_p2p64_items(const int32_t *__restrict__
 // as (x - com_leaf, y - com_leaf, m) in FP32 (written by P2M); a source leaf is moved
 // into the target's frame by one FP32 shift per leaf pair, formed in FP64 and rounded once.
 // 7 blocks per SM: 72 registers, no spills (left alone, ptxas picks 64 and spills)
-__global__ void __launch_bounds__(128, 7) k_p2p32_items(int64_t n_items, const int32_t *__restrict__ item_leaf,
+__global__ void __launch_bounds__(32 * WPB, 28 / WPB) k_p2p32_items(int64_t n_items, const int32_t *__restrict__ item_leaf,
                                                      const int64_t *__restrict__ item_qb, const int32_t *__restrict__ item_nq,
                                                      const float4 *__restrict__ pos, const double *__restrict__ comx,
                                                      const double *__restrict__ comy, const int32_t *__restrict__ bs,
@@ -1248,15 +1253,14 @@ __global__ void __launch_bounds__(128, 7) k_p2p32_items(int64_t n_items, const i
                                                      float eps2, int tchunks, float2 *__restrict__ part) {
     // staged sources, one row of 32 per warp, as x / y / m planes so that one
     // broadcast 16-byte load yields the x (or y, m) of four consecutive sources
-    __shared__ __align__(16) float sx[4][32], sy[4][32], sm[4][32];
+    __shared__ __align__(16) float sx[WPB][32], sy[WPB][32], sm[WPB][32];
     int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // one warp per item (a grid-stride loop, launched with one warp for every item)
-    const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < n_items; it += nwarps) {
+    const int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // one item a warp
+    if (it < n_items) {
         int32_t leaf = item_leaf[it];
         int64_t qb = item_qb[it];
         int nq = item_nq[it];
-        if (nq < 0) continue;  // an M2P item of the near-list split (k_m2p)
+        if (nq < 0) return;  // an M2P item of the near-list split (k_m2p)
         int32_t t0 = bs[leaf], t1 = be[leaf];
         double tcx = comx[leaf], tcy = comy[leaf];
         int sl = lane < nq ? src_idx[qb + lane] : -1;
@@ -1363,23 +1367,22 @@ __global__ void __launch_bounds__(128, 7) k_p2p32_items(int64_t n_items, const i
 // of at most 16 bodies (n_max <= 16), where the second target of k_p2p32_rows would be
 // empty and a row holds only half a warp of sources: partial rows run their whole
 // quads packed and the rest scalar.
-__global__ void __launch_bounds__(128, 8) k_p2p32_rows1(int64_t n_items, const int32_t *__restrict__ item_leaf,
+__global__ void __launch_bounds__(32 * WPB, 32 / WPB) k_p2p32_rows1(int64_t n_items, const int32_t *__restrict__ item_leaf,
                                                     const int64_t *__restrict__ item_qb, const int32_t *__restrict__ item_nq,
                                                     const float4 *__restrict__ pos, const double *__restrict__ comx,
                                                     const double *__restrict__ comy, const int32_t *__restrict__ bs,
                                                     const int32_t *__restrict__ be, const int32_t *__restrict__ src_idx,
                                                     float eps2, float2 *__restrict__ part) {
-    __shared__ __align__(16) float sx[4][32], sy[4][32], sm[4][32];
-    __shared__ __align__(16) int4 meta[4][32];  // per source leaf: begin, end, shift x, shift y (FP32 bits)
+    __shared__ __align__(16) float sx[WPB][32], sy[WPB][32], sm[WPB][32];
+    __shared__ __align__(16) int4 meta[WPB][32];  // per source leaf: begin, end, shift x, shift y (FP32 bits)
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < n_items; it += nwarps) {
+    const int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // one item a warp
+    if (it < n_items) {
         const int32_t leaf = item_leaf[it];
         const int nq = item_nq[it];
-        if (nq < 0) continue;  // an M2P item of the near-list split (k_m2p)
+        if (nq < 0) return;  // an M2P item of the near-list split (k_m2p)
         const int32_t t0 = bs[leaf], t1 = be[leaf];
         bool own_lane = false;
-        __syncwarp();  // the previous item's reads of meta[w] are done
         if (lane < nq) {
             int32_t sl = src_idx[item_qb[it] + lane];
             double tcx = comx[leaf], tcy = comy[leaf];
@@ -1472,24 +1475,23 @@ __global__ void __launch_bounds__(128, 8) k_p2p32_rows1(int64_t n_items, const i
 // broadcast load of four sources serves eight interactions; the two halves' sums of a
 // target are added (half 0 first) at the end of the item.  Same per-interaction
 // arithmetic as k_p2p32_items.
-__global__ void __launch_bounds__(128, 8) k_p2p32_rows(int64_t n_items, const int32_t *__restrict__ item_leaf,
+__global__ void __launch_bounds__(32 * WPB, 32 / WPB) k_p2p32_rows(int64_t n_items, const int32_t *__restrict__ item_leaf,
                                                     const int64_t *__restrict__ item_qb, const int32_t *__restrict__ item_nq,
                                                     const float4 *__restrict__ pos, const double *__restrict__ comx,
                                                     const double *__restrict__ comy, const int32_t *__restrict__ bs,
                                                     const int32_t *__restrict__ be, const int32_t *__restrict__ src_idx,
                                                     float eps2, float2 *__restrict__ part) {
-    __shared__ __align__(16) float sx[4][32], sy[4][32], sm[4][32];
-    __shared__ __align__(16) int4 meta[4][32];  // per source leaf: begin, end, shift x, shift y (FP32 bits)
+    __shared__ __align__(16) float sx[WPB][32], sy[WPB][32], sm[WPB][32];
+    __shared__ __align__(16) int4 meta[WPB][32];  // per source leaf: begin, end, shift x, shift y (FP32 bits)
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int half = lane >> 4, tl = lane & 15;  // lane: targets tl and tl + 16, source quads of its half
-    const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < n_items; it += nwarps) {
+    const int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // one item a warp
+    if (it < n_items) {
         const int32_t leaf = item_leaf[it];
         const int nq = item_nq[it];
-        if (nq < 0) continue;  // an M2P item of the near-list split (k_m2p)
+        if (nq < 0) return;  // an M2P item of the near-list split (k_m2p)
         const int32_t t0 = bs[leaf], t1 = be[leaf];
         bool own_lane = false;
-        __syncwarp();  // the previous item's reads of meta[w] are done
         if (lane < nq) {
             int32_t sl = src_idx[item_qb[it] + lane];
             double tcx = comx[leaf], tcy = comy[leaf];
@@ -1604,30 +1606,29 @@ __global__ void __launch_bounds__(128, 8) k_p2p32_rows(int64_t n_items, const in
 // stream when eps > 0 (each body's term on itself is exactly 0); with eps = 0 it runs
 // first, as the scalar own row of k_p2p32_rows.  With empty masks the stream is every body
 // of every row, so the same kernel serves the plain split.
-__global__ void __launch_bounds__(128, 8) k_p2p32_stream(
+__global__ void __launch_bounds__(32 * WPB, 32 / WPB) k_p2p32_stream(
     int64_t n_items, const int32_t *__restrict__ item_leaf, const int64_t *__restrict__ item_qb,
     const int32_t *__restrict__ item_nq, const float4 *__restrict__ pos, const double *__restrict__ comx,
     const double *__restrict__ comy, const int32_t *__restrict__ bs, const int32_t *__restrict__ be,
     const int32_t *__restrict__ src_idx, const uint32_t *__restrict__ p2p_mask, float eps2,
     float2 *__restrict__ part) {
-    __shared__ __align__(16) float sx[4][32], sy[4][32], sm[4][32];
-    __shared__ __align__(16) int4 meta[4][32];  // per source leaf: begin, end, shift x, shift y (FP32 bits)
-    __shared__ uint16_t strm[4][32 * 32];       // the item's kept bodies: (row << 5) | body
+    __shared__ __align__(16) float sx[WPB][32], sy[WPB][32], sm[WPB][32];
+    __shared__ __align__(16) int4 meta[WPB][32];  // per source leaf: begin, end, shift x, shift y (FP32 bits)
+    __shared__ uint16_t strm[WPB][32 * 32];       // the item's kept bodies: (row << 5) | body
     const unsigned full = 0xffffffffu;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const int half = lane >> 4, tl = lane & 15;  // lane: targets tl and tl + 16, source quads of its half
-    const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
     const float4 far4 = make_float4(1e18f, 1e18f, 0.f, 0.f);
     const bool self_in_stream = eps2 > 0.f;
-    for (int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < n_items; it += nwarps) {
+    const int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // one item a warp
+    if (it < n_items) {
         const int32_t leaf = item_leaf[it];
         const int nq = item_nq[it];
-        if (nq < 0) continue;  // an M2P item of the near-list split (k_m2p)
+        if (nq < 0) return;  // an M2P item of the near-list split (k_m2p)
         const int32_t t0 = bs[leaf], t1 = be[leaf];
         bool own_lane = false;
         uint32_t keep = 0;
-        __syncwarp();  // the previous item's reads of meta[w] and strm[w] are done
         if (lane < nq) {
             const int64_t q = item_qb[it] + lane;
             const int32_t sl = src_idx[q];
@@ -1850,7 +1851,7 @@ __device__ __forceinline__ void m2p_eval(T dx, T dy, T eps2, const V *w, T &fx, 
 // Writes the item's partial slot like a P2P item, so the ordered sum of the leaf's items
 // includes it.
 template <int P, class T, class V>
-__global__ void __launch_bounds__(128) k_m2p(int64_t n_list, const int32_t *__restrict__ list,
+__global__ void __launch_bounds__(32 * WPB) k_m2p(int64_t n_list, const int32_t *__restrict__ list,
                                              const int32_t *__restrict__ item_leaf,
                                              const int64_t *__restrict__ item_qb, const int32_t *__restrict__ item_nq,
                                              const float4 *__restrict__ pos, const double *__restrict__ X,
@@ -1861,7 +1862,7 @@ __global__ void __launch_bounds__(128) k_m2p(int64_t n_list, const int32_t *__re
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<T>(NC);
     constexpr int CPL = (NC + 31) / 32;  // coefficients a lane prepares
-    __shared__ V sw[4][NC];
+    __shared__ V sw[WPB][NC];
     const unsigned full = 0xffffffffu;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -1983,7 +1984,7 @@ __device__ __forceinline__ f2v rsqrt_x2(f2v r2) {
 // memory.  The halves' sums are added in a fixed order (half 0's first), as in the
 // two-target P2P rows.
 template <int P>
-__global__ void __launch_bounds__(128, 8) k_m2p_x2(int64_t n_list, const int32_t *__restrict__ list,
+__global__ void __launch_bounds__(32 * WPB, 32 / WPB) k_m2p_x2(int64_t n_list, const int32_t *__restrict__ list,
                                                 const int32_t *__restrict__ item_leaf,
                                                 const int64_t *__restrict__ item_qb,
                                                 const int32_t *__restrict__ item_nq, const float4 *__restrict__ pos,
@@ -1994,8 +1995,8 @@ __global__ void __launch_bounds__(128, 8) k_m2p_x2(int64_t n_list, const int32_t
     static_assert(P <= 5, "shared-memory moment rows are sized for p <= 5");
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<float>(NC);
-    __shared__ __align__(16) float4 smm[4][32][NC];  // (mx, mx, my, my) per moment
-    __shared__ __align__(8) float2 shf[4][32];        // com_a - com_s
+    __shared__ __align__(16) float4 smm[WPB][32][NC];  // (mx, mx, my, my) per moment
+    __shared__ __align__(8) float2 shf[WPB][32];        // com_a - com_s
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int half = lane >> 4, tl = lane & 15;
     const f2v E2 = f2splat(eps2);
@@ -2074,7 +2075,7 @@ constexpr int P2L_RING = 4;  // rounds of P2L source bodies in flight per warp (
 // coefficient sums stay pairs until the end (pair halves, then the warp, in a fixed
 // order).  Leaves above 32 bodies go through their further bodies 32 at a time.
 template <int P>
-__global__ void __launch_bounds__(128, 6) k_p2l_x2(int64_t n_units, const int32_t *__restrict__ uleaf,
+__global__ void __launch_bounds__(32 * WPB, 24 / WPB) k_p2l_x2(int64_t n_units, const int32_t *__restrict__ uleaf,
                                                 const int64_t *__restrict__ ustart, const int32_t *__restrict__ ulen,
                                                 const int32_t *__restrict__ src_idx, const float4 *__restrict__ pos,
                                                 const double *__restrict__ comx, const double *__restrict__ comy,
@@ -2083,7 +2084,7 @@ __global__ void __launch_bounds__(128, 6) k_p2l_x2(int64_t n_units, const int32_
     static_assert(P <= 5, "paired accumulators are sized for p <= 5");
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<float>(NC);
-    __shared__ __align__(16) float4 p2l_ring[4][P2L_RING][64];  // per warp: P2L_RING rounds x 64 bodies
+    __shared__ __align__(16) float4 p2l_ring[WPB][P2L_RING][64];  // per warp: P2L_RING rounds x 64 bodies
     const int lane = threadIdx.x & 31;
     const int half = lane >> 4, tl = lane & 15;
     const int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -2178,7 +2179,7 @@ __global__ void __launch_bounds__(128, 6) k_p2l_x2(int64_t n_units, const int32_
 // c + lane and c + 32 + lane), each with its row's com_a - com_s; a padding slot has zero
 // mass at a unit offset.  Writes the unit's partial like k_p2l_x2.
 template <int P>
-__global__ void __launch_bounds__(128, 6) k_p2l_body_x2(int64_t u_base, int64_t n_units,
+__global__ void __launch_bounds__(32 * WPB, 24 / WPB) k_p2l_body_x2(int64_t u_base, int64_t n_units,
                                                      const int32_t *__restrict__ uleaf,
                                                      const int64_t *__restrict__ ustart,
                                                      const int32_t *__restrict__ ulen,
@@ -2192,9 +2193,9 @@ __global__ void __launch_bounds__(128, 6) k_p2l_body_x2(int64_t u_base, int64_t 
     constexpr int RPL = GX_BODY_UNIT / 32;  // rows per lane
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<float>(NC);
-    __shared__ __align__(16) float2 rsh[4][GX_BODY_UNIT];  // per row: com_a - com_s in FP32
-    __shared__ int32_t rb0[4][GX_BODY_UNIT];               // per row: the source leaf's first body
-    __shared__ uint16_t strm[4][GX_BODY_UNIT * 32];        // the unit's masked bodies: (row << 5) | body
+    __shared__ __align__(16) float2 rsh[WPB][GX_BODY_UNIT];  // per row: com_a - com_s in FP32
+    __shared__ int32_t rb0[WPB][GX_BODY_UNIT];               // per row: the source leaf's first body
+    __shared__ uint16_t strm[WPB][GX_BODY_UNIT * 32];        // the unit's masked bodies: (row << 5) | body
     const unsigned full = 0xffffffffu;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t wu = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -2328,7 +2329,7 @@ __device__ __forceinline__ void p2l_body(T dx, T dy, T mj, T eps2, T *acc) {
 // the whole warp's evaluation for the third of a row that the masks keep: 14.0 -> 10.8 ms at
 // 1M, 8.7 ms of it the FP64 pipe's.)
 template <int P, class T>
-__global__ void __launch_bounds__(128) k_p2l_stream(int64_t n_units, const int32_t *__restrict__ uleaf,
+__global__ void __launch_bounds__(32 * WPB) k_p2l_stream(int64_t n_units, const int32_t *__restrict__ uleaf,
                                                     const int64_t *__restrict__ ustart, const int32_t *__restrict__ ulen,
                                                     const int32_t *__restrict__ src_idx,
                                                     const float4 *__restrict__ pos, const double *__restrict__ X,
@@ -2343,9 +2344,9 @@ __global__ void __launch_bounds__(128) k_p2l_stream(int64_t n_units, const int32
     static_assert(ROWS % 32 == 0 && ROWS * 32 <= 65536, "whole rows per lane, 16-bit entries");
     const int PP = gx_rt_order(P);
     const int NCr = (PP + 1) * (PP + 2) / 2;
-    __shared__ int32_t rb0[4][ROWS];       // per row: the source leaf's first body
-    __shared__ float2 rsh[4][ROWS];        // FP32: com_a - com_s
-    __shared__ uint16_t strm[4][ROWS * 32];
+    __shared__ int32_t rb0[WPB][ROWS];       // per row: the source leaf's first body
+    __shared__ float2 rsh[WPB][ROWS];        // FP32: com_a - com_s
+    __shared__ uint16_t strm[WPB][ROWS * 32];
     const unsigned full = 0xffffffffu;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -2419,7 +2420,7 @@ __global__ void __launch_bounds__(128) k_p2l_stream(int64_t n_units, const int32
 
 // P2L units over larger leaves (no body-level units there): a row at a time.
 template <int P, class T>
-__global__ void __launch_bounds__(128) k_p2l(int64_t n_units, const int32_t *__restrict__ uleaf,
+__global__ void __launch_bounds__(32 * WPB) k_p2l(int64_t n_units, const int32_t *__restrict__ uleaf,
                                              const int64_t *__restrict__ ustart, const int32_t *__restrict__ ulen,
                                              const int32_t *__restrict__ src_idx,
                                              const float4 *__restrict__ pos, const double *__restrict__ X,
@@ -2723,7 +2724,7 @@ int run_forces(gx_ctx *ctx, bool timed) {
     const gx_ctx::Items &I = mode == GX_MODE_ACCURATE ? ctx->items_acc : ctx->items_ref;
     const int tchunks = (int)std::max<int64_t>(1, (ctx->max_leaf + 31) / 32);
     const int32_t *src_idx = mode == GX_MODE_ACCURATE ? dptr<int32_t>(ctx->near_idx) : dptr<int32_t>(ctx->p2p_idx);
-    const unsigned gi = (unsigned)((I.n * 32 + 127) / 128);  // warp per item
+    const unsigned gi = gx_blocks(I.n, WPB);  // warp per item
     const bool split = mode == GX_MODE_ACCURATE && ctx->theta_w > 0.0;  // near-list split: M2P items, P2L units
     // body-level P2L of the P2P rows: masks in the plan, body-level P2L units
     const bool body = split && ctx->plan_body_split && gx_body_split_on(ctx);
@@ -2765,19 +2766,19 @@ int run_forces(gx_ctx *ctx, bool timed) {
             // two targets per lane pays when leaves fill most of a row; with leaves of at
             // most 16 bodies (n_max <= 16) the second target would be empty
             if (mixed && body)
-                k_p2p32_stream<<<gi, 128, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
+                k_p2p32_stream<<<gi, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
                                                              dptr<int32_t>(I.nq), pos, comx, comy, bs, be, src_idx,
                                                              p2p_mask, (float)eps2, dptr<float2>(ctx->part));
             else if (mixed && tchunks == 1 && ctx->max_leaf <= 16)
-                k_p2p32_rows1<<<gi, 128, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
+                k_p2p32_rows1<<<gi, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
                                                             dptr<int32_t>(I.nq), pos, comx, comy, bs, be, src_idx,
                                                             (float)eps2, dptr<float2>(ctx->part));
             else if (mixed && tchunks == 1)
-                k_p2p32_rows<<<gi, 128, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
+                k_p2p32_rows<<<gi, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
                                                            dptr<int32_t>(I.nq), pos, comx, comy, bs, be, src_idx,
                                                            (float)eps2, dptr<float2>(ctx->part));
             else if (mixed)
-                k_p2p32_items<<<gi, 128, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
+                k_p2p32_items<<<gi, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
                                                             dptr<int32_t>(I.nq), pos, comx, comy, bs, be, src_idx,
                                                             (float)eps2, tchunks, dptr<float2>(ctx->part));
             else
@@ -2788,11 +2789,11 @@ int run_forces(gx_ctx *ctx, bool timed) {
         }
         if (timed) GX_CUDA(ctx, cudaEventRecord(ctx->ev[15], ctx->stream2));  // the P2P kernel alone
         if (split && ctx->n_m2p_items > 0) {
-            const unsigned gm = (unsigned)((ctx->n_m2p_items * 32 + 127) / 128);  // warp per M2P item
+            const unsigned gm = gx_blocks(ctx->n_m2p_items, WPB);  // warp per M2P item
             // M2P items of the near-list split: their own slots of the same partial array
             if constexpr (P <= 5) {
                 if (mixed && tchunks == 1) {
-                    k_m2p_x2<P><<<gm, 128, 0, ctx->stream2>>>(ctx->n_m2p_items, dptr<int32_t>(ctx->m2p_list),
+                    k_m2p_x2<P><<<gm, 32 * WPB, 0, ctx->stream2>>>(ctx->n_m2p_items, dptr<int32_t>(ctx->m2p_list),
                                                               dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
                                                               dptr<int32_t>(I.nq), pos, comx, comy, bs, be, src_idx,
                                                               (float)eps2, reinterpret_cast<const float *>(M),
@@ -2801,12 +2802,12 @@ int run_forces(gx_ctx *ctx, bool timed) {
                 }
             }
             if (mixed)
-                k_m2p<P, float, float2><<<gm, 128, 0, ctx->stream2>>>(
+                k_m2p<P, float, float2><<<gm, 32 * WPB, 0, ctx->stream2>>>(
                     ctx->n_m2p_items, dptr<int32_t>(ctx->m2p_list), dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb), dptr<int32_t>(I.nq), pos, nullptr, nullptr, comx,
                     comy, bs, be, src_idx, (float)eps2, reinterpret_cast<const float *>(M), tchunks,
                     dptr<float2>(ctx->part));
             else
-                k_m2p<P, double, double2><<<gm, 128, 0, ctx->stream2>>>(
+                k_m2p<P, double, double2><<<gm, 32 * WPB, 0, ctx->stream2>>>(
                     ctx->n_m2p_items, dptr<int32_t>(ctx->m2p_list), dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb), dptr<int32_t>(I.nq), nullptr, X, Y, comx, comy, bs,
                     be, src_idx, eps2, reinterpret_cast<const double *>(M), tchunks, dptr<double2>(ctx->part));
         m2p_done:
@@ -2832,25 +2833,25 @@ int run_forces(gx_ctx *ctx, bool timed) {
         auto p2l_field = [&](cudaStream_t sp) -> int {
             if constexpr (P <= 5 && sizeof(T) == 4) {
                 if (PU.n_leafu > 0) {
-                    k_p2l_x2<P><<<gx_blocks(PU.n_leafu * 32, 128), 128, 0, sp>>>(
+                    k_p2l_x2<P><<<gx_blocks(PU.n_leafu, WPB), 32 * WPB, 0, sp>>>(
                         PU.n_leafu, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start), dptr<int32_t>(PU.len), src_idx,
                         pos, comx, comy, bs, be, (float)eps2, dptr<float>(ctx->p2l_part));
                     ctx->launches++;
                 }
                 if (body && PU.n_body > 0) {
-                    k_p2l_body_x2<P><<<gx_blocks(PU.n_body * 32, 128), 128, 0, sp>>>(
+                    k_p2l_body_x2<P><<<gx_blocks(PU.n_body, WPB), 32 * WPB, 0, sp>>>(
                         PU.n_leafu, PU.n_body, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start),
                         dptr<int32_t>(PU.len), src_idx, p2p_mask, pos, comx, comy, bs, (float)eps2,
                         dptr<float>(ctx->p2l_part));
                     ctx->launches++;
                 }
             } else if (ctx->max_leaf <= 32) {
-                k_p2l_stream<P, T><<<gx_blocks(PU.n * 32, 128), 128, 0, sp>>>(
+                k_p2l_stream<P, T><<<gx_blocks(PU.n, WPB), 32 * WPB, 0, sp>>>(
                     PU.n, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start), dptr<int32_t>(PU.len), src_idx, pos, X, Y,
                     Mb, comx, comy, bs, be, (T)eps2, p2p_mask, dptr<T>(ctx->p2l_part));
                 ctx->launches++;
             } else {
-                k_p2l<P, T><<<gx_blocks(PU.n * 32, 128), 128, 0, sp>>>(
+                k_p2l<P, T><<<gx_blocks(PU.n, WPB), 32 * WPB, 0, sp>>>(
                     PU.n, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start), dptr<int32_t>(PU.len), src_idx, pos, X, Y,
                     Mb, comx, comy, bs, be, (T)eps2, dptr<T>(ctx->p2l_part));
                 ctx->launches++;
@@ -2889,7 +2890,7 @@ int run_forces(gx_ctx *ctx, bool timed) {
             GX_TRY(gx_ensure(ctx, ctx->m2l_part, sizeof(T) * NS * (size_t)(U.n + 1)));
             if (U.n > 0) {
                 const int64_t *node_u = dptr<int64_t>(U.node_u);
-                k_m2l_units<P, T><<<(unsigned)((U.n * 32 + 127) / 128), 128, 0, st>>>(
+                k_m2l_units<P, T><<<gx_blocks(U.n, WPB), 32 * WPB, 0, st>>>(
                     U.n, dptr<int32_t>(U.node), dptr<int64_t>(U.start), dptr<int32_t>(U.len), node_u,
                     dptr<int32_t>(ctx->far_idx), comx, comy, mixed ? dptr<float4>(ctx->comhl) : nullptr, eps2, M, L,
                     dptr<T>(ctx->m2l_part), dptr<unsigned>(ctx->m2l_count));
