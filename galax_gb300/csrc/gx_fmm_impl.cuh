@@ -702,8 +702,11 @@ __device__ __forceinline__ bool nonzero_bits(double v) {
 // per output coefficient, as many sources side by side as fit (two at p = 4): a list of 23
 // sources, the mean at N = 200k, takes 12 x 15 multiply-adds a lane instead of a round of
 // 225 with a quarter of the lanes idle and a warp sum of each of the 15 coefficients, and a
-// derivative set is read as 15 neighbouring values instead of 32 sets at once.
-template <int P>
+// derivative set is read as 15 neighbouring values instead of 32 sets at once.  W warps share
+// a node's list, their sums added in order: four for a small tree, whose nodes do not fill the
+// GPU and where the longest list is the whole pass (N = 1000: 22 -> 10 us, 10,000: 61 -> 41),
+// one for a large one.
+template <int P, int W>
 __global__ void __launch_bounds__(128) k_m2l_ref_rows(int64_t nn, const uint32_t *__restrict__ vdata,
                                                       const uint8_t *__restrict__ vlen,
                                                       const int64_t *__restrict__ voff,
@@ -715,7 +718,9 @@ __global__ void __launch_bounds__(128) k_m2l_ref_rows(int64_t nn, const uint32_t
     constexpr int SIDE = 32 / NC;
     static_assert(SIDE >= 1 && GX_LIST_CAP <= 64, "a lane per coefficient, two list entries per lane");
     const unsigned full = 0xffffffffu;
-    const int64_t node = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    static_assert(W == 1 || W == 4, "a block of four warps: four nodes or one");
+    const int wn = W == 1 ? 0 : threadIdx.x >> 5;  // this warp's share of the node's list
+    const int64_t node = W == 1 ? ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5 : blockIdx.x;
     const int lane = threadIdx.x & 31;
     if (node >= nn) return;
     const int len = vlen[node];
@@ -728,7 +733,7 @@ __global__ void __launch_bounds__(128) k_m2l_ref_rows(int64_t nn, const uint32_t
     const int oj = k - n * (n + 1) / 2, oi = n - oj;
     const double *g0 = G + gx_kdi(oi, oj, P);
     double acc = 0.0;
-    for (int s0 = 0; s0 < len; s0 += SIDE) {
+    for (int s0 = wn * SIDE; s0 < len; s0 += W * SIDE) {
         const int s = s0 + slot;
         const int sa = __shfl_sync(full, srcA, s & 31), sb = __shfl_sync(full, srcB, s & 31);
         const int da = __shfl_sync(full, didA, s & 31), db = __shfl_sync(full, didB, s & 31);
@@ -748,6 +753,13 @@ __global__ void __launch_bounds__(128) k_m2l_ref_rows(int64_t nn, const uint32_t
     double v = acc;
 #pragma unroll
     for (int q = 1; q < SIDE; q++) v += __shfl_sync(full, acc, (lane + q * NC) & 31);
+    if constexpr (W > 1) {
+        __shared__ double sum[W][32];
+        sum[wn][lane] = v;
+        __syncthreads();
+        if (wn > 0) return;
+        v = (sum[0][lane] + sum[1][lane]) + (sum[2][lane] + sum[3][lane]);
+    }
     if (lane < NC) L[node * NS + lane] = v * tab_ifp<double>(oi, oj);
 }
 
@@ -2876,14 +2888,19 @@ int run_forces(gx_ctx *ctx, bool timed) {
         // M2L
         const unsigned gn = (unsigned)((nn * 32 + 127) / 128);
         if (mode == GX_MODE_REF && !mixed) {
-            const auto launch = [&](auto kernel) {
-                kernel<<<gn, 128, 0, st>>>(nn, dptr<uint32_t>(ctx->vdata), dptr<uint8_t>(ctx->vlen),
+            const auto launch = [&](auto kernel, unsigned grid) {
+                kernel<<<grid, 128, 0, st>>>(nn, dptr<uint32_t>(ctx->vdata), dptr<uint8_t>(ctx->vlen),
                                            dptr<int64_t>(ctx->ref_voff), dptr<int32_t>(ctx->ref_did),
                                            dptr<double>(ctx->ref_G), reinterpret_cast<const double *>(M),
                                            reinterpret_cast<double *>(L));
             };
-            if constexpr (NC <= 32) launch(k_m2l_ref_rows<P>);
-            else launch(k_m2l_ref<P>);
+            if constexpr (NC <= 32) {
+                // below some 100 nodes an SM a warp each leaves schedulers without one
+                if (nn <= (int64_t)ctx->sm_count * 100) launch(k_m2l_ref_rows<P, 4>, (unsigned)nn);
+                else launch(k_m2l_ref_rows<P, 1>, gn);
+            } else {
+                launch(k_m2l_ref<P>, gn);
+            }
         } else if (mode == GX_MODE_ACCURATE) {
             // nodes without far sources keep whatever L holds: has_far = 0 keeps L2L from reading it
             const gx_ctx::M2LUnits &U = ctx->m2l_units;
