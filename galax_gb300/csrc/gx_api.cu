@@ -108,11 +108,15 @@ void gx_tree_plan_free(gx_tree_plan &t) {
     }
 }
 
-static int sync_status(gx_ctx *ctx, unsigned *out) {
-    GX_CUDA(ctx, cudaMemcpyAsync(ctx->pin, ctx->status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+int gx_fetch(gx_ctx *ctx, void *dst, const void *src, size_t bytes) {
+    GX_CUDA(ctx, cudaMemcpyAsync(ctx->pin, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    *out = *ctx->pin;
+    std::memcpy(dst, ctx->pin, bytes);
     return GX_OK;
+}
+
+static int sync_status(gx_ctx *ctx, unsigned *out) {
+    return gx_fetch(ctx, out, ctx->status.p, sizeof(unsigned));
 }
 
 // ---- host arrays read and written by kernels ----
@@ -216,7 +220,7 @@ int gx_create(const gx_config *cfg, gx_ctx **out) {
         gx_destroy(ctx);
         return s;
     }
-    if (cudaMallocHost(&ctx->pin, 64) != cudaSuccess) {
+    if (cudaMallocHost(&ctx->pin, GX_PIN) != cudaSuccess) {
         cudaGetLastError();
         gx_destroy(ctx);
         return GX_ERR_ALLOC;

@@ -61,6 +61,10 @@ int gx_cuda_check(gx_ctx *ctx, cudaError_t e, const char *what);
 
 // Grow-only device allocation; contents are not preserved on growth.
 int gx_ensure(gx_ctx *ctx, DevBuf &b, size_t bytes);
+constexpr size_t GX_PIN = 4096;
+// bytes <= GX_PIN of device memory into dst, after what is on the stream.  Through page-locked
+// memory: a copy into ordinary memory goes by a staging buffer of the driver and takes longer.
+int gx_fetch(gx_ctx *ctx, void *dst, const void *src, size_t bytes);
 template <class T>
 inline T *dptr(const DevBuf &b) { return reinterpret_cast<T *>(b.p); }
 
@@ -89,7 +93,7 @@ struct gx_ctx {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr;
     std::string err;
     int sm_count = 0;
-    unsigned *pin = nullptr;  // 64 page-locked bytes: small results on their way to the host
+    void *pin = nullptr;  // GX_PIN page-locked bytes: small results on their way to the host (gx_fetch)
     long host_pages = 0;      // the host's page size where the GPU shares its page tables, else 0
 
     // tree (device, SoA); node ids are int32, body indices int32

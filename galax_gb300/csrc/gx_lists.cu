@@ -719,6 +719,20 @@ __global__ void k_chain_leaf_offsets(int64_t nl, int64_t up, int64_t near_cap, i
     ncnt[x] = ncnt[x + up];
 }
 
+// the lists before the first level: empty, but for the root's near list {root} at index 0
+__global__ void k_mac_open(int64_t nn, int64_t root, int32_t *fcnt, int32_t *ncnt, int64_t *nstart, int32_t *near_idx,
+                           int64_t *ctr) {
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nn) return;
+    fcnt[k] = 0;
+    ncnt[k] = k == root ? 1 : 0;
+    if (k == root) {
+        nstart[k] = 0;
+        near_idx[0] = (int32_t)root;
+        for (int q = 0; q < PC_N; q++) ctr[q] = q == PC_NEAR ? 1 : 0;
+    }
+}
+
 // The chain shortcut needs node x + l nl (levels 1 .. L) to have the single child
 // x + (l - 1) nl, as Tree::build numbers them; a tree given from the host that does not
 // flags OVF_CHAIN and is planned without the shortcut.
@@ -1007,8 +1021,7 @@ static int build_level(gx_ctx *ctx, int64_t s, int64_t e, DevBuf &storage, size_
     }
     GX_CUDA(ctx, cudaGetLastError());
     struct { unsigned nf; unsigned pad; double ma; } h{};
-    GX_CUDA(ctx, cudaMemcpyAsync(&h, nf, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-    GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    GX_TRY(gx_fetch(ctx, &h, nf, sizeof(h)));
     L.brute = h.nf > 0;
     L.maxabs = h.ma;
     return GX_OK;
@@ -1024,8 +1037,7 @@ static size_t bvh_bytes(int64_t cnt) {
 
 static int check_status(gx_ctx *ctx) {
     unsigned st = 0;
-    GX_CUDA(ctx, cudaMemcpyAsync(&st, dptr<unsigned>(ctx->status), sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
-    GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    GX_TRY(gx_fetch(ctx, &st, dptr<unsigned>(ctx->status), sizeof(unsigned)));
     if (st & GX_DEV_STACK_OVERFLOW) return gx_fail(ctx, GX_ERR_STATE, "list builder: traversal stack overflow");
     return GX_OK;
 }
@@ -1065,8 +1077,7 @@ int gx_lists_build_ref(gx_ctx *ctx) {
             k_cenv_up<<<gx_blocks(lo, 128), 128, 0, ctx->stream>>>(lo, 2 * lo, L.cbox, L.cmh);
             ctx->launches++;
         }
-        GX_CUDA(ctx, cudaMemcpyAsync(&L.cmax, cmax, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-        GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        GX_TRY(gx_fetch(ctx, &L.cmax, cmax, sizeof(double)));
         k_vlist_node<<<gx_blocks(e0 - s0, 64), 64, 0, ctx->stream>>>(s0, e0, L, dptr<int32_t>(ctx->parent),
                                                                     dptr<int4>(ctx->child), cx, cy, hw,
                                                                     dptr<uint32_t>(ctx->vdata), dptr<uint8_t>(ctx->vlen),
@@ -1106,8 +1117,7 @@ int gx_plan_ref(gx_ctx *ctx) {
                                                                     dptr<uint8_t>(ctx->ulen), cnt);
         GX_TRY(gx_exclusive_scan_i64(ctx, cnt, eoff, nl + 1));
         int64_t nk = 0;
-        GX_CUDA(ctx, cudaMemcpyAsync(&nk, eoff + nl, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-        GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        GX_TRY(gx_fetch(ctx, &nk, eoff + nl, sizeof(int64_t)));
         // keys and their sort buffers: scratch_a (keys, alt), scratch_b (values, alt)
         GX_TRY(gx_ensure(ctx, ctx->scratch_a, sizeof(uint64_t) * (size_t)(nk + 1) * 2));
         GX_TRY(gx_ensure(ctx, ctx->scratch_b, sizeof(uint32_t) * (size_t)(nk + 1) * 2));
@@ -1129,8 +1139,7 @@ int gx_plan_ref(gx_ctx *ctx) {
         int64_t *off = dptr<int64_t>(ctx->p2p_off);
         GX_TRY(gx_exclusive_scan_i64(ctx, len, off, nl + 1));
         int64_t tot = 0;
-        GX_CUDA(ctx, cudaMemcpyAsync(&tot, off + nl, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-        GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        GX_TRY(gx_fetch(ctx, &tot, off + nl, sizeof(int64_t)));
         GX_TRY(gx_ensure(ctx, ctx->p2p_idx, sizeof(int32_t) * (size_t)(tot + 1)));
         k_gather_fill<<<gx_blocks(nl, 256), 256, 0, ctx->stream>>>(nl, sk, kstart, off, dptr<int32_t>(ctx->p2p_idx));
         ctx->launches += 6;
@@ -1147,8 +1156,7 @@ int gx_plan_ref(gx_ctx *ctx) {
     k_u8_to_i64<<<gx_blocks(nn, 256), 256, 0, ctx->stream>>>(dptr<uint8_t>(ctx->vlen), len64, nn);
     GX_TRY(gx_exclusive_scan_i64(ctx, len64, voff, nn + 1));
     int64_t np = 0;
-    GX_CUDA(ctx, cudaMemcpyAsync(&np, voff + nn, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-    GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    GX_TRY(gx_fetch(ctx, &np, voff + nn, sizeof(int64_t)));
     ctx->n_v_pairs = np;
     GX_TRY(gx_ensure(ctx, ctx->ref_did, sizeof(int32_t) * (size_t)(np + 1)));
     if (np > 0) {
@@ -1289,7 +1297,7 @@ int gx_plan_accurate(gx_ctx *ctx) {
                                           ctx->hint_near + ctx->hint_near / 8});
     GX_TRY(gx_ensure(ctx, ctx->plan_ctr, sizeof(int64_t) * PC_N));
     int64_t *ctr = dptr<int64_t>(ctx->plan_ctr);
-    int64_t hc[PC_N] = {};
+    int64_t hc[PC_N];
     const unsigned gmac = (unsigned)(ctx->sm_count > 0 ? ctx->sm_count * 16 : 2432);  // grid-stride k_mac
     for (int attempt = 0;; attempt++) {
         if (attempt == 8) return gx_fail(ctx, GX_ERR_CAP_EXCEEDED, "accurate plan: list storage keeps overflowing");
@@ -1305,20 +1313,9 @@ int gx_plan_accurate(gx_ctx *ctx) {
         int32_t *unode = dptr<int32_t>(ctx->scratch_b), *uchunk = unode + (ucap + 1);
         int64_t *ufar = dptr<int64_t>(ctx->scratch_e), *unear = ufar + (ucap + 1), *ufo = unear + (ucap + 1),
                 *uno = ufo + (ucap + 1);
-        GX_CUDA(ctx, cudaMemsetAsync(fcnt, 0, sizeof(int32_t) * (size_t)nn, ctx->stream));
-        GX_CUDA(ctx, cudaMemsetAsync(ncnt, 0, sizeof(int32_t) * (size_t)nn, ctx->stream));
-        // root: near itself (near list {root} at index 0)
-        hc[PC_FAR] = 0;
-        hc[PC_NEAR] = 1;
-        hc[PC_NEAR_LAST] = 0;
-        hc[PC_OVF] = 0;
-        const int64_t zero = 0;
-        const int32_t one = 1, root32 = (int32_t)root;
-        GX_CUDA(ctx, cudaMemcpyAsync(ctr, hc, sizeof(hc), cudaMemcpyHostToDevice, ctx->stream));
-        GX_CUDA(ctx, cudaMemcpyAsync(nstart + root, &zero, sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
-        GX_CUDA(ctx, cudaMemcpyAsync(ncnt + root, &one, sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
-        GX_CUDA(ctx, cudaMemcpyAsync(dptr<int32_t>(ctx->near_idx), &root32, sizeof(int32_t), cudaMemcpyHostToDevice,
-                                     ctx->stream));
+        k_mac_open<<<gx_blocks(nn, 256), 256, 0, ctx->stream>>>(nn, root, fcnt, ncnt, nstart,
+                                                                dptr<int32_t>(ctx->near_idx), ctr);
+        ctx->launches++;
         if (lv_low >= 2) {
             k_chain_check<<<gx_blocks(nl0, 256), 256, 0, ctx->stream>>>(nl0, lv_low, dptr<int4>(ctx->child), ctr);
             ctx->launches++;
@@ -1365,8 +1362,7 @@ int gx_plan_accurate(gx_ctx *ctx) {
             ctx->launches += 3;
             GX_CUDA(ctx, cudaGetLastError());
         }
-        GX_CUDA(ctx, cudaMemcpyAsync(hc, ctr, sizeof(hc), cudaMemcpyDeviceToHost, ctx->stream));
-        GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        GX_TRY(gx_fetch(ctx, hc, ctr, sizeof(hc)));
         if (!hc[PC_OVF]) break;
         if (hc[PC_OVF] & OVF_CHAIN) {  // no shortcut for this tree; its radii per level
             ctx->chain_levels = lv_low = 0;
@@ -1864,6 +1860,16 @@ int gx_tree_balance(gx_ctx *ctx, int64_t n_max, const double bounds[4]) {
     return gx_tree_rebuild_with_splits(ctx, n_max, bounds, splits);
 }
 
+// the totals of the items, the M2L units and the split pairs, to the host in one launch
+// (three copies, each after a kernel of its own, kept the GPU waiting between them)
+static __global__ void k_items_totals(const int64_t *dtot, const int64_t *m2l_units, const int64_t *pairs,
+                                      int64_t *out) {
+    const int k = threadIdx.x;
+    if (k < 4) out[k] = dtot[k];
+    else if (k == 4) out[k] = m2l_units ? *m2l_units : 0;
+    else if (k < 9) out[k] = pairs ? pairs[k - 5] : 0;
+}
+
 // P2P work items of the current plan (REF gather lists or ACCURATE near lists).
 int gx_plan_items(gx_ctx *ctx, bool accurate) {
     gx_ctx::Items &I = accurate ? ctx->items_acc : ctx->items_ref;
@@ -1889,18 +1895,14 @@ int gx_plan_items(gx_ctx *ctx, bool accurate) {
     GX_TRY(gx_ensure(ctx, I.off, sizeof(int64_t) * (size_t)(nl + 1)));
     GX_TRY(gx_ensure(ctx, ctx->scratch_c, sizeof(int64_t) * 4));
     int64_t *dtot = dptr<int64_t>(ctx->scratch_c);
-    int64_t tot[5] = {0, 0, 0, 0, 0};  // items, M2P items, P2L units, body-level units, M2L units
-    unsigned long long stot[4] = {0, 0, 0, 0};
     gx_ctx::P2LUnits &PU = ctx->p2l_units;
     if (split) {
         GX_TRY(gx_ensure(ctx, ctx->m2p_off, sizeof(int64_t) * (size_t)(nl + 1)));
         GX_TRY(gx_ensure(ctx, PU.leaf_u, sizeof(int64_t) * (size_t)(nl + 1)));
         GX_TRY(gx_ensure(ctx, PU.body_u, sizeof(int64_t) * (size_t)(nl + 1)));
-        GX_CUDA(ctx, cudaMemcpyAsync(stot, ctx->split_tot.p, sizeof(stot), cudaMemcpyDeviceToHost, ctx->stream));
     }
     GX_TRY(cs_launch(ctx, nl, k_item_offsets, nl, K, KM, start, cnt, scnt, body ? 1 : 0, dptr<int64_t>(I.off),
                      dptr<int64_t>(ctx->m2p_off), dptr<int64_t>(PU.leaf_u), dptr<int64_t>(PU.body_u), dtot));
-    GX_CUDA(ctx, cudaMemcpyAsync(tot, dtot, sizeof(int64_t) * 4, cudaMemcpyDeviceToHost, ctx->stream));
     gx_ctx::M2LUnits &U = ctx->m2l_units;
     const int64_t *fstart = accurate ? dptr<int64_t>(ctx->far_off) : nullptr;
     const int32_t *fcnt = accurate ? reinterpret_cast<const int32_t *>(fstart + nn) : nullptr;
@@ -1910,11 +1912,18 @@ int gx_plan_items(gx_ctx *ctx, bool accurate) {
         int64_t *nu = dptr<int64_t>(ctx->m2l_cnt);
         k_m2l_units_count<<<gx_blocks(nn + 1, 256), 256, 0, ctx->stream>>>(nn, fcnt, nu);
         GX_TRY(gx_exclusive_scan_i64(ctx, nu, dptr<int64_t>(U.node_u), nn + 1));
-        GX_CUDA(ctx, cudaMemcpyAsync(&tot[4], dptr<int64_t>(U.node_u) + nn, sizeof(int64_t), cudaMemcpyDeviceToHost,
-                                     ctx->stream));
         ctx->launches++;
     }
+    // the totals by one kernel into the page-locked words
+    int64_t *ph = static_cast<int64_t *>(ctx->pin);
+    k_items_totals<<<1, 32, 0, ctx->stream>>>(dtot, accurate ? dptr<int64_t>(U.node_u) + nn : nullptr,
+                                              split ? dptr<int64_t>(ctx->split_tot) : nullptr, ph);
+    GX_CUDA(ctx, cudaGetLastError());
     GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    ctx->launches++;
+    int64_t tot[5], stot[4];  // items, M2P items, P2L units, body-level units, M2L units; pairs
+    std::copy(ph, ph + 5, tot);
+    std::copy(ph + 5, ph + 9, stot);
     // the partial sums index items in 31 bits
     if (tot[0] >= ((int64_t)1 << 31)) return gx_fail(ctx, GX_ERR_CAP_EXCEEDED, "more than 2^31 P2P work items");
     GX_TRY(gx_ensure(ctx, I.leaf, sizeof(int32_t) * (size_t)(tot[0] + 1)));

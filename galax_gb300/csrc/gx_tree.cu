@@ -114,10 +114,12 @@ struct Arrays7 {
     const double *in[7];
     double *out[7];
 };
-__global__ void k_permute7(const uint32_t *__restrict__ idx, int64_t n, int na, Arrays7 a) {
+// perm (or null) takes a copy of idx.
+__global__ void k_permute7(const uint32_t *__restrict__ idx, int64_t n, int na, Arrays7 a, uint32_t *perm) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t j = idx[i];
+    if (perm) perm[i] = j;
     double v[7];
 #pragma unroll
     for (int k = 0; k < 7; k++)
@@ -130,13 +132,44 @@ __global__ void k_permute7(const uint32_t *__restrict__ idx, int64_t n, int na, 
 __device__ __forceinline__ double fmin_rs(double a, double b) { return (a != a) ? b : ((b != b) ? a : (b < a ? b : a)); }
 __device__ __forceinline__ double fmax_rs(double a, double b) { return (a != a) ? b : ((b != b) ? a : (b > a ? b : a)); }
 
-// leaf nodes (lib.rs:228-267); one thread per leaf, sums in body order.
+// ---- parent rounds (lib.rs:269-354) ----
+// The rounds run without host round trips: the level bounds, the shift and the round's
+// segment and group counts live in a device state block, every kernel of a round reads
+// them there, and the host only waits once per batch of rounds.  A round whose new
+// level would not fit the node storage sets the overflow flag; the build is then redone
+// with more storage.
+enum {
+    TS_S = 0, TS_E = 1, TS_C = 2, TS_SHIFT = 3, TS_NSEG = 4, TS_NG = 5, TS_FLAGS = 6, TS_ROUNDS = 7,
+    TS_CHAIN_M = 8,  // min over adjacent leaves of the highest bit in which their first keys differ
+    TS_CHAIN_L = 9,  // single-child rounds built by k_chain_rounds
+    TS_BEFORE = 10,  // rounds built before k_rounds_cluster
+    TS_N = 11
+};
+enum { TS_DONE = 1, TS_OVERFLOW = 2, TS_STUCK = 4 };
+constexpr int TS_MAX_ROUNDS = 400;  // level starts kept: TS_MAX_ROUNDS + 2
+
+__device__ __forceinline__ void tree_state_init(int64_t nl, int64_t *st, int64_t *lstart) {
+    st[TS_S] = 0;
+    st[TS_E] = st[TS_C] = nl;
+    st[TS_SHIFT] = 2;
+    st[TS_NSEG] = st[TS_NG] = 0;
+    st[TS_FLAGS] = nl > 1 ? 0 : TS_DONE;
+    st[TS_ROUNDS] = 0;
+    st[TS_CHAIN_M] = 64;
+    st[TS_CHAIN_L] = st[TS_BEFORE] = 0;
+    lstart[0] = 0;
+    lstart[1] = nl;
+}
+
+// leaf nodes (lib.rs:228-267); one thread per leaf, sums in body order.  The first also sets
+// the build's state.
 __global__ void k_leaves(const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ m,
                          const int32_t *__restrict__ rs, const int32_t *__restrict__ re, int64_t nl, double *cx,
                          double *cy, double *hw, double *mass, double *comx, double *comy, int32_t *bs, int32_t *be,
-                         int4 *child, int32_t *parent, uint8_t *is_leaf) {
+                         int4 *child, int32_t *parent, uint8_t *is_leaf, int64_t *st, int64_t *lstart) {
     int64_t L = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (L >= nl) return;
+    if (L == 0) tree_state_init(nl, st, lstart);
     int32_t s = rs[L], e = re[L];
     double ms = 0.0, sx = 0.0, sy = 0.0;
     double bx0 = 1.7976931348623157e308, bx1 = -1.7976931348623157e308;
@@ -169,21 +202,6 @@ __global__ void k_chunk_ranges(int64_t n, int64_t n_max, int64_t nl, int32_t *rs
     re[L] = (int32_t)e;
 }
 
-// ---- parent rounds (lib.rs:269-354) ----
-// The rounds run without host round trips: the level bounds, the shift and the round's
-// segment and group counts live in a device state block, every kernel of a round reads
-// them there, and the host only waits once per batch of rounds.  A round whose new
-// level would not fit the node storage sets the overflow flag; the build is then redone
-// with more storage.
-enum {
-    TS_S = 0, TS_E = 1, TS_C = 2, TS_SHIFT = 3, TS_NSEG = 4, TS_NG = 5, TS_FLAGS = 6, TS_ROUNDS = 7,
-    TS_CHAIN_M = 8,  // min over adjacent leaves of the highest bit in which their first keys differ
-    TS_CHAIN_L = 9,  // single-child rounds built by k_chain_rounds
-    TS_BEFORE = 10,  // rounds built before k_rounds_cluster
-    TS_N = 11
-};
-enum { TS_DONE = 1, TS_OVERFLOW = 2, TS_STUCK = 4 };
-constexpr int TS_MAX_ROUNDS = 400;  // level starts kept: TS_MAX_ROUNDS + 2
 
 constexpr int TS_CLUSTER = 65536;  // levels of at most this many nodes: k_rounds_cluster
 // the multi-block round kernels do nothing once the build is over or the level is small
@@ -616,12 +634,8 @@ static int build_from_ranges(gx_ctx *ctx, const int32_t *rs, const int32_t *re, 
             dptr<double>(ctx->x), dptr<double>(ctx->y), dptr<double>(ctx->m), rs, re, nl, dptr<double>(ctx->cx),
             dptr<double>(ctx->cy), dptr<double>(ctx->hw), dptr<double>(ctx->mass), dptr<double>(ctx->comx),
             dptr<double>(ctx->comy), dptr<int32_t>(ctx->bs), dptr<int32_t>(ctx->be), dptr<int4>(ctx->child),
-            dptr<int32_t>(ctx->parent), dptr<uint8_t>(ctx->is_leaf));
+            dptr<int32_t>(ctx->parent), dptr<uint8_t>(ctx->is_leaf), st, lstart);
         ctx->launches++;
-        const int64_t init[TS_N] = {0, nl, nl, 2, 0, 0, nl > 1 ? 0 : TS_DONE, 0, 64, 0, 0};
-        const int64_t ls01[2] = {0, nl};
-        GX_CUDA(ctx, cudaMemcpyAsync(st, init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream));
-        GX_CUDA(ctx, cudaMemcpyAsync(lstart, ls01, sizeof(ls01), cudaMemcpyHostToDevice, ctx->stream));
         if (nl > 1) {
             k_chain_depth<<<gx_blocks(nl, 256), 256, 0, ctx->stream>>>(nl, dptr<uint64_t>(ctx->keys),
                                                                       dptr<int32_t>(ctx->bs), st);
@@ -684,8 +698,8 @@ static int build_from_ranges(gx_ctx *ctx, const int32_t *rs, const int32_t *re, 
             ctx->launches += 3 + large;
             GX_CUDA(ctx, cudaGetLastError());
             issued += batch;
-            GX_CUDA(ctx, cudaMemcpyAsync(hs, st, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream));
-            GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+            static_assert(sizeof(hs) <= GX_PIN, "the state and the level starts in one gx_fetch");
+            GX_TRY(gx_fetch(ctx, hs, st, sizeof(hs)));
             if (hs[TS_FLAGS] & TS_STUCK) return gx_fail(ctx, GX_ERR_STATE, "tree build did not converge");
             if (hs[TS_FLAGS] != 0) break;
             batch = 8;
@@ -743,6 +757,7 @@ int gx_tree_build_device(gx_ctx *ctx, int64_t n, int64_t n_max, const double bou
         // arrays per launch as fit in half of the 129 MB L2 together (all seven at 1M)
         DevBuf *arrs[7] = {&ctx->x, &ctx->y, &ctx->vx, &ctx->vy, &ctx->m, &ctx->ax, &ctx->ay};
         const int per = (int)std::max<int64_t>(1, std::min<int64_t>(7, ((int64_t)64 << 20) / (8 * n)));
+        GX_TRY(gx_ensure(ctx, ctx->perm, sizeof(uint32_t) * n));
         for (int k0 = 0; k0 < 7; k0 += per) {
             const int na = std::min(per, 7 - k0);
             Arrays7 a7{};
@@ -751,12 +766,11 @@ int gx_tree_build_device(gx_ctx *ctx, int64_t n, int64_t n_max, const double bou
                 a7.in[k] = dptr<double>(*arrs[k0 + k]);
                 a7.out[k] = dptr<double>(ctx->body_alt[k0 + k]);
             }
-            k_permute7<<<gx_blocks(n, 256), 256, 0, ctx->stream>>>(idx, n, na, a7);
+            k_permute7<<<gx_blocks(n, 256), 256, 0, ctx->stream>>>(
+                idx, n, na, a7, k0 == 0 ? dptr<uint32_t>(ctx->perm) : nullptr);
             ctx->launches++;
         }
         for (int k = 0; k < 7; k++) std::swap(*arrs[k], ctx->body_alt[k]);
-        GX_TRY(gx_ensure(ctx, ctx->perm, sizeof(uint32_t) * n));
-        GX_CUDA(ctx, cudaMemcpyAsync(ctx->perm.p, idx, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, ctx->stream));
         GX_CUDA(ctx, cudaGetLastError());
     }
     int64_t nl = (n + n_max - 1) / n_max;
