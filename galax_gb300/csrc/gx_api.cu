@@ -216,6 +216,8 @@ int gx_create(const gx_config *cfg, gx_ctx **out) {
     }
     // kernel-image check: the status allocation and a memset are the first device work
     int s = gx_ensure(ctx, ctx->status, 64);
+    if (s == GX_OK) s = gx_ensure(ctx, ctx->queues, 128 * GX_QUEUES);
+    if (s == GX_OK && cudaMemset(ctx->queues.p, 0, 128 * GX_QUEUES) != cudaSuccess) s = GX_ERR_CUDA;
     if (s != GX_OK) {
         gx_destroy(ctx);
         return s;
@@ -250,7 +252,7 @@ int gx_destroy(gx_ctx *ctx) {
                       &ctx->Lff32, &ctx->pos32, &ctx->fl32, &ctx->part, &ctx->items_ref.leaf, &ctx->items_ref.qb, &ctx->items_ref.nq, &ctx->items_ref.off, &ctx->items_acc.leaf, &ctx->items_acc.qb, &ctx->items_acc.nq, &ctx->items_acc.off, &ctx->scratch_a, &ctx->scratch_b, &ctx->scratch_c, &ctx->scratch_d,
                       &ctx->scratch_e, &ctx->scratch_f, &ctx->scratch_g, &ctx->status, &ctx->red, &ctx->flush, &ctx->adj_lx, &ctx->adj_ly, &ctx->adj_lvx, &ctx->adj_lvy, &ctx->adj_lm, &ctx->adj_gx, &ctx->adj_gy, &ctx->adj_gm, &ctx->adj_lax, &ctx->adj_lay, &ctx->adj_lf, &ctx->adj_dL, &ctx->adj_dM, &ctx->adj_dMleaf, &ctx->adj_lam32, &ctx->ckpt, &ctx->seg, &ctx->ids, &ctx->perm, &ctx->roll_perms, &ctx->radius32,
                       &ctx->m2l_units.node, &ctx->m2l_units.start, &ctx->m2l_units.len, &ctx->m2l_units.node_u,
-                      &ctx->m2l_part, &ctx->m2l_count, &ctx->plan_ctr, &ctx->tree_state, &ctx->m2l_cnt, &ctx->split_cnt,
+                      &ctx->queues, &ctx->m2l_part, &ctx->m2l_count, &ctx->plan_ctr, &ctx->tree_state, &ctx->m2l_cnt, &ctx->split_cnt,
                       &ctx->split_tot, &ctx->p2l_units.leaf, &ctx->p2l_units.start, &ctx->p2l_units.len,
                       &ctx->p2l_units.leaf_u, &ctx->p2l_units.body_u, &ctx->p2l_part, &ctx->m2p_list,
                       &ctx->m2p_off, &ctx->p2p_mask, &ctx->body_off32};

@@ -105,7 +105,25 @@ __device__ __forceinline__ T warp_sum_t(T v) {
     return v;
 }
 
-// Warps a block of the kernels that give a warp a work item or unit: one, as a block's place
+// The items of a kernel whose blocks, of one warp, take them from a queue: block b starts
+// with item b and, while it works on one, asks for the next.  Each item is asked for once, so
+// the counter wraps to 0 with the last and is ready for the next launch.  A block an item left
+// a third of the places on an SM empty at any time (Plummer 1M: 23 of 32 P2P blocks, the
+// launch of a block and its first loads against 25 us of work).
+struct ItemQueue {
+    unsigned it, n, *queue, asked;  // fewer than 2^31 items (a grid's limit, too)
+    __device__ __forceinline__ ItemQueue(unsigned *q, int64_t count) : it(blockIdx.x), n((unsigned)count), queue(q) { ask(); }
+    __device__ __forceinline__ void ask() {
+        if (gridDim.x < n && (threadIdx.x & 31) == 0) asked = gridDim.x + atomicInc(queue, n - 1);
+    }
+    __device__ __forceinline__ bool more() const { return it < n; }
+    __device__ __forceinline__ void next() {
+        __syncwarp();  // the last item's shared memory has been read
+        it = gridDim.x < n ? __shfl_sync(0xffffffffu, asked, 0) : n;
+        if (it < n) ask();
+    }
+};
+// Warps a block of the item and unit kernels: one, as a block's place
 // on an SM is free again only when its last warp is done, and items differ in length (disk 4M,
 // p = 6: 18.65 -> 17.9 ms an evaluation; Plummer 1M, whose items are mostly full, 2.40 -> 2.37).
 constexpr int WPB = 1;
@@ -916,34 +934,35 @@ __global__ void __launch_bounds__(32 * WPB, (sizeof(T) == 4 && P <= 4) ? 32 / WP
     int64_t n_units, const int32_t *__restrict__ unode, const int64_t *__restrict__ ustart,
     const int32_t *__restrict__ ulen, const int64_t *__restrict__ node_u, const int32_t *__restrict__ idx,
     const double *__restrict__ comx, const double *__restrict__ comy, const float4 *__restrict__ comhl, double eps2d,
-    const T *__restrict__ M, T *__restrict__ L, T *part, unsigned *count) {
+    const T *__restrict__ M, T *__restrict__ L, T *part, unsigned *count, unsigned *queue) {
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<T>(NC);
     const int PP = gx_rt_order(P);
     const int NCr = (PP + 1) * (PP + 2) / 2;
     (void)NCr;
-    int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
-    if (u >= n_units) return;
-    const int64_t node = unode[u];
-    float4 thl = make_float4(0.f, 0.f, 0.f, 0.f);
-    if constexpr (sizeof(T) == 4) thl = comhl[node];
-    T acc[NC];
+    for (ItemQueue items(queue, n_units); items.more(); items.next()) {
+        const int64_t u = items.it;
+        const int64_t node = unode[u];
+        float4 thl = make_float4(0.f, 0.f, 0.f, 0.f);
+        if constexpr (sizeof(T) == 4) thl = comhl[node];
+        T acc[NC];
 #pragma unroll
-    for (int k = 0; k < NCr; k++) acc[k] = T(0);
-    m2l_sources<P, T, int32_t>(idx, ustart[u], ulen[u], lane, comx[node], comy[node], thl, comx, comy, comhl,
-                               (T)eps2d, M, acc);
-    const int64_t u0 = node_u[node], u1 = node_u[node + 1];
-    const auto store = [&](int k, T v) {
-        int i, j;
-        mi_split(k, i, j);
-        L[node * NS + k] = v * -tab_ifp<T>(i, j);
-    };
-    if (u1 - u0 == 1) {
-        warp_coeffs<NC>(acc, store);
-    } else {
-        warp_coeffs<NC>(acc, [&](int k, T v) { part[u * NS + k] = v; });
-        last_unit_sums<NC, NS>(node, u0, u1, part, count, store);
+        for (int k = 0; k < NCr; k++) acc[k] = T(0);
+        m2l_sources<P, T, int32_t>(idx, ustart[u], ulen[u], lane, comx[node], comy[node], thl, comx, comy, comhl,
+                                   (T)eps2d, M, acc);
+        const int64_t u0 = node_u[node], u1 = node_u[node + 1];
+        const auto store = [&](int k, T v) {
+            int i, j;
+            mi_split(k, i, j);
+            L[node * NS + k] = v * -tab_ifp<T>(i, j);
+        };
+        if (u1 - u0 == 1) {
+            warp_coeffs<NC>(acc, store);
+        } else {
+            warp_coeffs<NC>(acc, [&](int k, T v) { part[u * NS + k] = v; });
+            last_unit_sums<NC, NS>(node, u0, u1, part, count, store);
+        }
     }
 }
 
@@ -1262,17 +1281,18 @@ __global__ void __launch_bounds__(32 * WPB, 28 / WPB) k_p2p32_items(int64_t n_it
                                                      const float4 *__restrict__ pos, const double *__restrict__ comx,
                                                      const double *__restrict__ comy, const int32_t *__restrict__ bs,
                                                      const int32_t *__restrict__ be, const int32_t *__restrict__ src_idx,
-                                                     float eps2, int tchunks, float2 *__restrict__ part) {
+                                                     float eps2, int tchunks, float2 *__restrict__ part,
+                                                     unsigned *queue) {
     // staged sources, one row of 32 per warp, as x / y / m planes so that one
     // broadcast 16-byte load yields the x (or y, m) of four consecutive sources
     __shared__ __align__(16) float sx[WPB][32], sy[WPB][32], sm[WPB][32];
     int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // one item a warp
-    if (it < n_items) {
+    for (ItemQueue items(queue, n_items); items.more(); items.next()) {
+        const int64_t it = items.it;
         int32_t leaf = item_leaf[it];
         int64_t qb = item_qb[it];
         int nq = item_nq[it];
-        if (nq < 0) return;  // an M2P item of the near-list split (k_m2p)
+        if (nq < 0) continue;  // an M2P item of the near-list split (k_m2p)
         int32_t t0 = bs[leaf], t1 = be[leaf];
         double tcx = comx[leaf], tcy = comy[leaf];
         int sl = lane < nq ? src_idx[qb + lane] : -1;
@@ -1384,15 +1404,15 @@ __global__ void __launch_bounds__(32 * WPB, 32 / WPB) k_p2p32_rows1(int64_t n_it
                                                     const float4 *__restrict__ pos, const double *__restrict__ comx,
                                                     const double *__restrict__ comy, const int32_t *__restrict__ bs,
                                                     const int32_t *__restrict__ be, const int32_t *__restrict__ src_idx,
-                                                    float eps2, float2 *__restrict__ part) {
+                                                    float eps2, float2 *__restrict__ part, unsigned *queue) {
     __shared__ __align__(16) float sx[WPB][32], sy[WPB][32], sm[WPB][32];
     __shared__ __align__(16) int4 meta[WPB][32];  // per source leaf: begin, end, shift x, shift y (FP32 bits)
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // one item a warp
-    if (it < n_items) {
+    for (ItemQueue items(queue, n_items); items.more(); items.next()) {
+        const int64_t it = items.it;
         const int32_t leaf = item_leaf[it];
         const int nq = item_nq[it];
-        if (nq < 0) return;  // an M2P item of the near-list split (k_m2p)
+        if (nq < 0) continue;  // an M2P item of the near-list split (k_m2p)
         const int32_t t0 = bs[leaf], t1 = be[leaf];
         bool own_lane = false;
         if (lane < nq) {
@@ -1492,16 +1512,16 @@ __global__ void __launch_bounds__(32 * WPB, 32 / WPB) k_p2p32_rows(int64_t n_ite
                                                     const float4 *__restrict__ pos, const double *__restrict__ comx,
                                                     const double *__restrict__ comy, const int32_t *__restrict__ bs,
                                                     const int32_t *__restrict__ be, const int32_t *__restrict__ src_idx,
-                                                    float eps2, float2 *__restrict__ part) {
+                                                    float eps2, float2 *__restrict__ part, unsigned *queue) {
     __shared__ __align__(16) float sx[WPB][32], sy[WPB][32], sm[WPB][32];
     __shared__ __align__(16) int4 meta[WPB][32];  // per source leaf: begin, end, shift x, shift y (FP32 bits)
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int half = lane >> 4, tl = lane & 15;  // lane: targets tl and tl + 16, source quads of its half
-    const int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // one item a warp
-    if (it < n_items) {
+    for (ItemQueue items(queue, n_items); items.more(); items.next()) {
+        const int64_t it = items.it;
         const int32_t leaf = item_leaf[it];
         const int nq = item_nq[it];
-        if (nq < 0) return;  // an M2P item of the near-list split (k_m2p)
+        if (nq < 0) continue;  // an M2P item of the near-list split (k_m2p)
         const int32_t t0 = bs[leaf], t1 = be[leaf];
         bool own_lane = false;
         if (lane < nq) {
@@ -1623,7 +1643,7 @@ __global__ void __launch_bounds__(32 * WPB, 32 / WPB) k_p2p32_stream(
     const int32_t *__restrict__ item_nq, const float4 *__restrict__ pos, const double *__restrict__ comx,
     const double *__restrict__ comy, const int32_t *__restrict__ bs, const int32_t *__restrict__ be,
     const int32_t *__restrict__ src_idx, const uint32_t *__restrict__ p2p_mask, float eps2,
-    float2 *__restrict__ part) {
+    float2 *__restrict__ part, unsigned *queue) {
     __shared__ __align__(16) float sx[WPB][32], sy[WPB][32], sm[WPB][32];
     __shared__ __align__(16) int4 meta[WPB][32];  // per source leaf: begin, end, shift x, shift y (FP32 bits)
     __shared__ uint16_t strm[WPB][32 * 32];       // the item's kept bodies: (row << 5) | body
@@ -1633,11 +1653,11 @@ __global__ void __launch_bounds__(32 * WPB, 32 / WPB) k_p2p32_stream(
     const int half = lane >> 4, tl = lane & 15;  // lane: targets tl and tl + 16, source quads of its half
     const float4 far4 = make_float4(1e18f, 1e18f, 0.f, 0.f);
     const bool self_in_stream = eps2 > 0.f;
-    const int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // one item a warp
-    if (it < n_items) {
+    for (ItemQueue items(queue, n_items); items.more(); items.next()) {
+        const int64_t it = items.it;
         const int32_t leaf = item_leaf[it];
         const int nq = item_nq[it];
-        if (nq < 0) return;  // an M2P item of the near-list split (k_m2p)
+        if (nq < 0) continue;  // an M2P item of the near-list split (k_m2p)
         const int32_t t0 = bs[leaf], t1 = be[leaf];
         bool own_lane = false;
         uint32_t keep = 0;
@@ -1870,14 +1890,14 @@ __global__ void __launch_bounds__(32 * WPB) k_m2p(int64_t n_list, const int32_t 
                                              const double *__restrict__ Y, const double *__restrict__ comx,
                                              const double *__restrict__ comy, const int32_t *__restrict__ bs,
                                              const int32_t *__restrict__ be, const int32_t *__restrict__ src_idx,
-                                             T eps2, const T *__restrict__ M, int tchunks, V *__restrict__ part) {
+                                             T eps2, const T *__restrict__ M, int tchunks, V *__restrict__ part,
+                                             unsigned *queue) {
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<T>(NC);
     constexpr int CPL = (NC + 31) / 32;  // coefficients a lane prepares
     __shared__ V sw[WPB][NC];
     const unsigned full = 0xffffffffu;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
     T scx[CPL], scy[CPL];
 #pragma unroll
     for (int c = 0; c < CPL; c++) {
@@ -1887,8 +1907,8 @@ __global__ void __launch_bounds__(32 * WPB) k_m2p(int64_t n_list, const int32_t 
         scx[c] = sign * tab_ff<T>(si + 1, sj);
         scy[c] = sign * tab_ff<T>(si, sj + 1);
     }
-    for (int64_t li = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; li < n_list; li += nwarps) {
-        const int64_t it = list[li];
+    for (ItemQueue items(queue, n_list); items.more(); items.next()) {
+        const int64_t it = list[items.it];
         const int nq0 = item_nq[it];
         if (nq0 >= 0) continue;
         const int nq = -nq0;
@@ -2003,7 +2023,8 @@ __global__ void __launch_bounds__(32 * WPB, 32 / WPB) k_m2p_x2(int64_t n_list, c
                                                 const double *__restrict__ comx, const double *__restrict__ comy,
                                                 const int32_t *__restrict__ bs, const int32_t *__restrict__ be,
                                                 const int32_t *__restrict__ src_idx, float eps2,
-                                                const float *__restrict__ M, float2 *__restrict__ part) {
+                                                const float *__restrict__ M, float2 *__restrict__ part,
+                                                unsigned *queue) {
     static_assert(P <= 5, "shared-memory moment rows are sized for p <= 5");
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<float>(NC);
@@ -2012,11 +2033,11 @@ __global__ void __launch_bounds__(32 * WPB, 32 / WPB) k_m2p_x2(int64_t n_list, c
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int half = lane >> 4, tl = lane & 15;
     const f2v E2 = f2splat(eps2);
-    const int64_t li = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // one item a warp
-    if (li < n_list) {
+    for (ItemQueue items(queue, n_list); items.more(); items.next()) {
+        const int64_t li = items.it;
         const int32_t it = list[li];
         const int nq0 = item_nq[it];
-        if (nq0 >= 0) return;
+        if (nq0 >= 0) continue;
         const int nq = -nq0;
         const int32_t leaf = item_leaf[it];
         if (lane < nq) {
@@ -2092,95 +2113,96 @@ __global__ void __launch_bounds__(32 * WPB, 24 / WPB) k_p2l_x2(int64_t n_units, 
                                                 const int32_t *__restrict__ src_idx, const float4 *__restrict__ pos,
                                                 const double *__restrict__ comx, const double *__restrict__ comy,
                                                 const int32_t *__restrict__ bs, const int32_t *__restrict__ be,
-                                                float eps2, float *__restrict__ ppart) {
+                                                float eps2, float *__restrict__ ppart, unsigned *queue) {
     static_assert(P <= 5, "paired accumulators are sized for p <= 5");
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<float>(NC);
     __shared__ __align__(16) float4 p2l_ring[WPB][P2L_RING][64];  // per warp: P2L_RING rounds x 64 bodies
     const int lane = threadIdx.x & 31;
     const int half = lane >> 4, tl = lane & 15;
-    const int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (u >= n_units) return;
-    const int32_t a = uleaf[u];
-    const int nq = ulen[u];
-    if (nq < 0) return;  // a body-level unit (k_p2l_body_x2)
-    int32_t sb = 0, se = 0;
-    float shx = 0.f, shy = 0.f;
-    if (lane < nq) {
-        const int32_t sl = src_idx[ustart[u] + lane];
-        sb = bs[sl];
-        se = be[sl];
-        shx = (float)(comx[a] - comx[sl]);
-        shy = (float)(comy[a] - comy[sl]);
-    }
-    const f2v E2 = f2splat(eps2);
-    f2v acc[NC];
-#pragma unroll
-    for (int k = 0; k < NC; k++) acc[k] = f2splat(0.f);
-    const int rounds = (nq + 1) >> 1;  // both halves run the same number of rounds
-    // round r: this half's source k = 2r + half (its first 32 bodies: lane tl loads bodies
-    // tl and tl + 16).  They are copied global -> shared by cp.async P2L_RING - 1 rounds
-    // ahead, each lane reading back only its own copies, so the loads in flight hold no
-    // registers; leaves above 32 bodies load the rest in place.
-    auto src = [&](int r, int32_t &j0, int32_t &j1, float &ox, float &oy) {
-        const int k = 2 * r + half;
-        const int kk = k < nq ? k : 0;
-        j0 = __shfl_sync(0xffffffffu, sb, kk);
-        const int32_t e1 = __shfl_sync(0xffffffffu, se, kk);
-        j1 = k < nq ? e1 : j0;  // the half without a source this round runs no body
-        ox = __shfl_sync(0xffffffffu, shx, kk);
-        oy = __shfl_sync(0xffffffffu, shy, kk);
-    };
-    auto body_pair = [&](const float4 &pA, const float4 &pB, float ox, float oy) {
-        // com_a - x_j = (com_a - com_s) - (x_j - com_s); an empty slot has m = 0 and
-        // sits at com_s, at the leaf pair's nonzero distance
-        const f2v dx = f2sub(f2splat(ox), f2pair(pA.x, pB.x)), dy = f2sub(f2splat(oy), f2pair(pA.y, pB.y));
-        const f2v ir = rsqrt_x2(f2fma(dx, dx, f2fma(dy, dy, E2)));
-        f2v c[NC];
-        taylor_1r_x2<P>(dx, dy, ir, f2mul(ir, ir), c);
-        const f2v mm = f2pair(pA.z, pB.z);
-#pragma unroll
-        for (int q = 0; q < NC; q++) acc[q] = f2fma(mm, c[q], acc[q]);
-    };
-    float4 *ring = &p2l_ring[threadIdx.x >> 5][0][0];
-    auto issue = [&](int r) {
-        if (r < rounds) {
-            int32_t j0, j1;
-            float ox, oy;
-            src(r, j0, j1, ox, oy);
-            const int32_t jA = j0 + tl, jB = j0 + tl + 16;
-            float4 *dst = ring + (r % P2L_RING) * 64 + lane;  // body A at lane, B at 32 + lane
-            cp_async16_zfill(dst, pos + (jA < j1 ? jA : 0), jA < j1);
-            cp_async16_zfill(dst + 32, pos + (jB < j1 ? jB : 0), jB < j1);
+    for (ItemQueue items(queue, n_units); items.more(); items.next()) {
+        const int64_t u = items.it;
+        const int32_t a = uleaf[u];
+        const int nq = ulen[u];
+        if (nq < 0) continue;  // a body-level unit (k_p2l_body_x2)
+        int32_t sb = 0, se = 0;
+        float shx = 0.f, shy = 0.f;
+        if (lane < nq) {
+            const int32_t sl = src_idx[ustart[u] + lane];
+            sb = bs[sl];
+            se = be[sl];
+            shx = (float)(comx[a] - comx[sl]);
+            shy = (float)(comy[a] - comy[sl]);
         }
-        cp_async_commit();  // an empty group past the last round keeps the count uniform
-    };
+        const f2v E2 = f2splat(eps2);
+        f2v acc[NC];
 #pragma unroll
-    for (int r = 0; r < P2L_RING - 1; r++) issue(r);
-    for (int r = 0; r < rounds; r++) {
-        issue(r + P2L_RING - 1);
-        cp_async_wait<P2L_RING - 1>();  // round r's copies have landed
-        int32_t c0, c1;
-        float cox, coy;
-        src(r, c0, c1, cox, coy);
-        const float4 *slot = ring + (r % P2L_RING) * 64 + lane;
-        if (c0 < c1) body_pair(slot[0], slot[32], cox, coy);
-        for (int32_t b0 = c0 + 32; b0 < c1; b0 += 32) {
-            const int32_t jA = b0 + tl, jB = b0 + tl + 16;
-            const float4 pA = jA < c1 ? pos[jA] : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float4 pB = jB < c1 ? pos[jB] : make_float4(0.f, 0.f, 0.f, 0.f);
-            body_pair(pA, pB, cox, coy);
+        for (int k = 0; k < NC; k++) acc[k] = f2splat(0.f);
+        const int rounds = (nq + 1) >> 1;  // both halves run the same number of rounds
+        // round r: this half's source k = 2r + half (its first 32 bodies: lane tl loads bodies
+        // tl and tl + 16).  They are copied global -> shared by cp.async P2L_RING - 1 rounds
+        // ahead, each lane reading back only its own copies, so the loads in flight hold no
+        // registers; leaves above 32 bodies load the rest in place.
+        auto src = [&](int r, int32_t &j0, int32_t &j1, float &ox, float &oy) {
+            const int k = 2 * r + half;
+            const int kk = k < nq ? k : 0;
+            j0 = __shfl_sync(0xffffffffu, sb, kk);
+            const int32_t e1 = __shfl_sync(0xffffffffu, se, kk);
+            j1 = k < nq ? e1 : j0;  // the half without a source this round runs no body
+            ox = __shfl_sync(0xffffffffu, shx, kk);
+            oy = __shfl_sync(0xffffffffu, shy, kk);
+        };
+        auto body_pair = [&](const float4 &pA, const float4 &pB, float ox, float oy) {
+            // com_a - x_j = (com_a - com_s) - (x_j - com_s); an empty slot has m = 0 and
+            // sits at com_s, at the leaf pair's nonzero distance
+            const f2v dx = f2sub(f2splat(ox), f2pair(pA.x, pB.x)), dy = f2sub(f2splat(oy), f2pair(pA.y, pB.y));
+            const f2v ir = rsqrt_x2(f2fma(dx, dx, f2fma(dy, dy, E2)));
+            f2v c[NC];
+            taylor_1r_x2<P>(dx, dy, ir, f2mul(ir, ir), c);
+            const f2v mm = f2pair(pA.z, pB.z);
+#pragma unroll
+            for (int q = 0; q < NC; q++) acc[q] = f2fma(mm, c[q], acc[q]);
+        };
+        float4 *ring = &p2l_ring[threadIdx.x >> 5][0][0];
+        auto issue = [&](int r) {
+            if (r < rounds) {
+                int32_t j0, j1;
+                float ox, oy;
+                src(r, j0, j1, ox, oy);
+                const int32_t jA = j0 + tl, jB = j0 + tl + 16;
+                float4 *dst = ring + (r % P2L_RING) * 64 + lane;  // body A at lane, B at 32 + lane
+                cp_async16_zfill(dst, pos + (jA < j1 ? jA : 0), jA < j1);
+                cp_async16_zfill(dst + 32, pos + (jB < j1 ? jB : 0), jB < j1);
+            }
+            cp_async_commit();  // an empty group past the last round keeps the count uniform
+        };
+#pragma unroll
+        for (int r = 0; r < P2L_RING - 1; r++) issue(r);
+        for (int r = 0; r < rounds; r++) {
+            issue(r + P2L_RING - 1);
+            cp_async_wait<P2L_RING - 1>();  // round r's copies have landed
+            int32_t c0, c1;
+            float cox, coy;
+            src(r, c0, c1, cox, coy);
+            const float4 *slot = ring + (r % P2L_RING) * 64 + lane;
+            if (c0 < c1) body_pair(slot[0], slot[32], cox, coy);
+            for (int32_t b0 = c0 + 32; b0 < c1; b0 += 32) {
+                const int32_t jA = b0 + tl, jB = b0 + tl + 16;
+                const float4 pA = jA < c1 ? pos[jA] : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 pB = jB < c1 ? pos[jB] : make_float4(0.f, 0.f, 0.f, 0.f);
+                body_pair(pA, pB, cox, coy);
+            }
         }
-    }
-    cp_async_wait<0>();
-    float sum[NC];
+        cp_async_wait<0>();
+        float sum[NC];
 #pragma unroll
-    for (int q = 0; q < NC; q++) {
-        float lo, hi;
-        upk2(acc[q].v, lo, hi);
-        sum[q] = lo + hi;
+        for (int q = 0; q < NC; q++) {
+            float lo, hi;
+            upk2(acc[q].v, lo, hi);
+            sum[q] = lo + hi;
+        }
+        warp_coeffs<NC>(sum, [&](int q, float v) { ppart[u * NS + q] = v; });
     }
-    warp_coeffs<NC>(sum, [&](int q, float v) { ppart[u * NS + q] = v; });
 }
 
 // Body-level P2L units, mixed form, p <= 5: a unit is up to GX_BODY_UNIT consecutive
@@ -2199,7 +2221,7 @@ __global__ void __launch_bounds__(32 * WPB, 24 / WPB) k_p2l_body_x2(int64_t u_ba
                                                      const uint32_t *__restrict__ p2p_mask,
                                                      const float4 *__restrict__ pos, const double *__restrict__ comx,
                                                      const double *__restrict__ comy, const int32_t *__restrict__ bs,
-                                                     float eps2, float *__restrict__ ppart) {
+                                                     float eps2, float *__restrict__ ppart, unsigned *queue) {
     static_assert(P <= 5, "paired accumulators are sized for p <= 5");
     static_assert(GX_BODY_UNIT % 32 == 0 && GX_BODY_UNIT * 32 <= 65536, "whole rows per lane, 16-bit entries");
     constexpr int RPL = GX_BODY_UNIT / 32;  // rows per lane
@@ -2210,104 +2232,105 @@ __global__ void __launch_bounds__(32 * WPB, 24 / WPB) k_p2l_body_x2(int64_t u_ba
     __shared__ uint16_t strm[WPB][GX_BODY_UNIT * 32];        // the unit's masked bodies: (row << 5) | body
     const unsigned full = 0xffffffffu;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t wu = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (wu >= n_units) return;
-    const int64_t u = u_base + wu;  // the body-level units follow the leaf-level ones
-    const int raw = ulen[u];
-    if (raw >= 0) return;  // a leaf-level unit (k_p2l_x2)
-    const int nq = -raw;
-    const int32_t a = uleaf[u];
-    const double acx = comx[a], acy = comy[a];
-    uint32_t take[RPL];
+    for (ItemQueue items(queue, n_units); items.more(); items.next()) {
+        const int64_t wu = items.it;
+        const int64_t u = u_base + wu;  // the body-level units follow the leaf-level ones
+        const int raw = ulen[u];
+        if (raw >= 0) continue;  // a leaf-level unit (k_p2l_x2)
+        const int nq = -raw;
+        const int32_t a = uleaf[u];
+        const double acx = comx[a], acy = comy[a];
+        uint32_t take[RPL];
 #pragma unroll
-    for (int h = 0; h < RPL; h++) {
-        take[h] = 0u;
-        const int r = 32 * h + lane;
-        if (r < nq) {
-            const int64_t q = ustart[u] + r;
-            const int32_t sl = src_idx[q];
-            take[h] = p2p_mask[q];  // 0 for the self row
-            rb0[w][r] = bs[sl];
-            rsh[w][r] = make_float2((float)(acx - comx[sl]), (float)(acy - comy[sl]));
+        for (int h = 0; h < RPL; h++) {
+            take[h] = 0u;
+            const int r = 32 * h + lane;
+            if (r < nq) {
+                const int64_t q = ustart[u] + r;
+                const int32_t sl = src_idx[q];
+                take[h] = p2p_mask[q];  // 0 for the self row
+                rb0[w][r] = bs[sl];
+                rsh[w][r] = make_float2((float)(acx - comx[sl]), (float)(acy - comy[sl]));
+            }
         }
-    }
-    // exclusive scan of the rows' counts (rows lane, then rows 32 + lane, ...)
-    int base = 0, T = 0;
-    int excl[RPL];
+        // exclusive scan of the rows' counts (rows lane, then rows 32 + lane, ...)
+        int base = 0, T = 0;
+        int excl[RPL];
 #pragma unroll
-    for (int h = 0; h < RPL; h++) {
-        const int c = __popc(take[h]);
-        int incl = c;
+        for (int h = 0; h < RPL; h++) {
+            const int c = __popc(take[h]);
+            int incl = c;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(full, incl, o);
-            if (lane >= o) incl += t;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(full, incl, o);
+                if (lane >= o) incl += t;
+            }
+            excl[h] = base + incl - c;
+            base += __shfl_sync(full, incl, 31);
         }
-        excl[h] = base + incl - c;
-        base += __shfl_sync(full, incl, 31);
-    }
-    T = base;
+        T = base;
 #pragma unroll
-    for (int h = 0; h < RPL; h++) {
-        uint32_t m = take[h];
-        int pp = excl[h];
-        const int r = 32 * h + lane;
-        while (m) {
-            const int j = __ffs(m) - 1;
-            m &= m - 1u;
-            strm[w][pp++] = (uint16_t)((r << 5) | j);
+        for (int h = 0; h < RPL; h++) {
+            uint32_t m = take[h];
+            int pp = excl[h];
+            const int r = 32 * h + lane;
+            while (m) {
+                const int j = __ffs(m) - 1;
+                m &= m - 1u;
+                strm[w][pp++] = (uint16_t)((r << 5) | j);
+            }
         }
-    }
-    __syncwarp();
-    const f2v E2 = f2splat(eps2);
-    f2v acc[NC];
+        __syncwarp();
+        const f2v E2 = f2splat(eps2);
+        f2v acc[NC];
 #pragma unroll
-    for (int k = 0; k < NC; k++) acc[k] = f2splat(0.f);
-    auto get = [&](int p, float4 &v, float2 &o) {
-        if (p < T) {
-            const int e = strm[w][p];
-            v = pos[rb0[w][e >> 5] + (e & 31)];
-            o = rsh[w][e >> 5];
-        } else {
-            v = make_float4(0.f, 0.f, 0.f, 0.f);
-            o = make_float2(1.f, 1.f);
+        for (int k = 0; k < NC; k++) acc[k] = f2splat(0.f);
+        auto get = [&](int p, float4 &v, float2 &o) {
+            if (p < T) {
+                const int e = strm[w][p];
+                v = pos[rb0[w][e >> 5] + (e & 31)];
+                o = rsh[w][e >> 5];
+            } else {
+                v = make_float4(0.f, 0.f, 0.f, 0.f);
+                o = make_float2(1.f, 1.f);
+            }
+        };
+        float4 cA = make_float4(0.f, 0.f, 0.f, 0.f), cB = cA;
+        float2 oA = make_float2(1.f, 1.f), oB = oA;
+        if (T > 0) {
+            get(lane, cA, oA);
+            get(32 + lane, cB, oB);
         }
-    };
-    float4 cA = make_float4(0.f, 0.f, 0.f, 0.f), cB = cA;
-    float2 oA = make_float2(1.f, 1.f), oB = oA;
-    if (T > 0) {
-        get(lane, cA, oA);
-        get(32 + lane, cB, oB);
-    }
-    for (int c0 = 0; c0 < T; c0 += 64) {
-        float4 nA = make_float4(0.f, 0.f, 0.f, 0.f), nB = nA;
-        float2 pA = make_float2(1.f, 1.f), pB = pA;
-        if (c0 + 64 < T) {
-            get(c0 + 64 + lane, nA, pA);
-            get(c0 + 96 + lane, nB, pB);
+        for (int c0 = 0; c0 < T; c0 += 64) {
+            float4 nA = make_float4(0.f, 0.f, 0.f, 0.f), nB = nA;
+            float2 pA = make_float2(1.f, 1.f), pB = pA;
+            if (c0 + 64 < T) {
+                get(c0 + 64 + lane, nA, pA);
+                get(c0 + 96 + lane, nB, pB);
+            }
+            // com_a - x_j = (com_a - com_s) - (x_j - com_s)
+            const f2v dx = f2sub(f2pair(oA.x, oB.x), f2pair(cA.x, cB.x));
+            const f2v dy = f2sub(f2pair(oA.y, oB.y), f2pair(cA.y, cB.y));
+            const f2v ir = rsqrt_x2(f2fma(dx, dx, f2fma(dy, dy, E2)));
+            f2v cf[NC];
+            taylor_1r_x2<P>(dx, dy, ir, f2mul(ir, ir), cf);
+            const f2v mm = f2pair(cA.z, cB.z);
+#pragma unroll
+            for (int q = 0; q < NC; q++) acc[q] = f2fma(mm, cf[q], acc[q]);
+            cA = nA;
+            cB = nB;
+            oA = pA;
+            oB = pB;
         }
-        // com_a - x_j = (com_a - com_s) - (x_j - com_s)
-        const f2v dx = f2sub(f2pair(oA.x, oB.x), f2pair(cA.x, cB.x));
-        const f2v dy = f2sub(f2pair(oA.y, oB.y), f2pair(cA.y, cB.y));
-        const f2v ir = rsqrt_x2(f2fma(dx, dx, f2fma(dy, dy, E2)));
-        f2v cf[NC];
-        taylor_1r_x2<P>(dx, dy, ir, f2mul(ir, ir), cf);
-        const f2v mm = f2pair(cA.z, cB.z);
+        float sum[NC];
 #pragma unroll
-        for (int q = 0; q < NC; q++) acc[q] = f2fma(mm, cf[q], acc[q]);
-        cA = nA;
-        cB = nB;
-        oA = pA;
-        oB = pB;
+        for (int q = 0; q < NC; q++) {
+            float lo, hi;
+            upk2(acc[q].v, lo, hi);
+            sum[q] = lo + hi;
+        }
+        warp_coeffs<NC>(sum, [&](int q, float v) { ppart[u * NS + q] = v; });
     }
-    float sum[NC];
-#pragma unroll
-    for (int q = 0; q < NC; q++) {
-        float lo, hi;
-        upk2(acc[q].v, lo, hi);
-        sum[q] = lo + hi;
-    }
-    warp_coeffs<NC>(sum, [&](int q, float v) { ppart[u * NS + q] = v; });
 }
 
 // P2L units: one warp per unit (a target leaf and at most GX_P2L_UNIT of its P2L source
@@ -2348,7 +2371,8 @@ __global__ void __launch_bounds__(32 * WPB) k_p2l_stream(int64_t n_units, const 
                                                     const double *__restrict__ Y, const double *__restrict__ Mb,
                                                     const double *__restrict__ comx, const double *__restrict__ comy,
                                                     const int32_t *__restrict__ bs, const int32_t *__restrict__ be, T eps2,
-                                                    const uint32_t *__restrict__ p2p_mask, T *__restrict__ ppart) {
+                                                    const uint32_t *__restrict__ p2p_mask, T *__restrict__ ppart,
+                                                    unsigned *queue) {
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<T>(NC);
     constexpr int ROWS = GX_BODY_UNIT > GX_P2L_UNIT ? GX_BODY_UNIT : GX_P2L_UNIT;
@@ -2361,73 +2385,74 @@ __global__ void __launch_bounds__(32 * WPB) k_p2l_stream(int64_t n_units, const 
     __shared__ uint16_t strm[WPB][ROWS * 32];
     const unsigned full = 0xffffffffu;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (u >= n_units) return;
-    const int32_t a = uleaf[u];
-    const int raw = ulen[u], nq = raw < 0 ? -raw : raw;  // a body-level unit's length is stored negated
-    const double tcx = comx[a], tcy = comy[a];
-    int total = 0;
+    for (ItemQueue items(queue, n_units); items.more(); items.next()) {
+        const int64_t u = items.it;
+        const int32_t a = uleaf[u];
+        const int raw = ulen[u], nq = raw < 0 ? -raw : raw;  // a body-level unit's length is stored negated
+        const double tcx = comx[a], tcy = comy[a];
+        int total = 0;
 #pragma unroll
-    for (int h = 0; h < RPL; h++) {
-        uint32_t take = 0u;
-        const int r = 32 * h + lane;
-        if (r < nq) {
-            const int64_t q = ustart[u] + r;
-            const int32_t sl = src_idx[q];
-            const int nb = be[sl] - bs[sl];
-            take = raw < 0 ? p2p_mask[q] : (nb >= 32 ? full : (1u << nb) - 1u);
-            rb0[w][r] = bs[sl];
-            if constexpr (sizeof(T) == 4)
-                rsh[w][r] = make_float2((float)(tcx - comx[sl]), (float)(tcy - comy[sl]));
-        }
-        const int c = __popc(take);
-        int incl = c;
+        for (int h = 0; h < RPL; h++) {
+            uint32_t take = 0u;
+            const int r = 32 * h + lane;
+            if (r < nq) {
+                const int64_t q = ustart[u] + r;
+                const int32_t sl = src_idx[q];
+                const int nb = be[sl] - bs[sl];
+                take = raw < 0 ? p2p_mask[q] : (nb >= 32 ? full : (1u << nb) - 1u);
+                rb0[w][r] = bs[sl];
+                if constexpr (sizeof(T) == 4)
+                    rsh[w][r] = make_float2((float)(tcx - comx[sl]), (float)(tcy - comy[sl]));
+            }
+            const int c = __popc(take);
+            int incl = c;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(full, incl, o);
-            if (lane >= o) incl += v;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(full, incl, o);
+                if (lane >= o) incl += v;
+            }
+            int at = total + incl - c;
+            total += __shfl_sync(full, incl, 31);
+            while (take) {
+                const int j = __ffs(take) - 1;
+                take &= take - 1u;
+                strm[w][at++] = (uint16_t)((r << 5) | j);
+            }
         }
-        int at = total + incl - c;
-        total += __shfl_sync(full, incl, 31);
-        while (take) {
-            const int j = __ffs(take) - 1;
-            take &= take - 1u;
-            strm[w][at++] = (uint16_t)((r << 5) | j);
+        __syncwarp();
+        T acc[NC];
+#pragma unroll
+        for (int k = 0; k < NCr; k++) acc[k] = T(0);
+        // com_a - x_j and m_j of stream entry p (past the end: a unit offset and no mass)
+        const auto get = [&](int p, T &dx, T &dy, T &m) {
+            dx = dy = T(1);
+            m = T(0);
+            if (p >= total) return;
+            const int e = strm[w][p], j = rb0[w][e >> 5] + (e & 31);
+            if constexpr (sizeof(T) == 4) {
+                const float4 v = pos[j];
+                const float2 o = rsh[w][e >> 5];
+                dx = o.x - v.x;
+                dy = o.y - v.y;
+                m = v.z;
+            } else {
+                dx = tcx - X[j];
+                dy = tcy - Y[j];
+                m = Mb[j];
+            }
+        };
+        T dx, dy, m;
+        get(lane, dx, dy, m);
+        for (int p = 0; p < total; p += 32) {
+            T nx, ny, nm;
+            get(p + 32 + lane, nx, ny, nm);
+            p2l_body<P, T>(dx, dy, m, eps2, acc);
+            dx = nx;
+            dy = ny;
+            m = nm;
         }
+        warp_coeffs<NC>(acc, [&](int k, T v) { ppart[u * NS + k] = v; });
     }
-    __syncwarp();
-    T acc[NC];
-#pragma unroll
-    for (int k = 0; k < NCr; k++) acc[k] = T(0);
-    // com_a - x_j and m_j of stream entry p (past the end: a unit offset and no mass)
-    const auto get = [&](int p, T &dx, T &dy, T &m) {
-        dx = dy = T(1);
-        m = T(0);
-        if (p >= total) return;
-        const int e = strm[w][p], j = rb0[w][e >> 5] + (e & 31);
-        if constexpr (sizeof(T) == 4) {
-            const float4 v = pos[j];
-            const float2 o = rsh[w][e >> 5];
-            dx = o.x - v.x;
-            dy = o.y - v.y;
-            m = v.z;
-        } else {
-            dx = tcx - X[j];
-            dy = tcy - Y[j];
-            m = Mb[j];
-        }
-    };
-    T dx, dy, m;
-    get(lane, dx, dy, m);
-    for (int p = 0; p < total; p += 32) {
-        T nx, ny, nm;
-        get(p + 32 + lane, nx, ny, nm);
-        p2l_body<P, T>(dx, dy, m, eps2, acc);
-        dx = nx;
-        dy = ny;
-        m = nm;
-    }
-    warp_coeffs<NC>(acc, [&](int k, T v) { ppart[u * NS + k] = v; });
 }
 
 // P2L units over larger leaves (no body-level units there): a row at a time.
@@ -2439,85 +2464,86 @@ __global__ void __launch_bounds__(32 * WPB) k_p2l(int64_t n_units, const int32_t
                                              const double *__restrict__ Y, const double *__restrict__ Mb,
                                              const double *__restrict__ comx, const double *__restrict__ comy,
                                              const int32_t *__restrict__ bs, const int32_t *__restrict__ be, T eps2,
-                                             T *__restrict__ ppart) {
+                                             T *__restrict__ ppart, unsigned *queue) {
     constexpr int NC = nc2(P);
     constexpr int NS = row_stride<T>(NC);
     const int PP = gx_rt_order(P);
     const int NCr = (PP + 1) * (PP + 2) / 2;
     (void)NCr;
     const int lane = threadIdx.x & 31;
-    const int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (u >= n_units) return;
-    const int32_t a = uleaf[u];
-    const int nq = ulen[u];
-    const double tcx = comx[a], tcy = comy[a];
-    T acc[NC];
+    for (ItemQueue items(queue, n_units); items.more(); items.next()) {
+        const int64_t u = items.it;
+        const int32_t a = uleaf[u];
+        const int nq = ulen[u];
+        const double tcx = comx[a], tcy = comy[a];
+        T acc[NC];
 #pragma unroll
-    for (int k = 0; k < NCr; k++) acc[k] = T(0);
-    // the unit's rows 32 at a time
-    for (int g0 = 0; g0 < nq; g0 += 32) {
-        const int ng = min(32, nq - g0);
-        int32_t sb = 0, se = 0;
-        T shx = T(0), shy = T(0);
-        double scx = 0.0, scy = 0.0;
-        if (lane < ng) {
-            const int64_t q = ustart[u] + g0 + lane;
-            const int32_t sl = src_idx[q];
-            sb = bs[sl];
-            se = be[sl];
-            scx = comx[sl];
-            scy = comy[sl];
-            shx = (T)(tcx - scx);
-            shy = (T)(tcy - scy);
-        }
-        // one body of source k per lane (the first 32 of the leaf): relative position, mass
-        auto fetch = [&](int k, T &px, T &py, T &pm) {
-            const int32_t j = __shfl_sync(0xffffffffu, sb, k) + lane, j1 = __shfl_sync(0xffffffffu, se, k);
-            if constexpr (sizeof(T) == 4) {
-                const float4 v = j < j1 ? pos[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-                px = v.x;
-                py = v.y;
-                pm = v.z;
-            } else {
-                const double cx = __shfl_sync(0xffffffffu, scx, k), cy = __shfl_sync(0xffffffffu, scy, k);
-                px = j < j1 ? X[j] - cx : 0.0;
-                py = j < j1 ? Y[j] - cy : 0.0;
-                pm = j < j1 ? Mb[j] : 0.0;
+        for (int k = 0; k < NCr; k++) acc[k] = T(0);
+        // the unit's rows 32 at a time
+        for (int g0 = 0; g0 < nq; g0 += 32) {
+            const int ng = min(32, nq - g0);
+            int32_t sb = 0, se = 0;
+            T shx = T(0), shy = T(0);
+            double scx = 0.0, scy = 0.0;
+            if (lane < ng) {
+                const int64_t q = ustart[u] + g0 + lane;
+                const int32_t sl = src_idx[q];
+                sb = bs[sl];
+                se = be[sl];
+                scx = comx[sl];
+                scy = comy[sl];
+                shx = (T)(tcx - scx);
+                shy = (T)(tcy - scy);
             }
-        };
-        T cx_ = T(0), cy_ = T(0), cm = T(0);
-        fetch(0, cx_, cy_, cm);
-        for (int k = 0; k < ng; k++) {
-            T nx = T(0), ny = T(0), nm = T(0);
-            if (k + 1 < ng) fetch(k + 1, nx, ny, nm);
-            const T ox = __shfl_sync(0xffffffffu, shx, k), oy = __shfl_sync(0xffffffffu, shy, k);
-            const int32_t j0 = __shfl_sync(0xffffffffu, sb, k), j1 = __shfl_sync(0xffffffffu, se, k);
-            const double ckx = __shfl_sync(0xffffffffu, scx, k), cky = __shfl_sync(0xffffffffu, scy, k);
-            (void)ckx;
-            (void)cky;
-            // com_a - x_j = (com_a - com_s) - (x_j - com_s)
-            if (j0 + lane < j1) p2l_body<P, T>(ox - cx_, oy - cy_, cm, eps2, acc);
-            // the rest of the source's bodies
-            for (int32_t j = j0 + 32 + lane; j < j1; j += 32) {
-                T px, py, pm;
+            // one body of source k per lane (the first 32 of the leaf): relative position, mass
+            auto fetch = [&](int k, T &px, T &py, T &pm) {
+                const int32_t j = __shfl_sync(0xffffffffu, sb, k) + lane, j1 = __shfl_sync(0xffffffffu, se, k);
                 if constexpr (sizeof(T) == 4) {
-                    const float4 v = pos[j];
+                    const float4 v = j < j1 ? pos[j] : make_float4(0.f, 0.f, 0.f, 0.f);
                     px = v.x;
                     py = v.y;
                     pm = v.z;
                 } else {
-                    px = X[j] - ckx;
-                    py = Y[j] - cky;
-                    pm = Mb[j];
+                    const double cx = __shfl_sync(0xffffffffu, scx, k), cy = __shfl_sync(0xffffffffu, scy, k);
+                    px = j < j1 ? X[j] - cx : 0.0;
+                    py = j < j1 ? Y[j] - cy : 0.0;
+                    pm = j < j1 ? Mb[j] : 0.0;
                 }
-                p2l_body<P, T>(ox - px, oy - py, pm, eps2, acc);
+            };
+            T cx_ = T(0), cy_ = T(0), cm = T(0);
+            fetch(0, cx_, cy_, cm);
+            for (int k = 0; k < ng; k++) {
+                T nx = T(0), ny = T(0), nm = T(0);
+                if (k + 1 < ng) fetch(k + 1, nx, ny, nm);
+                const T ox = __shfl_sync(0xffffffffu, shx, k), oy = __shfl_sync(0xffffffffu, shy, k);
+                const int32_t j0 = __shfl_sync(0xffffffffu, sb, k), j1 = __shfl_sync(0xffffffffu, se, k);
+                const double ckx = __shfl_sync(0xffffffffu, scx, k), cky = __shfl_sync(0xffffffffu, scy, k);
+                (void)ckx;
+                (void)cky;
+                // com_a - x_j = (com_a - com_s) - (x_j - com_s)
+                if (j0 + lane < j1) p2l_body<P, T>(ox - cx_, oy - cy_, cm, eps2, acc);
+                // the rest of the source's bodies
+                for (int32_t j = j0 + 32 + lane; j < j1; j += 32) {
+                    T px, py, pm;
+                    if constexpr (sizeof(T) == 4) {
+                        const float4 v = pos[j];
+                        px = v.x;
+                        py = v.y;
+                        pm = v.z;
+                    } else {
+                        px = X[j] - ckx;
+                        py = Y[j] - cky;
+                        pm = Mb[j];
+                    }
+                    p2l_body<P, T>(ox - px, oy - py, pm, eps2, acc);
+                }
+                cx_ = nx;
+                cy_ = ny;
+                cm = nm;
             }
-            cx_ = nx;
-            cy_ = ny;
-            cm = nm;
         }
+        warp_coeffs<NC>(acc, [&](int k, T v) { ppart[u * NS + k] = v; });
     }
-    warp_coeffs<NC>(acc, [&](int k, T v) { ppart[u * NS + k] = v; });
 }
 
 // Folding of long item ranges.  A wide halo leaf can have ~1000 P2P items (977 at 1M
@@ -2736,7 +2762,7 @@ int run_forces(gx_ctx *ctx, bool timed) {
     const gx_ctx::Items &I = mode == GX_MODE_ACCURATE ? ctx->items_acc : ctx->items_ref;
     const int tchunks = (int)std::max<int64_t>(1, (ctx->max_leaf + 31) / 32);
     const int32_t *src_idx = mode == GX_MODE_ACCURATE ? dptr<int32_t>(ctx->near_idx) : dptr<int32_t>(ctx->p2p_idx);
-    const unsigned gi = gx_blocks(I.n, WPB);  // warp per item
+    const unsigned gq = gx_item_grid(ctx, I.n);
     const bool split = mode == GX_MODE_ACCURATE && ctx->theta_w > 0.0;  // near-list split: M2P items, P2L units
     // body-level P2L of the P2P rows: masks in the plan, body-level P2L units
     const bool body = split && ctx->plan_body_split && gx_body_split_on(ctx);
@@ -2778,21 +2804,25 @@ int run_forces(gx_ctx *ctx, bool timed) {
             // two targets per lane pays when leaves fill most of a row; with leaves of at
             // most 16 bodies (n_max <= 16) the second target would be empty
             if (mixed && body)
-                k_p2p32_stream<<<gi, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
+                k_p2p32_stream<<<gq, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
                                                              dptr<int32_t>(I.nq), pos, comx, comy, bs, be, src_idx,
-                                                             p2p_mask, (float)eps2, dptr<float2>(ctx->part));
+                                                             p2p_mask, (float)eps2, dptr<float2>(ctx->part),
+                                                             gx_queue(ctx, GX_Q_P2P));
             else if (mixed && tchunks == 1 && ctx->max_leaf <= 16)
-                k_p2p32_rows1<<<gi, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
+                k_p2p32_rows1<<<gq, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
                                                             dptr<int32_t>(I.nq), pos, comx, comy, bs, be, src_idx,
-                                                            (float)eps2, dptr<float2>(ctx->part));
+                                                            (float)eps2, dptr<float2>(ctx->part),
+                                                            gx_queue(ctx, GX_Q_P2P));
             else if (mixed && tchunks == 1)
-                k_p2p32_rows<<<gi, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
+                k_p2p32_rows<<<gq, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
                                                            dptr<int32_t>(I.nq), pos, comx, comy, bs, be, src_idx,
-                                                           (float)eps2, dptr<float2>(ctx->part));
+                                                           (float)eps2, dptr<float2>(ctx->part),
+                                                           gx_queue(ctx, GX_Q_P2P));
             else if (mixed)
-                k_p2p32_items<<<gi, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
+                k_p2p32_items<<<gq, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
                                                             dptr<int32_t>(I.nq), pos, comx, comy, bs, be, src_idx,
-                                                            (float)eps2, tchunks, dptr<float2>(ctx->part));
+                                                            (float)eps2, tchunks, dptr<float2>(ctx->part),
+                                                            gx_queue(ctx, GX_Q_P2P));
             else
                 k_p2p64_items<<<(unsigned)I.n, 128, 0, ctx->stream2>>>(dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
                                                                        dptr<int32_t>(I.nq), X, Y, Mb, bs, be, src_idx,
@@ -2801,7 +2831,7 @@ int run_forces(gx_ctx *ctx, bool timed) {
         }
         if (timed) GX_CUDA(ctx, cudaEventRecord(ctx->ev[15], ctx->stream2));  // the P2P kernel alone
         if (split && ctx->n_m2p_items > 0) {
-            const unsigned gm = gx_blocks(ctx->n_m2p_items, WPB);  // warp per M2P item
+            const unsigned gm = gx_item_grid(ctx, ctx->n_m2p_items);
             // M2P items of the near-list split: their own slots of the same partial array
             if constexpr (P <= 5) {
                 if (mixed && tchunks == 1) {
@@ -2809,7 +2839,7 @@ int run_forces(gx_ctx *ctx, bool timed) {
                                                               dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
                                                               dptr<int32_t>(I.nq), pos, comx, comy, bs, be, src_idx,
                                                               (float)eps2, reinterpret_cast<const float *>(M),
-                                                              dptr<float2>(ctx->part));
+                                                              dptr<float2>(ctx->part), gx_queue(ctx, GX_Q_M2P));
                     goto m2p_done;
                 }
             }
@@ -2817,11 +2847,12 @@ int run_forces(gx_ctx *ctx, bool timed) {
                 k_m2p<P, float, float2><<<gm, 32 * WPB, 0, ctx->stream2>>>(
                     ctx->n_m2p_items, dptr<int32_t>(ctx->m2p_list), dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb), dptr<int32_t>(I.nq), pos, nullptr, nullptr, comx,
                     comy, bs, be, src_idx, (float)eps2, reinterpret_cast<const float *>(M), tchunks,
-                    dptr<float2>(ctx->part));
+                    dptr<float2>(ctx->part), gx_queue(ctx, GX_Q_M2P));
             else
                 k_m2p<P, double, double2><<<gm, 32 * WPB, 0, ctx->stream2>>>(
                     ctx->n_m2p_items, dptr<int32_t>(ctx->m2p_list), dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb), dptr<int32_t>(I.nq), nullptr, X, Y, comx, comy, bs,
-                    be, src_idx, eps2, reinterpret_cast<const double *>(M), tchunks, dptr<double2>(ctx->part));
+                    be, src_idx, eps2, reinterpret_cast<const double *>(M), tchunks, dptr<double2>(ctx->part),
+                    gx_queue(ctx, GX_Q_M2P));
         m2p_done:
             ctx->launches++;
         }
@@ -2845,27 +2876,27 @@ int run_forces(gx_ctx *ctx, bool timed) {
         auto p2l_field = [&](cudaStream_t sp) -> int {
             if constexpr (P <= 5 && sizeof(T) == 4) {
                 if (PU.n_leafu > 0) {
-                    k_p2l_x2<P><<<gx_blocks(PU.n_leafu, WPB), 32 * WPB, 0, sp>>>(
+                    k_p2l_x2<P><<<gx_item_grid(ctx, PU.n_leafu), 32 * WPB, 0, sp>>>(
                         PU.n_leafu, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start), dptr<int32_t>(PU.len), src_idx,
-                        pos, comx, comy, bs, be, (float)eps2, dptr<float>(ctx->p2l_part));
+                        pos, comx, comy, bs, be, (float)eps2, dptr<float>(ctx->p2l_part), gx_queue(ctx, GX_Q_P2L));
                     ctx->launches++;
                 }
                 if (body && PU.n_body > 0) {
-                    k_p2l_body_x2<P><<<gx_blocks(PU.n_body, WPB), 32 * WPB, 0, sp>>>(
+                    k_p2l_body_x2<P><<<gx_item_grid(ctx, PU.n_body), 32 * WPB, 0, sp>>>(
                         PU.n_leafu, PU.n_body, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start),
                         dptr<int32_t>(PU.len), src_idx, p2p_mask, pos, comx, comy, bs, (float)eps2,
-                        dptr<float>(ctx->p2l_part));
+                        dptr<float>(ctx->p2l_part), gx_queue(ctx, GX_Q_P2L));
                     ctx->launches++;
                 }
             } else if (ctx->max_leaf <= 32) {
-                k_p2l_stream<P, T><<<gx_blocks(PU.n, WPB), 32 * WPB, 0, sp>>>(
+                k_p2l_stream<P, T><<<gx_item_grid(ctx, PU.n), 32 * WPB, 0, sp>>>(
                     PU.n, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start), dptr<int32_t>(PU.len), src_idx, pos, X, Y,
-                    Mb, comx, comy, bs, be, (T)eps2, p2p_mask, dptr<T>(ctx->p2l_part));
+                    Mb, comx, comy, bs, be, (T)eps2, p2p_mask, dptr<T>(ctx->p2l_part), gx_queue(ctx, GX_Q_P2L));
                 ctx->launches++;
             } else {
-                k_p2l<P, T><<<gx_blocks(PU.n, WPB), 32 * WPB, 0, sp>>>(
+                k_p2l<P, T><<<gx_item_grid(ctx, PU.n), 32 * WPB, 0, sp>>>(
                     PU.n, dptr<int32_t>(PU.leaf), dptr<int64_t>(PU.start), dptr<int32_t>(PU.len), src_idx, pos, X, Y,
-                    Mb, comx, comy, bs, be, (T)eps2, dptr<T>(ctx->p2l_part));
+                    Mb, comx, comy, bs, be, (T)eps2, dptr<T>(ctx->p2l_part), gx_queue(ctx, GX_Q_P2L));
                 ctx->launches++;
             }
             return GX_OK;
@@ -2907,10 +2938,10 @@ int run_forces(gx_ctx *ctx, bool timed) {
             GX_TRY(gx_ensure(ctx, ctx->m2l_part, sizeof(T) * NS * (size_t)(U.n + 1)));
             if (U.n > 0) {
                 const int64_t *node_u = dptr<int64_t>(U.node_u);
-                k_m2l_units<P, T><<<gx_blocks(U.n, WPB), 32 * WPB, 0, st>>>(
+                k_m2l_units<P, T><<<gx_item_grid(ctx, U.n), 32 * WPB, 0, st>>>(
                     U.n, dptr<int32_t>(U.node), dptr<int64_t>(U.start), dptr<int32_t>(U.len), node_u,
                     dptr<int32_t>(ctx->far_idx), comx, comy, mixed ? dptr<float4>(ctx->comhl) : nullptr, eps2, M, L,
-                    dptr<T>(ctx->m2l_part), dptr<unsigned>(ctx->m2l_count));
+                    dptr<T>(ctx->m2l_part), dptr<unsigned>(ctx->m2l_count), gx_queue(ctx, GX_Q_M2L));
             }
         } else {
             k_m2l_exact<P, T, uint32_t><<<gn, 128, 0, st>>>(nn, dptr<uint32_t>(ctx->vdata), nullptr, nullptr,

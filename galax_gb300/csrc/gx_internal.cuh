@@ -152,6 +152,7 @@ struct gx_ctx {
         DevBuf node, start, len, node_u;  // int32, int64, int32, int64[n_nodes+1]
         int64_t n = 0;
     } m2l_units;
+    DevBuf queues;     // GX_QUEUES counters of the item kernels' queues, 128 bytes apart, 0 between launches
     DevBuf m2l_part;   // per-unit partial locals of nodes cut into several units
     DevBuf m2l_count;  // uint32 per node: its units that have finished (zero between evaluations)
     // ACCURATE near-list split (theta_w > 0): every leaf's near list is partitioned in
@@ -261,6 +262,18 @@ int gx_forces_device(gx_ctx *ctx, bool timed);
 // gx_api.cu: device rebuild with the last build's parameters (permutes the resident
 // bodies and ids; invalidates the plans), plan check, ids reset
 int gx_rebuild_internal(gx_ctx *ctx);
+// The queues of the kernels whose one-warp blocks take their items in turn (one launch of a
+// kind runs at a time), and their grids: 24 blocks an SM from 16 items a block on, else a
+// block an item.  Evaluations with 24 / a block an item: Plummer 1M 1.91 / 1.985 ms (16: 1.96,
+// 64: 1.90), disk 4M, p = 6 14.8 / 15.8 (15.5, 15.0), but uniform 50,000, with two items a
+// block, 0.131 / 0.117: the far field's small launches wait for places then and the blocks
+// finish unevenly.
+enum { GX_Q_P2P, GX_Q_M2P, GX_Q_P2L, GX_Q_M2L, GX_QUEUES };
+inline unsigned *gx_queue(gx_ctx *ctx, int which) { return static_cast<unsigned *>(ctx->queues.p) + 32 * which; }
+inline unsigned gx_item_grid(const gx_ctx *ctx, int64_t n) {
+    const int64_t grid = (ctx->sm_count > 0 ? ctx->sm_count : 152) * (int64_t)24;
+    return (unsigned)(n < 16 * grid ? n : grid);
+}
 int gx_ensure_plan_public(gx_ctx *ctx);
 int gx_ids_reset(gx_ctx *ctx);
 int gx_poly_table_host(int p, double eps, std::vector<double> &out);
