@@ -7,12 +7,14 @@
 //
 //   P2M   (lib.rs:848-887)   warp per leaf, lane per body, warp-shuffle reduction
 //   M2M   (lib.rs:890-938)   four lanes per parent, one child each; small levels in one launch
-//   M2L   (lib.rs:1199-1259) warp per target node, lane per list entry, warp reduction
+//   M2L   (lib.rs:1199-1259) REF: warp per target node, lane per output coefficient; other
+//                            modes: warp per unit of a far list, lane per source
 //   L2L   (lib.rs:1262-1302) REF: node-id-ascending order means every leaf receives
 //                            its own M2L local plus one shift of its parent's M2L local;
-//                            other modes: top-down per level
-//   L2P   (lib.rs:1308-1355) + P2P (lib.rs:1395-1462) fused: warp per target leaf,
-//                            lane per body, source leaves staged in shared memory
+//                            other modes: every ancestor's straight to the leaf
+//   L2P   (lib.rs:1308-1355) with L2L in the mixed form, else with the final sum
+//   P2P   (lib.rs:1395-1462) items of a target leaf and up to 32 source leaves, staged in
+//                            shared memory; partial sums added in order
 //
 // M2L contraction.  With M'[S] = (-1)^|S| M[S] and the kernel derivatives G, the
 // reference's plan (lib.rs:1160-1196) is L[T] = (1/T!) sum_S M'[S] G[S+T]; the 1/T!

@@ -154,8 +154,9 @@ int gx_plan_info(gx_ctx *ctx, int64_t *n_far_pairs, int64_t *n_near_pairs, int64
  * x, y, m (tree order), runs the six passes, writes ax, ay.  Inputs are sanitised
  * on the device like compute_fmm_force (lib.rs:1474-1482).  Page-locked ax, ay
  * (gx_host_alloc, cudaHostAlloc, cudaHostRegister) are written by the device
- * directly, and page-locked x, y, m read directly once the plan exists; other
- * memory is copied before and after the evaluation. */
+ * directly, and page-locked x, y, m read directly once the plan exists.  On a host
+ * whose page tables the GPU shares, kernels read and write ordinary arrays of up to
+ * 128 pages (8 MB) too; other memory is copied before and after the evaluation. */
 int gx_compute_forces(gx_ctx *ctx, const double *x, const double *y, const double *m, double *ax, double *ay);
 
 /* Device-resident state (no per-step host traffic). */
@@ -237,9 +238,11 @@ int gx_rollout_backward(gx_ctx *ctx, const double *lx, const double *ly, const d
                         double *gx0, double *gy0, double *gvx0, double *gvy0, double *gm, int64_t *peak_bytes);
 
 /* Device time of the last force evaluation per pass, in ms:
- * {total, prepare, p2m, m2m, m2l, l2l, l2p+p2p}; returns 7 entries.  The near field
- * (P2P) runs on a second, lower-priority stream beside m2m..l2l, so those passes
- * include the slots it takes, and the last entry is the wait for it plus L2P. */
+ * {total, prepare, p2m, m2m, m2l, l2l, l2p+p2p}; returns 7 entries.  Sanitising is
+ * part of p2m where the leaves cover the bodies.  The near field (P2P, M2P) and P2L run
+ * on a second and a third, lower-priority stream beside m2m..m2l, so those passes
+ * include the slots they take; l2l includes the wait for P2L and, mixed, L2P, and the
+ * last entry is the wait for the near field plus the final sum. */
 int gx_last_timings(gx_ctx *ctx, double out[7]);
 /* Number of kernels the last force evaluation launched. */
 int gx_last_launch_count(gx_ctx *ctx, int64_t *count);
