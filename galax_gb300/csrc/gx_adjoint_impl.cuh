@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(128) k_adj_l2p(int64_t nl, const double *__res
 // partials in unit order.  Nodes without far entries are not written: has_far = 0 keeps A4
 // from reading them.
 template <int P, class T>
-__global__ void __launch_bounds__(32 * WPB, (sizeof(T) == 4 && P <= 4) ? 32 / WPB : 1)
+__global__ void __launch_bounds__(32 * WPB, m2l_warps<P, T>() / WPB)
     k_adj_m2l(int64_t n_units, const int32_t *__restrict__ unode, const int64_t *__restrict__ ustart,
               const int32_t *__restrict__ ulen, const int64_t *__restrict__ node_u, const int32_t *__restrict__ idx,
               const double *__restrict__ comx, const double *__restrict__ comy, const float4 *__restrict__ comhl,

@@ -927,12 +927,21 @@ __device__ __forceinline__ void last_unit_sums(int64_t node, int64_t u0, int64_t
     if (lane == 0) count[node] = 0;
 }
 
+// Warps an SM keeps of a kernel around m2l_fused: what its registers allow with few spills or
+// none (64, 80 and 128 of them).  Left alone at p = 5 and 6 in FP32 ptxas takes 151 and 225, for
+// 12 and 8 warps: evaluations of Plummer 1M 2.53 -> 2.40 and 3.41 -> 3.24 ms, disk 4M 12.8 ->
+// 12.5 and 14.7 -> 14.3.  FP64 is bound by its pipe at any number.
+template <int P, class T>
+constexpr int m2l_warps() {
+    return sizeof(T) == 8 || P > 6 ? WPB : P <= 4 ? 32 : P == 5 ? 24 : 16;
+}
+
 // ACCURATE M2L over work units: every far list is cut into units of at most
 // GX_M2L_UNIT sources (one warp each), so a node near the centre of a wide halo, with
 // tens of thousands of far sources, is spread over many warps instead of running as
 // one straggler.  A node with one unit writes its local directly, the others as above.
 template <int P, class T>
-__global__ void __launch_bounds__(32 * WPB, (sizeof(T) == 4 && P <= 4) ? 32 / WPB : 1) k_m2l_units(
+__global__ void __launch_bounds__(32 * WPB, m2l_warps<P, T>() / WPB) k_m2l_units(
     int64_t n_units, const int32_t *__restrict__ unode, const int64_t *__restrict__ ustart,
     const int32_t *__restrict__ ulen, const int64_t *__restrict__ node_u, const int32_t *__restrict__ idx,
     const double *__restrict__ comx, const double *__restrict__ comy, const float4 *__restrict__ comhl, double eps2d,
