@@ -133,9 +133,10 @@ constexpr size_t GX_DIRECT_PAGES = 128;  // of an array; above, touching them co
 // The device address of a host array of bytes bytes, or null where it takes a copy: page-locked
 // memory (cudaHostAlloc or cudaHostRegister: its first and its last byte must resolve to the
 // same allocation, as a registered range shorter than the array would let a kernel run past
-// it), or few pages of ordinary memory on a host as above.
+// it), or few pages of ordinary memory on a host as above.  Kernels load and store the arrays'
+// 8-byte elements whole, so their address has to be a multiple of 8; a copy takes any.
 static void *direct_host(const gx_ctx *ctx, const void *p, size_t bytes, bool write) {
-    if (!p || bytes == 0) return nullptr;
+    if (!p || bytes == 0 || reinterpret_cast<uintptr_t>(p) % 8 != 0) return nullptr;
     const char *first = static_cast<const char *>(p), *last = first + bytes - 1;
     cudaPointerAttributes at{}, at_last{};
     if (cudaPointerGetAttributes(&at, first) != cudaSuccess || cudaPointerGetAttributes(&at_last, last) != cudaSuccess) {
