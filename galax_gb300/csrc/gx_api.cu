@@ -456,10 +456,14 @@ int gx_upload_bodies(gx_ctx *ctx, int64_t n, const double *x, const double *y, c
     GX_TRY(check_ctx(ctx));
     if (!x || !y || !m) return gx_fail(ctx, GX_ERR_INVALID_ARG, "x, y and m are required");
     if (ctx->have_tree && n != ctx->n_bodies) return gx_fail(ctx, GX_ERR_INVALID_ARG, "n differs from the tree's body count");
-    GX_TRY(upload_bodies_impl(ctx, n, x, y, vx, vy, m, ax, ay));
-    ctx->n_bodies = n;
-    GX_TRY(gx_ids_reset(ctx));
-    GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    int rc = upload_bodies_impl(ctx, n, x, y, vx, vy, m, ax, ay);
+    if (rc == GX_OK) {
+        ctx->n_bodies = n;
+        rc = gx_ids_reset(ctx);
+    }
+    const cudaError_t e = cudaStreamSynchronize(ctx->stream);  // the caller's arrays have been read, whatever failed
+    GX_TRY(rc);
+    GX_CUDA(ctx, e);
     return GX_OK;
 }
 

@@ -71,3 +71,23 @@ c = count("fake_copies")
 ctx._check(G.lib().gx_body_ids(ctx._h, G._p(ids, G._I64)))
 assert count("fake_copies") == c + 1
 """)
+
+
+def test_a_failed_upload_has_read_its_arrays(run):
+    """An upload that fails behind its kernel (no memory for the ids) waits before it returns:
+    the caller may free the arrays then."""
+    run("""
+n = 1000
+ctx = G.GpuContext(G.GpuConfig(max_n=n))
+fail.value = 4 * n + 4 * n // 8                       # the ids, with gx_ensure's eighth
+w, c = count("fake_waits"), count("fake_copies")
+try:
+    ctx.upload_bodies(bodies(n))
+    raise SystemExit("the upload did not fail")
+except G.GpuError as e:
+    assert e.code == 3, e
+assert count("fake_copies") == c and count("fake_waits") == w + 1
+fail.value = 0
+ctx.upload_bodies(bodies(n))
+assert count("fake_waits") == w + 2
+""")
