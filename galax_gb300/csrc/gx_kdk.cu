@@ -116,9 +116,11 @@ __global__ void __launch_bounds__(RED_THREADS) k_n2_sampled(int64_t n, const dou
 #pragma unroll 2
     for (int64_t j = (int64_t)rank * blockDim.x + threadIdx.x; j < n; j += (int64_t)nb * blockDim.x) {
         const double mj = m[j], dx = x[j] - xi, dy = y[j] - yi;
-        const double f = j == i ? 0.0 : gx_mass_r3(fma(dx, dx, fma(dy, dy, eps2)), gx_mass_split(mj), mj);
-        fx = fma(f, dx, fx);
-        fy = fma(f, dy, fy);
+        const double f = gx_mass_r3(fma(dx, dx, fma(dy, dy, eps2)), gx_mass_split(mj), mj);
+        if (j != i) {  // the target itself adds nothing, not even where dx = x - x is NaN
+            fx = fma(f, dx, fx);
+            fy = fma(f, dy, fy);
+        }
     }
     const double tx = block_sum(fx, sh);
     const double ty = block_sum(fy, sh);
