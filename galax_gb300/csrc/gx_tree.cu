@@ -442,19 +442,33 @@ __global__ void __launch_bounds__(RC_THREADS) k_rounds_cluster(int64_t *st, int6
     const int per = (int)((c + nb * RC_THREADS - 1) / (nb * RC_THREADS));
     int i0 = (int)min(c, (int64_t)(rank * RC_THREADS + t) * per), n = (int)min(c, (int64_t)i0 + per) - i0;
     uint64_t dv = 0;
-    if (n > 0) {
-        uint64_t p = i0 > 0 ? keys[bs[s + i0 - 1]] : 0;
+    const auto load_d = [&](const auto &key) {
+        dv = 0;
+        uint64_t p = n > 0 && i0 > 0 ? key(s + i0 - 1) : 0;
         for (int k = 0; k < n; k++) {
-            const uint64_t g = keys[bs[s + i0 + k]], x = g ^ p;
+            const uint64_t g = key(s + i0 + k), x = g ^ p;
             const int d1 = i0 + k == 0 ? 255 : (x ? 64 - __clzll((long long)x) : 0);
             dv |= (uint64_t)d1 << (8 * k);
             p = g;
         }
-    }
+    };
+    load_d([&](int64_t q) { return keys[bs[q]]; });
     const auto mx = [](int a, int b) { return max(a, b); };
     const auto sm = [](int a, int b) { return a + b; };
     for (int par = 0; flags == 0; par ^= 1) {
-        const int sh = (int)min(shift, (int64_t)63);
+        // The reference's shift is taken modulo 64 (a tree of more than 4^11 leaves in an order
+        // without runs gets there): at 0 again, the d of the nodes' own first keys count, which
+        // are those of their first leaves.
+        const int sh = (int)(shift & 63);
+        if (sh == 0) {
+            cl.sync();  // the last round's child slots are written
+            const int64_t nl = level_start[1];
+            const auto key = [&](int64_t q) {
+                while (q >= nl) q = child[4 * q];
+                return keys[bs[q]];
+            };
+            load_d(key);
+        }
         // the last segment head before this thread's run
         int last = -1;
         for (int k = 0; k < n; k++)
