@@ -605,13 +605,24 @@ __host__ __device__ constexpr double ff_const(int k, int l) {
     return r;
 }
 
-template <int P, int N, class T>
+template <int P, int N, bool WIDE, class T>
 __device__ __forceinline__ void m2l_order(T X, T Y, T ir2, T *a, const T *in, T *out) {
     if constexpr (N <= 2 * P) {
         // c1x a_{k-1,l} + c1y a_{k,l-1} + c2 (a_{k-2,l} + a_{k,l-2}); with X = dx / R^2 and
-        // Y = dy / R^2 formed once, three multiplies an order (none at order 1)
-        constexpr double q1 = -(double)(2 * N - 1) / N, q2 = -(double)(N - 1) / N;
-        const T c1x = (T)q1 * X, c1y = (T)q1 * Y, c2 = (T)q2 * ir2;
+        // Y = dy / R^2 formed once, three multiplies an order (none at order 1).  WIDE: X = dx
+        // and Y = dy, multiplied by 1/R^2 order by order.
+        T c1x, c1y, c2;
+        if constexpr (WIDE) {
+            const T in_ = tab_inv<T>(N) * ir2, c1 = -(T)(2 * N - 1) * in_;
+            c1x = c1 * X;
+            c1y = c1 * Y;
+            c2 = -(T)(N - 1) * in_;
+        } else {
+            constexpr double q1 = -(double)(2 * N - 1) / N, q2 = -(double)(N - 1) / N;
+            c1x = (T)q1 * X;
+            c1y = (T)q1 * Y;
+            c2 = (T)q2 * ir2;
+        }
 #pragma unroll
         for (int k = 0; k <= N; k++) {
             const int l = N - k;
@@ -633,11 +644,11 @@ __device__ __forceinline__ void m2l_order(T X, T Y, T ir2, T *a, const T *in, T 
                     if (yi + yj <= P && xi + xj <= P) out[gx_mi(xi, xj)] += in[gx_mi(yi, yj)] * Av;
                 }
         }
-        m2l_order<P, N + 1, T>(X, Y, ir2, a, in, out);
+        m2l_order<P, N + 1, WIDE, T>(X, Y, ir2, a, in, out);
     }
 }
 
-template <int P, class T>
+template <int P, bool WIDE, class T>
 __device__ __forceinline__ void m2l_fused_core(T dx, T dy, T eps2, const T *in, T *out) {
     T r2 = dx * dx + dy * dy + eps2;
     T ir = rsqrt_t<T>(r2);
@@ -646,7 +657,8 @@ __device__ __forceinline__ void m2l_fused_core(T dx, T dy, T eps2, const T *in, 
     if constexpr (P <= 8) {
         T a[nc2(2 * P)];
         a[0] = ir;
-        m2l_order<P, 1, T>(dx * ir2, dy * ir2, ir2, a, in, out);
+        if constexpr (WIDE) m2l_order<P, 1, true, T>(dx, dy, ir2, a, in, out);
+        else m2l_order<P, 1, false, T>(dx * ir2, dy * ir2, ir2, a, in, out);
     } else {
         // high orders: run-time loop bounds keep the code size bounded
         const int PP = gx_rt_order(P);
@@ -681,7 +693,11 @@ __device__ __forceinline__ void m2l_fused_core(T dx, T dy, T eps2, const T *in, 
 // range for R ~ 0.1.  The 1/R kernel is homogeneous of degree -1 in (d, eps), so the
 // derivatives are formed at unit distance, d' = d/R, and the powers of 1/R go to the
 // operands:  out[X] += R^-(1+|X|) sum_Y (in[Y] R^-|Y|) A'[X+Y].
-template <int P, class T>
+// WIDE: for lists that no opening angle bounds (the reference's, whose pairs may be closer than
+// the nodes are wide, so that the terms grow with the order).  The rounding of X and Y is the
+// same at every order and adds up over them: there it made the mixed form's error 1.2 to 1.3
+// times as large at p = 4 to 8, while under an opening angle the fewer roundings win.
+template <int P, class T, bool WIDE = false>
 __device__ __forceinline__ void m2l_fused(T dx, T dy, T eps2, const T *in, T *out) {
     if constexpr (sizeof(T) == 4 && P >= 6) {
         constexpr int NC = nc2(P);
@@ -699,13 +715,13 @@ __device__ __forceinline__ void m2l_fused(T dx, T dy, T eps2, const T *in, T *ou
                 sin_[gx_mi(yi, yj)] = in[gx_mi(yi, yj)] * pw[yi + yj];
                 sout[gx_mi(yi, yj)] = T(0);
             }
-        m2l_fused_core<P, T>(dx * ir, dy * ir, eps2 * (ir * ir), sin_, sout);
+        m2l_fused_core<P, WIDE, T>(dx * ir, dy * ir, eps2 * (ir * ir), sin_, sout);
 #pragma unroll
         for (int xi = 0; xi <= PP; xi++)
 #pragma unroll
             for (int xj = 0; xj <= PP - xi; xj++) out[gx_mi(xi, xj)] += sout[gx_mi(xi, xj)] * pw[1 + xi + xj];
     } else {
-        m2l_fused_core<P, T>(dx, dy, eps2, in, out);
+        m2l_fused_core<P, WIDE, T>(dx, dy, eps2, in, out);
     }
 }
 
@@ -833,7 +849,7 @@ __global__ void __launch_bounds__(128) k_m2l_ref(int64_t nn, const uint32_t *__r
 
 // EXACT / ACCURATE M2L of one target over its sources idx[st .. st + len): lane l takes
 // sources l, l + 32, ...; acc holds the lane's unscaled sum over M'[S] A[S+T].
-template <int P, class T, class IDX>
+template <int P, class T, class IDX, bool WIDE>
 __device__ __forceinline__ void m2l_sources(const IDX *__restrict__ idx, int64_t st, int len, int lane, double tcx,
                                             double tcy, float4 thl, const double *__restrict__ comx,
                                             const double *__restrict__ comy, const float4 *__restrict__ comhl, T eps2,
@@ -865,7 +881,7 @@ __device__ __forceinline__ void m2l_sources(const IDX *__restrict__ idx, int64_t
 #pragma unroll
             for (int j = 0; j <= PP - i; j++)
                 if ((i + j) & 1) ms[gx_mi(i, j)] = -ms[gx_mi(i, j)];
-        m2l_fused<P, T>(dx, dy, eps2, ms, acc);
+        m2l_fused<P, T, WIDE>(dx, dy, eps2, ms, acc);
         src = nsrc;
     }
 }
@@ -894,7 +910,7 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && P <= 4) ? 8 : 1) k_m2l
     T acc[NC];
 #pragma unroll
     for (int k = 0; k < NCr; k++) acc[k] = T(0);
-    m2l_sources<P, T, IDX>(idx, st, len, lane, comx[node], comy[node], thl, comx, comy, comhl, (T)eps2d, M, acc);
+    m2l_sources<P, T, IDX, true>(idx, st, len, lane, comx[node], comy[node], thl, comx, comy, comhl, (T)eps2d, M, acc);
     // G = -A: L[T] = -(1/T!) sum_S M'[S] A[S+T]
     warp_coeffs<NC>(acc, [&](int k, T v) {
         int i, j;
@@ -960,7 +976,7 @@ __global__ void __launch_bounds__(32 * WPB, m2l_warps<P, T>() / WPB) k_m2l_units
         T acc[NC];
 #pragma unroll
         for (int k = 0; k < NCr; k++) acc[k] = T(0);
-        m2l_sources<P, T, int32_t>(idx, ustart[u], ulen[u], lane, comx[node], comy[node], thl, comx, comy, comhl,
+        m2l_sources<P, T, int32_t, false>(idx, ustart[u], ulen[u], lane, comx[node], comy[node], thl, comx, comy, comhl,
                                    (T)eps2d, M, acc);
         const int64_t u0 = node_u[node], u1 = node_u[node + 1];
         const auto store = [&](int k, T v) {
