@@ -836,7 +836,8 @@ int gx_plan_info(gx_ctx *ctx, int64_t *n_far_pairs, int64_t *n_near_pairs, int64
             idxp = dptr<int32_t>(ctx->near_idx);
             GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
             tot_idx = 0;
-            for (int64_t a = 0; a < nl; a++) tot_idx = std::max(tot_idx, st[a] + cnt[a]);
+            for (int64_t a = 0; a < nl; a++)  // a leaf without entries (one that no node has as a child) has no start
+                if (cnt[a] > 0) tot_idx = std::max(tot_idx, st[a] + cnt[a]);
         } else {
             GX_CUDA(ctx, cudaMemcpyAsync(st.data(), ctx->p2p_off.p, 8 * (nl + 1), cudaMemcpyDeviceToHost, ctx->stream));
             GX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
