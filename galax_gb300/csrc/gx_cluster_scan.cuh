@@ -7,7 +7,8 @@
 // the sums through distributed shared memory at a cluster barrier, and scan their shares;
 // the caller's load and store functions make the entries and use their offsets in the same
 // pass.  Beyond CS_MAX_N entries the three launches over the whole GPU are faster: at 331k one
-// cluster takes 27 us.
+// cluster takes 27 us, and the plan of 2,000,000 leaves spent 3.6 of its 44 ms in scans by one
+// cluster.  cs_scan takes the one form or the other.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -148,5 +149,97 @@ int cs_launch(gx_ctx *ctx, int64_t n, void (*kernel)(Params...), Args... args) {
     cfg.gridDim = dim3(blocks);
     GX_CUDA(ctx, cudaLaunchKernelEx(&cfg, kernel, Params(args)...));
     ctx->launches++;
+    return GX_OK;
+}
+
+// ---- one scan in either form ----
+// F describes it: off() (true: nothing is to be done), count() entries, load(i), store(i,
+// prefix, value) as above, and total(sum of all), called by one thread.
+template <int K, class F>
+__global__ void __launch_bounds__(CS_THREADS) k_scan_one_cluster(F f) {
+    if (f.off()) return;
+    const CsVec<K> all = cluster_scan<K>(
+        f.count(), [&](int64_t i) { return f.load(i); },
+        [&](int64_t i, const CsVec<K> &p, const CsVec<K> &v) { f.store(i, p, v); });
+    if (blockIdx.x == 0 && threadIdx.x == 0) f.total(all);
+}
+
+constexpr int64_t CS_TILE = CS_THREADS * CS_ITEMS;
+
+template <int K, class F>
+__global__ void __launch_bounds__(CS_THREADS) k_scan_tile_sums(F f, CsVec<K> *sums) {
+    __shared__ CsVec<K> sh[33];
+    if (f.off()) return;
+    const int64_t n = f.count(), base = blockIdx.x * CS_TILE;
+    if (base >= n) return;
+    CsVec<K> sum{}, total;
+    for (int q = 0; q < CS_ITEMS; q++) {
+        const int64_t i = base + q * CS_THREADS + threadIdx.x;
+        if (i >= n) break;
+        const CsVec<K> x = f.load(i);
+#pragma unroll
+        for (int k = 0; k < K; k++) sum.v[k] += x.v[k];
+    }
+    cs_block_scan<K>(sum, sh, total);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+template <int K, class F>
+__global__ void __launch_bounds__(CS_THREADS) k_scan_tile_tops(F f, CsVec<K> *sums) {
+    __shared__ CsVec<K> sh[33];
+    if (f.off()) return;
+    const int64_t nb = (f.count() + CS_TILE - 1) / CS_TILE;
+    CsVec<K> run{}, total;
+    for (int64_t base = 0; base < nb; base += CS_THREADS) {
+        const int64_t i = base + threadIdx.x;
+        CsVec<K> p = cs_block_scan<K>(i < nb ? sums[i] : CsVec<K>{}, sh, total);
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            p.v[k] += run.v[k];
+            run.v[k] += total.v[k];
+        }
+        if (i < nb) sums[i] = p;
+    }
+    __syncthreads();  // off() has been read: total may change it
+    if (threadIdx.x == 0) f.total(run);
+}
+
+template <int K, class F>
+__global__ void __launch_bounds__(CS_THREADS) k_scan_tile_stores(F f, const CsVec<K> *sums) {
+    __shared__ CsVec<K> sh[33];
+    if (f.off()) return;
+    const int64_t n = f.count(), base = blockIdx.x * CS_TILE + (int64_t)threadIdx.x * CS_ITEMS;
+    if (blockIdx.x * CS_TILE >= n) return;
+    CsVec<K> v[CS_ITEMS], s{}, total;
+#pragma unroll
+    for (int q = 0; q < CS_ITEMS; q++) {
+        v[q] = base + q < n ? f.load(base + q) : CsVec<K>{};
+#pragma unroll
+        for (int k = 0; k < K; k++) s.v[k] += v[q].v[k];
+    }
+    CsVec<K> p = cs_block_scan<K>(s, sh, total);
+    const CsVec<K> before = sums[blockIdx.x];
+#pragma unroll
+    for (int k = 0; k < K; k++) p.v[k] += before.v[k];
+#pragma unroll
+    for (int q = 0; q < CS_ITEMS; q++) {
+        if (base + q < n) f.store(base + q, p, v[q]);
+#pragma unroll
+        for (int k = 0; k < K; k++) p.v[k] += v[q].v[k];
+    }
+}
+
+// About n entries, n_cap at most.
+template <int K, class F>
+int cs_scan(gx_ctx *ctx, int64_t n, int64_t n_cap, const F &f) {
+    if (n <= CS_MAX_N) return cs_launch(ctx, n, k_scan_one_cluster<K, F>, f);
+    const int64_t nb = (n_cap + CS_TILE - 1) / CS_TILE;
+    GX_TRY(gx_ensure(ctx, ctx->scratch_g, sizeof(CsVec<K>) * (size_t)nb));
+    CsVec<K> *sums = dptr<CsVec<K>>(ctx->scratch_g);
+    k_scan_tile_sums<K, F><<<(unsigned)nb, CS_THREADS, 0, ctx->stream>>>(f, sums);
+    k_scan_tile_tops<K, F><<<1, CS_THREADS, 0, ctx->stream>>>(f, sums);
+    k_scan_tile_stores<K, F><<<(unsigned)nb, CS_THREADS, 0, ctx->stream>>>(f, sums);
+    ctx->launches += 3;
+    GX_CUDA(ctx, cudaGetLastError());
     return GX_OK;
 }

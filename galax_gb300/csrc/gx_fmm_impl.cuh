@@ -1155,7 +1155,7 @@ __global__ void __launch_bounds__(128) k_l2l_ref_leaves(int64_t nl, const int32_
 // keeping the common loop free of the self test.
 
 // Work items: the source list of every target leaf is cut into items of at most
-// P2P_K source leaves; one warp per item writes per-body partial accelerations to
+// 32 source leaves; one warp per item writes per-body partial accelerations to
 // its own slot, so the work per warp is bounded however uneven the lists are
 // (Plummer core leaves have hundreds of near leaves, halo leaves a few).  A second
 // kernel evaluates L2P and adds the partials of each leaf in item order, so the

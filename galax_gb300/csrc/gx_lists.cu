@@ -515,24 +515,25 @@ enum {
 };
 enum { OVF_UNITS = 1, OVF_FAR = 2, OVF_NEAR = 4, OVF_CHAIN = 8 };
 
-// The level's units, chunks of the nodes' candidate lists (their parents' near lists), counted
-// and scanned by one cluster: uoff[x - s] the first unit of node x, uoff[e - s] their number.
 __device__ __forceinline__ int64_t mac_chunks(int32_t P, const int32_t *near_cnt) {
     return P >= 0 ? ((int64_t)near_cnt[P] + MAC_CHUNK - 1) / MAC_CHUNK : 0;
 }
-__global__ void __launch_bounds__(CS_THREADS) k_mac_units(int64_t s, int64_t e, const int32_t *parent,
-                                                          const int32_t *near_cnt, int64_t *uoff, int64_t ucap,
-                                                          int64_t *ctr) {
-    if (ctr[PC_OVF]) return;
-    const CsVec<1> all = cluster_scan<1>(
-        e - s, [&](int64_t i) { return CsVec<1>{{mac_chunks(parent[s + i], near_cnt)}}; },
-        [&](int64_t i, const CsVec<1> &p, const CsVec<1> &) { uoff[i] = p.v[0]; });
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+// The level's units, chunks of the nodes' candidate lists (their parents' near lists): uoff[x -
+// s] the first unit of node x, uoff[e - s] their number.
+struct MacUnits {
+    int64_t s, e;
+    const int32_t *parent, *near_cnt;
+    int64_t *uoff, ucap, *ctr;
+    __device__ bool off() const { return ctr[PC_OVF] != 0; }
+    __device__ int64_t count() const { return e - s; }
+    __device__ CsVec<1> load(int64_t i) const { return {{mac_chunks(parent[s + i], near_cnt)}}; }
+    __device__ void store(int64_t i, const CsVec<1> &p, const CsVec<1> &) const { uoff[i] = p.v[0]; }
+    __device__ void total(const CsVec<1> &all) const {
         uoff[e - s] = all.v[0];
         if (all.v[0] > ucap)
             atomicOr(reinterpret_cast<unsigned long long *>(ctr + PC_OVF), (unsigned long long)OVF_UNITS);
     }
-}
+};
 // unit -> (node, chunk): over the whole GPU, as a wide halo node has dozens
 __global__ void k_mac_unit_nodes(int64_t s, int64_t e, const int64_t *uoff, int32_t *unode, int32_t *uchunk,
                                  const int64_t *ctr) {
@@ -546,31 +547,32 @@ __global__ void k_mac_unit_nodes(int64_t s, int64_t e, const int64_t *uoff, int3
     }
 }
 
-// After the counting pass, by one cluster: the units' offsets within the level (ufo, uno; one
-// more entry, the totals) and the running totals moved past the level.
-__global__ void __launch_bounds__(CS_THREADS) k_mac_offsets(const int64_t *Uptr, const int64_t *ufar,
-                                                            const int64_t *unear, int64_t *ufo, int64_t *uno,
-                                                            int64_t far_cap, int64_t near_cap, int64_t *ctr) {
-    if (ctr[PC_OVF]) return;
-    const int64_t U = *Uptr, far0 = ctr[PC_FAR], near0 = ctr[PC_NEAR];
-    const CsVec<2> all = cluster_scan<2>(
-        U, [&](int64_t u) { return CsVec<2>{{ufar[u], unear[u]}}; },
-        [&](int64_t u, const CsVec<2> &p, const CsVec<2> &) {
-            ufo[u] = p.v[0];
-            uno[u] = p.v[1];
-        });
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;  // all threads have read the totals before the scan's barriers
-    ufo[U] = all.v[0];
-    uno[U] = all.v[1];
-    ctr[PC_FAR0] = far0;
-    ctr[PC_NEAR0] = near0;
-    ctr[PC_FAR] = far0 + all.v[0];
-    ctr[PC_NEAR] = near0 + all.v[1];
-    ctr[PC_NEAR_LAST] = all.v[1];
-    const unsigned long long bad =
-        (far0 + all.v[0] > far_cap ? OVF_FAR : 0) | (near0 + all.v[1] > near_cap ? OVF_NEAR : 0);
-    if (bad) atomicOr(reinterpret_cast<unsigned long long *>(ctr + PC_OVF), bad);
-}
+// After the counting pass: the units' offsets within the level (ufo, uno; one more entry, the
+// totals) and the running totals moved past the level.
+struct MacOffsets {
+    const int64_t *units, *ufar, *unear;
+    int64_t *ufo, *uno, far_cap, near_cap, *ctr;
+    __device__ bool off() const { return ctr[PC_OVF] != 0; }
+    __device__ int64_t count() const { return *units; }
+    __device__ CsVec<2> load(int64_t u) const { return {{ufar[u], unear[u]}}; }
+    __device__ void store(int64_t u, const CsVec<2> &p, const CsVec<2> &) const {
+        ufo[u] = p.v[0];
+        uno[u] = p.v[1];
+    }
+    __device__ void total(const CsVec<2> &all) const {
+        const int64_t U = *units, far0 = ctr[PC_FAR], near0 = ctr[PC_NEAR];
+        ufo[U] = all.v[0];
+        uno[U] = all.v[1];
+        ctr[PC_FAR0] = far0;
+        ctr[PC_NEAR0] = near0;
+        ctr[PC_FAR] = far0 + all.v[0];
+        ctr[PC_NEAR] = near0 + all.v[1];
+        ctr[PC_NEAR_LAST] = all.v[1];
+        const unsigned long long bad =
+            (far0 + all.v[0] > far_cap ? OVF_FAR : 0) | (near0 + all.v[1] > near_cap ? OVF_NEAR : 0);
+        if (bad) atomicOr(reinterpret_cast<unsigned long long *>(ctr + PC_OVF), bad);
+    }
+};
 
 __device__ __forceinline__ bool mac_far_v(const float4 A, float Ra, const float4 B, float Rb, float theta2) {
     const float ex = __fadd_rn(__fsub_rn(A.x, B.x), __fsub_rn(A.y, B.y));
@@ -583,24 +585,25 @@ __device__ __forceinline__ bool mac_far_v(const float4 A, float Ra, const float4
 // pass 0: per-unit counts (ufar, unear), and each candidate's decisions in dec (one word
 // per lane and unit: byte k holds candidate k * 32 + lane's far mask in the low nibble and
 // its near mask in the high one, one bit per child slot); pass 1: the children written at
-// the running totals plus the per-unit offsets, from dec without testing again, and every
-// node's list starts and counts.  A grid-stride loop over the level's units, one warp per unit; each lane loads its
-// MAC_ROUNDS candidates, then their children, then tests them, so that the gathers of a
-// unit are in flight together.
+// the running totals plus the per-unit offsets, from dec without testing again, and with LISTS
+// every node's list starts and counts.  Whole levels that do not fit have set PC_OVF before.  A
+// grid-stride loop over the level's units, one warp per unit; each lane loads its MAC_ROUNDS
+// candidates, then their children, then tests them, so that the gathers of a unit are in flight
+// together.
 constexpr int MAC_ROUNDS = MAC_CHUNK / 32;
-__global__ void __launch_bounds__(128) k_mac(const int64_t *Uptr, int pass, const int32_t *unode,
+template <int PASS, bool LISTS>
+__global__ void __launch_bounds__(128) k_mac(const int64_t *Uptr, const int32_t *unode,
                                              const int32_t *uchunk, const int32_t *parent, const int4 *child,
                                              const float4 *hl, const float *R32, float theta2,
                                              int64_t *near_start, int32_t *near_cnt, int64_t *far_start,
                                              int32_t *far_cnt, const int32_t *near_idx_in, int64_t *ufar, int64_t *unear,
-                                             int32_t *far_idx, int32_t *near_idx, int64_t far_cap, int64_t near_cap,
-                                             uint32_t *dec, int64_t *ctr) {
+                                             int32_t *far_idx, int32_t *near_idx, uint32_t *dec, const int64_t *ctr) {
     const unsigned full = 0xffffffffu;
     if (ctr[PC_OVF]) return;
     const int64_t n_units = *Uptr;
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    const int64_t far0 = pass ? ctr[PC_FAR0] : 0, near0 = pass ? ctr[PC_NEAR0] : 0;
+    const int64_t far0 = PASS ? ctr[PC_FAR0] : 0, near0 = PASS ? ctr[PC_NEAR0] : 0;
     for (int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n_units; u += nwarps) {
         const int32_t x = unode[u];
         const int32_t P = parent[x];
@@ -610,17 +613,10 @@ __global__ void __launch_bounds__(128) k_mac(const int64_t *Uptr, int pass, cons
         const int64_t qa = near_start[P] + (int64_t)uchunk[u] * MAC_CHUNK;
         const int qn = (int)min((int64_t)MAC_CHUNK, near_start[P] + (int64_t)near_cnt[P] - qa);
         int64_t fb = 0, nb = 0;
-        if (pass) {
-            // this unit's whole range must fit; otherwise flag and write nothing
+        if constexpr (PASS) {
             fb = far0 + ufar[u];
             nb = near0 + unear[u];
-            const int64_t fe = far0 + ufar[u + 1], ne = near0 + unear[u + 1];
-            const unsigned long long bad = (fe > far_cap ? OVF_FAR : 0) | (ne > near_cap ? OVF_NEAR : 0);
-            if (bad) {
-                if (lane == 0) atomicOr(reinterpret_cast<unsigned long long *>(ctr + PC_OVF), bad);
-                continue;
-            }
-            if (uchunk[u] == 0 && lane == 0) {  // the node's first unit (every node has one: it is near itself)
+            if (LISTS && uchunk[u] == 0 && lane == 0) {  // the node's first unit (every node has one: it is near itself)
                 const int64_t last = u + mac_chunks(P, near_cnt);
                 far_start[x] = fb;
                 near_start[x] = nb;
@@ -635,7 +631,7 @@ __global__ void __launch_bounds__(128) k_mac(const int64_t *Uptr, int pass, cons
 #pragma unroll
         for (int k = 0; k < MAC_ROUNDS; k++) c4[k] = cand[k] >= 0 ? child[cand[k]] : make_int4(-1, -1, -1, -1);
         uint32_t d = 0;
-        if (pass) {
+        if constexpr (PASS) {
             d = dec[u * 32 + lane];
         } else {
             const float4 A = hl[x];
@@ -717,6 +713,21 @@ __global__ void k_chain_leaf_offsets(int64_t nl, int64_t up, int64_t near_cap, i
     if (ctr[PC_OVF] || dst + n > near_cap) return;
     nstart[x] = dst + (nstart[x + up] - (dst - n));
     ncnt[x] = ncnt[x + up];
+}
+
+// Pass 1's list starts and counts, a thread per node, for levels above CS_MAX_N nodes: within the
+// pass they save a launch and cost its warps three dependent loads a node.  At 2,000,000 leaves
+// the passes take 21.9 ms with them here (0.13) and compiled apart, 24.5 with all in one kernel.
+__global__ void k_mac_node_lists(int64_t s, int64_t e, const int64_t *uoff, const int64_t *ufo, const int64_t *uno,
+                                 const int64_t *ctr, int64_t *fstart, int32_t *fcnt, int64_t *nstart, int32_t *ncnt) {
+    if (ctr[PC_OVF]) return;
+    const int64_t x = s + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= e) return;
+    const int64_t a = uoff[x - s], b = uoff[x - s + 1];
+    fstart[x] = ctr[PC_FAR0] + ufo[a];
+    nstart[x] = ctr[PC_NEAR0] + uno[a];
+    fcnt[x] = (int32_t)(ufo[b] - ufo[a]);
+    ncnt[x] = (int32_t)(uno[b] - uno[a]);
 }
 
 // the lists before the first level: empty, but for the root's near list {root} at index 0
@@ -1338,18 +1349,25 @@ int gx_plan_accurate(gx_ctx *ctx) {
         for (int lv = lv_big; lv >= lv_low; lv--) {
             const int64_t s = ctx->level_start[lv], e = ctx->level_start[lv + 1], c = e - s;
             // units: chunks of each node's candidate list
-            GX_TRY(cs_launch(ctx, c, k_mac_units, s, e, dptr<int32_t>(ctx->parent), ncnt, uoff, ucap, ctr));
+            GX_TRY(cs_scan<1>(ctx, c, c, MacUnits{s, e, dptr<int32_t>(ctx->parent), ncnt, uoff, ucap, ctr}));
             k_mac_unit_nodes<<<gx_blocks(c, 256), 256, 0, ctx->stream>>>(s, e, uoff, unode, uchunk, ctr);
             const int64_t *Ud = uoff + c;  // the level's unit count, on the device
-            k_mac<<<gmac, 128, 0, ctx->stream>>>(Ud, 0, unode, uchunk, dptr<int32_t>(ctx->parent),
-                                                 dptr<int4>(ctx->child), hl, R32, theta2, nstart, ncnt, fstart, fcnt,
-                                                 dptr<int32_t>(ctx->near_idx), ufar, unear, nullptr, nullptr, far_cap,
-                                                 near_cap, dec, ctr);
-            GX_TRY(cs_launch(ctx, CS_MAX_N, k_mac_offsets, Ud, ufar, unear, ufo, uno, far_cap, near_cap, ctr));
-            k_mac<<<gmac, 128, 0, ctx->stream>>>(Ud, 1, unode, uchunk, dptr<int32_t>(ctx->parent),
-                                                 dptr<int4>(ctx->child), hl, R32, theta2, nstart, ncnt, fstart, fcnt,
-                                                 dptr<int32_t>(ctx->near_idx), ufo, uno, dptr<int32_t>(ctx->far_idx),
-                                                 dptr<int32_t>(ctx->near_idx), far_cap, near_cap, dec, ctr);
+            k_mac<0, false><<<gmac, 128, 0, ctx->stream>>>(
+                Ud, unode, uchunk, dptr<int32_t>(ctx->parent), dptr<int4>(ctx->child), hl, R32, theta2, nstart, ncnt,
+                nullptr, nullptr, dptr<int32_t>(ctx->near_idx), ufar, unear, nullptr, nullptr, dec, ctr);
+            // a unit for every node or more: their number is on the device only
+            GX_TRY(cs_scan<2>(ctx, std::max(c, CS_MAX_N), ucap,
+                              MacOffsets{Ud, ufar, unear, ufo, uno, far_cap, near_cap, ctr}));
+            const bool apart = c > CS_MAX_N;
+            if (apart) {
+                k_mac_node_lists<<<gx_blocks(c, 256), 256, 0, ctx->stream>>>(s, e, uoff, ufo, uno, ctr, fstart, fcnt,
+                                                                            nstart, ncnt);
+                ctx->launches++;
+            }
+            (apart ? k_mac<1, false> : k_mac<1, true>)<<<gmac, 128, 0, ctx->stream>>>(
+                Ud, unode, uchunk, dptr<int32_t>(ctx->parent), dptr<int4>(ctx->child), hl, R32, theta2, nstart, ncnt,
+                fstart, fcnt, dptr<int32_t>(ctx->near_idx), ufo, uno, dptr<int32_t>(ctx->far_idx),
+                dptr<int32_t>(ctx->near_idx), dec, ctr);
             ctx->launches += 3;
             GX_CUDA(ctx, cudaGetLastError());
         }
@@ -1414,21 +1432,26 @@ __device__ __forceinline__ int near_kind(const float4 A, float Ra, const float4 
 constexpr int NS_CHUNK = 256;
 constexpr int NS_ROUNDS = NS_CHUNK / 32;
 
-// unit -> (leaf, chunk, entries), by one cluster; uoff[nl]: their number
-__global__ void __launch_bounds__(CS_THREADS) k_ns_units(int64_t nl, const int32_t *ncnt, int64_t *uoff, int4 *unit,
-                                                         int32_t *split_cnt) {
-    const CsVec<1> all = cluster_scan<1>(
-        nl, [&](int64_t a) { return CsVec<1>{{(ncnt[a] + NS_CHUNK - 1) / NS_CHUNK}}; },
-        [&](int64_t a, const CsVec<1> &p, const CsVec<1> &) {
-            const int32_t c = ncnt[a];
-            const int64_t u0 = p.v[0];
-            uoff[a] = u0;
-            for (int32_t j = 0; j * NS_CHUNK < c; j++)
-                unit[u0 + j] = make_int4((int32_t)a, j, min(NS_CHUNK, c - j * NS_CHUNK), 0);
-            if (c == 0) split_cnt[2 * a] = split_cnt[2 * a + 1] = 0;  // no unit writes them
-        });
-    if (blockIdx.x == 0 && threadIdx.x == 0) uoff[nl] = all.v[0];
-}
+// unit -> (leaf, chunk, entries); uoff[nl]: their number
+struct SplitUnits {
+    int64_t nl;
+    const int32_t *ncnt;
+    int64_t *uoff;
+    int4 *unit;
+    int32_t *split_cnt;
+    __device__ bool off() const { return false; }
+    __device__ int64_t count() const { return nl; }
+    __device__ CsVec<1> load(int64_t a) const { return {{(ncnt[a] + NS_CHUNK - 1) / NS_CHUNK}}; }
+    __device__ void store(int64_t a, const CsVec<1> &p, const CsVec<1> &) const {
+        const int32_t c = ncnt[a];
+        const int64_t u0 = p.v[0];
+        uoff[a] = u0;
+        for (int32_t j = 0; j * NS_CHUNK < c; j++)
+            unit[u0 + j] = make_int4((int32_t)a, j, min(NS_CHUNK, c - j * NS_CHUNK), 0);
+        if (c == 0) split_cnt[2 * a] = split_cnt[2 * a + 1] = 0;  // no unit writes them
+    }
+    __device__ void total(const CsVec<1> &all) const { uoff[nl] = all.v[0]; }
+};
 
 __global__ void __launch_bounds__(128) k_ns_kinds(const int64_t *__restrict__ Ud, const int4 *__restrict__ unit,
                                                    const int64_t *__restrict__ nstart,
@@ -1565,7 +1588,7 @@ int gx_plan_near_split(gx_ctx *ctx) {
         GX_TRY(gx_ensure(ctx, ctx->scratch_d, sizeof(int4) * (size_t)ucap));
         int64_t *uoff = dptr<int64_t>(ctx->scratch_a);
         int4 *unit = dptr<int4>(ctx->scratch_b), *ucnt = dptr<int4>(ctx->scratch_d);
-        GX_TRY(cs_launch(ctx, nl, k_ns_units, nl, ncnt, uoff, unit, dptr<int32_t>(ctx->split_cnt)));
+        GX_TRY(cs_scan<1>(ctx, nl, nl, SplitUnits{nl, ncnt, uoff, unit, dptr<int32_t>(ctx->split_cnt)}));
         const unsigned g = (unsigned)(ctx->sm_count > 0 ? ctx->sm_count * 16 : 2432);  // grid-stride, 4 warps a block
         k_ns_kinds<<<g, 128, 0, ctx->stream>>>(uoff + nl, unit, nstart, dptr<int32_t>(ctx->near_idx),
                                                dptr<int32_t>(ctx->scratch_f), dptr<float4>(ctx->comhl),
@@ -1580,23 +1603,25 @@ int gx_plan_near_split(gx_ctx *ctx) {
 }
 
 namespace {
-constexpr int P2P_K = 32;  // most source leaves per P2P (or M2P) work item
+constexpr int P2P_KB = 5;  // log2 of the most source leaves per P2P (or M2P) item
 
-// Source leaves per P2P item: a small problem's lists are cut finer, down to one leaf an
-// item, until there are enough items for the GPU to balance: 8 an SM for the reference's
+// log2 of the source leaves per P2P item: a small problem's lists are cut finer, down to one leaf
+// an item, until there are enough items for the GPU to balance: 8 an SM for the reference's
 // lists (FP64; at N = 1000 their 306 near pairs were 32 items), 2 an SM for the
 // opening-angle lists, whose mixed form gains less from it than its final sum pays for the
 // extra partials (N = 10,000, 14,561 near pairs, 8 an SM: P2P 28 -> 20 us beside the far
 // field, sum 8 -> 10 us after it).
-static int p2p_item_leaves(const gx_ctx *ctx, int64_t near_pairs, bool accurate) {
+static int p2p_item_leaves_log2(const gx_ctx *ctx, int64_t near_pairs, bool accurate) {
     const int64_t want = (int64_t)ctx->sm_count * (accurate ? 2 : 8);
-    int k = P2P_K;
-    while (k > 1 && near_pairs / k < want) k /= 2;
+    int k = P2P_KB;
+    while (k > 0 && (near_pairs >> k) < want) k--;
     return k;
 }
-// Source leaves per M2P item: not below eight (k_m2p_x2 sets up its moments a lane per
+// The same per M2P item: not below eight leaves (k_m2p_x2 sets up its moments a lane per
 // source and its half-warps take every other one).
-static int m2p_item_leaves(int p2p_leaves) { return p2p_leaves < 8 ? 8 : p2p_leaves; }
+static int m2p_item_leaves_log2(int p2p) { return p2p < 3 ? 3 : p2p; }
+// ceil(v / 2^k)
+__device__ __forceinline__ int64_t ceil_shift(int64_t v, int k) { return (v + ((1 << k) - 1)) >> k; }
 
 // ancestor table: anc[level * nl + leaf] = the leaf's ancestor at that level
 __global__ void k_ancestors(int64_t nl, int n_levels, const int32_t *parent, int32_t *anc) {
@@ -1621,42 +1646,41 @@ __global__ void k_comhl(int64_t nn, const double *comx, const double *comy, floa
 // per leaf: number of items; start/count from either list layout.  With the near-list
 // split (split != null) the leaf's P2P items are followed by its M2P items, whose
 // source count is stored negated; split[2a] is the leaf's M2P count.
-// Per leaf, scanned together by one cluster: its work items (K source leaves each of its P2P
-// sources, KM of its M2P ones), its M2P items, its P2L units (of at most GX_P2L_UNIT source
-// leaves) and with the body-level P2L its units of at most GX_BODY_UNIT of its P2P rows.
-// Each array's entry nl is the total; tot receives all four.
-__global__ void __launch_bounds__(CS_THREADS) k_item_offsets(int64_t nl, int K, int KM, const int64_t *start,
-                                                             const int32_t *cnt, const int32_t *split, int body,
-                                                             int64_t *off, int64_t *m2p_off, int64_t *leaf_u,
-                                                             int64_t *body_u, int64_t *tot) {
-    const CsVec<4> all = cluster_scan<4>(
-        nl,
-        [&](int64_t a) {
-            const int64_t c = cnt ? cnt[a] : start[a + 1] - start[a];
-            const int64_t cm = split ? split[2 * a] : 0, cl = split ? split[2 * a + 1] : 0, m = (cm + KM - 1) / KM;
-            return CsVec<4>{{(c + K - 1) / K + m, m, (cl + GX_P2L_UNIT - 1) / GX_P2L_UNIT,
-                             body ? (c + GX_BODY_UNIT - 1) / GX_BODY_UNIT : 0}};
-        },
-        [&](int64_t a, const CsVec<4> &p, const CsVec<4> &) {
-            off[a] = p.v[0];
-            if (split) {
-                m2p_off[a] = p.v[1];
-                leaf_u[a] = p.v[2];
-                if (body) body_u[a] = p.v[3];
-            }
-        });
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    off[nl] = all.v[0];
-    if (split) {
-        m2p_off[nl] = all.v[1];
-        leaf_u[nl] = all.v[2];
-        if (body) body_u[nl] = all.v[3];
+// Per leaf, scanned together: its work items (K source leaves each of its P2P sources, KM of its
+// M2P ones), its M2P items, its P2L units (of at most GX_P2L_UNIT source leaves) and with the
+// body-level P2L its units of at most GX_BODY_UNIT of its P2P rows.  Each array's entry nl is
+// the total; tot receives all four.
+struct ItemOffsets {
+    int64_t nl;
+    int kb, kmb;  // log2 of K and KM
+    const int64_t *start;
+    const int32_t *cnt, *split;
+    int body;
+    int64_t *item_off, *m2p_off, *leaf_u, *body_u, *tot;
+    __device__ bool off() const { return false; }
+    __device__ int64_t count() const { return nl; }
+    __device__ CsVec<4> load(int64_t a) const {
+        const int64_t c = cnt ? cnt[a] : start[a + 1] - start[a];
+        const int64_t cm = split ? split[2 * a] : 0, cl = split ? split[2 * a + 1] : 0, m = ceil_shift(cm, kmb);
+        return {{ceil_shift(c, kb) + m, m, (cl + GX_P2L_UNIT - 1) / GX_P2L_UNIT,
+                 body ? (c + GX_BODY_UNIT - 1) / GX_BODY_UNIT : 0}};
     }
-    for (int k = 0; k < 4; k++) tot[k] = all.v[k];
-}
+    __device__ void put(int64_t a, const CsVec<4> &p) const {
+        item_off[a] = p.v[0];
+        if (!split) return;
+        m2p_off[a] = p.v[1];
+        leaf_u[a] = p.v[2];
+        if (body) body_u[a] = p.v[3];
+    }
+    __device__ void store(int64_t a, const CsVec<4> &p, const CsVec<4> &) const { put(a, p); }
+    __device__ void total(const CsVec<4> &all) const {
+        put(nl, all);
+        for (int k = 0; k < 4; k++) tot[k] = all.v[k];
+    }
+};
 
 // one warp per leaf, lanes over its items: the widest halo leaves have ~1000 items
-__global__ void k_items_fill(int64_t nl, int K, int KM, const int64_t *start, const int32_t *cnt, const int32_t *split,
+__global__ void k_items_fill(int64_t nl, int kb, int kmb, const int64_t *start, const int32_t *cnt, const int32_t *split,
                              const int64_t *off, int32_t *leaf, int64_t *qb, int32_t *nq, const int64_t *m2p_off,
                              int32_t *m2p_list) {
     const int64_t a = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1664,18 +1688,20 @@ __global__ void k_items_fill(int64_t nl, int K, int KM, const int64_t *start, co
     if (a >= nl) return;
     const int64_t s0 = start[a];
     const int64_t c = cnt ? cnt[a] : start[a + 1] - start[a];
-    const int64_t it0 = off[a], np = (c + K - 1) / K;
+    const int64_t K = 1 << kb, KM = 1 << kmb, it0 = off[a], np = ceil_shift(c, kb);
+#pragma unroll 1  // mostly one turn: registers for more leaves at once
     for (int64_t k = lane; k < np; k += 32) {
         leaf[it0 + k] = (int32_t)a;
         qb[it0 + k] = s0 + k * K;
-        nq[it0 + k] = (int32_t)min((int64_t)K, c - k * K);
+        nq[it0 + k] = (int32_t)min(K, c - k * K);
     }
-    const int64_t cm = split ? split[2 * a] : 0, nm = (cm + KM - 1) / KM;
+    const int64_t cm = split ? split[2 * a] : 0, nm = ceil_shift(cm, kmb);
+#pragma unroll 1
     for (int64_t k = lane; k < nm; k += 32) {
         const int64_t it = it0 + np + k;
         leaf[it] = (int32_t)a;
         qb[it] = s0 + c + k * KM;
-        nq[it] = -(int32_t)min((int64_t)KM, cm - k * KM);
+        nq[it] = -(int32_t)min(KM, cm - k * KM);
         m2p_list[m2p_off[a] + k] = (int32_t)it;
     }
 }
@@ -1890,8 +1916,8 @@ int gx_plan_items(gx_ctx *ctx, bool accurate) {
     const bool body = split && nl > 0 && gx_body_split_on(ctx);  // body-level P2L units after the leaf-level ones
     if (accurate) ctx->plan_body_split = false;  // the masks follow these items (gx_plan_body_masks)
     const int32_t *scnt = split ? dptr<int32_t>(ctx->split_cnt) : nullptr;
-    const int K = p2p_item_leaves(ctx, accurate ? ctx->n_near_pairs : ctx->n_p2p_pairs, accurate);
-    const int KM = m2p_item_leaves(K);
+    const int kb = p2p_item_leaves_log2(ctx, accurate ? ctx->n_near_pairs : ctx->n_p2p_pairs, accurate);
+    const int kmb = m2p_item_leaves_log2(kb);
     GX_TRY(gx_ensure(ctx, I.off, sizeof(int64_t) * (size_t)(nl + 1)));
     GX_TRY(gx_ensure(ctx, ctx->scratch_c, sizeof(int64_t) * 4));
     int64_t *dtot = dptr<int64_t>(ctx->scratch_c);
@@ -1901,8 +1927,9 @@ int gx_plan_items(gx_ctx *ctx, bool accurate) {
         GX_TRY(gx_ensure(ctx, PU.leaf_u, sizeof(int64_t) * (size_t)(nl + 1)));
         GX_TRY(gx_ensure(ctx, PU.body_u, sizeof(int64_t) * (size_t)(nl + 1)));
     }
-    GX_TRY(cs_launch(ctx, nl, k_item_offsets, nl, K, KM, start, cnt, scnt, body ? 1 : 0, dptr<int64_t>(I.off),
-                     dptr<int64_t>(ctx->m2p_off), dptr<int64_t>(PU.leaf_u), dptr<int64_t>(PU.body_u), dtot));
+    GX_TRY(cs_scan<4>(ctx, nl, nl,
+                      ItemOffsets{nl, kb, kmb, start, cnt, scnt, body ? 1 : 0, dptr<int64_t>(I.off),
+                                  dptr<int64_t>(ctx->m2p_off), dptr<int64_t>(PU.leaf_u), dptr<int64_t>(PU.body_u), dtot}));
     gx_ctx::M2LUnits &U = ctx->m2l_units;
     const int64_t *fstart = accurate ? dptr<int64_t>(ctx->far_off) : nullptr;
     const int32_t *fcnt = accurate ? reinterpret_cast<const int32_t *>(fstart + nn) : nullptr;
@@ -1931,7 +1958,7 @@ int gx_plan_items(gx_ctx *ctx, bool accurate) {
     GX_TRY(gx_ensure(ctx, I.nq, sizeof(int32_t) * (size_t)(tot[0] + 1)));
     if (split) GX_TRY(gx_ensure(ctx, ctx->m2p_list, sizeof(int32_t) * (size_t)(tot[1] + 1)));
     k_items_fill<<<gx_blocks(nl * 32, 256), 256, 0, ctx->stream>>>(
-        nl, K, KM, start, cnt, scnt, dptr<int64_t>(I.off), dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb), dptr<int32_t>(I.nq),
+        nl, kb, kmb, start, cnt, scnt, dptr<int64_t>(I.off), dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb), dptr<int32_t>(I.nq),
         split ? dptr<int64_t>(ctx->m2p_off) : nullptr, split ? dptr<int32_t>(ctx->m2p_list) : nullptr);
     ctx->launches++;
     I.n = tot[0];
