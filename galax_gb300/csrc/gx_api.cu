@@ -415,7 +415,7 @@ static int upload_bodies_impl(gx_ctx *ctx, int64_t n, const double *x, const dou
     bool same_n = ctx->have_bodies && ctx->n_bodies == n;
     bool keep[7];
     const double *dsrc[7];
-    bool direct = n > 0;
+    bool direct = n > 0 && n <= GX_COPY_KERNEL;
     for (int k = 0; k < 7; k++) {
         void *before = dst[k]->p;
         GX_TRY(gx_ensure(ctx, *dst[k], bytes));
@@ -423,7 +423,7 @@ static int upload_bodies_impl(gx_ctx *ctx, int64_t n, const double *x, const dou
     }
     for (int k = 0; k < 7 && direct; k++) {
         dsrc[k] = src[k] ? static_cast<const double *>(direct_host(ctx, src[k], sizeof(double) * n, false)) : nullptr;
-        direct = !src[k] || (dsrc[k] && n <= GX_COPY_KERNEL);
+        direct = !src[k] || dsrc[k];
     }
     if (direct) {
         Copy7 c;

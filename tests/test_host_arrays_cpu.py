@@ -91,3 +91,17 @@ fail.value = 0
 ctx.upload_bodies(bodies(n))
 assert count("fake_waits") == w + 2
 """)
+
+
+def test_large_uploads_do_not_look_at_the_pages(run):
+    """Above the kernel copy's limit the arrays are copied whatever they are: their pages are
+    neither asked after nor touched."""
+    run("""
+n = 262_145
+ctx = G.GpuContext(G.GpuConfig(max_n=n))
+b = bodies(n)
+q, c = count("fake_queries"), count("fake_copies")
+ctx.upload_bodies(b)
+ctx.download_bodies(b)
+assert count("fake_queries") == q and count("fake_copies") == c + 14
+""")
