@@ -548,19 +548,23 @@ int gx_upload_tree(gx_ctx *ctx, int64_t n_nodes, int64_t n_bodies, const double 
     // round contiguously, which the device passes rely on.
     std::vector<int32_t> lev((size_t)n_nodes);
     std::vector<int32_t> bs32((size_t)n_nodes), be32((size_t)n_nodes);
-    int32_t maxlev = 0;
+    int32_t maxlev = 0, not_unary = INT32_MAX;
     int64_t nl = 0;
     for (int64_t i = 0; i < n_nodes; i++) {
-        int32_t l = 0;
+        int32_t l = 0, kids = 0;
         for (int k = 0; k < 4; k++) {
             int32_t c = child[4 * i + k];
             if (c >= 0) {
                 if (c >= i) return gx_fail(ctx, GX_ERR_INVALID_ARG, "child id must precede its parent");
                 l = std::max(l, lev[c] + 1);
+                kids++;
             }
         }
         lev[i] = l;
         maxlev = std::max(maxlev, l);
+        // the lowest level with a node that is not the one parent of the node nl before it (nl
+        // is final there: the leaves come first)
+        if (l > 0 && l < not_unary && (kids != 1 || child[4 * i] != i - nl)) not_unary = l;
         if (is_leaf[i]) {
             if (l != 0) return gx_fail(ctx, GX_ERR_INVALID_ARG, "leaf with children");
             nl++;
@@ -600,19 +604,22 @@ int gx_upload_tree(gx_ctx *ctx, int64_t n_nodes, int64_t n_bodies, const double 
     ctx->max_leaf = 0;
     for (int64_t i = 0; i < nl; i++) ctx->max_leaf = std::max(ctx->max_leaf, body_end[i] - body_start[i]);
     ctx->unary_levels = 0;
-    for (int l = 1; l < ctx->n_levels; l++) {  // single-child levels, checked node by node
-        bool chain = ls[l + 1] - ls[l] == nl;
-        for (int64_t i = ls[l]; chain && i < ls[l + 1]; i++)
-            chain = child[4 * i] == i - nl && child[4 * i + 1] < 0 && child[4 * i + 2] < 0 && child[4 * i + 3] < 0;
-        if (!chain) break;
-        ctx->unary_levels = l;
+    while (ctx->unary_levels + 1 < std::min(ctx->n_levels, not_unary) &&
+           ls[ctx->unary_levels + 2] - ls[ctx->unary_levels + 1] == nl)
+        ctx->unary_levels++;
+    // how far the leaves' ranges go without a gap: in id order, which is body order in the
+    // trees that Tree::build makes, else sorted
+    int64_t reach = 0, i = 0;
+    for (; i < nl && body_start[i] <= reach; i++) reach = std::max(reach, body_end[i]);
+    if (i < nl) {
+        std::vector<std::pair<int64_t, int64_t>> lr;
+        lr.reserve((size_t)nl);
+        for (i = 0; i < nl; i++) lr.emplace_back(body_start[i], body_end[i]);
+        std::sort(lr.begin(), lr.end());
+        reach = 0;
+        for (const auto &r : lr)
+            if (r.first <= reach) reach = std::max(reach, r.second);
     }
-    std::vector<std::pair<int64_t, int64_t>> lr;  // the leaves' ranges, in body order
-    for (int64_t i = 0; i < nl; i++) lr.emplace_back(body_start[i], body_end[i]);
-    std::sort(lr.begin(), lr.end());
-    int64_t reach = 0;
-    for (const auto &r : lr)
-        if (r.first <= reach) reach = std::max(reach, r.second);
     ctx->leaves_cover = reach == n_bodies;
     ctx->ref_lists_valid = true;  // the caller's lists
     ctx->have_tree = true;
