@@ -27,7 +27,7 @@
 
 namespace {
 
-// Factorials, binomials and reciprocals come from a constant-memory table, filled by
+// Factorials, their products and reciprocals come from a constant-memory table, filled by
 // static initialization from a constexpr builder, in both FP64 and FP32 (each FP32
 // entry is the FP64 value rounded once).  A table read is one constant-bank operand
 // when the loop around it is unrolled and one constant load when it is not; no
@@ -37,8 +37,6 @@ namespace {
 struct GxTables {
     double fact[34];
     double invfact[34];
-    double binom[17][17];
-    float binom_f[17][17];
     double ifp[17][17];  // 1/(i! j!) as the FP64 product of 1/i! and 1/j!
     float ifp_f[17][17];
     double inv[34];  // 1/n
@@ -51,11 +49,6 @@ __host__ __device__ constexpr GxTables gx_make_tables() {
     t.fact[0] = 1.0;
     for (int i = 1; i < 34; i++) t.fact[i] = t.fact[i - 1] * (double)i;
     for (int i = 0; i < 34; i++) t.invfact[i] = 1.0 / t.fact[i];
-    for (int n = 0; n < 17; n++) {
-        t.binom[n][0] = 1.0;
-        for (int k = 1; k <= n; k++) t.binom[n][k] = t.binom[n - 1][k - 1] + (k < n ? t.binom[n - 1][k] : 0.0);
-        for (int k = 0; k < 17; k++) t.binom_f[n][k] = (float)t.binom[n][k];
-    }
     for (int i = 0; i < 17; i++)
         for (int j = 0; j < 17; j++) {
             t.ifp[i][j] = t.invfact[i] * t.invfact[j];
@@ -75,13 +68,7 @@ __host__ __device__ constexpr GxTables gx_make_tables() {
     return t;
 }
 __constant__ GxTables c_tab = gx_make_tables();
-__device__ __forceinline__ double cfact(int n) { return c_tab.fact[n]; }
-__device__ __forceinline__ double cinvfact(int n) { return c_tab.invfact[n]; }
-__device__ __forceinline__ double cbinom(int n, int k) { return (k < 0 || k > n) ? 0.0 : c_tab.binom[n][k]; }
-// typed reads: C(n, k), 1/(i! j!), 1/n
-template <class T> __device__ __forceinline__ T tab_binom(int n, int k);
-template <> __device__ __forceinline__ double tab_binom<double>(int n, int k) { return c_tab.binom[n][k]; }
-template <> __device__ __forceinline__ float tab_binom<float>(int n, int k) { return c_tab.binom_f[n][k]; }
+// typed reads: 1/(i! j!), k! l!, 1/n
 template <class T> __device__ __forceinline__ T tab_ifp(int i, int j);
 template <> __device__ __forceinline__ double tab_ifp<double>(int i, int j) { return c_tab.ifp[i][j]; }
 template <> __device__ __forceinline__ float tab_ifp<float>(int i, int j) { return c_tab.ifp_f[i][j]; }
@@ -94,7 +81,7 @@ template <> __device__ __forceinline__ float tab_inv<float>(int n) { return c_ta
 __host__ __device__ constexpr int nc2(int q) { return (q + 1) * (q + 2) / 2; }  // entries with k+l <= q
 
 // Loops over expansion indices are fully unrolled (coefficient arrays stay in
-// registers) for orders up to 5; above that the bound is made a runtime value
+// registers) for orders up to 8; above that the bound is made a runtime value
 // (a zero the compiler cannot see through) so the loops stay rolled and the
 // translation units compile in seconds.
 __constant__ int g_rt_zero = 0;
@@ -1302,7 +1289,7 @@ __global__ void __launch_bounds__(128) k_p2p64_items(const int32_t *__restrict__
 // FP32 partials on coordinates relative to the target leaf's COM.  Bodies come packed
 // as (x - com_leaf, y - com_leaf, m) in FP32 (written by P2M); a source leaf is moved
 // into the target's frame by one FP32 shift per leaf pair, formed in FP64 and rounded once.
-// 7 blocks per SM: 72 registers, no spills (left alone, ptxas picks 64 and spills)
+// 28 warps an SM: 72 registers, no spills (left alone, ptxas picks 64 and spills)
 __global__ void __launch_bounds__(32 * WPB, 28 / WPB) k_p2p32_items(int64_t n_items, const int32_t *__restrict__ item_leaf,
                                                      const int64_t *__restrict__ item_qb, const int32_t *__restrict__ item_nq,
                                                      const float4 *__restrict__ pos, const double *__restrict__ comx,

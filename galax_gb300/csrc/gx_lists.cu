@@ -26,7 +26,6 @@
 #include "gx_internal.cuh"
 
 int gx_tree_rebuild_with_splits(gx_ctx *ctx, int64_t n_max, const double bounds[4], const std::vector<int64_t> &splits);
-int gx_add_offsets(gx_ctx *ctx, const int64_t *o, int64_t *dst, int64_t c, int64_t add);
 
 namespace {
 
@@ -1826,19 +1825,7 @@ __global__ void k_m2l_units_fill(int64_t nn, const int64_t *fstart, const int32_
         ulen[u] = min(GX_M2L_UNIT, fcnt[a] - k);
     }
 }
-
-__global__ void k_add_offsets(const int64_t *o, int64_t *dst, int64_t c, int64_t add) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < c) dst[i] = o[i] + add;
-}
 }  // namespace
-
-int gx_add_offsets(gx_ctx *ctx, const int64_t *o, int64_t *dst, int64_t c, int64_t add) {
-    k_add_offsets<<<gx_blocks(c, 256), 256, 0, ctx->stream>>>(o, dst, c, add);
-    ctx->launches++;
-    GX_CUDA(ctx, cudaGetLastError());
-    return GX_OK;
-}
 
 // build_constrained (lib.rs:541-588) on the device: up to 10 rebuilds with split
 // points; the per-leaf neighbour search runs on the GPU, the split-point set (a

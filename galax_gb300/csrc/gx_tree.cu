@@ -789,7 +789,7 @@ int gx_tree_build_device(gx_ctx *ctx, int64_t n, int64_t n_max, const double bou
     }
     int64_t nl = (n + n_max - 1) / n_max;
     GX_TRY(gx_ensure(ctx, ctx->scratch_f, sizeof(int32_t) * (size_t)(2 * nl + 2) + 64));
-    // scratch_f is also the radix-sort flag; the sort is finished at this point
+    // scratch_f held the sort's digit totals; the sort is finished at this point
     int32_t *rs = dptr<int32_t>(ctx->scratch_f), *re = rs + nl;
     k_chunk_ranges<<<gx_blocks(nl, 256), 256, 0, ctx->stream>>>(n, n_max, nl, rs, re);
     ctx->launches++;
