@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(128) k_adj_l2p(int64_t nl, const double *__res
 // partials in unit order.  Nodes without far entries are not written: has_far = 0 keeps A4
 // from reading them.
 template <int P, class T>
-__global__ void __launch_bounds__(32 * WPB, m2l_warps<P, T>() / WPB)
+__global__ void __launch_bounds__(32 * m2l_block<P, T>(), m2l_warps<P, T>() / m2l_block<P, T>())
     k_adj_m2l(int64_t n_units, const int32_t *__restrict__ unode, const int64_t *__restrict__ ustart,
               const int32_t *__restrict__ ulen, const int64_t *__restrict__ node_u, const int32_t *__restrict__ idx,
               const double *__restrict__ comx, const double *__restrict__ comy, const float4 *__restrict__ comhl,
@@ -669,7 +669,8 @@ int run_force_vjp(gx_ctx *ctx, const double *X, const double *Y, const void *lf_
     if (U.n > 0) {
         const int64_t *node_u = dptr<int64_t>(U.node_u);
         GX_TRY(gx_ensure(ctx, ctx->m2l_part, sizeof(T) * NS * (size_t)(U.n + 1)));
-        k_adj_m2l<P, T><<<gx_blocks(U.n, WPB), 32 * WPB, 0, st>>>(
+        constexpr int B = m2l_block<P, T>();
+        k_adj_m2l<P, T><<<gx_blocks(U.n, B), 32 * B, 0, st>>>(
             U.n, dptr<int32_t>(U.node), dptr<int64_t>(U.start), dptr<int32_t>(U.len), node_u,
             dptr<int32_t>(ctx->far_idx), comx, comy, F32 ? dptr<float4>(ctx->comhl) : nullptr, eps2, dL, dM,
             dptr<T>(ctx->m2l_part), dptr<unsigned>(ctx->m2l_count));

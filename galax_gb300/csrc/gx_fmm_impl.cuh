@@ -930,13 +930,27 @@ __device__ __forceinline__ void last_unit_sums(int64_t node, int64_t u0, int64_t
     if (lane == 0) count[node] = 0;
 }
 
-// Warps an SM keeps of a kernel around m2l_fused: what its registers allow with few spills or
+// Warps a block of a kernel around m2l_fused: four in FP32 at p = 8, whose unrolled pair is some
+// 3,000 instructions: the warps of a block start together and share what is fetched of them
+// (Plummer 1M: M2L 9.9 ms one warp a block from the queue, 8.6 one without, 7.9 four).
+template <int P, class T>
+constexpr int m2l_block() {
+    return sizeof(T) == 4 && P == 8 ? 4 : WPB;
+}
+// Whether large launches take their units from a queue: up to the orders whose pair stays in
+// registers, or nearly.  Above, the kernel around the loop is the slower one: M2L alone at Plummer
+// 1M with / without it FP32 195.6 / 170.6 ms at p = 9 and 637 / 597 at 12, FP64 179.8 / 167.8 at 8.
+template <int P, class T>
+constexpr bool m2l_queued() {
+    return P <= (sizeof(T) == 4 ? 7 : 6);
+}
+// Warps an SM keeps of such a kernel: what its registers allow with few spills or
 // none (64, 80 and 128 of them).  Left alone at p = 5 and 6 in FP32 ptxas takes 151 and 225, for
 // 12 and 8 warps: evaluations of Plummer 1M 2.53 -> 2.40 and 3.41 -> 3.24 ms, disk 4M 12.8 ->
 // 12.5 and 14.7 -> 14.3.  FP64 is bound by its pipe at any number.
 template <int P, class T>
 constexpr int m2l_warps() {
-    return sizeof(T) == 8 || P > 6 ? WPB : P <= 4 ? 32 : P == 5 ? 24 : 16;
+    return sizeof(T) == 8 || P > 6 ? m2l_block<P, T>() : P <= 4 ? 32 : P == 5 ? 24 : 16;
 }
 
 // ACCURATE M2L over work units: every far list is cut into units of at most
@@ -944,7 +958,7 @@ constexpr int m2l_warps() {
 // tens of thousands of far sources, is spread over many warps instead of running as
 // one straggler.  A node with one unit writes its local directly, the others as above.
 template <int P, class T>
-__global__ void __launch_bounds__(32 * WPB, m2l_warps<P, T>() / WPB) k_m2l_units(
+__global__ void __launch_bounds__(32 * m2l_block<P, T>(), m2l_warps<P, T>() / m2l_block<P, T>()) k_m2l_units(
     int64_t n_units, const int32_t *__restrict__ unode, const int64_t *__restrict__ ustart,
     const int32_t *__restrict__ ulen, const int64_t *__restrict__ node_u, const int32_t *__restrict__ idx,
     const double *__restrict__ comx, const double *__restrict__ comy, const float4 *__restrict__ comhl, double eps2d,
@@ -955,8 +969,7 @@ __global__ void __launch_bounds__(32 * WPB, m2l_warps<P, T>() / WPB) k_m2l_units
     const int NCr = (PP + 1) * (PP + 2) / 2;
     (void)NCr;
     int lane = threadIdx.x & 31;
-    for (ItemQueue items(queue, n_units); items.more(); items.next()) {
-        const int64_t u = items.it;
+    const auto unit = [&](int64_t u) {
         const int64_t node = unode[u];
         float4 thl = make_float4(0.f, 0.f, 0.f, 0.f);
         if constexpr (sizeof(T) == 4) thl = comhl[node];
@@ -977,6 +990,12 @@ __global__ void __launch_bounds__(32 * WPB, m2l_warps<P, T>() / WPB) k_m2l_units
             warp_coeffs<NC>(acc, [&](int k, T v) { part[u * NS + k] = v; });
             last_unit_sums<NC, NS>(node, u0, u1, part, count, store);
         }
+    };
+    if constexpr (m2l_queued<P, T>()) {
+        for (ItemQueue items(queue, n_units); items.more(); items.next()) unit(items.it);
+    } else {
+        const int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+        if (u < n_units) unit(u);
     }
 }
 
@@ -2915,9 +2934,13 @@ int run_forces(gx_ctx *ctx, bool timed) {
             }
             return GX_OK;
         };
-        // the near field starts beside the far-field chain; for a measurement of the
-        // near field alone (gx_bench_forces) it starts after the chain
-        if (!ctx->near_after_far) {
+        // The near field starts beside the far-field chain, up to p = 8.  Above, M2L lives on local
+        // memory, is nearly all of the evaluation, and loses more beside kernels that take L1 for
+        // shared memory than they gain (disk 1M, n_max = 16, p = 9 with the split: 548 to 679 ms
+        // beside it, 397 after it).  For a measurement of the near field alone (gx_bench_forces) it
+        // starts after the chain at any order.
+        const bool near_after_far = ctx->near_after_far || P > 8;
+        if (!near_after_far) {
             GX_TRY(near_field());
             if (p2l) {
                 GX_CUDA(ctx, cudaStreamWaitEvent(ctx->stream3, ctx->ev_fork, 0));
@@ -2952,7 +2975,8 @@ int run_forces(gx_ctx *ctx, bool timed) {
             GX_TRY(gx_ensure(ctx, ctx->m2l_part, sizeof(T) * NS * (size_t)(U.n + 1)));
             if (U.n > 0) {
                 const int64_t *node_u = dptr<int64_t>(U.node_u);
-                k_m2l_units<P, T><<<gx_item_grid(ctx, U.n), 32 * WPB, 0, st>>>(
+                constexpr int B = m2l_block<P, T>();
+                k_m2l_units<P, T><<<m2l_queued<P, T>() ? gx_item_grid(ctx, U.n) : gx_blocks(U.n, B), 32 * B, 0, st>>>(
                     U.n, dptr<int32_t>(U.node), dptr<int64_t>(U.start), dptr<int32_t>(U.len), node_u,
                     dptr<int32_t>(ctx->far_idx), comx, comy, mixed ? dptr<float4>(ctx->comhl) : nullptr, eps2, M, L,
                     dptr<T>(ctx->m2l_part), dptr<unsigned>(ctx->m2l_count), gx_queue(ctx, GX_Q_M2L));
@@ -2970,8 +2994,8 @@ int run_forces(gx_ctx *ctx, bool timed) {
             GX_TRY(gx_ensure(ctx, ctx->fl32, sizeof(float2) * (size_t)n));
             fl = dptr<float2>(ctx->fl32);
         }
-        if (p2l && ctx->near_after_far) GX_TRY(p2l_field(st));
-        if (p2l && !ctx->near_after_far) GX_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_join3, 0));
+        if (p2l && near_after_far) GX_TRY(p2l_field(st));
+        if (p2l && !near_after_far) GX_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_join3, 0));
         if (mode == GX_MODE_REF && !mixed)
             k_l2l_ref_leaves<P, T><<<gx_blocks(nl, 128), 128, 0, st>>>(nl, parent, comx, comy, L, Lf);
         else  // REF lists: the leaf's own local and its parent's
@@ -2982,7 +3006,7 @@ int run_forces(gx_ctx *ctx, bool timed) {
                 dptr<T>(ctx->p2l_part), Lf, pos, bs, be, fl);
         ctx->launches++;
         tm.mark();  // 5
-        if (ctx->near_after_far) GX_TRY(near_field());
+        if (near_after_far) GX_TRY(near_field());
         // join the near field, then the ordered sum of the P2P partials (+ L2P in FP64)
         GX_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_join, 0));
         if (mixed) {
