@@ -267,11 +267,13 @@ int gx_rebuild_internal(gx_ctx *ctx);
 // block an item.  Evaluations with 24 / a block an item: Plummer 1M 1.91 / 1.985 ms (16: 1.96,
 // 64: 1.90), disk 4M, p = 6 14.8 / 15.8 (15.5, 15.0), but uniform 50,000, with two items a
 // block, 0.131 / 0.117: the far field's small launches wait for places then and the blocks
-// finish unevenly.
+// finish unevenly.  k_p2p32_items, whose registers let an SM hold 28 of its blocks, takes 28: with
+// 24, disk 4M without the split, n_max = 64, went from 19.8 (a block an item) to 20.2 ms, with 28 to
+// 18.0; with the split 13.0, 11.4 and 10.9.
 enum { GX_Q_P2P, GX_Q_M2P, GX_Q_P2L, GX_Q_M2L, GX_QUEUES };
 inline unsigned *gx_queue(gx_ctx *ctx, int which) { return static_cast<unsigned *>(ctx->queues.p) + 32 * which; }
-inline unsigned gx_item_grid(const gx_ctx *ctx, int64_t n) {
-    const int64_t grid = (ctx->sm_count > 0 ? ctx->sm_count : 152) * (int64_t)24;
+inline unsigned gx_item_grid(const gx_ctx *ctx, int64_t n, int per_sm = 24) {
+    const int64_t grid = (ctx->sm_count > 0 ? ctx->sm_count : 152) * (int64_t)per_sm;
     return (unsigned)(n < 16 * grid ? n : grid);
 }
 int gx_ensure_plan_public(gx_ctx *ctx);

@@ -156,7 +156,8 @@ int gx_plan_info(gx_ctx *ctx, int64_t *n_far_pairs, int64_t *n_near_pairs, int64
  * (gx_host_alloc, cudaHostAlloc, cudaHostRegister) are written by the device
  * directly, and page-locked x, y, m read directly once the plan exists.  On a host
  * whose page tables the GPU shares, kernels read and write ordinary arrays of up to
- * 128 pages (8 MB) too; other memory is copied before and after the evaluation. */
+ * 128 pages (8 MB) too; other memory, and arrays whose address is not a multiple of 8,
+ * are copied before and after the evaluation. */
 int gx_compute_forces(gx_ctx *ctx, const double *x, const double *y, const double *m, double *ax, double *ay);
 
 /* Device-resident state (no per-step host traffic). */
