@@ -2847,7 +2847,7 @@ int run_forces(gx_ctx *ctx, bool timed) {
                                                             (float)eps2, dptr<float2>(ctx->part),
                                                             gx_queue(ctx, GX_Q_P2P));
             else if (mixed && tchunks == 1)
-                k_p2p32_rows<<<gq, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
+                k_p2p32_rows<<<(unsigned)I.n, 32 * WPB, 0, ctx->stream2>>>(I.n, dptr<int32_t>(I.leaf), dptr<int64_t>(I.qb),
                                                            dptr<int32_t>(I.nq), pos, comx, comy, bs, be, src_idx,
                                                            (float)eps2, dptr<float2>(ctx->part),
                                                            gx_queue(ctx, GX_Q_P2P));

@@ -271,8 +271,9 @@ int gx_rebuild_internal(gx_ctx *ctx);
 // 24, disk 4M without the split, n_max = 64, went from 19.8 (a block an item) to 20.2 ms, with 28 to
 // 18.0; with the split 13.0, 11.4 and 10.9.  k_p2p32_rows1 takes its 32: with 24 an evaluation without the
 // split had two speeds, by how its blocks and M2L's came to lie (Plummer 1M, n_max = 16: 3.98 or 4.83 ms, a
-// block an item 4.33, with 32 always 4.07; uniform 3.27 or 3.91, 3.57, 3.34).  k_p2p32_rows is better
-// with 24 (disk 4M 9.32 and 9.87 with 32, 10.1 a block an item).
+// block an item 4.33, with 32 always 4.07; uniform 3.27 or 3.91, 3.57, 3.34).  k_p2p32_rows, the one of
+// leaves of 17 to 32 bodies without the body-level P2L, gives every item a block: disk 2M at p = 4 9.19 ms at n_max
+// = 24 (24: 11.3, 32: 9.15) and 5.28 at 32 (32: 5.38), Plummer 1M 2.74 (24: 2.74, 32: 2.82).
 enum { GX_Q_P2P, GX_Q_M2P, GX_Q_P2L, GX_Q_M2L, GX_QUEUES };
 inline unsigned *gx_queue(gx_ctx *ctx, int which) { return static_cast<unsigned *>(ctx->queues.p) + 32 * which; }
 inline unsigned gx_item_grid(const gx_ctx *ctx, int64_t n, int per_sm = 24) {
